@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <mutex>
 #include <string>
+#include "engine.cuh"
 #include "starsh-b200.h"
 
 namespace b200 {
@@ -23,7 +24,7 @@ struct DeviceBuffer {
 struct Context {
     int device = -1;
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;   // second stream for overlapping launches
+    SvdLanes lanes;                // streams the small SVD's size ranges overlap on
     cudaStream_t copy = nullptr;   // device-to-host copies of finished batches
     DeviceBuffer workspace;    // per-slot scratch of the engine
     DeviceBuffer tiles;        // TileWork array of a batch

@@ -65,6 +65,17 @@ static thread_local std::string t_error;
 static thread_local starsh_b200_stats t_stats;
 static std::atomic<long long> g_launches{0};
 
+static bool create_lanes(SvdLanes &l)
+{
+    for (cudaStream_t &s : l.s)
+        if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess)
+            return false;
+    for (cudaEvent_t &e : l.done)
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+            return false;
+    return cudaEventCreateWithFlags(&l.fork, cudaEventDisableTiming) == cudaSuccess;
+}
+
 // A context a thread has made its own (a serving worker's), or null.
 static thread_local Context *t_ctx = nullptr;
 
@@ -92,10 +103,9 @@ Context *context()
         g_ctx.device = dev;
         if (cudaStreamCreateWithFlags(&g_ctx.stream, cudaStreamNonBlocking)
                 != cudaSuccess ||
-            cudaStreamCreateWithFlags(&g_ctx.side, cudaStreamNonBlocking)
-                != cudaSuccess ||
             cudaStreamCreateWithFlags(&g_ctx.copy, cudaStreamNonBlocking)
-                != cudaSuccess) {
+                != cudaSuccess ||
+            !create_lanes(g_ctx.lanes)) {
             cudaGetLastError();
             set_error("cudaStreamCreate failed");
             return;
@@ -161,8 +171,8 @@ Context *context_new_private()
     c->workspace_cap = cap_mb << 20;
     cudaSetDevice(c->device);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking) != cudaSuccess) {
+        cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking) != cudaSuccess ||
+        !create_lanes(c->lanes)) {
         cudaGetLastError();
         delete c;
         return nullptr;
@@ -175,7 +185,7 @@ void context_free_private(Context *c)
     if (c == nullptr) return;
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
-    cudaStreamSynchronize(c->side);
+    for (cudaStream_t l : c->lanes.s) cudaStreamSynchronize(l);
     cudaStreamSynchronize(c->copy);
     {
         std::lock_guard<std::mutex> g(g_idle_mu);
@@ -199,7 +209,9 @@ void context_free_private(Context *c)
         if (c->tiles_pin[i]) host_pinned_free(c->tiles_pin[i]);
     }
     cudaStreamDestroy(c->stream);
-    cudaStreamDestroy(c->side);
+    for (cudaStream_t l : c->lanes.s) cudaStreamDestroy(l);
+    cudaEventDestroy(c->lanes.fork);
+    for (cudaEvent_t e : c->lanes.done) cudaEventDestroy(e);
     cudaStreamDestroy(c->copy);
     delete c;
 }
@@ -935,26 +947,26 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         cudaEventRecord(ev[1], s);
         // basis: pass A
         if ((info = gemm(STEP_GRAM_Y, true, false, nt, k_max, k_max, none))) break;
-        launch_pivchol(0, dt, dt, nt, ws, s);
+        launch_pivchol(0, dt, nt, ws, s);
         launch_gather_cols(0, dt, nt, ws, s);
         count_launch(2);
         if ((info = gemm(STEP_Q1, false, false, nt, m_max, k_max, none))) break;
         if ((info = gemm(STEP_GRAM_Q1, true, false, nt, k_max, k_max, none))) break;
-        launch_chol_inv(0, dt, nt, ws, s);
+        launch_chol_inv(0, dt, nt, ws, k_max, s);
         count_launch();
         if ((info = gemm(STEP_Q, false, false, nt, m_max, k_max, none))) break;
         // basis: pass B (tiles that do not need it have empty GEMMs)
         if ((info = gemm(STEP_RES_Z, true, false, nt, k_max, k_max, none))) break;
         if ((info = gemm(STEP_RES_Y, false, false, nt, m_max, k_max, none))) break;
         if ((info = gemm(STEP_GRAM_YR, true, false, nt, k_max, k_max, none))) break;
-        launch_pivchol(1, dt, dt, nt, ws, s);
+        launch_pivchol(1, dt, nt, ws, s);
         launch_gather_cols(1, dt, nt, ws, s);
         count_launch(2);
         if ((info = gemm(STEP_Q1B, false, false, nt, m_max, k_max, none))) break;
         if ((info = gemm(STEP_RES_Z2, true, false, nt, k_max, k_max, none))) break;
         if ((info = gemm(STEP_RES_Q1B, false, false, nt, m_max, k_max, none))) break;
         if ((info = gemm(STEP_GRAM_Q1B, true, false, nt, k_max, k_max, none))) break;
-        launch_chol_inv(1, dt, nt, ws, s);
+        launch_chol_inv(1, dt, nt, ws, k_max, s);
         count_launch();
         if ((info = gemm(STEP_QB, false, false, nt, m_max, k_max, none))) break;
         launch_merge_basis(dt, nt, s);
@@ -990,7 +1002,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             if ((e = gemm(STEP_A_ORTH_Z, true, false, nt, k_max, bmax, none))) return e;
             if ((e = gemm(STEP_A_ORTH_R, false, false, nt, m_max, bmax, none))) return e;
             if ((e = gemm(STEP_A_GRAM_R, true, false, nt, bmax, bmax, none))) return e;
-            launch_chol_inv(1, dt, rcount(), ws, s, ract());
+            launch_chol_inv(1, dt, rcount(), ws, bmax, s, ract());
             count_launch();
             if ((e = gemm(STEP_A_QB, false, false, nt, m_max, bmax, none))) return e;
             launch_merge_basis(dt, nt, s);
@@ -1042,7 +1054,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
                 if ((info = gemm(STEP_A_RES_Y, false, false, nt, m_max, bmax, none))) break;
             }
             if ((info = gemm(STEP_A_GRAM, true, false, nt, bmax, bmax, none))) break;
-            launch_round_pivchol(dt, rcount(), ws, 0, s, ract());
+            launch_round_pivchol(dt, rcount(), ws, 0, bmax, s, ract());
             count_launch();
             if ((info = append(bmax))) break;
             if (may_repeat) {
@@ -1050,7 +1062,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
                 if ((info = gemm(STEP_A_RES_Z2, true, false, nt, k_max, bmax, none))) break;
                 if ((info = gemm(STEP_A_RES_Y2, false, false, nt, m_max, bmax, none))) break;
                 if ((info = gemm(STEP_A_GRAM2, true, false, nt, bmax, bmax, none))) break;
-                launch_round_pivchol(dt, rcount(), ws, 1, s, ract());
+                launch_round_pivchol(dt, rcount(), ws, 1, bmax, s, ract());
                 count_launch();
                 if ((info = append(bmax))) break;
             }
@@ -1082,8 +1094,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         if ((info = gemm(STEP_PROJECT, true, false, nt, k_max, plan[pi].n, none))) break;
         cudaEventRecord(ev[3], s);
         if ((info = gemm(STEP_GRAM_B, false, true, nt, k_max, k_max, none))) break;
-        count_launch(launch_pivchol(2, dt, dt, nt, ws, s));
-        count_launch(launch_jacobi(dt, nt, ws, s, ctx.side));
+        count_launch(launch_small_svd(dt, nt, ws, s, ctx.lanes));
         if ((info = gemm(STEP_ROTATE, true, false, nt, k_max, plan[pi].n, none))) break;
         launch_rank_cut(dt, nt, ws, s);
         count_launch();

@@ -153,18 +153,27 @@ void make_gemm_descs(GemmStep step, const TileWork *d_tiles, int ntiles,
 void launch_gen_tiles(const DevKernel *d_kernels, const TileWork *d_tiles,
                       int ntiles, Workspace ws, cudaStream_t stream,
                       int need = 0, int family = 0);
-// launch_pivchol and launch_jacobi return the number of kernels launched.
-int launch_pivchol(int phase, const TileWork *d_tiles, TileWork *d_tiles_rw,
-                   int ntiles, Workspace ws, cudaStream_t s);
+// Phases A (0) and B (1) of the pivoted Cholesky.
+void launch_pivchol(int phase, TileWork *d_tiles, int ntiles, Workspace ws,
+                    cudaStream_t s);
+// Streams and events the small SVD spreads its size ranges over (all null:
+// one stream).
+struct SvdLanes {
+    cudaStream_t s[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t fork = nullptr;
+    cudaEvent_t done[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+};
+// Gram factor and Jacobi SVD of B B^T (in S): W, k2, tail_h; returns the
+// number of kernels launched.
+int launch_small_svd(TileWork *d_tiles, int ntiles, Workspace ws,
+                     cudaStream_t stream, const SvdLanes &lanes);
 // `act` (optional): the launch covers the `ntiles` tiles listed there (a
 // round's sampling tiles) instead of the first `ntiles` of the batch.
 void launch_gather_cols(int phase, const TileWork *d_tiles, int ntiles,
                         Workspace ws, cudaStream_t stream,
                         const int *act = nullptr);
 void launch_chol_inv(int phase, TileWork *d_tiles, int ntiles, Workspace ws,
-                     cudaStream_t stream, const int *act = nullptr);
-int launch_jacobi(TileWork *d_tiles, int ntiles, Workspace ws,
-                  cudaStream_t stream, cudaStream_t side);
+                     int nmax, cudaStream_t stream, const int *act = nullptr);
 void launch_rank_cut(TileWork *d_tiles, int ntiles, Workspace ws,
                      cudaStream_t stream);
 void launch_merge_basis(TileWork *d_tiles, int ntiles, cudaStream_t stream);
@@ -178,7 +187,7 @@ void launch_round_setup(TileWork *d_tiles, int ntiles, int block,
 void launch_round_end(TileWork *d_tiles, int ntiles, int verify,
                       cudaStream_t stream);
 void launch_round_pivchol(TileWork *d_tiles, int ntiles, Workspace ws,
-                          int repeat, cudaStream_t stream,
+                          int repeat, int bmax, cudaStream_t stream,
                           const int *act = nullptr);
 void launch_select_w(const TileWork *d_tiles, int ntiles, Workspace ws,
                      cudaStream_t stream);

@@ -164,28 +164,27 @@ extern "C" int starsh_b200_dense_rsvd_noalloc(const double *dD, int nrows,
     const int m = nrows, n = ncols;
     if ((info = gemm(STEP_SKETCH, false, false, m, k, none))) return info;
     if ((info = gemm(STEP_GRAM_Y, true, false, k, k, none))) return info;
-    launch_pivchol(0, dt, dt, 1, ws, s);
+    launch_pivchol(0, dt, 1, ws, s);
     launch_gather_cols(0, dt, 1, ws, s);
     if ((info = gemm(STEP_Q1, false, false, m, k, none))) return info;
     if ((info = gemm(STEP_GRAM_Q1, true, false, k, k, none))) return info;
-    launch_chol_inv(0, dt, 1, ws, s);
+    launch_chol_inv(0, dt, 1, ws, k, s);
     if ((info = gemm(STEP_Q, false, false, m, k, none))) return info;
     if ((info = gemm(STEP_RES_Z, true, false, k, k, none))) return info;
     if ((info = gemm(STEP_RES_Y, false, false, m, k, none))) return info;
     if ((info = gemm(STEP_GRAM_YR, true, false, k, k, none))) return info;
-    launch_pivchol(1, dt, dt, 1, ws, s);
+    launch_pivchol(1, dt, 1, ws, s);
     launch_gather_cols(1, dt, 1, ws, s);
     if ((info = gemm(STEP_Q1B, false, false, m, k, none))) return info;
     if ((info = gemm(STEP_RES_Z2, true, false, k, k, none))) return info;
     if ((info = gemm(STEP_RES_Q1B, false, false, m, k, none))) return info;
     if ((info = gemm(STEP_GRAM_Q1B, true, false, k, k, none))) return info;
-    launch_chol_inv(1, dt, 1, ws, s);
+    launch_chol_inv(1, dt, 1, ws, k, s);
     if ((info = gemm(STEP_QB, false, false, m, k, none))) return info;
     launch_merge_basis(dt, 1, s);
     if ((info = gemm(STEP_PROJECT, true, false, k, n, none))) return info;
     if ((info = gemm(STEP_GRAM_B, false, true, k, k, none))) return info;
-    launch_pivchol(2, dt, dt, 1, ws, s);
-    launch_jacobi(dt, 1, ws, s, nullptr);
+    launch_small_svd(dt, 1, ws, s, SvdLanes{});
     if ((info = gemm(STEP_ROTATE, true, false, k, n, none))) return info;
     launch_rank_cut(dt, 1, ws, s);
     // One tile: its factors start at offset 0 of the caller's buffers, so

@@ -745,10 +745,7 @@ __device__ double block_sum(double x, double *red)
 enum : int { PH_A = 0, PH_B = 1, PH_H = 2, PH_R = 3, PH_R2 = 4 };
 
 constexpr int kSmallThreads = 256;
-#ifndef PIVCHOL_H_LANES
-#define PIVCHOL_H_LANES 4
-#endif
-constexpr int kPivcholLanes = PIVCHOL_H_LANES;   // lanes per row, large phase-H factors
+constexpr int kPivcholLanes = 4;                 // lanes per row, large phase-H factors
 constexpr int kPivcholSplit = 128;               // "large": more rows than this
 constexpr int kMaxK = 1024;   // largest sketch width handled by one CTA
 
@@ -988,11 +985,314 @@ k_pivchol(TileWork *__restrict__ tiles, Workspace ws, int phase, int nn_lo,
     }
 }
 
-void launch_round_pivchol(TileWork *d_tiles, int ntiles, Workspace ws,
-                          int repeat, cudaStream_t stream, const int *act)
+// Columns of an upper triangular inverse in shared memory, row-packed: row b
+// holds columns b .. cnt - 1, so lanes of consecutive columns read
+// consecutive doubles.
+__device__ __forceinline__ int tri_at(int b, int c, int cnt)
 {
-    k_pivchol<1><<<ntiles, kSmallThreads, 0, stream>>>(
-        d_tiles, ws, repeat ? PH_R2 : PH_R, 0, INT_MAX, act);
+    return b * cnt - b * (b - 1) / 2 + c - b;
+}
+
+// X = R^{-1} for the upper triangular R(a, b) = R[a * ra + b * rb], a <= b <
+// cnt, in shared memory, one thread per column (its back substitution sums
+// b = a + 1 .. c in that order, a chain of dependent products: the entry
+// just found stays in a register, the others' loads run ahead of the
+// chain), then T(:, 0:cnt) = X with zeros below the diagonal.  Called by
+// the whole block.
+__device__ __forceinline__ void tri_inverse(const double *R, int ra, int rb,
+                                            int cnt, double *X, double *T, int ld)
+{
+    for (int c = threadIdx.x; c < cnt; c += blockDim.x) {
+        double x = 1.0 / R[c * ra + c * rb];
+        X[tri_at(c, c, cnt)] = x;
+        for (int a = c - 1; a >= 0; --a) {
+            const double *r = R + a * ra + (a + 1) * rb;
+            double acc = fma(*r, x, 0.0);
+            int at = tri_at(a + 2, c, cnt);
+            #pragma unroll 8
+            for (int b = a + 2; b <= c; ++b) {
+                r += rb;
+                acc = fma(*r, X[at], acc);
+                at += cnt - b - 1;
+            }
+            x = -acc / R[a * ra + a * rb];
+            X[tri_at(a, c, cnt)] = x;
+        }
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int c = threadIdx.x >> 5; c < cnt; c += blockDim.x >> 5)
+        for (int a = lane; a < cnt; a += 32)
+            T[(size_t)c * ld + a] = a <= c ? X[tri_at(a, c, cnt)] : 0.0;
+}
+
+// Order-preserving 64-bit key of a double.
+__device__ __forceinline__ unsigned long long order_key(double v)
+{
+    const long long b = __double_as_longlong(v);
+    return (unsigned long long)(b < 0 ? ~b : b | (long long)0x8000000000000000ull);
+}
+
+__device__ __forceinline__ double key_value(unsigned long long k)
+{
+    return __longlong_as_double((long long)(k >> 63 ? k & 0x7fffffffffffffffull : ~k));
+}
+
+// Block sum of one value per row in the order of block_sum (tree over the
+// 32 rows of a warp, tree over the warps): every thread gets it.
+template <int W>
+__device__ __forceinline__ double row_sum(double x, double *red)
+{
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if constexpr (W == 1) return x;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+    __syncthreads();
+    if constexpr (W == 2) return red[0] + red[1];
+    if constexpr (W == 3) return (red[0] + red[2]) + red[1];
+    return (red[0] + red[2]) + (red[1] + red[3]);
+}
+
+// The same factorisation for at most 32 W rows: the Gram sits in shared
+// memory, one thread per row, the diagonal in a register.  Step j's column
+// of L takes slot j; the Gram column that was there moves to the slot of
+// the pivot's column, which no later step reads (each thread moves its own
+// row).  What bounds it is the chain of dependent steps -- pivot search,
+// the left-looking product, quotient -- so the search is three integer
+// warp reductions on an order-preserving key, the product walks
+// consecutive slots (addresses known ahead, so its loads overlap), and a
+// step has one block barrier (none for W = 1); the kernel above takes
+// about 6 us a step (five barriers, the Gram and L read from L2).
+// Every sum keeps the order of the kernel above (four partial sums of the
+// left-looking product, trees over 32 rows and over warps), so both give
+// the same bits.  Phases R, R2 (nn <= the round's columns) and H (tiles of
+// 32 (W - 1) < nn <= 32 W rows: nn_lo, nn_hi).  81 tiles, 64 columns:
+// 215 -> 30 us; 81 tiles of up to 128 rows in phase H 286 -> 49 us.
+template <int W>
+__global__ void __launch_bounds__(32 * W)
+k_pivchol_rows(TileWork *__restrict__ tiles, Workspace ws, int phase, int nn_lo,
+               int nn_hi, const int *__restrict__ act)
+{
+    extern __shared__ double pc_sm[];
+    __shared__ double redd[4];
+    __shared__ unsigned long long redk[2][4];
+    __shared__ int redi[2][4];
+    __shared__ int spiv[32 * W];
+    __shared__ int pos[32 * W], at[32 * W];   // Gram column -> slot, and back
+    TileWork &tw = tiles[act ? act[blockIdx.x] : blockIdx.x];
+    const int s = tw.slot;
+    const double tol = tw.tol;
+    int nn;
+    if (phase == PH_H) nn = tw.k1;
+    else if (phase == PH_R) nn = tw.bcur;
+    else nn = tw.need_pass_b ? tw.bcur : 0;
+    const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
+    if (nn < nn_lo || nn > nn_hi) return;
+    if (phase != PH_H && nn <= 0) {
+        if (i == 0) {
+            tw.kb = 0;
+            if (phase == PH_R) tw.kround = 0;
+            if (phase == PH_R2) tw.need_pass_b = 0;
+        }
+        return;
+    }
+    const double dn = tw.dnorm2, var0 = tw.omega_var;
+    const int room = tw.k - tw.k1;
+    constexpr int LD = 32 * W + 1;
+    const double *G = ws.S(s);
+    const int ld = ws.ldK();
+    if (i < nn)
+        for (int c = 0; c < nn; ++c) {
+            const unsigned d = (unsigned)__cvta_generic_to_shared(pc_sm + c * LD + i);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
+                         :: "r"(d), "l"(G + (size_t)c * ld + i));
+        }
+    asm volatile("cp.async.commit_group;");
+    pos[i] = at[i] = i;
+    asm volatile("cp.async.wait_group 0;");
+    __syncthreads();
+    double dg = i < nn ? pc_sm[i * LD + i] : 0.0;
+    bool open = i < nn;                    // not a pivot yet
+    const double trace = row_sum<W>(dg, redd);
+
+    // Largest value and its (smallest) row over the open rows, as keys;
+    // values not above -DBL_MAX (NaN) never win.
+    unsigned long long bk;
+    int bi;
+    auto search = [&](int par) {
+        const bool in = open && dg > -DBL_MAX;
+        const unsigned long long k = order_key(in ? dg : -DBL_MAX);
+        const unsigned hi = (unsigned)(k >> 32), lo = (unsigned)k;
+        const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+        const unsigned row = in && hi == mh && lo == ml ? (unsigned)i : 1u << 30;
+        bi = (int)__reduce_min_sync(0xffffffffu, row);
+        bk = ((unsigned long long)mh << 32) | ml;
+        if constexpr (W > 1) {
+            if (lane == 0) {
+                redk[par][warp] = bk;
+                redi[par][warp] = bi;
+            }
+            __syncthreads();
+            bk = redk[par][0];
+            bi = redi[par][0];
+            #pragma unroll
+            for (int w = 1; w < W; ++w)
+                if (redk[par][w] > bk) {
+                    bk = redk[par][w];
+                    bi = redi[par][w];
+                }
+        } else {
+            __syncwarp();
+        }
+    };
+    search(1);
+    const double dmax = key_value(bk);
+
+    double thr;
+    int cap = nn;
+    double stop_trace = -1.0;
+    if (phase != PH_H) {
+        const double noise = 1e-15 * dmax;
+        const double var = var0 > 0.0 ? var0 : 1.0;
+        const double floor_ = 0.01 * tol * tol * dn * var;
+        thr = fmax(noise, floor_);
+        cap = min(nn, room);
+        if (i == 0)
+            tw.need_pass_b = phase == PH_R && noise > floor_ &&
+                             0.01 * tol * tol < 1e-15;
+    } else {
+        thr = 1e-18 * dmax;
+        if (i == 0) tw.tr_h = trace;
+        const double energy = dn > 0.0 ? fmax(dn, trace) : trace;
+        stop_trace = 0.01 * tol * tol * energy;
+        if (dn > 0.0 &&
+            fmax(0.0, dn - trace - 2e-15 * dn) > tol * tol * fmax(dn, trace)) {
+            if (i == 0) {
+                tw.k2 = 0;
+                tw.tail_h = trace;
+                tw.status |= TILE_TAIL_LEFT;
+            }
+            return;
+        }
+    }
+    if (!(dmax > 0.0)) thr = DBL_MAX;
+
+    int j = 0;
+    for (; j < cap; ++j) {
+        search(j & 1);
+        if (stop_trace >= 0.0) {
+            const double total = row_sum<W>(open ? fmax(0.0, dg) : 0.0, redd);
+            if (total <= stop_trace) break;
+        }
+        const double best = key_value(bk);
+        if (!(best > thr)) break;
+        const int p = bi;
+        const double sp = sqrt(best);
+        const int q = pos[p];
+        double *colq = pc_sm + q * LD + i, *colj = pc_sm + j * LD + i;
+        double v = 0.0, gq = 0.0;
+        if (i < nn) {
+            gq = *colq;                // the pivot's Gram column, this row
+            *colq = *colj;             // slot j's column moves there
+        }
+        if (i == p) {
+            v = sp;
+            open = false;
+            spiv[j] = p;
+        } else if (open) {
+            double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+            const double *li = pc_sm + i, *lp = pc_sm + p;
+            int l = 0;
+            #pragma unroll 4
+            for (; l + 3 < j; l += 4, li += 4 * LD, lp += 4 * LD) {
+                a0 = fma(li[0], lp[0], a0);
+                a1 = fma(li[LD], lp[LD], a1);
+                a2 = fma(li[2 * LD], lp[2 * LD], a2);
+                a3 = fma(li[3 * LD], lp[3 * LD], a3);
+            }
+            for (; l < j; ++l, li += LD, lp += LD) a0 = fma(*li, *lp, a0);
+            const double acc = gq - ((a0 + a1) + (a2 + a3));
+            v = acc / sp;
+            dg -= v * v;
+        }
+        if (i < nn) *colj = v;
+        // pos and at of the moved column: every thread has read pos[p]
+        // before the barrier of the next search; the entries written here
+        // are read after it
+        if constexpr (W == 1) __syncwarp();
+        if (i == 0) {
+            const int r = at[j];
+            pos[r] = q;
+            at[q] = r;
+        }
+        if constexpr (W == 1) __syncwarp();
+    }
+    const int cnt = j;
+    __syncthreads();
+    if (i == 0) {
+        if (phase == PH_H) tw.k2 = cnt;
+        else tw.kb = cnt;
+        if (phase == PH_R) {
+            tw.kround = cnt;
+            if (cnt == 0) tw.need_pass_b = 0;
+        }
+    }
+    if (phase == PH_H) {
+        const double rest = row_sum<W>(open ? fmax(0.0, dg) : 0.0, redd);
+        if (i == 0) tw.tail_h = cnt > 0 ? rest : trace;
+        double *L = ws.L(s);
+        if (i < nn)
+            for (int c = 0; c < cnt; ++c) L[(size_t)c * ld + i] = pc_sm[c * LD + i];
+        return;
+    }
+    int *piv = ws.Piv(s);
+    const int mine = i < cnt ? spiv[i] : 0;
+    if (i < cnt) piv[i] = mine;
+    // rows in pivot order: slot a then holds R11(a, b) = L(piv[b], a)
+    for (int a0 = 0; a0 < cnt; a0 += 8) {
+        double v[8];
+        #pragma unroll
+        for (int u = 0; u < 8; ++u)
+            v[u] = a0 + u < cnt ? pc_sm[(a0 + u) * LD + mine] : 0.0;
+        __syncthreads();
+        #pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (a0 + u < cnt && i < cnt) pc_sm[(a0 + u) * LD + i] = v[u];
+    }
+    __syncthreads();
+    // T = R11^{-1} (upper triangular)
+    tri_inverse(pc_sm, LD, 1, cnt, pc_sm + nn_hi * LD, ws.T(s), ld);
+}
+
+template <int W>
+static void pivchol_rows_launch(TileWork *d_tiles, int ntiles, Workspace ws,
+                                int phase, int nn_lo, int nn_hi,
+                                cudaStream_t stream, const int *act)
+{
+    const int tri = phase == PH_H ? 0 : nn_hi * (nn_hi + 1) / 2;
+    const size_t smem = ((size_t)nn_hi * (32 * W + 1) + tri) * sizeof(double);
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(k_pivchol_rows<W>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_pivchol_rows<W><<<ntiles, 32 * W, smem, stream>>>(d_tiles, ws, phase, nn_lo,
+                                                        nn_hi, act);
+}
+
+// A round's pivoted Cholesky; `bmax` bounds the round's columns.
+void launch_round_pivchol(TileWork *d_tiles, int ntiles, Workspace ws,
+                          int repeat, int bmax, cudaStream_t stream,
+                          const int *act)
+{
+    const int phase = repeat ? PH_R2 : PH_R;
+    if (bmax <= 32)
+        pivchol_rows_launch<1>(d_tiles, ntiles, ws, phase, INT_MIN, 32, stream, act);
+    else if (bmax <= 64)
+        pivchol_rows_launch<2>(d_tiles, ntiles, ws, phase, INT_MIN, 64, stream, act);
+    else
+        k_pivchol<1><<<ntiles, kSmallThreads, 0, stream>>>(d_tiles, ws, phase, 0,
+                                                           INT_MAX, act);
 }
 
 // ||D||_F^2 of every block from the generator's per-CTA partial sums, in a
@@ -1083,21 +1383,11 @@ void launch_round_end(TileWork *d_tiles, int ntiles, int verify,
                                                           verify);
 }
 
-int launch_pivchol(int phase, const TileWork *, TileWork *d_tiles_rw,
-                    int ntiles, Workspace ws, cudaStream_t s)
+void launch_pivchol(int phase, TileWork *d_tiles, int ntiles, Workspace ws,
+                    cudaStream_t s)
 {
-    if (phase == PH_H && kPivcholLanes > 1) {
-        // small factors one lane per row, large ones kPivcholLanes
-        k_pivchol<1><<<ntiles, kSmallThreads, 0, s>>>(d_tiles_rw, ws, phase, 0,
-                                                      kPivcholSplit, nullptr);
-        k_pivchol<kPivcholLanes><<<ntiles, kSmallThreads * kPivcholLanes, 0, s>>>(
-            d_tiles_rw, ws, phase, kPivcholSplit + 1, INT_MAX, nullptr);
-        return 2;
-    } else {
-        k_pivchol<1><<<ntiles, kSmallThreads, 0, s>>>(d_tiles_rw, ws, phase, 0,
-                                                      INT_MAX, nullptr);
-        return 1;
-    }
+    k_pivchol<1><<<ntiles, kSmallThreads, 0, s>>>(d_tiles, ws, phase, 0, INT_MAX,
+                                                  nullptr);
 }
 
 // Gathers the pivot columns of Y into the Q buffer (phase A) or the Q1
@@ -1133,13 +1423,13 @@ void launch_gather_cols(int phase, const TileWork *d_tiles, int ntiles,
 // T(slot) = R^{-1}.  For phase B the new columns are appended to the basis
 // afterwards by the caller's merge step.
 __global__ void __launch_bounds__(kSmallThreads)
-k_chol_inv(TileWork *__restrict__ tiles, Workspace ws, int phase,
+k_chol_inv(TileWork *__restrict__ tiles, Workspace ws, int phase, int nn_lo,
            const int *__restrict__ act)
 {
     TileWork &tw = tiles[act ? act[blockIdx.x] : blockIdx.x];
     const int s = tw.slot;
     const int nn = phase == PH_A ? tw.k1 : tw.kb;
-    if (nn <= 0) return;
+    if (nn < nn_lo) return;
     const double *G = ws.S(s);
     double *R = ws.L(s);
     double *T = ws.T(s);
@@ -1194,10 +1484,79 @@ k_chol_inv(TileWork *__restrict__ tiles, Workspace ws, int phase,
     }
 }
 
-void launch_chol_inv(int phase, TileWork *d_tiles, int ntiles, Workspace ws,
-                     cudaStream_t stream, const int *act)
+// The same for nn <= kCholSmall: the Gram sits in shared memory and is
+// factored right-looking, so a step is one square root, one quotient and
+// one update per entry instead of a chain of j of them; every entry still
+// subtracts its products in the order l = 0, 1, ..., so both kernels give
+// the same bits.  81 tiles with up to 64 columns: 150 -> 35 us.
+constexpr int kCholSmall = 64;
+
+__global__ void __launch_bounds__(256)
+k_chol_inv_small(TileWork *__restrict__ tiles, Workspace ws, int phase,
+                 int nn_hi, const int *__restrict__ act)
 {
-    k_chol_inv<<<ntiles, kSmallThreads, 0, stream>>>(d_tiles, ws, phase, act);
+    extern __shared__ double ci_sm[];
+    __shared__ double gd[kCholSmall];
+    TileWork &tw = tiles[act ? act[blockIdx.x] : blockIdx.x];
+    const int s = tw.slot;
+    const int nn = phase == PH_A ? tw.k1 : tw.kb;
+    if (nn <= 0 || nn > nn_hi) return;
+    constexpr int LD = kCholSmall + 1;
+    double *A = ci_sm, *X = ci_sm + kCholSmall * LD;
+    const double *G = ws.S(s);
+    const int ld = ws.ldK();
+    // thread (c, q): column c, rows j = q, q + 4, ...
+    const int c = threadIdx.x & 63, q = threadIdx.x >> 6;
+    for (int e = threadIdx.x; e < nn * 64; e += 256) {
+        const int row = e & 63, col = e >> 6;
+        if (row <= col) A[col * LD + row] = G[(size_t)col * ld + row];
+    }
+    __syncthreads();
+    if (threadIdx.x < nn) gd[threadIdx.x] = A[threadIdx.x * LD + threadIdx.x];
+    __syncthreads();
+    int nn_ok = nn;
+    for (int l = 0; l < nn; ++l) {
+        const double acc = A[l * LD + l];
+        // a column numerically inside the span of the previous ones ends
+        // the factor (as above); the test is the same for every thread
+        if (!(acc > 1e-14 * gd[l])) { nn_ok = l; break; }
+        const double r = sqrt(fmax(acc, 0.0));
+        // every thread forms its column's R(l, c) itself; one of the four
+        // stores it, and the diagonal is read by all before it is stored
+        double rc = 0.0;
+        if (c > l && c < nn) rc = A[c * LD + l] / r;
+        __syncthreads();
+        if (q == 0 && c < nn) {
+            if (c == l) A[l * LD + l] = r;
+            else if (c > l) A[c * LD + l] = rc;
+        }
+        __syncthreads();
+        if (c < nn)
+            for (int j = l + 1 + q; j <= c; j += 4)
+                A[c * LD + j] -= A[j * LD + l] * rc;
+        __syncthreads();
+    }
+    tri_inverse(A, 1, LD, nn_ok, X, ws.T(s), ld);
+    if (threadIdx.x == 0 && nn_ok < nn) {
+        if (phase == PH_A) tw.k1 = nn_ok;
+        else tw.kb = nn_ok;
+        tw.trunc_round = 1;
+        tw.status |= TILE_CHOL_TRUNC;
+    }
+}
+
+// `nmax` bounds the columns of every tile.
+void launch_chol_inv(int phase, TileWork *d_tiles, int ntiles, Workspace ws,
+                     int nmax, cudaStream_t stream, const int *act)
+{
+    constexpr size_t smem = ((size_t)kCholSmall * (kCholSmall + 1) +
+                             kCholSmall * (kCholSmall + 1) / 2) * sizeof(double);
+    cudaFuncSetAttribute(k_chol_inv_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem);
+    k_chol_inv_small<<<ntiles, 256, smem, stream>>>(d_tiles, ws, phase, kCholSmall, act);
+    if (nmax > kCholSmall)
+        k_chol_inv<<<ntiles, kSmallThreads, 0, stream>>>(d_tiles, ws, phase,
+                                                         kCholSmall + 1, act);
 }
 
 // -------------------------------------------------- one-sided Jacobi
@@ -1264,23 +1623,66 @@ __device__ __forceinline__ bool jacobi_unchanged(const int *lastrot, int a,
     return lastrot[a] < since && lastrot[b] < since;
 }
 
-// Rotation of the column pair (ca, cb) by the G lanes of one group (gl =
-// lane within the group).  Every lane of the warp calls this (inactive
-// groups with valid = false) because the reductions shuffle across the
-// whole warp.  Returns true if the pair was rotated.
-template <int G, int E>
-__device__ __forceinline__ bool jacobi_rotate(double *ca, double *cb, int rows,
-                                              int gl, bool valid, double eps2)
+// Where a lane keeps its E rows (gl + G q, q < E) of a column in shared
+// memory.  PAIRED: rows q and q + 1 (q even) side by side, so that a lane
+// moves two rows per 16-byte access and the column is padded with zero rows
+// to G E (zeros change no sum); else row i at i, rows past `rows` skipped.
+template <int G, bool PAIRED>
+__device__ __forceinline__ int jacobi_at(int i)
 {
-    double xa[E], xb[E];
-    double al = 0.0, be = 0.0, ga = 0.0;
-    #pragma unroll
-    for (int q = 0; q < E; ++q) {
-        const int i = gl + G * q;
-        const bool in = valid && i < rows;
-        xa[q] = in ? ca[i] : 0.0;
-        xb[q] = in ? cb[i] : 0.0;
+    if constexpr (!PAIRED) return i;
+    const int q = i / G;
+    return (q >> 1) * 2 * G + (i - q * G) * 2 + (q & 1);
+}
+
+template <int G, int E, bool PAIRED>
+__device__ __forceinline__ void jacobi_load(double (&x)[E], const double *col,
+                                            int rows, int gl, bool valid)
+{
+    if constexpr (PAIRED) {
+        static_assert(E % 2 == 0, "row pairs");
+        const double2 *p = reinterpret_cast<const double2 *>(col) + gl;
+        #pragma unroll
+        for (int q = 0; q < E; q += 2) {
+            const double2 v = valid ? p[q / 2 * G] : make_double2(0.0, 0.0);
+            x[q] = v.x;
+            x[q + 1] = v.y;
+        }
+    } else {
+        #pragma unroll
+        for (int q = 0; q < E; ++q) {
+            const int i = gl + G * q;
+            x[q] = valid && i < rows ? col[i] : 0.0;
+        }
     }
+}
+
+template <int G, int E, bool PAIRED>
+__device__ __forceinline__ void jacobi_store(const double (&x)[E], double *col,
+                                             int rows, int gl)
+{
+    if constexpr (PAIRED) {
+        double2 *p = reinterpret_cast<double2 *>(col) + gl;
+        #pragma unroll
+        for (int q = 0; q < E; q += 2) p[q / 2 * G] = make_double2(x[q], x[q + 1]);
+    } else {
+        #pragma unroll
+        for (int q = 0; q < E; ++q) {
+            const int i = gl + G * q;
+            if (i < rows) col[i] = x[q];
+        }
+    }
+}
+
+// Rotation of a column pair whose rows are spread over the G lanes of one
+// group, E per lane.  Every lane of the warp calls this (inactive groups
+// with zero columns) because the reductions shuffle across the whole warp.
+// Returns true if the pair was rotated.
+template <int G, int E>
+__device__ __forceinline__ bool jacobi_rotate(double (&xa)[E], double (&xb)[E],
+                                              double eps2)
+{
+    double al = 0.0, be = 0.0, ga = 0.0;
     #pragma unroll
     for (int q = 0; q < E; ++q) {
         al = fma(xa[q], xa[q], al);
@@ -1306,11 +1708,9 @@ __device__ __forceinline__ bool jacobi_rotate(double *ca, double *cb, int rows,
     const double sn = c * t;
     #pragma unroll
     for (int q = 0; q < E; ++q) {
-        const int i = gl + G * q;
-        if (i < rows) {
-            ca[i] = c * xa[q] - sn * xb[q];
-            cb[i] = sn * xa[q] + c * xb[q];
-        }
+        const double a = xa[q], b = xb[q];
+        xa[q] = c * a - sn * b;
+        xb[q] = sn * a + c * b;
     }
     return true;
 }
@@ -1350,17 +1750,39 @@ __device__ bool jacobi_rotate_stream(double *ca, double *cb, int rows,
     return true;
 }
 
-template <int CLASS, int G, int E, int THREADS, bool SMEM>
-__global__ void __launch_bounds__(THREADS, THREADS <= 128 ? 512 / THREADS : 1)
-k_jacobi(TileWork *__restrict__ tiles, Workspace ws)
+// Doubles between the columns of the shared-memory kernel: padded to whole
+// row pairs of the G lanes (PAIRED), and for G = 4, whose eight-lane access
+// phases take two neighbouring columns, an odd multiple of 8 so that the
+// two use different banks; else the row count, odd.
+template <int G, int E, bool PAIRED>
+__host__ __device__ constexpr int jacobi_stride(int rows)
 {
-    extern __shared__ double sm[];
+    return !PAIRED ? (rows | 1) : G == 4 ? (E * G / 8 | 1) * 8 : E * G;
+}
+
+// The factor in shared memory (SMEM) or streamed from global memory (E = 0).
+// The launch takes the tiles with rows_lo <= k1 <= rows_hi <= G E (of the
+// classes 3 and 5 those that fit).  Shared-memory traffic and the FP64
+// pipe bound a step, and with one CTA per SM its latency: the row pairs
+// halve the accesses, the padding removes their bank conflicts (columns an
+// odd number of doubles apart shared banks between the groups of a warp),
+// E close to the row count leaves few lanes on padding, and the narrower
+// ranges fit two CTAs on an SM.
+template <int CLASS, int G, int E, int THREADS, int MINB, bool PAIRED>
+__global__ void __launch_bounds__(THREADS, MINB)
+k_jacobi(TileWork *__restrict__ tiles, Workspace ws, int rows_lo, int rows_hi)
+{
+    constexpr bool SMEM = E > 0;
+    constexpr int EE = SMEM ? E : 1;
+    extern __shared__ double2 jac_sm[];
+    double *sm = reinterpret_cast<double *>(jac_sm);
     __shared__ int rotated[2];
     __shared__ int lastrot[jacobi_class_cols(CLASS)];
     TileWork &tw = tiles[blockIdx.x];
     const int s = tw.slot;
     const int rows = tw.k1, cols = tw.k2;
-    if (cols <= 0 || jacobi_class(rows, cols) != CLASS) return;   // uniform
+    if (cols <= 0 || rows < rows_lo || rows > rows_hi ||
+        jacobi_class(rows, cols) != CLASS) return;   // uniform
     for (int c = threadIdx.x; c < cols; c += THREADS) lastrot[c] = -1;
     // Relative orthogonality the rotations stop at: the rank cut needs the
     // left singular vectors orthonormal to well below tol (their overlap
@@ -1369,21 +1791,21 @@ k_jacobi(TileWork *__restrict__ tiles, Workspace ws)
     const double eps = fmax(1e-15, fmin(1e-7, 0.01 * tw.tol));
     const double eps2 = eps * eps;
     const int ldg = ws.ldK();
-    const int lds = rows | 1;   // odd stride: fewer bank conflicts
     double *A = SMEM ? sm : ws.L(s);
-    const int lda = SMEM ? lds : ldg;
+    const int lda = SMEM ? jacobi_stride<G, EE, PAIRED>(rows) : ldg;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kWarps = THREADS / 32;
     if (SMEM) {
         const double *Lg = ws.L(s);
-        for (int e = threadIdx.x; e < rows * cols; e += THREADS) {
-            const int c = e / rows, i = e - c * rows;
-            A[(size_t)c * lda + i] = Lg[(size_t)c * ldg + i];
-        }
+        const int fill = PAIRED ? G * EE : rows;
+        for (int c = warp; c < cols; c += kWarps)
+            for (int i = lane; i < fill; i += 32)
+                A[(size_t)c * lda + jacobi_at<G, PAIRED>(i)] =
+                    i < rows ? Lg[(size_t)c * ldg + i] : 0.0;
     }
     if (threadIdx.x == 0) rotated[0] = rotated[1] = 0;
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kGroupsPerWarp = 32 / G;
-    constexpr int kWarps = THREADS / 32;
     const int gw = lane / G, gl = lane % G;
     const int nc = cols + (cols & 1);      // players, with a bye if odd
     const int npairs = nc / 2;
@@ -1412,10 +1834,18 @@ k_jacobi(TileWork *__restrict__ tiles, Workspace ws)
                 if (!__any_sync(0xffffffffu, valid)) continue;   // warp-uniform
                 double *ca = A + (size_t)a * lda, *cb = A + (size_t)b * lda;
                 bool rot;
-                if constexpr (E > 0)
-                    rot = jacobi_rotate<G, E>(ca, cb, rows, gl, valid, eps2);
-                else
+                if constexpr (SMEM) {
+                    double xa[EE], xb[EE];
+                    jacobi_load<G, EE, PAIRED>(xa, ca, rows, gl, valid);
+                    jacobi_load<G, EE, PAIRED>(xb, cb, rows, gl, valid);
+                    rot = jacobi_rotate<G, EE>(xa, xb, eps2);
+                    if (rot) {
+                        jacobi_store<G, EE, PAIRED>(xa, ca, rows, gl);
+                        jacobi_store<G, EE, PAIRED>(xb, cb, rows, gl);
+                    }
+                } else {
                     rot = jacobi_rotate_stream(ca, cb, rows, lane, valid, eps2);
+                }
                 if (rot && gl == 0) lastrot[a] = lastrot[b] = now;
                 any |= rot;
             }
@@ -1433,11 +1863,15 @@ k_jacobi(TileWork *__restrict__ tiles, Workspace ws)
     for (int c = warp; c < cols; c += kWarps) {
         const double *ca = A + (size_t)c * lda;
         double nrm = 0.0;
-        for (int i = lane; i < rows; i += 32) nrm = fma(ca[i], ca[i], nrm);
+        for (int i = lane; i < rows; i += 32) {
+            const double x = ca[jacobi_at<G, PAIRED>(i)];
+            nrm = fma(x, x, nrm);
+        }
         #pragma unroll
         for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
         const double inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
-        for (int i = lane; i < rows; i += 32) W[(size_t)c * ldg + i] = ca[i] * inv;
+        for (int i = lane; i < rows; i += 32)
+            W[(size_t)c * ldg + i] = ca[jacobi_at<G, PAIRED>(i)] * inv;
         if (lane == 0) sig[c] = nrm;
     }
     if (threadIdx.x == 0) {
@@ -1577,31 +2011,55 @@ k_jacobi_block(TileWork *__restrict__ tiles, Workspace ws)
                                            column(b, b0, b1) < cols &&
                                            !jacobi_unchanged(lr, a, b, now - T);
                         if (__any_sync(0xffffffffu, valid)) {
-                            const bool rot = jacobi_rotate<G, E>(
-                                sm + (size_t)a * lds, sm + (size_t)b * lds, rows,
-                                gl, valid, eps2);
-                            if (rot && gl == 0) lr[a] = lr[b] = now;
+                            double *ca = sm + (size_t)a * lds, *cb = sm + (size_t)b * lds;
+                            double xa[E], xb[E];
+                            jacobi_load<G, E, false>(xa, ca, rows, gl, valid);
+                            jacobi_load<G, E, false>(xb, cb, rows, gl, valid);
+                            const bool rot = jacobi_rotate<G, E>(xa, xb, eps2);
+                            if (rot) {
+                                jacobi_store<G, E, false>(xa, ca, rows, gl);
+                                jacobi_store<G, E, false>(xb, cb, rows, gl);
+                                if (gl == 0) lr[a] = lr[b] = now;
+                            }
                             any |= rot;
                         }
                         __syncthreads();
                     }
                 }
                 if (!bye) {
-                    // the cross pairs: slot gw with slot B + (gw + step) mod B
+                    // the cross pairs: slot gw with slot B + (gw + step) mod
+                    // B.  A group's own column a stays in its registers for
+                    // the B steps (no other group touches it).
+                    const int a = gw;
+                    const bool in_a = column(a, b0, b1) < cols;
+                    double *ca = sm + (size_t)a * lds;
+                    double xa[E];
+                    bool moved = false;
+                    jacobi_load<G, E, false>(xa, ca, rows, gl, in_a);
                     for (int step = 0; step < B; ++step, ++now) {
-                        const int a = gw, b = B + (gw + step) % B;
-                        const bool valid = column(a, b0, b1) < cols &&
-                                           column(b, b0, b1) < cols &&
+                        const int b = B + (gw + step) % B;
+                        const bool valid = in_a && column(b, b0, b1) < cols &&
                                            !jacobi_unchanged(lr, a, b, now - T);
                         if (__any_sync(0xffffffffu, valid)) {
-                            const bool rot = jacobi_rotate<G, E>(
-                                sm + (size_t)a * lds, sm + (size_t)b * lds, rows,
-                                gl, valid, eps2);
-                            if (rot && gl == 0) lr[a] = lr[b] = now;
+                            double *cb = sm + (size_t)b * lds;
+                            double xb[E];
+                            // an inactive group's zero column b is never
+                            // rotated
+                            jacobi_load<G, E, false>(xb, cb, rows, gl, valid);
+                            const bool rot = jacobi_rotate<G, E>(xa, xb, eps2);
+                            if (rot) {
+                                jacobi_store<G, E, false>(xb, cb, rows, gl);
+                                if (gl == 0) lr[a] = lr[b] = now;
+                                moved = true;
+                            }
                             any |= rot;
                         }
                         __syncthreads();
                     }
+                    if (moved) {
+                        jacobi_store<G, E, false>(xa, ca, rows, gl);
+                    }
+                    __syncthreads();
                 }
                 for (int e = threadIdx.x; e < nslots * rows; e += THREADS) {
                     const int q = e / rows, i = e - q * rows;
@@ -1673,82 +2131,117 @@ static void jacobi_block_launch(TileWork *d_tiles, int ntiles, Workspace ws,
     cudaLaunchKernelEx(&cfg, fn, d_tiles, ws);
 }
 
-template <int CLASS, int G, int E, int THREADS, bool SMEM>
-static void jacobi_class_launch(TileWork *d_tiles, int ntiles, Workspace ws,
-                                size_t smem, cudaStream_t stream)
+// Tiles with rows_lo <= k1 <= rows_hi of the class (k1 <= kmax, the batch's
+// widest factor; k2 <= k1).
+template <int CLASS, int G, int E, int THREADS, int MINB, bool PAIRED>
+static int jacobi_rows_launch(TileWork *d_tiles, int ntiles, Workspace ws,
+                              int rows_lo, int rows_hi, cudaStream_t stream)
 {
-    auto *fn = k_jacobi<CLASS, G, E, THREADS, SMEM>;
-    if (SMEM && smem > 48 * 1024)
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    fn<<<ntiles, THREADS, SMEM ? smem : 0, stream>>>(d_tiles, ws);
+    const int kmax = ws.k_max;
+    if (kmax < rows_lo) return 0;
+    auto *fn = k_jacobi<CLASS, G, E, THREADS, MINB, PAIRED>;
+    size_t smem = 0;
+    if (E > 0) {
+        const int r = std::min(rows_hi, kmax);
+        smem = (size_t)jacobi_stride<G, (E > 0 ? E : 1), PAIRED>(r) * r * sizeof(double);
+        if (!PAIRED) smem = std::min(smem, kJacobiSmemMax);
+        if (smem > 48 * 1024)
+            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem);
+    }
+    fn<<<ntiles, THREADS, smem, stream>>>(d_tiles, ws, rows_lo, rows_hi);
+    return 1;
 }
 
-int launch_jacobi(TileWork *d_tiles, int ntiles, Workspace ws,
-                  cudaStream_t stream, cudaStream_t side)
+// Phase H of the pivoted Cholesky and the Jacobi SVD on its factor, by
+// ranges of rows on their own streams: the ranges are independent chains of
+// a few long launches that seldom fill the GPU one by one (81 tiles: 1.40
+// ms of Jacobi one after another, the longest of them 1.12 ms).  `lanes`
+// may hold null streams (everything then runs on `stream`).
+int launch_small_svd(TileWork *d_tiles, int ntiles, Workspace ws,
+                     cudaStream_t stream, const SvdLanes &lanes)
 {
-    // Classes a batch can reach, from the largest factor it may hold
-    // (k1, k2 <= k_max).  Shared memory is sized for the class's largest
-    // tile that fits.
     const int kmax = ws.k_max;
-    auto smem_for = [&](int rows) {
-        const int r = std::min(rows, kmax);
-        const size_t full = (size_t)(r | 1) * std::min(r, kmax) * sizeof(double);
-        return std::min(full, kJacobiSmemMax);
-    };
-    // The block classes (one CTA per SM, long-running) run on `side`, the
-    // others on `stream`, overlapping them.
-    cudaStream_t big = side ? side : stream;
-    cudaEvent_t fork = nullptr, join = nullptr;
-    if (side && kmax > 64) {
-        cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
-        cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
-        cudaEventRecord(fork, stream);
-        cudaStreamWaitEvent(side, fork, 0);
-    }
-    // the block classes (factor in global memory) on `side`; the classes
-    // whose factor sits in shared memory on `stream`, filling the SMs the
-    // last wave of the block classes leaves idle
-    if (kmax > 128)
-        jacobi_block_launch<4, 16, 12>(d_tiles, ntiles, ws,
-                                       std::min(kmax, 192), big);
-    if (kmax > 192)
-        jacobi_block_launch<6, 16, 16>(d_tiles, ntiles, ws,
-                                       std::min(kmax, 256), big);
-    if (kmax > 256)
-        jacobi_block_launch<7, 16, 18>(d_tiles, ntiles, ws,
-                                       std::min(kmax, 288), big);
-    if (kmax > 288)
-        jacobi_block_launch<8, 16, 20>(d_tiles, ntiles, ws,
-                                       std::min(kmax, 320), big);
-    if (kmax > 320)
-        jacobi_block_launch<9, 32, 16>(d_tiles, ntiles, ws,
-                                       std::min(kmax, 512), big);
-    if (kmax > 512)
-        jacobi_class_launch<10, 32, 0, 1024, false>(d_tiles, ntiles, ws, 0,
-                                                    big);
-    if (kmax > 192)
-        jacobi_class_launch<5, 16, 16, 512, true>(d_tiles, ntiles, ws,
-                                                  smem_for(256), stream);
-    if (kmax > 128)
-        jacobi_class_launch<3, 16, 12, 512, true>(d_tiles, ntiles, ws,
-                                                  smem_for(192), stream);
-    if (kmax > 64)
-        jacobi_class_launch<2, 8, 16, 512, true>(d_tiles, ntiles, ws,
-                                                 smem_for(128), stream);
-    jacobi_class_launch<0, 4, 8, 64, true>(d_tiles, ntiles, ws,
-                                           smem_for(32), stream);
-    if (kmax > 32)
-        jacobi_class_launch<1, 4, 16, 128, true>(d_tiles, ntiles, ws,
-                                                 smem_for(64), stream);
+    int count = 0;
+    const bool fork = lanes.fork != nullptr && kmax > 64;
+    cudaStream_t l1 = stream, l2 = stream, big = stream, mid = stream;
     if (fork) {
-        cudaEventRecord(join, side);
-        cudaStreamWaitEvent(stream, join, 0);
-        cudaEventDestroy(fork);
-        cudaEventDestroy(join);
+        l1 = lanes.s[0];
+        l2 = lanes.s[1];
+        big = lanes.s[2];
+        mid = lanes.s[3];
+        cudaEventRecord(lanes.fork, stream);
     }
-    return 1 + (kmax > 32) + (kmax > 64) + 2 * (kmax > 128) + 2 * (kmax > 192) +
-           (kmax > 256) + (kmax > 288) + (kmax > 320) + (kmax > 512);
+    auto start = [&](cudaStream_t s) {
+        if (fork) cudaStreamWaitEvent(s, lanes.fork, 0);
+    };
+    // above 128 rows: the block classes (factor in global memory), the
+    // longest chains, first; beside them the classes whose factor fits in
+    // shared memory
+    if (kmax > kPivcholSplit) {
+        start(big);
+        k_pivchol<kPivcholLanes><<<ntiles, kSmallThreads * kPivcholLanes, 0, big>>>(
+            d_tiles, ws, PH_H, kPivcholSplit + 1, INT_MAX, nullptr);
+        ++count;
+        if (fork) {
+            cudaEventRecord(lanes.done[4], big);
+            cudaStreamWaitEvent(mid, lanes.done[4], 0);
+        }
+        jacobi_block_launch<4, 16, 12>(d_tiles, ntiles, ws, std::min(kmax, 192), big);
+        ++count;
+        if (kmax > 192) {
+            jacobi_block_launch<6, 16, 16>(d_tiles, ntiles, ws, std::min(kmax, 256), big);
+            ++count;
+        }
+        if (kmax > 256) {
+            jacobi_block_launch<7, 16, 18>(d_tiles, ntiles, ws, std::min(kmax, 288), big);
+            ++count;
+        }
+        if (kmax > 288) {
+            jacobi_block_launch<8, 16, 20>(d_tiles, ntiles, ws, std::min(kmax, 320), big);
+            ++count;
+        }
+        if (kmax > 320) {
+            jacobi_block_launch<9, 32, 16>(d_tiles, ntiles, ws, std::min(kmax, 512), big);
+            ++count;
+        }
+        if (kmax > 512)
+            count += jacobi_rows_launch<10, 32, 0, 1024, 1, false>(
+                d_tiles, ntiles, ws, 513, kMaxK, big);
+        count += jacobi_rows_launch<5, 16, 16, 512, 1, false>(d_tiles, ntiles, ws, 193, 256, mid);
+        count += jacobi_rows_launch<3, 16, 12, 512, 1, false>(d_tiles, ntiles, ws, 161, 192, mid);
+        count += jacobi_rows_launch<3, 16, 10, 512, 1, false>(d_tiles, ntiles, ws, 129, 160, mid);
+    }
+    if (kmax > 96) {
+        start(l2);
+        pivchol_rows_launch<4>(d_tiles, ntiles, ws, PH_H, 97, 128, l2, nullptr);
+        ++count;
+        count += jacobi_rows_launch<2, 8, 16, 512, 1, true>(d_tiles, ntiles, ws, 113, 128, l2);
+        count += jacobi_rows_launch<2, 8, 14, 448, 1, true>(d_tiles, ntiles, ws, 97, 112, l2);
+    }
+    if (kmax > 64) {
+        start(l1);
+        pivchol_rows_launch<3>(d_tiles, ntiles, ws, PH_H, 65, 96, l1, nullptr);
+        ++count;
+        count += jacobi_rows_launch<2, 8, 12, 384, 2, true>(d_tiles, ntiles, ws, 81, 96, l1);
+        count += jacobi_rows_launch<2, 8, 10, 320, 2, true>(d_tiles, ntiles, ws, 65, 80, l1);
+    }
+    pivchol_rows_launch<2>(d_tiles, ntiles, ws, PH_H, INT_MIN, 64, stream, nullptr);
+    ++count;
+    count += jacobi_rows_launch<1, 4, 16, 128, 4, true>(d_tiles, ntiles, ws, 49, 64, stream);
+    count += jacobi_rows_launch<1, 4, 12, 96, 5, true>(d_tiles, ntiles, ws, 33, 48, stream);
+    count += jacobi_rows_launch<0, 4, 8, 64, 8, true>(d_tiles, ntiles, ws, 1, 32, stream);
+    if (fork) {
+        const cudaStream_t used[4] = {l1, kmax > 96 ? l2 : nullptr,
+                                      kmax > kPivcholSplit ? big : nullptr,
+                                      kmax > kPivcholSplit ? mid : nullptr};
+        for (int q = 0; q < 4; ++q)
+            if (used[q]) {
+                cudaEventRecord(lanes.done[q], used[q]);
+                cudaStreamWaitEvent(stream, lanes.done[q], 0);
+            }
+    }
+    return count;
 }
 
 // Appends the residual-pass columns to the basis: k1 += kb.
