@@ -73,7 +73,8 @@ static bool create_lanes(SvdLanes &l)
     for (cudaEvent_t &e : l.done)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
             return false;
-    return cudaEventCreateWithFlags(&l.fork, cudaEventDisableTiming) == cudaSuccess;
+    return cudaEventCreateWithFlags(&l.fork, cudaEventDisableTiming) == cudaSuccess &&
+           cudaEventCreateWithFlags(&l.large, cudaEventDisableTiming) == cudaSuccess;
 }
 
 // A context a thread has made its own (a serving worker's), or null.
@@ -211,6 +212,7 @@ void context_free_private(Context *c)
     cudaStreamDestroy(c->stream);
     for (cudaStream_t l : c->lanes.s) cudaStreamDestroy(l);
     cudaEventDestroy(c->lanes.fork);
+    cudaEventDestroy(c->lanes.large);
     for (cudaEvent_t e : c->lanes.done) cudaEventDestroy(e);
     cudaStreamDestroy(c->copy);
     delete c;
@@ -607,9 +609,10 @@ __global__ void k_store_to_host(const unsigned long long *__restrict__ src,
         dst[i] = src[i];
 }
 
-__global__ void k_count_to_host(const int *__restrict__ src, int *dst)
+// The counts of a round's set-up.
+__global__ void k_counts_to_host(const int *__restrict__ src, int *dst)
 {
-    *dst = *src;
+    if (threadIdx.x < 1 + kSvdBins) dst[threadIdx.x] = src[threadIdx.x];
 }
 
 // Runs the device pipeline over the far blocks of every problem of `jobs`
@@ -819,7 +822,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     if (!ctx.tiles.reserve((size_t)max_slots * sizeof(TileWork), s) ||
         !ctx.descs.reserve((size_t)max_slots * sizeof(GemmDesc), s) ||
         !ctx.flag.reserve(256, s) ||
-        !ctx.act.reserve((size_t)max_slots * sizeof(int), s))
+        !ctx.act.reserve((size_t)max_slots * (1 + kSvdBins) * sizeof(int), s))
         return cuda_fail(cudaErrorMemoryAllocation, "batch arrays");
     const size_t pin_need = (size_t)max_slots * sizeof(TileWork);
     if (ctx.tiles_pin_bytes < pin_need) {
@@ -916,7 +919,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         cudaEventRecord(ev[4], s);
         if (fused) {
             launch_round_setup(dt, nt, ep.block, (int *)ctx.flag.ptr,
-                               (int *)ctx.act.ptr, s);
+                               (int *)ctx.act.ptr, nt, s);
             if (any_separate) {
                 launch_gen_tiles(d_kernels, dt, nt, ws, s, TILE_GEN_SEPARATE,
                                  one_family);
@@ -1015,16 +1018,16 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             const bool pre_sketched = fused && round == 0;
             round_count = -1;
             if (!pre_sketched) {
-            launch_round_setup(dt, nt, block, d_active, (int *)ctx.act.ptr, s);
+            launch_round_setup(dt, nt, block, d_active, (int *)ctx.act.ptr, nt, s);
             count_launch();
             // round 0 samples every tile with a sketch width (known on
             // the host): the round is enqueued behind the generation
             // without waiting for the flag; later rounds read how many
             // tiles sample and run their GEMMs over those alone
             if (round > 0 || !any_width) {
-                k_count_to_host<<<1, 1, 0, s>>>(d_active, (int *)ctx.mapped_dev);
+                k_counts_to_host<<<1, 32, 0, s>>>(d_active, (int *)ctx.mapped_dev);
                 count_launch();
-                B200_CUDA(cudaGetLastError(), "k_count_to_host");
+                B200_CUDA(cudaGetLastError(), "k_counts_to_host");
                 B200_CUDA(cudaStreamSynchronize(s), "round flag");
                 const int active = *(volatile int *)ctx.mapped;
                 if (!active) break;
@@ -1094,7 +1097,13 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         if ((info = gemm(STEP_PROJECT, true, false, nt, k_max, plan[pi].n, none))) break;
         cudaEventRecord(ev[3], s);
         if ((info = gemm(STEP_GRAM_B, false, true, nt, k_max, k_max, none))) break;
-        count_launch(launch_small_svd(dt, nt, ws, s, ctx.lanes));
+        // the adaptive engine's last round set-up, which the host has read,
+        // counted and listed the tiles by basis size
+        const bool listed = ep.engine == STARSH_B200_MIXED;
+        int bins[kSvdBins];
+        if (listed) memcpy(bins, (const int *)ctx.mapped + 1, sizeof(bins));
+        count_launch(launch_small_svd(dt, nt, ws, s, ctx.lanes, listed ? bins : nullptr,
+                                      listed ? (const int *)ctx.act.ptr + nt : nullptr, nt));
         if ((info = gemm(STEP_ROTATE, true, false, nt, k_max, plan[pi].n, none))) break;
         launch_rank_cut(dt, nt, ws, s);
         count_launch();

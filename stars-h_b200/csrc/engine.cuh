@@ -156,17 +156,33 @@ void launch_gen_tiles(const DevKernel *d_kernels, const TileWork *d_tiles,
 // Phases A (0) and B (1) of the pivoted Cholesky.
 void launch_pivchol(int phase, TileWork *d_tiles, int ntiles, Workspace ws,
                     cudaStream_t s);
+// Ranges of basis sizes (rows of the small SVD's factor) that share a
+// kernel: bin b holds svd_bin_lo(b) .. svd_bin_hi(b) rows.
+constexpr int kSvdBins = 14;
+enum : int { kBin32 = 0, kBin48, kBin64, kBin80, kBin96, kBin112, kBin128, kSvdBinLarge };
+__host__ __device__ constexpr int svd_bin_hi(int b)
+{
+    return b == 0 ? 32 : b <= 6 ? 32 + 16 * b : b == 7 ? 160 : b == 8 ? 192
+         : b == 9 ? 256 : b == 10 ? 288 : b == 11 ? 320 : b == 12 ? 512 : 1 << 30;
+}
+__host__ __device__ constexpr int svd_bin_lo(int b) { return b == 0 ? 0 : svd_bin_hi(b - 1) + 1; }
+__host__ __device__ int svd_bin(int rows);
+
 // Streams and events the small SVD spreads its size ranges over (all null:
-// one stream).
+// one stream): one for each range above 64 rows, and one more.
 struct SvdLanes {
-    cudaStream_t s[4] = {nullptr, nullptr, nullptr, nullptr};
-    cudaEvent_t fork = nullptr;
-    cudaEvent_t done[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    static constexpr int kStreams = kSvdBins - kSvdBinLarge + 5;
+    cudaStream_t s[kStreams] = {};
+    cudaEvent_t fork = nullptr, large = nullptr;
+    cudaEvent_t done[kStreams] = {};
 };
 // Gram factor and Jacobi SVD of B B^T (in S): W, k2, tail_h; returns the
-// number of kernels launched.
+// number of kernels launched.  count / list (optional): the tiles of every
+// bin, as collected by the round set-up.
 int launch_small_svd(TileWork *d_tiles, int ntiles, Workspace ws,
-                     cudaStream_t stream, const SvdLanes &lanes);
+                     cudaStream_t stream, const SvdLanes &lanes,
+                     const int *count = nullptr, const int *list = nullptr,
+                     int list_ld = 0);
 // `act` (optional): the launch covers the `ntiles` tiles listed there (a
 // round's sampling tiles) instead of the first `ntiles` of the batch.
 void launch_gather_cols(int phase, const TileWork *d_tiles, int ntiles,
@@ -178,12 +194,13 @@ void launch_rank_cut(TileWork *d_tiles, int ntiles, Workspace ws,
                      cudaStream_t stream);
 void launch_merge_basis(TileWork *d_tiles, int ntiles, cudaStream_t stream);
 // Adaptive sketch: squared Frobenius norms of the generated blocks, round
-// set-up (returns through d_active whether any tile still samples) and the
-// per-round pivoted Cholesky of the residual block's Gram.
+// set-up (d_counts: tiles that still sample, then the tiles of every svd
+// bin; d_act: their lists, ld entries each) and the per-round pivoted
+// Cholesky of the residual block's Gram.
 void launch_block_norms(const TileWork *d_tiles, TileWork *d_rw, int ntiles,
                         Workspace ws, cudaStream_t stream);
 void launch_round_setup(TileWork *d_tiles, int ntiles, int block,
-                        int *d_active, int *d_act, cudaStream_t stream);
+                        int *d_counts, int *d_act, int ld, cudaStream_t stream);
 void launch_round_end(TileWork *d_tiles, int ntiles, int verify,
                       cudaStream_t stream);
 void launch_round_pivchol(TileWork *d_tiles, int ntiles, Workspace ws,

@@ -985,45 +985,90 @@ k_pivchol(TileWork *__restrict__ tiles, Workspace ws, int phase, int nn_lo,
     }
 }
 
-// Columns of an upper triangular inverse in shared memory, row-packed: row b
-// holds columns b .. cnt - 1, so lanes of consecutive columns read
-// consecutive doubles.
-__device__ __forceinline__ int tri_at(int b, int c, int cnt)
+// acc += sum of N products x[u sx] y[u sy], u ascending, all loads first.
+template <int N>
+__device__ __forceinline__ void chain_block(double &acc, const double *x, int sx,
+                                            const double *y, int sy)
 {
-    return b * cnt - b * (b - 1) / 2 + c - b;
+    double xv[N], yv[N];
+    #pragma unroll
+    for (int u = 0; u < N; ++u) {
+        xv[u] = x[u * sx];
+        yv[u] = y[u * sy];
+    }
+    #pragma unroll
+    for (int u = 0; u < N; ++u) acc = fma(xv[u], yv[u], acc);
 }
 
-// X = R^{-1} for the upper triangular R(a, b) = R[a * ra + b * rb], a <= b <
-// cnt, in shared memory, one thread per column (its back substitution sums
-// b = a + 1 .. c in that order, a chain of dependent products: the entry
-// just found stays in a register, the others' loads run ahead of the
-// chain), then T(:, 0:cnt) = X with zeros below the diagonal.  Called by
-// the whole block.
-__device__ __forceinline__ void tri_inverse(const double *R, int ra, int rb,
-                                            int cnt, double *X, double *T, int ld)
+// a[u mod C] += x[u s] y[u s] for u = 0 .. N - 1, all loads first.
+template <int C, int N>
+__device__ __forceinline__ void chains_block(double (&a)[C], const double *x,
+                                             const double *y, int s)
 {
-    for (int c = threadIdx.x; c < cnt; c += blockDim.x) {
-        double x = 1.0 / R[c * ra + c * rb];
-        X[tri_at(c, c, cnt)] = x;
-        for (int a = c - 1; a >= 0; --a) {
-            const double *r = R + a * ra + (a + 1) * rb;
-            double acc = fma(*r, x, 0.0);
-            int at = tri_at(a + 2, c, cnt);
-            #pragma unroll 8
-            for (int b = a + 2; b <= c; ++b) {
-                r += rb;
-                acc = fma(*r, X[at], acc);
-                at += cnt - b - 1;
+    double xv[N], yv[N];
+    #pragma unroll
+    for (int u = 0; u < N; ++u) {
+        xv[u] = x[u * s];
+        yv[u] = y[u * s];
+    }
+    #pragma unroll
+    for (int u = 0; u < N; ++u) a[u % C] = fma(xv[u], yv[u], a[u % C]);
+}
+
+// X = R^{-1} for the upper triangular R(a, b) = R[a * ld_r + b] (a < b < cnt,
+// diagonal in `diag`), in shared memory, one thread per column; X is stored
+// as rows of ldx doubles, zero below the diagonal, and copied to
+// T(:, 0:cnt).  A column's back substitution sums b = a + 1 .. c in that
+// order, a chain of dependent products; a warp runs its 32 columns in step
+// (the zeros change no sum), so the chain's loads go in whole blocks.
+// Called by the whole block.
+__device__ __forceinline__ void tri_inverse(const double *R, int ld_r,
+                                            const double *diag, int cnt,
+                                            double *X, int ldx, double *T, int ld)
+{
+    const int c = threadIdx.x, c_hi = min(cnt - 1, c | 31);
+    const int lane = threadIdx.x & 31;
+    if ((c & ~31) < cnt) {
+        const bool in = c < cnt;
+        double x = 0.0;                       // X(a + 1, c)
+        for (int a = c_hi; a >= 0; --a) {
+            double v = 0.0;
+            if (a < c_hi) {
+                const double *r = R + a * ld_r + a + 1;
+                double acc = fma(*r, x, 0.0);
+                const double *xp = X + (a + 2) * ldx + c;
+                int n = c_hi - a - 1;
+                ++r;
+                for (; n >= 16; n -= 16, r += 16, xp += 16 * ldx)
+                    chain_block<16>(acc, r, 1, xp, ldx);
+                if (n & 8) {
+                    chain_block<8>(acc, r, 1, xp, ldx);
+                    r += 8;
+                    xp += 8 * ldx;
+                }
+                if (n & 4) {
+                    chain_block<4>(acc, r, 1, xp, ldx);
+                    r += 4;
+                    xp += 4 * ldx;
+                }
+                if (n & 2) {
+                    chain_block<2>(acc, r, 1, xp, ldx);
+                    r += 2;
+                    xp += 2 * ldx;
+                }
+                if (n & 1) acc = fma(*r, *xp, acc);
+                v = -acc;
             }
-            x = -acc / R[a * ra + a * rb];
-            X[tri_at(a, c, cnt)] = x;
+            if (a == c) v = 1.0;
+            x = a <= c && in ? v / diag[a] : 0.0;
+            if (in) X[a * ldx + c] = x;
         }
+        if (in)
+            for (int a = c_hi + 1; a < cnt; ++a) X[a * ldx + c] = 0.0;
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    for (int c = threadIdx.x >> 5; c < cnt; c += blockDim.x >> 5)
-        for (int a = lane; a < cnt; a += 32)
-            T[(size_t)c * ld + a] = a <= c ? X[tri_at(a, c, cnt)] : 0.0;
+    for (int q = threadIdx.x >> 5; q < cnt; q += blockDim.x >> 5)
+        for (int a = lane; a < cnt; a += 32) T[(size_t)q * ld + a] = X[a * ldx + q];
 }
 
 // Order-preserving 64-bit key of a double.
@@ -1202,19 +1247,30 @@ k_pivchol_rows(TileWork *__restrict__ tiles, Workspace ws, int phase, int nn_lo,
             open = false;
             spiv[j] = p;
         } else if (open) {
-            double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+            // blocks of sixteen, eight and four products, four chains; the
+            // one to three left over join the first chain
+            double a[4] = {};
             const double *li = pc_sm + i, *lp = pc_sm + p;
-            int l = 0;
-            #pragma unroll 4
-            for (; l + 3 < j; l += 4, li += 4 * LD, lp += 4 * LD) {
-                a0 = fma(li[0], lp[0], a0);
-                a1 = fma(li[LD], lp[LD], a1);
-                a2 = fma(li[2 * LD], lp[2 * LD], a2);
-                a3 = fma(li[3 * LD], lp[3 * LD], a3);
+            int n = j;
+            for (; n >= 16; n -= 16, li += 16 * LD, lp += 16 * LD)
+                chains_block<4, 16>(a, li, lp, LD);
+            if (n & 8) {
+                chains_block<4, 8>(a, li, lp, LD);
+                li += 8 * LD;
+                lp += 8 * LD;
             }
-            for (; l < j; ++l, li += LD, lp += LD) a0 = fma(*li, *lp, a0);
-            const double acc = gq - ((a0 + a1) + (a2 + a3));
-            v = acc / sp;
+            if (n & 4) {
+                chains_block<4, 4>(a, li, lp, LD);
+                li += 4 * LD;
+                lp += 4 * LD;
+            }
+            if (n & 2) {
+                chain_block<2>(a[0], li, LD, lp, LD);
+                li += 2 * LD;
+                lp += 2 * LD;
+            }
+            if (n & 1) a[0] = fma(*li, *lp, a[0]);
+            v = (gq - ((a[0] + a[1]) + (a[2] + a[3]))) / sp;
             dg -= v * v;
         }
         if (i < nn) *colj = v;
@@ -1248,8 +1304,12 @@ k_pivchol_rows(TileWork *__restrict__ tiles, Workspace ws, int phase, int nn_lo,
         return;
     }
     int *piv = ws.Piv(s);
+    __shared__ double diag[32 * W];
     const int mine = i < cnt ? spiv[i] : 0;
-    if (i < cnt) piv[i] = mine;
+    if (i < cnt) {
+        piv[i] = mine;
+        diag[i] = pc_sm[i * LD + mine];
+    }
     // rows in pivot order: slot a then holds R11(a, b) = L(piv[b], a)
     for (int a0 = 0; a0 < cnt; a0 += 8) {
         double v[8];
@@ -1263,7 +1323,7 @@ k_pivchol_rows(TileWork *__restrict__ tiles, Workspace ws, int phase, int nn_lo,
     }
     __syncthreads();
     // T = R11^{-1} (upper triangular)
-    tri_inverse(pc_sm, LD, 1, cnt, pc_sm + nn_hi * LD, ws.T(s), ld);
+    tri_inverse(pc_sm, LD, diag, cnt, pc_sm + nn_hi * LD, LD, ws.T(s), ld);
 }
 
 template <int W>
@@ -1271,13 +1331,285 @@ static void pivchol_rows_launch(TileWork *d_tiles, int ntiles, Workspace ws,
                                 int phase, int nn_lo, int nn_hi,
                                 cudaStream_t stream, const int *act)
 {
-    const int tri = phase == PH_H ? 0 : nn_hi * (nn_hi + 1) / 2;
-    const size_t smem = ((size_t)nn_hi * (32 * W + 1) + tri) * sizeof(double);
+    const size_t smem = (size_t)(phase == PH_H ? 1 : 2) * nn_hi * (32 * W + 1) *
+                        sizeof(double);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(k_pivchol_rows<W>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_pivchol_rows<W><<<ntiles, 32 * W, smem, stream>>>(d_tiles, ws, phase, nn_lo,
                                                         nn_hi, act);
+}
+
+// Phase H for factors above kPivcholSplit rows: a cluster of CTAs shares the
+// rows in chunks of 32 (chunk w in CTA w mod CS), each CTA holding its rows
+// of the Gram, and then of L, in its own shared memory.  A step exchanges
+// the warps' pivot candidates and remaining-trace sums through distributed
+// shared memory (one cluster barrier), reads the pivot's row of L from the
+// CTA that owns it, and updates its rows.  Sums keep the order of
+// k_pivchol<4> (eight partial sums of the product by l mod 8, lanes' trees
+// over chunks), so both give the same bits; that kernel reads L from L2 in
+// one CTA: about 9 us a step at 150 .. 270 rows, 1.5 ms and more for a
+// launch with a few such tiles.
+constexpr int kClusterRows = 128;     // most rows of one CTA of the cluster
+constexpr int kClusterMaxChunks = 16;
+
+template <int CS>
+__host__ __device__ constexpr int pivchol_cluster_warps(int nn)
+{
+    return ((nn + 31) / 32 + CS - 1) / CS;
+}
+
+template <int CS>
+__global__ void __launch_bounds__(kClusterRows)
+k_pivchol_cluster(TileWork *__restrict__ tiles, Workspace ws, int nn_lo, int nn_hi,
+                  const int *__restrict__ act)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ double pk_sm[];          // [slot][own rows]
+    __shared__ unsigned long long ck[2][kClusterMaxChunks];
+    __shared__ int ci[2][kClusterMaxChunks];
+    __shared__ double cs[2][kClusterMaxChunks];
+    __shared__ int pos[32 * kClusterMaxChunks], at[32 * kClusterMaxChunks];
+    __shared__ __align__(16) double lp[32 * kClusterMaxChunks + 16];
+    const int rank = (int)cl.block_rank();
+    TileWork &tw = tiles[act ? act[blockIdx.x / CS] : blockIdx.x / CS];
+    const int s = tw.slot, nn = tw.k1;
+    if (nn < nn_lo || nn > nn_hi) return;       // cluster-uniform
+    const double tol = tw.tol, dn = tw.dnorm2;
+    const int nchunk = (nn + 31) / 32;
+    const int nw = pivchol_cluster_warps<CS>(nn), rl = 32 * nw;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int chunk = warp * CS + rank;         // this warp's rows
+    const int i = chunk * 32 + lane;
+    const bool mine = warp < nw && i < nn;
+    const double *G = ws.S(s);
+    const int ld = ws.ldK();
+    if (mine)
+        for (int c = 0; c < nn; ++c) {
+            const unsigned d = (unsigned)__cvta_generic_to_shared(pk_sm + c * rl + t);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
+                         :: "r"(d), "l"(G + (size_t)c * ld + i));
+        }
+    asm volatile("cp.async.commit_group;");
+    for (int q = t; q < 32 * kClusterMaxChunks; q += kClusterRows) pos[q] = at[q] = q;
+    for (int q = t; q < 2 * kClusterMaxChunks; q += kClusterRows) {
+        ck[q / kClusterMaxChunks][q % kClusterMaxChunks] = 0;
+        ci[q / kClusterMaxChunks][q % kClusterMaxChunks] = 1 << 30;
+        cs[q / kClusterMaxChunks][q % kClusterMaxChunks] = 0.0;
+    }
+    asm volatile("cp.async.wait_group 0;");
+    cl.sync();
+    double dg = mine ? pk_sm[i * rl + t] : 0.0;
+    bool open = mine;
+    // The chunks' best candidates and sums to every CTA, then the overall
+    // best (largest value, then smallest row) and the sum in block_sum's
+    // order (tree over the chunks).
+    // (two sets of slots in turn: a set is written again only after the
+    // barrier of the exchange between, which every reader has passed)
+    unsigned long long bk;
+    int bi, par = 1;
+    double total;
+    auto exchange = [&](double x) {
+        par ^= 1;
+        const bool in = open && dg > -DBL_MAX;
+        const unsigned long long k = order_key(in ? dg : -DBL_MAX);
+        const unsigned hi = (unsigned)(k >> 32), lo = (unsigned)k;
+        const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+        const unsigned row = in && hi == mh && lo == ml ? (unsigned)i : 1u << 30;
+        const int wi = (int)__reduce_min_sync(0xffffffffu, row);
+        #pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (warp < nw && chunk < nchunk && lane < CS) {
+            *cl.map_shared_rank(&ck[par][chunk], lane) =
+                ((unsigned long long)mh << 32) | ml;
+            *cl.map_shared_rank(&ci[par][chunk], lane) = wi;
+            *cl.map_shared_rank(&cs[par][chunk], lane) = x;
+        }
+        cl.sync();
+        const int w = lane & (kClusterMaxChunks - 1);
+        const unsigned long long kk = ck[par][w];
+        const unsigned kh = (unsigned)(kk >> 32), kl = (unsigned)kk;
+        const unsigned gh = __reduce_max_sync(0xffffffffu, kh);
+        const unsigned gl = __reduce_max_sync(0xffffffffu, kh == gh ? kl : 0u);
+        bi = (int)__reduce_min_sync(0xffffffffu,
+                                    kh == gh && kl == gl ? (unsigned)ci[par][w] : 1u << 30);
+        bk = ((unsigned long long)gh << 32) | gl;
+        total = lane < kClusterMaxChunks ? cs[par][w] : 0.0;
+        #pragma unroll
+        for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    };
+    exchange(dg);
+    const double trace = total;
+    const double dmax = key_value(bk);
+    double thr = 1e-18 * dmax;
+    const bool lead = rank == 0 && t == 0;
+    if (lead) tw.tr_h = trace;
+    const double energy = dn > 0.0 ? fmax(dn, trace) : trace;
+    const double stop_trace = 0.01 * tol * tol * energy;
+    if (dn > 0.0 &&
+        fmax(0.0, dn - trace - 2e-15 * dn) > tol * tol * fmax(dn, trace)) {
+        if (lead) {
+            tw.k2 = 0;
+            tw.tail_h = trace;
+            tw.status |= TILE_TAIL_LEFT;
+        }
+        return;
+    }
+    if (!(dmax > 0.0)) thr = DBL_MAX;
+    int j = 0;
+    for (; j < nn; ++j) {
+        exchange(open ? fmax(0.0, dg) : 0.0);
+        if (total <= stop_trace) break;
+        const double best = key_value(bk);
+        if (!(best > thr)) break;
+        const int p = bi;
+        const double sp = sqrt(best);
+        // row p of L from its CTA (chunk p / 32 is warp (p / 32) / CS of CTA
+        // (p / 32) mod CS there)
+        {
+            const double *src = cl.map_shared_rank(pk_sm, (p >> 5) % CS) +
+                                ((p >> 5) / CS * 32 + (p & 31));
+            for (int l = t; l < j + 16; l += kClusterRows)
+                lp[l] = l < j ? src[(size_t)l * rl] : 0.0;
+        }
+        const int q = pos[p], r = at[j];
+        double gq = 0.0;
+        if (mine) {
+            gq = pk_sm[q * rl + t];
+            pk_sm[q * rl + t] = pk_sm[j * rl + t];
+        }
+        __syncthreads();
+        double v = 0.0;
+        if (mine) {
+            if (i == p) {
+                v = sp;
+                open = false;
+            } else if (open) {
+                // lane q of the replaced kernel summed l = q, q + 8, ... and
+                // l = q + 4, q + 12, ...
+                double a[8] = {};
+                const double *li = pk_sm + t;
+                const double2 *l2 = reinterpret_cast<const double2 *>(lp);
+                int l = 0;
+                for (; l + 15 < j; l += 16) {
+                    double x[16];
+                    double2 y[8];
+                    #pragma unroll
+                    for (int u = 0; u < 16; ++u) x[u] = li[(l + u) * rl];
+                    #pragma unroll
+                    for (int u = 0; u < 8; ++u) y[u] = l2[l / 2 + u];
+                    #pragma unroll
+                    for (int u = 0; u < 16; ++u)
+                        a[u & 7] = fma(x[u], u & 1 ? y[u / 2].y : y[u / 2].x, a[u & 7]);
+                }
+                {
+                    // up to fifteen more (lp is zero past j)
+                    double x[16];
+                    #pragma unroll
+                    for (int u = 0; u < 16; ++u)
+                        x[u] = l + u < j ? li[(l + u) * rl] : 0.0;
+                    #pragma unroll
+                    for (int u = 0; u < 15; ++u) a[u & 7] = fma(x[u], lp[l + u], a[u & 7]);
+                }
+                const double p0 = a[0] + a[4], p1 = a[1] + a[5];
+                const double p2 = a[2] + a[6], p3 = a[3] + a[7];
+                v = (gq - ((p0 + p2) + (p1 + p3))) / sp;
+                dg -= v * v;
+            }
+            pk_sm[j * rl + t] = v;
+        }
+        // the moved column's place (every thread has read pos and at)
+        if (t == 0) {
+            pos[r] = q;
+            at[q] = r;
+        }
+    }
+    const int cnt = j;
+    if (lead) {
+        tw.k2 = cnt;
+        if (cnt == 0) tw.tail_h = trace;
+    }
+    exchange(open ? fmax(0.0, dg) : 0.0);
+    if (lead && cnt > 0) tw.tail_h = total;
+    double *L = ws.L(s);
+    if (mine)
+        for (int c = 0; c < cnt; ++c) L[(size_t)c * ld + i] = pk_sm[c * rl + t];
+    cl.sync();     // no CTA leaves while another may still read its rows
+}
+
+// Most rows k_pivchol_cluster<CS> takes: a CTA's share of the Gram within
+// its shared memory (kJacobiSmemMax).
+template <int CS>
+static int pivchol_cluster_fit(int kmax)
+{
+    int nn = std::min(kmax, 32 * kClusterMaxChunks);
+    while (nn > 0 && (pivchol_cluster_warps<CS>(nn) * 32 > kClusterRows ||
+                      (size_t)nn * 32 * pivchol_cluster_warps<CS>(nn) * sizeof(double) >
+                          208 * 1024))
+        --nn;
+    return nn;
+}
+
+template <int CS>
+static void pivchol_cluster_launch(TileWork *d_tiles, int ntiles, Workspace ws,
+                                   int nn_lo, int nn_hi, cudaStream_t stream,
+                                   const int *act)
+{
+    size_t smem = 0;
+    for (int nn = nn_lo; nn <= nn_hi; ++nn)
+        smem = std::max(smem, (size_t)nn * 32 * pivchol_cluster_warps<CS>(nn) * sizeof(double));
+    auto *fn = k_pivchol_cluster<CS>;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(ntiles * CS));
+    cfg.blockDim = dim3(kClusterRows);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CS;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, fn, d_tiles, ws, nn_lo, nn_hi, act);
+}
+
+// Phase H above kPivcholSplit rows, `count` tiles (of `act`, or the first
+// ones of the batch).  A few tiles: clusters of four as far as their shared
+// memory reaches (at least 256 rows), of eight beyond; a cluster keeps four
+// SMs to itself, so with more tiles than about two rounds of clusters the
+// one-CTA kernel, two tiles to an SM, has more throughput (134 mixed tiles:
+// 1.51 -> 0.59 ms with clusters; 641 tiles of a batch: 4.70 ms against
+// 4.98).  Returns the number of launches.
+constexpr int kPivcholClusterTiles = 74;
+
+static int pivchol_large_launch(TileWork *d_tiles, int count, Workspace ws,
+                                cudaStream_t stream, const int *act)
+{
+    const int kmax = ws.k_max;
+    int lo = kPivcholSplit + 1, launches = 0;
+    if (count <= kPivcholClusterTiles) {
+        const int fit4 = pivchol_cluster_fit<4>(kmax), fit8 = pivchol_cluster_fit<8>(kmax);
+        if (fit4 >= lo) {
+            pivchol_cluster_launch<4>(d_tiles, count, ws, lo, fit4, stream, act);
+            lo = fit4 + 1;
+            ++launches;
+        }
+        if (kmax >= lo && fit8 >= lo) {
+            pivchol_cluster_launch<8>(d_tiles, count, ws, lo, fit8, stream, act);
+            lo = fit8 + 1;
+            ++launches;
+        }
+    }
+    if (kmax >= lo) {
+        k_pivchol<kPivcholLanes><<<count, kSmallThreads * kPivcholLanes, 0, stream>>>(
+            d_tiles, ws, PH_H, lo, INT_MAX, act);
+        ++launches;
+    }
+    return launches;
 }
 
 // A round's pivoted Cholesky; `bmax` bounds the round's columns.
@@ -1324,14 +1656,18 @@ void launch_block_norms(const TileWork *, TileWork *d_rw, int ntiles,
 }
 
 // Start of a sampling round: tiles not done sample min(block, k - cols)
-// more columns; *active counts them (each takes the next round slot, in
-// any order: a slot only places the tile's GEMM descriptors).
+// more columns; counts[0] counts them (each takes the next round slot, in
+// any order: a slot only places the tile's GEMM descriptors).  counts[1 + b]
+// and the lists after act[0 .. ld - 1] collect the tiles by basis size
+// (svd_bin), for the small SVD when no tile samples any more.
 __global__ void k_round_setup(TileWork *__restrict__ tiles, int ntiles,
-                              int block, int *active, int *act)
+                              int block, int *counts, int *act, int ld)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntiles) return;
     TileWork &tw = tiles[t];
+    const int b = svd_bin(tw.k1);
+    act[(size_t)(1 + b) * ld + atomicAdd(counts + 1 + b, 1)] = t;
     if (tw.done || tw.cols_done >= tw.k) {
         tw.bcur = 0;
         tw.done = 1;
@@ -1341,17 +1677,16 @@ __global__ void k_round_setup(TileWork *__restrict__ tiles, int ntiles,
     tw.bcur = min(block, tw.k - tw.cols_done);
     tw.k1_round = tw.k1;
     tw.trunc_round = 0;
-    tw.round_slot = atomicAdd(active, 1);
+    tw.round_slot = atomicAdd(counts, 1);
     act[tw.round_slot] = t;
 }
 
 void launch_round_setup(TileWork *d_tiles, int ntiles, int block,
-                        int *d_active, int *d_act, cudaStream_t stream)
+                        int *d_counts, int *d_act, int ld, cudaStream_t stream)
 {
-    cudaMemsetAsync(d_active, 0, sizeof(int), stream);
-    k_round_setup<<<(ntiles + 127) / 128, 128, 0, stream>>>(d_tiles, ntiles,
-                                                            block, d_active,
-                                                            d_act);
+    cudaMemsetAsync(d_counts, 0, (1 + kSvdBins) * sizeof(int), stream);
+    k_round_setup<<<(ntiles + 127) / 128, 128, 0, stream>>>(d_tiles, ntiles, block,
+                                                            d_counts, d_act, ld);
 }
 
 // End of a round: the new orthonormal columns join the basis.  The tile is
@@ -1484,59 +1819,63 @@ k_chol_inv(TileWork *__restrict__ tiles, Workspace ws, int phase, int nn_lo,
     }
 }
 
-// The same for nn <= kCholSmall: the Gram sits in shared memory and is
-// factored right-looking, so a step is one square root, one quotient and
-// one update per entry instead of a chain of j of them; every entry still
-// subtracts its products in the order l = 0, 1, ..., so both kernels give
-// the same bits.  81 tiles with up to 64 columns: 150 -> 35 us.
+// The same for nn <= N, right-looking: thread (c, q) keeps the rows q, q +
+// 4, ... of column c in registers, so a step is one square root, one
+// quotient and one product per entry instead of a chain of l of them; every
+// entry still subtracts its products in the order l = 0, 1, ..., so both
+// kernels give the same bits.  Rows of the trailing matrix that are done,
+// and entries below the diagonal, are updated along with the others and
+// never read.
 constexpr int kCholSmall = 64;
 
-__global__ void __launch_bounds__(256)
+template <int N>
+__global__ void __launch_bounds__(4 * N)
 k_chol_inv_small(TileWork *__restrict__ tiles, Workspace ws, int phase,
-                 int nn_hi, const int *__restrict__ act)
+                 const int *__restrict__ act)
 {
+    constexpr int LD = N + 1, E = N / 4;
+    __shared__ double next[N], gd[N], diag[N];
     extern __shared__ double ci_sm[];
-    __shared__ double gd[kCholSmall];
     TileWork &tw = tiles[act ? act[blockIdx.x] : blockIdx.x];
     const int s = tw.slot;
     const int nn = phase == PH_A ? tw.k1 : tw.kb;
-    if (nn <= 0 || nn > nn_hi) return;
-    constexpr int LD = kCholSmall + 1;
-    double *A = ci_sm, *X = ci_sm + kCholSmall * LD;
+    if (nn <= 0 || nn > N) return;
+    double *R = ci_sm, *X = ci_sm + N * LD;     // R by rows
     const double *G = ws.S(s);
     const int ld = ws.ldK();
-    // thread (c, q): column c, rows j = q, q + 4, ...
-    const int c = threadIdx.x & 63, q = threadIdx.x >> 6;
-    for (int e = threadIdx.x; e < nn * 64; e += 256) {
-        const int row = e & 63, col = e >> 6;
-        if (row <= col) A[col * LD + row] = G[(size_t)col * ld + row];
+    const int c = threadIdx.x % N, q = threadIdx.x / N;
+    double a[E];
+    #pragma unroll
+    for (int u = 0; u < E; ++u) {
+        const int row = q + 4 * u;
+        a[u] = row <= c && c < nn ? G[(size_t)c * ld + row] : 0.0;
+        if (row == c) gd[c] = a[u];
     }
-    __syncthreads();
-    if (threadIdx.x < nn) gd[threadIdx.x] = A[threadIdx.x * LD + threadIdx.x];
+    for (int e = threadIdx.x; e < N * LD; e += 4 * N) R[e] = 0.0;
+    if (q == 0) next[c] = a[0];
     __syncthreads();
     int nn_ok = nn;
     for (int l = 0; l < nn; ++l) {
-        const double acc = A[l * LD + l];
+        const double acc = next[l];
         // a column numerically inside the span of the previous ones ends
         // the factor (as above); the test is the same for every thread
         if (!(acc > 1e-14 * gd[l])) { nn_ok = l; break; }
         const double r = sqrt(fmax(acc, 0.0));
-        // every thread forms its column's R(l, c) itself; one of the four
-        // stores it, and the diagonal is read by all before it is stored
-        double rc = 0.0;
-        if (c > l && c < nn) rc = A[c * LD + l] / r;
+        // each of a column's four threads forms its R(l, c), one stores it
+        const double rc = c > l && c < nn ? next[c] / r : 0.0;
+        if (q == 0) R[l * LD + c] = rc;
+        if (threadIdx.x == 0) diag[l] = r;
         __syncthreads();
-        if (q == 0 && c < nn) {
-            if (c == l) A[l * LD + l] = r;
-            else if (c > l) A[c * LD + l] = rc;
-        }
-        __syncthreads();
-        if (c < nn)
-            for (int j = l + 1 + q; j <= c; j += 4)
-                A[c * LD + j] -= A[j * LD + l] * rc;
+        #pragma unroll
+        for (int u = 0; u < E; ++u)
+            if (4 * u + 3 > l) {                 // uniform
+                const int j = q + 4 * u;
+                a[u] -= R[l * LD + j] * rc;
+                if (j == l + 1) next[c] = a[u];
+            }
         __syncthreads();
     }
-    tri_inverse(A, 1, LD, nn_ok, X, ws.T(s), ld);
+    tri_inverse(R, LD, diag, nn_ok, X, LD, ws.T(s), ld);
     if (threadIdx.x == 0 && nn_ok < nn) {
         if (phase == PH_A) tw.k1 = nn_ok;
         else tw.kb = nn_ok;
@@ -1545,15 +1884,25 @@ k_chol_inv_small(TileWork *__restrict__ tiles, Workspace ws, int phase,
     }
 }
 
+template <int N>
+static void chol_small_launch(int phase, TileWork *d_tiles, int ntiles,
+                              Workspace ws, cudaStream_t stream, const int *act)
+{
+    constexpr size_t smem = (size_t)2 * N * (N + 1) * sizeof(double);
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(k_chol_inv_small<N>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_chol_inv_small<N><<<ntiles, 4 * N, smem, stream>>>(d_tiles, ws, phase, act);
+}
+
 // `nmax` bounds the columns of every tile.
 void launch_chol_inv(int phase, TileWork *d_tiles, int ntiles, Workspace ws,
                      int nmax, cudaStream_t stream, const int *act)
 {
-    constexpr size_t smem = ((size_t)kCholSmall * (kCholSmall + 1) +
-                             kCholSmall * (kCholSmall + 1) / 2) * sizeof(double);
-    cudaFuncSetAttribute(k_chol_inv_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-    k_chol_inv_small<<<ntiles, 256, smem, stream>>>(d_tiles, ws, phase, kCholSmall, act);
+    if (nmax <= 32)
+        chol_small_launch<32>(phase, d_tiles, ntiles, ws, stream, act);
+    else
+        chol_small_launch<kCholSmall>(phase, d_tiles, ntiles, ws, stream, act);
     if (nmax > kCholSmall)
         k_chol_inv<<<ntiles, kSmallThreads, 0, stream>>>(d_tiles, ws, phase,
                                                          kCholSmall + 1, act);
@@ -1770,7 +2119,8 @@ __host__ __device__ constexpr int jacobi_stride(int rows)
 // ranges fit two CTAs on an SM.
 template <int CLASS, int G, int E, int THREADS, int MINB, bool PAIRED>
 __global__ void __launch_bounds__(THREADS, MINB)
-k_jacobi(TileWork *__restrict__ tiles, Workspace ws, int rows_lo, int rows_hi)
+k_jacobi(TileWork *__restrict__ tiles, Workspace ws, int rows_lo, int rows_hi,
+         const int *__restrict__ act)
 {
     constexpr bool SMEM = E > 0;
     constexpr int EE = SMEM ? E : 1;
@@ -1778,7 +2128,7 @@ k_jacobi(TileWork *__restrict__ tiles, Workspace ws, int rows_lo, int rows_hi)
     double *sm = reinterpret_cast<double *>(jac_sm);
     __shared__ int rotated[2];
     __shared__ int lastrot[jacobi_class_cols(CLASS)];
-    TileWork &tw = tiles[blockIdx.x];
+    TileWork &tw = tiles[act ? act[blockIdx.x] : blockIdx.x];
     const int s = tw.slot;
     const int rows = tw.k1, cols = tw.k2;
     if (cols <= 0 || rows < rows_lo || rows > rows_hi ||
@@ -1907,13 +2257,14 @@ k_jacobi(TileWork *__restrict__ tiles, Workspace ws, int rows_lo, int rows_hi)
 // read past L1 (__ldcg).
 constexpr int kJacobiClusterMax = 8;
 
-// CTAs per tile: 4 for the classes above 256 rows and for every block
-// class of a batch that holds such factors (kmax > 256: its large tiles
-// bound the batch), 2 otherwise (measured: on batches whose factors stay
-// below 257 rows, 4 CTAs per tile take SMs from the shared-memory classes
-// beside them and lose, on batches with larger factors they win);
+// CTAs per tile.  With few tiles the chain of one tile is what the launch
+// takes: one CTA for each meeting of a round (blocks of 512 / G columns, at
+// most k1 of them).  With more tiles than SMs, meetings queue on the SMs
+// anyway and a CTA per meeting only adds idle ones: 2, or 4 for the classes
+// above 256 rows.  Without the tile count (no list) the batch's widest
+// factor decides, as measured: 4 where kmax > 256, else 2.
 // STARSH_B200_JACOBI_CLUSTER (1 .. 8) sets one size for all.
-static int jacobi_cluster(int cls, int kmax)
+static int jacobi_cluster(int cls, int kmax, int count, bool known)
 {
     static const int forced = [] {
         int v = 0;
@@ -1921,12 +2272,19 @@ static int jacobi_cluster(int cls, int kmax)
             v = std::max(1, std::min(kJacobiClusterMax, atoi(e)));
         return v;
     }();
-    return forced ? forced : (cls >= 7 || kmax > 256) ? 4 : 2;
+    if (forced) return forced;
+    if (known && count <= 148) {
+        const int b = cls == 9 ? 16 : 32;
+        const int nb = (std::min(kmax, jacobi_class_cols(cls)) + b - 1) / b;
+        return std::max(2, std::min(kJacobiClusterMax, (nb + 1) / 2));
+    }
+    return cls >= 7 || (!known && kmax > 256) ? 4 : 2;
 }
 
 template <int CLASS, int G, int E>
 __global__ void __launch_bounds__(512, 1)
-k_jacobi_block(TileWork *__restrict__ tiles, Workspace ws)
+k_jacobi_block(TileWork *__restrict__ tiles, Workspace ws,
+               const int *__restrict__ act)
 {
     constexpr int THREADS = 512;
     constexpr int B = THREADS / G;          // columns per block, pairs per step
@@ -1937,7 +2295,7 @@ k_jacobi_block(TileWork *__restrict__ tiles, Workspace ws)
     extern __shared__ double sm[];
     __shared__ int rotated[2];              // in the cluster's first CTA
     __shared__ int lr[P2];                  // lastrot of the meeting's slots
-    TileWork &tw = tiles[blockIdx.x / csize];
+    TileWork &tw = tiles[act ? act[blockIdx.x / csize] : blockIdx.x / csize];
     const int s = tw.slot;
     const int rows = tw.k1, cols = tw.k2;
     if (cols <= 0 || jacobi_class(rows, cols) != CLASS) return;   // cluster-uniform
@@ -2108,7 +2466,7 @@ k_jacobi_block(TileWork *__restrict__ tiles, Workspace ws)
 
 template <int CLASS, int G, int E>
 static void jacobi_block_launch(TileWork *d_tiles, int ntiles, Workspace ws,
-                                int max_rows, cudaStream_t stream)
+                                int max_rows, cudaStream_t stream, const int *act)
 {
     const int kmax = ws.k_max;
     auto *fn = k_jacobi_block<CLASS, G, E>;
@@ -2116,7 +2474,7 @@ static void jacobi_block_launch(TileWork *d_tiles, int ntiles, Workspace ws,
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
     cudaLaunchConfig_t cfg = {};
-    const int cs = jacobi_cluster(CLASS, kmax);
+    const int cs = jacobi_cluster(CLASS, kmax, ntiles, act != nullptr);
     cfg.gridDim = dim3((unsigned)(ntiles * cs));
     cfg.blockDim = dim3(512);
     cfg.dynamicSmemBytes = smem;
@@ -2128,120 +2486,163 @@ static void jacobi_block_launch(TileWork *d_tiles, int ntiles, Workspace ws,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, fn, d_tiles, ws);
+    cudaLaunchKernelEx(&cfg, fn, d_tiles, ws, act);
 }
 
 // Tiles with rows_lo <= k1 <= rows_hi of the class (k1 <= kmax, the batch's
 // widest factor; k2 <= k1).
 template <int CLASS, int G, int E, int THREADS, int MINB, bool PAIRED>
-static int jacobi_rows_launch(TileWork *d_tiles, int ntiles, Workspace ws,
-                              int rows_lo, int rows_hi, cudaStream_t stream)
+static void jacobi_rows_launch(TileWork *d_tiles, int ntiles, Workspace ws,
+                               int rows_lo, int rows_hi, cudaStream_t stream,
+                               const int *act)
 {
-    const int kmax = ws.k_max;
-    if (kmax < rows_lo) return 0;
     auto *fn = k_jacobi<CLASS, G, E, THREADS, MINB, PAIRED>;
     size_t smem = 0;
     if (E > 0) {
-        const int r = std::min(rows_hi, kmax);
+        const int r = std::min(rows_hi, ws.k_max);
         smem = (size_t)jacobi_stride<G, (E > 0 ? E : 1), PAIRED>(r) * r * sizeof(double);
         if (!PAIRED) smem = std::min(smem, kJacobiSmemMax);
         if (smem > 48 * 1024)
             cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
     }
-    fn<<<ntiles, THREADS, smem, stream>>>(d_tiles, ws, rows_lo, rows_hi);
-    return 1;
+    fn<<<ntiles, THREADS, smem, stream>>>(d_tiles, ws, rows_lo, rows_hi, act);
+}
+
+__host__ __device__ int svd_bin(int rows)
+{
+    int b = 0;
+    while (b + 1 < kSvdBins && rows > svd_bin_hi(b)) ++b;
+    return b;
 }
 
 // Phase H of the pivoted Cholesky and the Jacobi SVD on its factor, by
-// ranges of rows on their own streams: the ranges are independent chains of
-// a few long launches that seldom fill the GPU one by one (81 tiles: 1.40
-// ms of Jacobi one after another, the longest of them 1.12 ms).  `lanes`
-// may hold null streams (everything then runs on `stream`).
+// ranges of rows (svd_bin) on their own streams: the ranges are independent
+// chains of a few long launches that seldom fill the GPU one by one (81
+// tiles: 1.40 ms of Jacobi one after another, the longest of them 1.12 ms).
+// `count` (host) and `list` (device, kSvdBins lists of `list_ld` tiles) tell
+// the tiles of each range, so that only they are launched; null: every
+// range is launched over the whole batch, each CTA taking its tile or
+// leaving it.  Without lanes everything runs on `stream`.
 int launch_small_svd(TileWork *d_tiles, int ntiles, Workspace ws,
-                     cudaStream_t stream, const SvdLanes &lanes)
+                     cudaStream_t stream, const SvdLanes &lanes,
+                     const int *count, const int *list, int list_ld)
 {
     const int kmax = ws.k_max;
-    int count = 0;
+    int launches = 0;
     const bool fork = lanes.fork != nullptr && kmax > 64;
-    cudaStream_t l1 = stream, l2 = stream, big = stream, mid = stream;
-    if (fork) {
-        l1 = lanes.s[0];
-        l2 = lanes.s[1];
-        big = lanes.s[2];
-        mid = lanes.s[3];
-        cudaEventRecord(lanes.fork, stream);
-    }
-    auto start = [&](cudaStream_t s) {
-        if (fork) cudaStreamWaitEvent(s, lanes.fork, 0);
+    if (fork) cudaEventRecord(lanes.fork, stream);
+    bool used[SvdLanes::kStreams] = {};
+    // stream q of the lanes, waiting for the fork at its first use
+    auto lane = [&](int q) {
+        if (!fork) return stream;
+        if (!used[q]) {
+            cudaStreamWaitEvent(lanes.s[q], lanes.fork, 0);
+            used[q] = true;
+        }
+        return lanes.s[q];
     };
-    // above 128 rows: the block classes (factor in global memory), the
-    // longest chains, first; beside them the classes whose factor fits in
-    // shared memory
-    if (kmax > kPivcholSplit) {
-        start(big);
-        k_pivchol<kPivcholLanes><<<ntiles, kSmallThreads * kPivcholLanes, 0, big>>>(
-            d_tiles, ws, PH_H, kPivcholSplit + 1, INT_MAX, nullptr);
-        ++count;
-        if (fork) {
-            cudaEventRecord(lanes.done[4], big);
-            cudaStreamWaitEvent(mid, lanes.done[4], 0);
-        }
-        jacobi_block_launch<4, 16, 12>(d_tiles, ntiles, ws, std::min(kmax, 192), big);
-        ++count;
-        if (kmax > 192) {
-            jacobi_block_launch<6, 16, 16>(d_tiles, ntiles, ws, std::min(kmax, 256), big);
-            ++count;
-        }
-        if (kmax > 256) {
-            jacobi_block_launch<7, 16, 18>(d_tiles, ntiles, ws, std::min(kmax, 288), big);
-            ++count;
-        }
-        if (kmax > 288) {
-            jacobi_block_launch<8, 16, 20>(d_tiles, ntiles, ws, std::min(kmax, 320), big);
-            ++count;
-        }
-        if (kmax > 320) {
-            jacobi_block_launch<9, 32, 16>(d_tiles, ntiles, ws, std::min(kmax, 512), big);
-            ++count;
-        }
-        if (kmax > 512)
-            count += jacobi_rows_launch<10, 32, 0, 1024, 1, false>(
-                d_tiles, ntiles, ws, 513, kMaxK, big);
-        count += jacobi_rows_launch<5, 16, 16, 512, 1, false>(d_tiles, ntiles, ws, 193, 256, mid);
-        count += jacobi_rows_launch<3, 16, 12, 512, 1, false>(d_tiles, ntiles, ws, 161, 192, mid);
-        count += jacobi_rows_launch<3, 16, 10, 512, 1, false>(d_tiles, ntiles, ws, 129, 160, mid);
-    }
-    if (kmax > 96) {
-        start(l2);
-        pivchol_rows_launch<4>(d_tiles, ntiles, ws, PH_H, 97, 128, l2, nullptr);
-        ++count;
-        count += jacobi_rows_launch<2, 8, 16, 512, 1, true>(d_tiles, ntiles, ws, 113, 128, l2);
-        count += jacobi_rows_launch<2, 8, 14, 448, 1, true>(d_tiles, ntiles, ws, 97, 112, l2);
-    }
-    if (kmax > 64) {
-        start(l1);
-        pivchol_rows_launch<3>(d_tiles, ntiles, ws, PH_H, 65, 96, l1, nullptr);
-        ++count;
-        count += jacobi_rows_launch<2, 8, 12, 384, 2, true>(d_tiles, ntiles, ws, 81, 96, l1);
-        count += jacobi_rows_launch<2, 8, 10, 320, 2, true>(d_tiles, ntiles, ws, 65, 80, l1);
-    }
-    pivchol_rows_launch<2>(d_tiles, ntiles, ws, PH_H, INT_MIN, 64, stream, nullptr);
-    ++count;
-    count += jacobi_rows_launch<1, 4, 16, 128, 4, true>(d_tiles, ntiles, ws, 49, 64, stream);
-    count += jacobi_rows_launch<1, 4, 12, 96, 5, true>(d_tiles, ntiles, ws, 33, 48, stream);
-    count += jacobi_rows_launch<0, 4, 8, 64, 8, true>(d_tiles, ntiles, ws, 1, 32, stream);
-    if (fork) {
-        const cudaStream_t used[4] = {l1, kmax > 96 ? l2 : nullptr,
-                                      kmax > kPivcholSplit ? big : nullptr,
-                                      kmax > kPivcholSplit ? mid : nullptr};
-        for (int q = 0; q < 4; ++q)
-            if (used[q]) {
-                cudaEventRecord(lanes.done[q], used[q]);
-                cudaStreamWaitEvent(stream, lanes.done[q], 0);
+    // the tiles of bin b: how many, and their list (null: the whole batch)
+    auto num = [&](int b) {
+        return svd_bin_lo(b) > kmax ? 0 : count ? count[b] : ntiles;
+    };
+    auto act = [&](int b) { return count ? list + (size_t)b * list_ld : nullptr; };
+    // Above 128 rows first: the longest chains.  Their Gram factors run in
+    // one launch per range, or one for the batch; the Jacobi SVDs of every
+    // range follow on streams of their own: the block classes (factor in
+    // global memory), and beside them the classes whose factor fits in
+    // shared memory.
+    for (int b = kSvdBinLarge; b < kSvdBins; ++b) {
+        const int n = num(b);
+        if (n == 0) continue;
+        const int rows = std::min(kmax, svd_bin_hi(b));
+        const cudaStream_t s = lane(count ? b - kSvdBinLarge : 0);
+        if (count || b == kSvdBinLarge)
+            launches += pivchol_large_launch(d_tiles, n, ws, s, act(b));
+        switch (b) {
+        case kSvdBinLarge:          // 129 .. 160
+        case kSvdBinLarge + 1: {    // 161 .. 192
+            const cudaStream_t m = count ? s : lane(SvdLanes::kStreams - 1);
+            if (fork && !count && b == kSvdBinLarge) {
+                cudaEventRecord(lanes.large, s);
+                cudaStreamWaitEvent(m, lanes.large, 0);
             }
+            if (b == kSvdBinLarge) {
+                jacobi_rows_launch<3, 16, 10, 512, 1, false>(d_tiles, n, ws, 129, 160, m, act(b));
+            } else {
+                jacobi_rows_launch<3, 16, 12, 512, 1, false>(d_tiles, n, ws, 161, 192, m, act(b));
+                jacobi_block_launch<4, 16, 12>(d_tiles, n, ws, rows, s, act(b));
+                ++launches;
+            }
+            break;
+        }
+        case kSvdBinLarge + 2:      // 193 .. 256
+            jacobi_block_launch<6, 16, 16>(d_tiles, n, ws, rows, s, act(b));
+            jacobi_rows_launch<5, 16, 16, 512, 1, false>(
+                d_tiles, n, ws, 193, 256, count ? s : lane(SvdLanes::kStreams - 1), act(b));
+            ++launches;
+            break;
+        case kSvdBinLarge + 3:      // 257 .. 288
+            jacobi_block_launch<7, 16, 18>(d_tiles, n, ws, rows, s, act(b));
+            break;
+        case kSvdBinLarge + 4:      // 289 .. 320
+            jacobi_block_launch<8, 16, 20>(d_tiles, n, ws, rows, s, act(b));
+            break;
+        case kSvdBinLarge + 5:      // 321 .. 512
+            jacobi_block_launch<9, 32, 16>(d_tiles, n, ws, rows, s, act(b));
+            break;
+        default:                    // above 512
+            jacobi_rows_launch<10, 32, 0, 1024, 1, false>(d_tiles, n, ws, 513, kMaxK, s, act(b));
+        }
+        ++launches;
     }
-    return count;
+    // 65 .. 128 rows: two ranges of the Gram factor, four of the Jacobi
+    constexpr int kLane2 = kSvdBins - kSvdBinLarge, kLane1 = kLane2 + 1;
+    if (num(kBin128)) {
+        const cudaStream_t s = lane(kLane2);
+        pivchol_rows_launch<4>(d_tiles, num(kBin128), ws, PH_H, 113, 128, s, act(kBin128));
+        jacobi_rows_launch<2, 8, 16, 512, 1, true>(d_tiles, num(kBin128), ws, 113, 128, s, act(kBin128));
+        launches += 2;
+    }
+    if (num(kBin112)) {
+        const cudaStream_t s = lane(kLane2 + 2);
+        pivchol_rows_launch<4>(d_tiles, num(kBin112), ws, PH_H, 97, 112, s, act(kBin112));
+        jacobi_rows_launch<2, 8, 14, 448, 1, true>(d_tiles, num(kBin112), ws, 97, 112, s, act(kBin112));
+        launches += 2;
+    }
+    if (num(kBin96)) {
+        const cudaStream_t s = lane(kLane1);
+        pivchol_rows_launch<3>(d_tiles, num(kBin96), ws, PH_H, 81, 96, s, act(kBin96));
+        jacobi_rows_launch<2, 8, 12, 384, 2, true>(d_tiles, num(kBin96), ws, 81, 96, s, act(kBin96));
+        launches += 2;
+    }
+    if (num(kBin80)) {
+        const cudaStream_t s = lane(kLane1 + 2);
+        pivchol_rows_launch<3>(d_tiles, num(kBin80), ws, PH_H, 65, 80, s, act(kBin80));
+        jacobi_rows_launch<2, 8, 10, 320, 2, true>(d_tiles, num(kBin80), ws, 65, 80, s, act(kBin80));
+        launches += 2;
+    }
+    if (num(kBin64)) {
+        pivchol_rows_launch<2>(d_tiles, num(kBin64), ws, PH_H, 49, 64, stream, act(kBin64));
+        jacobi_rows_launch<1, 4, 16, 128, 4, true>(d_tiles, num(kBin64), ws, 49, 64, stream, act(kBin64));
+        launches += 2;
+    }
+    if (num(kBin48)) {
+        pivchol_rows_launch<2>(d_tiles, num(kBin48), ws, PH_H, 33, 48, stream, act(kBin48));
+        jacobi_rows_launch<1, 4, 12, 96, 5, true>(d_tiles, num(kBin48), ws, 33, 48, stream, act(kBin48));
+        launches += 2;
+    }
+    if (num(kBin32)) {
+        pivchol_rows_launch<1>(d_tiles, num(kBin32), ws, PH_H, INT_MIN, 32, stream, act(kBin32));
+        jacobi_rows_launch<0, 4, 8, 64, 8, true>(d_tiles, num(kBin32), ws, 1, 32, stream, act(kBin32));
+        launches += 2;
+    }
+    for (int q = 0; q < SvdLanes::kStreams; ++q)
+        if (used[q]) {
+            cudaEventRecord(lanes.done[q], lanes.s[q]);
+            cudaStreamWaitEvent(stream, lanes.done[q], 0);
+        }
+    return launches;
 }
 
 // Appends the residual-pass columns to the basis: k1 += kb.
