@@ -49,6 +49,9 @@ struct Context {
     // engine behind the batch downloads of `copy`
     void *mapped = nullptr;
     void *mapped_dev = nullptr;
+    // the second lane of the library context's larger calls
+    bool may_help = false;
+    Context *helper = nullptr;
     std::mutex lock;           // one approximation / dmml at a time
 };
 

@@ -126,6 +126,7 @@ Context *context()
                                     &no);
         }
         cudaGetLastError();
+        g_ctx.may_help = true;
         g_ctx_ok = true;
     });
     if (!g_ctx_ok) return nullptr;
@@ -219,6 +220,24 @@ void context_free_private(Context *c)
 }
 
 void set_thread_context(Context *c) { t_ctx = c; }
+
+// The context of ctx's second lane, made at its first use; null if its
+// streams cannot be created.
+static Context *context_helper(Context &ctx)
+{
+    if (ctx.helper != nullptr) return ctx.helper;
+    Context *c = new Context();
+    c->device = ctx.device;
+    if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking) != cudaSuccess ||
+        !create_lanes(c->lanes)) {
+        cudaGetLastError();
+        delete c;
+        return nullptr;
+    }
+    ctx.helper = c;
+    return c;
+}
 
 void *pool_alloc(size_t bytes, cudaStream_t s)
 {
@@ -615,6 +634,31 @@ __global__ void k_counts_to_host(const int *__restrict__ src, int *dst)
     if (threadIdx.x < 1 + kSvdBins) dst[threadIdx.x] = src[threadIdx.x];
 }
 
+// Adds what one lane of a call measured and counted.
+static void add_stats(starsh_b200_stats &a, const starsh_b200_stats &b)
+{
+    a.sketch_ms += b.sketch_ms;
+    a.project_ms += b.project_ms;
+    a.sketch_flops += b.sketch_flops;
+    a.project_flops += b.project_flops;
+    a.tiles += b.tiles;
+    a.batches += b.batches;
+    a.sketch_launches += b.sketch_launches;
+    a.gen_ms += b.gen_ms;
+    a.basis_ms += b.basis_ms;
+    a.svd_ms += b.svd_ms;
+    a.output_ms += b.output_ms;
+    a.sketch_bytes += b.sketch_bytes;
+    a.fused_ms += b.fused_ms;
+    a.fused_launches += b.fused_launches;
+    a.fused_bytes += b.fused_bytes;
+    a.resketch_tiles += b.resketch_tiles;
+    a.mirror_wait_ms += b.mirror_wait_ms;
+}
+
+// Calls with fewer matrix entries run on one lane.
+constexpr long long kLaneEntries = 200000000;
+
 // Runs the device pipeline over the far blocks of every problem of `jobs`
 // in shared batches: tiles of different problems (kernels, sizes, tol,
 // maxrank) share every launch.  Fills each job's ranks and the per-block
@@ -624,20 +668,7 @@ __global__ void k_counts_to_host(const int *__restrict__ src, int *dst)
 static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
                           const EngineParams &ep)
 {
-    // every return waits for the batch downloads still in flight (their
-    // device sources are freed with the records on failure)
-    struct CopyDrain {
-        cudaStream_t c;
-        ~CopyDrain()
-        {
-            const auto t0 = std::chrono::steady_clock::now();
-            cudaStreamSynchronize(c);
-            thread_stats().mirror_wait_ms += std::chrono::duration<double, std::milli>(
-                std::chrono::steady_clock::now() - t0).count();
-        }
-    } drain{ctx.copy};
     cudaStream_t s = ctx.stream;
-    if (const int e = mapped_area(ctx)) return e;
     starsh_b200_stats &st = thread_stats();
     std::vector<TileWork> all;
     std::vector<std::pair<int, STARSH_int>> owner;   // (job, far block)
@@ -784,6 +815,30 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     if (const char *e = getenv("STARSH_B200_WORKSPACE_MB"))
         budget = std::min<size_t>(budget, (size_t)atoll(e) << 20);
     budget = std::min(budget, ctx.workspace_cap);
+    // Two lanes: the batches are dealt, as they come free, to two host
+    // threads with their own streams and workspaces, so that the chains of
+    // small launches of one batch's rounds and small SVDs run beside the
+    // other's full-width kernels, and neither waits for the host's reads.
+    // A call that would be one batch is cut in three (the first part, the
+    // near-diagonal tiles, has the longest rounds and SVDs).  Calls below
+    // kLaneEntries matrix entries are bound by the chain of one batch, which
+    // more parts do not shorten (7e7 entries: 4.74 against 4.54 ms, 1.2e8:
+    // 14.2 against 13.9 .. 15.3), and stay on one lane; above it 3e8 entries
+    // go from 10.9 to 10.8 ms, with host mirrors 8.8 to 7.8 (the first parts
+    // download early), 24 mixed problems 68.7 to 58.7, N = 65536 1/r 108.1
+    // to 102.1, N = 102400 square exponential 116.8 to 112.5.  A serving
+    // worker's context has the other workers beside it.
+    // STARSH_B200_LANES (1 or 2) sets the number.
+    int lanes = ctx.may_help && st.entries >= kLaneEntries && ntot >= 64 ? 2 : 1;
+    long long part = ntot;
+    if (const char *e = getenv("STARSH_B200_LANES"))
+        lanes = ctx.may_help ? std::max(1, std::min(2, atoi(e))) : 1;
+    Context *helper = lanes > 1 ? context_helper(ctx) : nullptr;
+    if (helper == nullptr) lanes = 1;
+    if (lanes > 1) {
+        budget /= 2;
+        part = (ntot + 2) / 3;
+    }
     // Batch plan: each batch takes as many tiles as fit the budget with
     // the layout of its largest dimensions (at most 4096).
     struct BatchPlan { long long b0; int nt; int m, n, k; size_t stride; };
@@ -801,7 +856,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         int bm = all[b0].m, bn = all[b0].n, bk = all[b0].k;
         size_t stride = workspace_layout(probe, bm, bn, bk, true, proj_i8);
         long long cap = (long long)(budget / (stride * sizeof(double)));
-        cap = std::max<long long>(1, std::min<long long>({cap, ntot - b0, kMaxBatchTiles}));
+        cap = std::max<long long>(1, std::min<long long>({cap, ntot - b0, kMaxBatchTiles, part}));
         for (long long q = b0; q < b0 + cap; ++q) {
             bm = std::max(bm, all[q].m);
             bn = std::max(bn, all[q].n);
@@ -817,6 +872,34 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         max_slots = std::max<long long>(max_slots, nt);
         b0 += nt;
     }
+    // what the lanes' streams read was uploaded on this one
+    cudaEvent_t ready = nullptr;
+    if (lanes > 1) {
+        B200_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming), "lane event");
+        cudaEventRecord(ready, s);
+    }
+    std::atomic<size_t> next_batch{0};
+    std::atomic<bool> failed{false};
+    std::mutex rec_lock;      // the records' lists of parts
+    auto run_lane = [&](Context &ctx, starsh_b200_stats &st) -> int {
+    // every return waits for what the lane still has in flight: the batch
+    // downloads, and on failure kernels (what they touch is freed with the
+    // records)
+    struct Drain {
+        cudaStream_t s, c;
+        starsh_b200_stats &st;
+        ~Drain()
+        {
+            cudaStreamSynchronize(s);
+            const auto t0 = std::chrono::steady_clock::now();
+            cudaStreamSynchronize(c);
+            st.mirror_wait_ms += std::chrono::duration<double, std::milli>(
+                std::chrono::steady_clock::now() - t0).count();
+        }
+    } drain{ctx.stream, ctx.copy, st};
+    cudaStream_t s = ctx.stream;
+    if (const int e = mapped_area(ctx)) return e;
+    if (ready) cudaStreamWaitEvent(s, ready, 0);
     if (!ctx.workspace.reserve(ws_need, s))
         return cuda_fail(cudaErrorMemoryAllocation, "workspace");
     if (!ctx.tiles.reserve((size_t)max_slots * sizeof(TileWork), s) ||
@@ -888,7 +971,8 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
                    : cuda_fail(cudaGetLastError(), "gemm_f64_batched");
     };
 
-    for (size_t pi = 0; pi < plan.size() && info == STARSH_SUCCESS; ++pi) {
+    for (size_t pi; info == STARSH_SUCCESS && !failed &&
+                    (pi = next_batch++) < plan.size();) {
         const long long b0 = plan[pi].b0;
         const int nt = plan[pi].nt;
         const int m_max = plan[pi].m, k_max = plan[pi].k;
@@ -1197,14 +1281,18 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             rec->dV[owner[b0 + t].second] = base + w.off_v;
         }
         std::vector<size_t> part_of(jobs.size(), 0);
-        for (size_t p = 0; p < jobs.size(); ++p) {
-            if (nu[p] + nv[p] == 0) continue;
-            Record *rec = jobs[p].rec;
-            rec->shared.push_back(chunk);
-            part_of[p] = rec->parts.size();
-            rec->parts.push_back({base + u0[p], nu[p], base + v0[p], nv[p]});
-            rec->u_total += nu[p];
-            rec->v_total += nv[p];
+        {
+            std::lock_guard<std::mutex> g(rec_lock);
+            for (size_t p = 0; p < jobs.size(); ++p) {
+                if (nu[p] + nv[p] == 0) continue;
+                Record *rec = jobs[p].rec;
+                rec->shared.push_back(chunk);
+                part_of[p] = rec->parts.size();
+                rec->parts.push_back({base + u0[p], nu[p], base + v0[p], nv[p]});
+                rec->parts.back().batch = pi;
+                rec->u_total += nu[p];
+                rec->v_total += nv[p];
+            }
         }
         if (total > 0) {
             OutArena out{base, base};
@@ -1230,6 +1318,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
                                               (nu[p] + nv[p]) * sizeof(double),
                                               cudaMemcpyDeviceToHost, ctx.copy),
                               "mirror copy");
+                    std::lock_guard<std::mutex> g(rec_lock);
                     Record::Part &pt = jobs[p].rec->parts[part_of[p]];
                     pt.hU = h;
                     pt.hV = h + nu[p];
@@ -1256,6 +1345,42 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         if (output_pending) st.output_ms += phase_ms(7, 8);
     }
     for (auto &e : ev) cudaEventDestroy(e);
+    return info;
+    };
+
+    if (lanes == 1 || plan.size() == 1) {
+        const int info = run_lane(ctx, st);
+        if (ready) cudaEventDestroy(ready);
+        return info;
+    }
+    // the helper's lane; its error text and statistics join this thread's
+    int info2 = STARSH_SUCCESS;
+    std::string error2;
+    starsh_b200_stats st2;
+    memset(&st2, 0, sizeof(st2));
+    std::thread other([&] {
+        cudaSetDevice(helper->device);
+        info2 = run_lane(*helper, st2);
+        if (info2) {
+            failed = true;
+            error2 = t_error;
+        }
+    });
+    int info = run_lane(ctx, st);
+    if (info) failed = true;
+    other.join();
+    cudaEventDestroy(ready);
+    add_stats(st, st2);
+    if (info == STARSH_SUCCESS && info2) {
+        info = info2;
+        t_error = error2;
+    }
+    // the parts in the order of the batches, whichever lane was first
+    for (ProblemJob &jb : jobs)
+        std::stable_sort(jb.rec->parts.begin(), jb.rec->parts.end(),
+                         [](const Record::Part &a, const Record::Part &b) {
+                             return a.batch < b.batch;
+                         });
     return info;
 }
 

@@ -60,6 +60,7 @@ struct Record {
     struct Part {
         const double *U; size_t nu; const double *V; size_t nv;
         double *hU = nullptr, *hV = nullptr;
+        size_t batch = 0;              // batch of the call it came from
     };
     std::vector<Part> parts;
     size_t u_total = 0, v_total = 0, d_total = 0;
