@@ -1,6 +1,6 @@
 // Batched FP64 GEMM (see gemm_f64.cuh).
 //
-// CTA tile 64 x 64, 32 x 128 or 128 x 32, K step 16, 8 warps of 32 x 16
+// CTA tile 64 x 64 or 128 x 32, K step 16, 8 warps of 32 x 16
 // output each (4 x 2 fragments of the m8n8k4 DMMA).  Operand tiles are staged
 // in shared memory double-buffered, the next K tile is fetched into
 // registers while the current one is multiplied.  Global loads are
@@ -44,7 +44,7 @@ k_gemm_f64(const GemmDesc *__restrict__ descs, int tiles_n)
     if (m0 >= d.M || n0 >= d.N) return;
 
     // [2][BM * kGemmLds] then [2][BN * kGemmLds], dynamic (above 48 KB
-    // for the 32 x 128 and 128 x 32 shapes)
+    // for the 128 x 32 shape)
     extern __shared__ double gemm_smem[];
     double (*As)[BM * kGemmLds] = reinterpret_cast<double (*)[BM * kGemmLds]>(gemm_smem);
     double (*Bs)[BN * kGemmLds] =
@@ -200,24 +200,19 @@ k_gemm_f64(const GemmDesc *__restrict__ descs, int tiles_n)
     }
 }
 
-// A^T B with 64 x 64 or 32 x 128 CTA tiles and a three-stage cp.async
-// pipeline: the transposed products (Grams and projections onto the basis
-// in the rounds; the projection B = Q^T D and rotation C = W^T B of the
-// small SVD, 32 x 128) have outputs of a few tiles and K = the tile
-// height, so one CTA walks a long K; the register-staged kernel above keeps
-// one K step in flight and waits on memory latency every step.  Operand
-// tiles land in shared memory directly (16-byte cp.async, k contiguous in
-// both operands), two steps ahead of the multiply (60 or 75 KB of shared
-// memory).  Where a tile fills every warp's output region, the per-element
-// accumulation order is that of k_gemm_f64 (K steps of 16 in order, the
-// DMMA's k-order inside a step), so results are identical to it; in a
-// launch that asks for it (split_k), a 64 x 64 tile with at most 32 rows or
-// 48 columns of its own splits K over the spare warps (fixed slice order,
-// deterministic).
-#ifndef GEMM_TN_STAGES
-#define GEMM_TN_STAGES 3      // four measured slower on the projection
-#endif
-constexpr int kTnStages = GEMM_TN_STAGES;
+// A^T B with 64 x 64 CTA tiles and a three-stage cp.async pipeline: the
+// transposed products (Grams and projections onto the basis in the rounds)
+// have outputs of a few tiles and K = the tile height, so one CTA walks a
+// long K; the register-staged kernel above keeps one K step in flight and
+// waits on memory latency every step.  Operand tiles land in shared memory
+// directly (16-byte cp.async, k contiguous in both operands), two steps
+// ahead of the multiply (60 KB of shared memory).  Where a tile fills every
+// warp's output region, the per-element accumulation order is that of
+// k_gemm_f64 (K steps of 16 in order, the DMMA's k-order inside a step), so
+// results are identical to it; in a launch that asks for it (split_k), a
+// tile with at most 32 rows or 48 columns of its own splits K over the
+// spare warps (fixed slice order, deterministic).
+constexpr int kTnStages = 3;
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool pred)
 {
@@ -227,12 +222,10 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool pr
                  :: "r"(sa), "l"(gmem), "r"(n));
 }
 
-template <int BM, int BN>
 __global__ void __launch_bounds__(kGemmThreads)
 k_gemm_f64_tn_pipe(const GemmDesc *__restrict__ descs, int tiles_n, int split_k)
 {
-    constexpr int WARPS_M = BM / 32;
-    static_assert(WARPS_M * (BN / 16) == kGemmThreads / 32, "warp grid");
+    constexpr int BM = 64, BN = 64, WARPS_M = BM / 32;
     // 16-byte pieces of the two operand tiles (BM and BN rows of 16 k)
     constexpr int PA = BM * kGemmBK / 2, PIECES = (BM + BN) * kGemmBK / 2;
     const GemmDesc d = descs[blockIdx.y];
@@ -255,7 +248,7 @@ k_gemm_f64_tn_pipe(const GemmDesc *__restrict__ descs, int tiles_n, int split_k)
     // through shared memory.  Every scheduler keeps the same share of the
     // DMMA work.
     int rh = WARPS_M, rp = 8, nsl = 1;
-    if constexpr (BM == 64 && BN == 64) if (split_k) {
+    if (split_k) {
         rh = d.M - m0 > 32 ? 2 : 1;
         const int cq = min(4, (d.N - n0 + 15) / 16);
         const int nreg = rh * cq;
@@ -379,6 +372,116 @@ k_gemm_f64_tn_pipe(const GemmDesc *__restrict__ descs, int tiles_n, int split_k)
                 *c = v;
             }
         }
+    }
+}
+
+// A^T B for wide outputs whose rows are a basis of a tile (the projection
+// B = Q^T D, K = the tile height, and the rotation C = W^T B): a CTA takes
+// 128 columns and up to 64 rows, each warp 16 columns and all of the rows,
+// in 8 MF rows fitted to the tile's own basis (a loop compiled per MF).
+// The DMMA pipe bounds a tile of many rows and the read of D one of few:
+// with 32 x 128 CTA tiles the pipe multiplied the padding up to 32 rows and
+// a basis of 33 .. 64 rows read D twice.  Per element the K order is that of
+// k_gemm_f64 (bit-identical).  Three stages (90 KB), two CTAs per SM.
+constexpr int kWideN = 128, kWideM = 64;
+
+template <int MF>
+__device__ __forceinline__ void tn_wide(const GemmDesc &d, int m0, int n0,
+                                        double *smem)
+{
+    constexpr int STAGE = (kWideM + kWideN) * kGemmLds;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int g = lane >> 2, tig = lane & 3, wn = warp * 16;
+    const bool evenA = (d.lda & 1) == 0 && ((uintptr_t)d.A & 15) == 0;
+    const bool evenB = (d.ldb & 1) == 0 && ((uintptr_t)d.B & 15) == 0;
+    // 16-byte pieces: row t / 8 + 32 r, k pair t % 8
+    const int row = t >> 3, kk = (t & 7) * 2;
+    auto piece = [&](double *dst, const double *src, int ld, int gr, int lim, int gk,
+                     bool even) {
+        const double *p = src + (size_t)gr * ld + gk;
+        if (even && gr < lim && gk + 1 < d.K) {
+            cp_async16(dst, p, true);
+        } else {
+            dst[0] = gr < lim && gk < d.K ? p[0] : 0.0;
+            dst[1] = gr < lim && gk + 1 < d.K ? p[1] : 0.0;
+        }
+    };
+    auto issue = [&](int kt) {
+        double *A = smem + kt % kTnStages * STAGE, *B = A + kWideM * kGemmLds;
+        const int gk = kt * kGemmBK + kk;
+        #pragma unroll
+        for (int r = 0; r < (MF + 3) / 4; ++r)
+            if (r * 32 + row < MF * 8)
+                piece(A + (r * 32 + row) * kGemmLds + kk, d.A, d.lda, m0 + r * 32 + row,
+                      d.M, gk, evenA);
+        #pragma unroll
+        for (int r = 0; r < kWideN / 32; ++r)
+            piece(B + (r * 32 + row) * kGemmLds + kk, d.B, d.ldb, n0 + r * 32 + row,
+                  d.N, gk, evenB);
+        asm volatile("cp.async.commit_group;");
+    };
+    double acc[MF][2][2] = {};
+    const int ktiles = (d.K + kGemmBK - 1) / kGemmBK;
+    #pragma unroll
+    for (int p = 0; p < kTnStages - 1; ++p) {
+        if (p < ktiles) issue(p);
+        else asm volatile("cp.async.commit_group;");
+    }
+    for (int kt = 0; kt < ktiles; ++kt) {
+        asm volatile("cp.async.wait_group %0;" :: "n"(kTnStages - 2));
+        __syncthreads();
+        if (kt + kTnStages - 1 < ktiles) issue(kt + kTnStages - 1);
+        else asm volatile("cp.async.commit_group;");
+        const double *A = smem + kt % kTnStages * STAGE, *B = A + kWideM * kGemmLds;
+        #pragma unroll
+        for (int k4 = 0; k4 < kGemmBK; k4 += 4) {
+            double af[MF], bf[2];
+            #pragma unroll
+            for (int j = 0; j < 2; ++j) bf[j] = B[(wn + j * 8 + g) * kGemmLds + k4 + tig];
+            #pragma unroll
+            for (int i = 0; i < MF; ++i) af[i] = A[(i * 8 + g) * kGemmLds + k4 + tig];
+            #pragma unroll
+            for (int i = 0; i < MF; ++i)
+                #pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    dmma_8x8x4(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;");
+    #pragma unroll
+    for (int i = 0; i < MF; ++i) {
+        const int gm = m0 + i * 8 + g;
+        if (gm >= d.M) continue;
+        #pragma unroll
+        for (int j = 0; j < 2; ++j)
+            #pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int gn = n0 + wn + j * 8 + 2 * tig + h;
+                if (gn >= d.N) continue;
+                double *c = d.C + (size_t)gn * d.ldc + gm;
+                double v = d.alpha * acc[i][j][h];
+                if (d.beta != 0.0) v += d.beta * *c;
+                *c = v;
+            }
+    }
+}
+
+__global__ void __launch_bounds__(kGemmThreads, 2)
+k_gemm_f64_tn_wide(const GemmDesc *__restrict__ descs, int tiles_n)
+{
+    extern __shared__ double gemm_smem[];
+    const GemmDesc d = descs[blockIdx.y];
+    const int m0 = blockIdx.x / tiles_n * kWideM, n0 = blockIdx.x % tiles_n * kWideN;
+    if (m0 >= d.M || n0 >= d.N) return;
+    switch (min(kWideM, d.M - m0) + 7 >> 3) {
+    case 1: tn_wide<1>(d, m0, n0, gemm_smem); break;
+    case 2: tn_wide<2>(d, m0, n0, gemm_smem); break;
+    case 3: tn_wide<3>(d, m0, n0, gemm_smem); break;
+    case 4: tn_wide<4>(d, m0, n0, gemm_smem); break;
+    case 5: tn_wide<5>(d, m0, n0, gemm_smem); break;
+    case 6: tn_wide<6>(d, m0, n0, gemm_smem); break;
+    case 7: tn_wide<7>(d, m0, n0, gemm_smem); break;
+    default: tn_wide<8>(d, m0, n0, gemm_smem);
     }
 }
 
@@ -549,40 +652,38 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmDesc *d_desc,
 {
     if (batch <= 0 || max_m <= 0 || max_n <= 0) return cudaSuccess;
     split_k = split_k && ta != tb;
-    // CTA shape: 64 x 64, or 32 x 128 when the output is wide and (as for
-    // the projection B = Q^T D and the rotation C = W^T B) its rows are a
-    // basis much narrower than the batch maximum, or 128 x 32 for narrow
-    // outputs (sketch blocks of 32 columns); 64 x 64 always with split_k
-    int bm = 64, bn = 64;
-    if (split_k) { }
-    else if (ta && !tb && max_n >= 256) { bm = 32; bn = 128; }
-    else if (max_n <= 32 && max_m >= 128) { bm = 128; bn = 32; }
+    // CTA shape: 64 x 64 (always with split_k); for A^T B whose output is
+    // wide and (as for the projection B = Q^T D and the rotation C = W^T B)
+    // has a basis much narrower than the batch maximum as its rows, the
+    // fitted 64 x 128 kernel; 128 x 32 for narrow outputs (sketch blocks of
+    // 32 columns)
+    const bool wide = ta && !tb && !split_k && max_n >= 256;
+    const int bm = !wide && !split_k && max_n <= 32 && max_m >= 128 ? 128 : 64;
+    const int bn = wide ? kWideN : bm == 128 ? 32 : 64;
     const int tiles_m = (max_m + bm - 1) / bm;
     const int tiles_n = (max_n + bn - 1) / bn;
-    // transposed products (64 x 64 and 32 x 128 tiles): the pipelined kernel
-    const bool pipe = ta && !tb && (bm == 64 || bm == 32);
     for (int b0 = 0; b0 < batch; b0 += 65535) {
         const int nb = batch - b0 < 65535 ? batch - b0 : 65535;
         const GemmDesc *dd = d_desc + b0;
-        if (pipe) {
-            dim3 grid(tiles_m * tiles_n, nb);
-            constexpr size_t smem64 = (size_t)kTnStages * 128 * kGemmLds * sizeof(double);
-            constexpr size_t smem32 = (size_t)kTnStages * 160 * kGemmLds * sizeof(double);
+        dim3 grid(tiles_m * tiles_n, nb);
+        if (ta && !tb && bm == 64) {
+            constexpr size_t smem = (size_t)kTnStages * 128 * kGemmLds * sizeof(double);
+            constexpr size_t smem_wide =
+                (size_t)kTnStages * (kWideM + kWideN) * kGemmLds * sizeof(double);
             static std::once_flag attr;
             std::call_once(attr, [] {
-                cudaFuncSetAttribute(k_gemm_f64_tn_pipe<64, 64>,
+                cudaFuncSetAttribute(k_gemm_f64_tn_pipe,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem64);
-                cudaFuncSetAttribute(k_gemm_f64_tn_pipe<32, 128>,
+                                     (int)smem);
+                cudaFuncSetAttribute(k_gemm_f64_tn_wide,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem32);
+                                     (int)smem_wide);
             });
-            if (bm == 64)
-                k_gemm_f64_tn_pipe<64, 64><<<grid, kGemmThreads, smem64, stream>>>(dd, tiles_n, split_k ? 1 : 0);
+            if (wide)
+                k_gemm_f64_tn_wide<<<grid, kGemmThreads, smem_wide, stream>>>(dd, tiles_n);
             else
-                k_gemm_f64_tn_pipe<32, 128><<<grid, kGemmThreads, smem32, stream>>>(dd, tiles_n, 0);
+                k_gemm_f64_tn_pipe<<<grid, kGemmThreads, smem, stream>>>(dd, tiles_n, split_k ? 1 : 0);
         } else if (!ta && tb && bm == 64) {
-            dim3 grid(tiles_m * tiles_n, nb);
             constexpr size_t smem = (size_t)kTnStages * 2 * kGemmBK * kNtLds * sizeof(double);
             static std::once_flag attr_nt;
             std::call_once(attr_nt, [] {
@@ -591,8 +692,7 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmDesc *d_desc,
                                      (int)smem);
             });
             k_gemm_f64_nt_pipe<<<grid, kGemmThreads, smem, stream>>>(dd, tiles_n, split_k ? 1 : 0);
-        } else if (bm == 32) launch_shape<32, 128>(ta, tb, dd, nb, tiles_m, tiles_n, stream);
-        else if (bm == 128) launch_shape<128, 32>(ta, tb, dd, nb, tiles_m, tiles_n, stream);
+        } else if (bm == 128) launch_shape<128, 32>(ta, tb, dd, nb, tiles_m, tiles_n, stream);
         else launch_shape<64, 64>(ta, tb, dd, nb, tiles_m, tiles_n, stream);
     }
     return cudaGetLastError();
