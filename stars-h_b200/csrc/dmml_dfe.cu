@@ -73,7 +73,7 @@ struct Job1 {          // phase 1: up to 128 rows of T that share A_j
 };
 
 struct NearPiece {
-    int block;         // near block (its D pointer is given per call)
+    long long off;     // its D, doubles after the first near block's
     int trans;         // 1: the mirrored block of a symmetric format
     int K;             // columns of op(D)
     int ld;            // leading dimension of D
@@ -207,14 +207,22 @@ k_prod_t(const Job1 *__restrict__ jobs, const double *const *__restrict__ vcol,
     }
 }
 
+// *out = alpha v + beta *out (not read when beta is 0).
+__device__ __forceinline__ void update(double *out, double alpha, double v,
+                                       double beta)
+{
+    const double old = beta == 0.0 ? 0.0 : beta * *out;
+    *out = fma(alpha, v, old);
+}
+
 // Phase 2: rows m0 .. m0 + rows - 1 of one output block row.
 template <int FN>
 __global__ void __launch_bounds__(256, 2)
 k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
          const double *__restrict__ T, int nrhs,
-         const NearPiece *__restrict__ near, const double *const *__restrict__ nearD,
+         const NearPiece *__restrict__ near, const double *__restrict__ nearD,
          const double *__restrict__ A, int lda, double *__restrict__ B, int ldb,
-         double alpha)
+         double alpha, double beta)
 {
     constexpr int BN = 16 * FN;
     constexpr int STAGE = prod_stage_doubles<FN>();
@@ -271,7 +279,7 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
             }
         } else {
             const NearPiece np = near[piece];
-            const double *D = nearD[np.block];
+            const double *D = nearD + np.off;
             #pragma unroll
             for (int q = 0; q < 4; ++q)
                 #pragma unroll
@@ -323,7 +331,7 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
             #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int col = n0 + wn + 8 * j + 2 * tig + h;
-                if (col < nrhs) out[(size_t)col * ldb] += alpha * acc[i][j][h];
+                if (col < nrhs) update(out + (size_t)col * ldb, alpha, acc[i][j][h], beta);
             }
     }
 }
@@ -332,9 +340,9 @@ template <int FN>
 static void launch_products(const Job1 *j1, int n1, const double *const *vcol,
                             const RowT *rowt, const Job2 *j2, int n2,
                             const double *const *ucol, const NearPiece *near,
-                            const double *const *nearD, const double *A, int lda,
+                            const double *nearD, const double *A, int lda,
                             double *T, double *B, int ldb, int nrhs, double alpha,
-                            cudaStream_t s)
+                            double beta, cudaStream_t s)
 {
     constexpr size_t smem = (size_t)kPStages * prod_stage_doubles<FN>() * sizeof(double);
     static std::once_flag attr;
@@ -352,7 +360,263 @@ static void launch_products(const Job1 *j1, int n1, const double *const *vcol,
     }
     if (n2 > 0) {
         k_prod_b<FN><<<dim3((unsigned)n2, ny), 256, smem, s>>>(
-            j2, ucol, T, nrhs, near, nearD, A, lda, B, ldb, alpha);
+            j2, ucol, T, nrhs, near, nearD, A, lda, B, ldb, alpha, beta);
+        count_launch();
+    }
+}
+
+// ------------------------------------------------ a few right-hand sides
+//
+// With up to kGemvRhs columns the product is bound by the read of the
+// factors, and the tiles above spend their 16 columns on padding and their
+// steps on 256-thread barriers (N = 25600 symmetric, one column: 39 + 68
+// us, here 35 + 51; N = 10000 with many dense blocks 35 + 50, here 14 + 39;
+// five and more columns are faster there).  Here a thread owns one element of T, or one output row, per column
+// and sums it alone; its operands come through a ring of cp.async stages in
+// shared memory deep enough to cover the memory latency, private to a warp.
+// An FP64 mma.sync adds its four products to the accumulator one after
+// another (k = 0, 1, 2, 3, each rounded), so a chain of FMAs over the whole
+// K gives the same bits as the tiles above: an iterative solver takes the
+// same iterations whichever kernels its products run on.
+constexpr int kGemvRhs = 4;
+constexpr int kGvKT = 64;            // phase 1: K of a stage
+constexpr int kGvLd = kGvKT + 1;     // ... doubles per row of it
+constexpr int kGvRowsT = 64;         // ... rows of T of a CTA
+constexpr int kGvStagesT = 3;
+constexpr int kGvKB = 32;            // phase 2: K of a stage
+constexpr int kGvRowsB = 64;         // ... rows of a CTA
+constexpr int kGvStagesB = 4;
+constexpr int kGvAhead = 3;          // ... stages a column pointer is read ahead
+
+// doubles of a stage: operand tile, then the other operand's NR rows
+template <int NR>
+constexpr int gv_stage_t() { return kGvRowsT * kGvLd + NR * kGvKT; }
+template <int NR>
+constexpr int gv_stage_b() { return kGvRowsB * kGvKB + NR * kGvKB; }
+
+// Phase 1: a CTA takes 64 rows of T (factor columns); its four warps copy 64
+// consecutive k of every row per stage (512 contiguous bytes: 128 left the
+// HBM at 1.8 TB/s), two of them own the 64 chains, a row per lane.  The odd
+// row stride keeps the lanes' reads on different banks.
+template <int NR>
+__global__ void __launch_bounds__(128)
+k_gemv_t(const Job1 *__restrict__ jobs, const double *const *__restrict__ vcol,
+         const RowT *__restrict__ rowt, const double *__restrict__ A, int lda,
+         double *__restrict__ T, int nrhs)
+{
+    extern __shared__ double sm[];
+    __shared__ const double *rowp[kGvRowsT];
+    const Job1 jb = jobs[blockIdx.x];
+    const int r0 = blockIdx.y * kGvRowsT, rows = min(kGvRowsT, jb.rows - r0);
+    if (rows <= 0) return;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t < kGvRowsT) rowp[t] = t < rows ? vcol[jb.rho0 + r0 + t] : nullptr;
+    __syncthreads();
+    constexpr int STAGE = gv_stage_t<NR>();
+    const double *Aj = A + jb.in0;
+    const int steps = (jb.K + kGvKT - 1) / kGvKT;
+    auto issue = [&](int st) {
+        double *S = sm + st % kGvStagesT * STAGE, *X = S + kGvRowsT * kGvLd;
+        const int k = st * kGvKT + lane;
+        #pragma unroll 4
+        for (int q = warp; q < rows; q += 4) {
+            const double *p = rowp[q];
+            cp_async8(S + q * kGvLd + lane, k < jb.K ? p + k : A, k < jb.K);
+            cp_async8(S + q * kGvLd + 32 + lane, k + 32 < jb.K ? p + k + 32 : A,
+                      k + 32 < jb.K);
+        }
+        for (int c = warp; c < NR; c += 4) {
+            const double *p = Aj + (size_t)c * lda;
+            const bool ok = c < nrhs;
+            cp_async8(X + c * kGvKT + lane, ok && k < jb.K ? p + k : A, ok && k < jb.K);
+            cp_async8(X + c * kGvKT + 32 + lane, ok && k + 32 < jb.K ? p + k + 32 : A,
+                      ok && k + 32 < jb.K);
+        }
+    };
+    double acc[NR] = {};
+    #pragma unroll
+    for (int p = 0; p < kGvStagesT - 1; ++p) {
+        if (p < steps) issue(p);
+        cp_async_commit();
+    }
+    for (int st = 0; st < steps; ++st) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kGvStagesT - 2));
+        __syncthreads();               // landed for all; the refilled one is consumed
+        if (st + kGvStagesT - 1 < steps) issue(st + kGvStagesT - 1);
+        cp_async_commit();
+        if (t < kGvRowsT) {
+            const double *S = sm + st % kGvStagesT * STAGE, *X = S + kGvRowsT * kGvLd;
+            #pragma unroll
+            for (int h = 0; h < kGvKT; h += 16) {
+                double v[16];
+                #pragma unroll
+                for (int k = 0; k < 16; ++k) v[k] = S[t * kGvLd + h + k];
+                #pragma unroll
+                for (int c = 0; c < NR; ++c)
+                    #pragma unroll
+                    for (int k = 0; k < 16; ++k)
+                        acc[c] = fma(v[k], X[c * kGvKT + h + k], acc[c]);
+            }
+        }
+    }
+    if (t >= rows) return;
+    const RowT rt = rowt[jb.rho0 + r0 + t];
+    double *out = T + (size_t)nrhs * rt.base + rt.kappa;
+    #pragma unroll
+    for (int c = 0; c < NR; ++c)
+        if (c < nrhs) out[(size_t)c * rt.ld] = acc[c];
+}
+
+// One stage of phase 2, as its copying warps see it.
+struct GvStage {
+    const double *col;   // lane u: the column at K index u of the stage
+    const double *x;     // the other operand there, `ldx` between columns
+    int ldx, k, rs;      // K indices in use; doubles between rows of col
+};
+
+// Phase 2: 64 output rows (K over the row's left-factor columns, then its
+// near blocks).  Two warps own the chains, a row per lane, and do nothing
+// else; the other two keep the ring filled, their column pointers read
+// three stages ahead.
+template <int NR>
+__global__ void __launch_bounds__(128)
+k_gemv_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
+         const double *__restrict__ T, int nrhs,
+         const NearPiece *__restrict__ near, const double *__restrict__ nearD,
+         const double *__restrict__ A, int lda, double *__restrict__ B, int ldb,
+         double alpha, double beta)
+{
+    extern __shared__ __align__(16) double gvb_sm[];
+    const Job2 jb = jobs[blockIdx.x];
+    const int r0 = blockIdx.y * kGvRowsB, rows = min(kGvRowsB, jb.rows - r0);
+    if (rows <= 0) return;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    constexpr int STAGE = gv_stage_b<NR>();
+    int total = (jb.kfar + kGvKB - 1) / kGvKB;
+    for (int q = jb.near0; q < jb.near1; ++q) total += (near[q].K + kGvKB - 1) / kGvKB;
+    if (warp >= 2) {
+        const int row = (warp - 2) * 32 + lane;
+        const int m = jb.m0 + r0 + min(row, rows - 1);
+        const double *Tf = T + (size_t)nrhs * jb.kap0;
+        // next stage to describe: piece (-1: the factors, else a near piece)
+        // and k0
+        int piece = jb.kfar > 0 ? -1 : jb.near0, k0 = 0;
+        auto describe = [&]() {
+            GvStage g{nullptr, A, 0, 0, 0};
+            if (piece >= jb.near1) return g;
+            int K;
+            if (piece < 0) {
+                K = jb.kfar;
+                g.k = min(kGvKB, K - k0);
+                if (lane < g.k) g.col = ucol[jb.kap0 + k0 + lane];
+                g.x = Tf + k0;
+                g.ldx = jb.kfar;
+                g.rs = 1;
+            } else {
+                const NearPiece np = near[piece];
+                K = np.K;
+                g.k = min(kGvKB, K - k0);
+                g.col = nearD + np.off + (size_t)(k0 + min(lane, g.k - 1)) * (np.trans ? 1 : np.ld);
+                g.x = A + np.in0 + k0;
+                g.ldx = lda;
+                g.rs = np.trans ? np.ld : 1;
+            }
+            k0 += kGvKB;
+            if (k0 >= K) {
+                piece = piece < 0 ? jb.near0 : piece + 1;
+                k0 = 0;
+            }
+            return g;
+        };
+        auto issue = [&](const GvStage &g, int st) {
+            double *S = gvb_sm + st % kGvStagesB * STAGE, *X = S + kGvRowsB * kGvKB;
+            const size_t mo = (size_t)m * g.rs;
+            #pragma unroll
+            for (int u = 0; u < kGvKB; ++u) {
+                const double *p = (const double *)__shfl_sync(
+                    0xffffffffu, (unsigned long long)g.col, u);
+                cp_async8(S + u * kGvRowsB + row, u < g.k ? p + mo : A, u < g.k);
+            }
+            for (int c = warp - 2; c < NR; c += 2) {
+                const bool ok = lane < g.k && c < nrhs;
+                cp_async8(X + c * kGvKB + lane, ok ? g.x + lane + (size_t)c * g.ldx : A, ok);
+            }
+        };
+        GvStage g[kGvAhead];
+        #pragma unroll
+        for (int q = 0; q < kGvAhead; ++q) g[q] = describe();
+        static_assert(kGvStagesB - 1 == kGvAhead, "the prologue issues what it described");
+        #pragma unroll
+        for (int q = 0; q < kGvStagesB - 1; ++q) {
+            if (q < total) issue(g[q], q);
+            cp_async_commit();
+            g[q] = describe();
+        }
+        for (int st0 = 0; st0 < total; st0 += kGvAhead)
+            #pragma unroll
+            for (int q = 0; q < kGvAhead; ++q) {
+                const int st = st0 + q;
+                if (st >= total) break;
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(kGvStagesB - 2));
+                __syncthreads();
+                if (st + kGvStagesB - 1 < total) {
+                    issue(g[q], st + kGvStagesB - 1);
+                    g[q] = describe();
+                }
+                cp_async_commit();
+            }
+        asm volatile("cp.async.wait_group 0;\n" ::);
+        return;
+    }
+    double acc[NR] = {};
+    for (int st = 0; st < total; ++st) {
+        __syncthreads();               // landed, and the refilled one consumed
+        const double *S = gvb_sm + st % kGvStagesB * STAGE + t;
+        const double2 *X = reinterpret_cast<const double2 *>(
+            gvb_sm + st % kGvStagesB * STAGE + kGvRowsB * kGvKB);
+        double v[kGvKB];
+        #pragma unroll
+        for (int k = 0; k < kGvKB; ++k) v[k] = S[k * kGvRowsB];
+        #pragma unroll
+        for (int c = 0; c < NR; ++c)
+            #pragma unroll
+            for (int k = 0; k < kGvKB; k += 2) {
+                const double2 x = X[(c * kGvKB + k) / 2];
+                acc[c] = fma(v[k], x.x, acc[c]);
+                acc[c] = fma(v[k + 1], x.y, acc[c]);
+            }
+    }
+    if (t >= rows) return;
+    #pragma unroll
+    for (int c = 0; c < NR; ++c)
+        if (c < nrhs) update(B + jb.out0 + r0 + t + (size_t)c * ldb, alpha, acc[c], beta);
+}
+
+template <int NR>
+static void launch_gemv(const Job1 *j1, int n1, const double *const *vcol,
+                        const RowT *rowt, const Job2 *j2, int n2,
+                        const double *const *ucol, const NearPiece *near,
+                        const double *nearD, const double *A, int lda, double *T,
+                        double *B, int ldb, int nrhs, double alpha, double beta,
+                        cudaStream_t s)
+{
+    constexpr size_t smem_t = (size_t)kGvStagesT * gv_stage_t<NR>() * sizeof(double);
+    constexpr size_t smem_b = (size_t)kGvStagesB * gv_stage_b<NR>() * sizeof(double);
+    static std::once_flag attr;
+    std::call_once(attr, [] {
+        cudaFuncSetAttribute(k_gemv_t<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem_t);
+        cudaFuncSetAttribute(k_gemv_b<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem_b);
+    });
+    if (n1 > 0) {
+        k_gemv_t<NR><<<dim3((unsigned)n1, kPBM / kGvRowsT), 128, smem_t, s>>>(
+            j1, vcol, rowt, A, lda, T, nrhs);
+        count_launch();
+    }
+    if (n2 > 0) {
+        k_gemv_b<NR><<<dim3((unsigned)n2, kPBM / kGvRowsB), 128, smem_b, s>>>(
+            j2, ucol, T, nrhs, near, nearD, A, lda, B, ldb, alpha, beta);
         count_launch();
     }
 }
@@ -452,6 +716,8 @@ struct ProductPlan {
     Job2 *j2 = nullptr;
     NearPiece *near = nullptr;
     int n1 = 0, n2 = 0, nnear = 0;
+    bool covers = false;       // phase 2 writes every output row
+    size_t near_total = 0;     // doubles of the near blocks
     long long trows = 0;       // rows of T over all block rows
     cudaEvent_t ready = nullptr;   // the upload has completed
     ~ProductPlan()
@@ -530,18 +796,28 @@ static int build_plan(STARSH_blrm *M, const Record &rec, cudaStream_t s,
             j1.push_back(Job1{rho0 + r0, std::min(kPBM, cnt - r0), q0.n, q0.in0});
     }
     // near pieces per output row, in near-block order
+    // (stored blocks by their place after the first one, regenerated ones
+    // in list order)
     std::vector<std::vector<NearPiece>> rownear(nbr);
+    size_t near_total = 0;
     for (STARSH_int b = 0; b < F->nblocks_near; ++b) {
         const STARSH_int i = F->block_near[2 * b], j = F->block_near[2 * b + 1];
         const int m = (int)R->size[i], n = (int)C->size[j];
-        rownear[i].push_back(NearPiece{(int)b, 0, n, m, (long long)C->start[j]});
+        const long long off = M->onfly ? (long long)near_total
+                                       : (long long)(rec.dD[b] - rec.dD[0]);
+        near_total += (size_t)m * n;
+        rownear[i].push_back(NearPiece{off, 0, n, m, (long long)C->start[j]});
         if (symm && i != j)
-            rownear[j].push_back(NearPiece{(int)b, 1, m, m, (long long)R->start[i]});
+            rownear[j].push_back(NearPiece{off, 1, m, m, (long long)R->start[i]});
     }
+    bool covers = true;
     std::vector<NearPiece> near;
     std::vector<Job2> j2;
     for (STARSH_int i = 0; i < nbr; ++i) {
-        if (S[i] == 0 && rownear[i].empty()) continue;
+        if (S[i] == 0 && rownear[i].empty()) {
+            covers = false;
+            continue;
+        }
         const int near0 = (int)near.size();
         near.insert(near.end(), rownear[i].begin(), rownear[i].end());
         const int mi = (int)R->size[i];
@@ -586,6 +862,8 @@ static int build_plan(STARSH_blrm *M, const Record &rec, cudaStream_t s,
     plan->n2 = (int)j2.size();
     plan->nnear = (int)near.size();
     plan->trows = trows;
+    plan->covers = covers;
+    plan->near_total = near_total;
     *out = plan;
     return STARSH_SUCCESS;
 }
@@ -608,9 +886,13 @@ int dmml_device(STARSH_blrm *M, int nrhs, double alpha,
     if (info) return info;
     cudaStream_t s = ctx.stream;
     // Order the user's stream before ours and ours before the user's.
-    cudaEvent_t ev;
-    cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    struct Order {
+        cudaEvent_t ev = nullptr;
+        ~Order() { if (ev) cudaEventDestroy(ev); }
+    } order;
+    cudaEvent_t &ev = order.ev;
     if (user_stream != s) {
+        B200_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "dmml event");
         cudaEventRecord(ev, user_stream);
         cudaStreamWaitEvent(s, ev, 0);
     }
@@ -619,10 +901,7 @@ int dmml_device(STARSH_blrm *M, int nrhs, double alpha,
         std::lock_guard<std::mutex> g(rec->plan_lock);
         if (!rec->plan) {
             ProductPlan *built = nullptr;
-            if ((info = build_plan(M, *rec, s, &built))) {
-                cudaEventDestroy(ev);
-                return info;
-            }
+            if ((info = build_plan(M, *rec, s, &built))) return info;
             rec->plan = std::shared_ptr<void>(built, [](void *q) {
                 delete (ProductPlan *)q;
             });
@@ -630,24 +909,21 @@ int dmml_device(STARSH_blrm *M, int nrhs, double alpha,
         plan = (ProductPlan *)rec->plan.get();
     }
     if (plan->ready) cudaStreamWaitEvent(s, plan->ready, 0);
-    {
+    // beta: with the product's last step, or first where it skips rows
+    if (!plan->covers) {
         const long long tot = (long long)nrows * nrhs;
         k_scale_cols<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(
             dB, ldb, (int)nrows, nrhs, beta);
         count_launch();
+        beta = 1.0;
     }
     // near blocks: dense D (stored, or regenerated when onfly)
     double *onfly_buf = nullptr;
-    std::vector<const double *> nearD(F->nblocks_near, nullptr);
+    const double *nearD = nullptr;
     if (F->nblocks_near > 0) {
         if (M->onfly) {
-            size_t tot = 0;
-            for (STARSH_int b = 0; b < F->nblocks_near; ++b)
-                tot += (size_t)R->size[F->block_near[2 * b]] *
-                       C->size[F->block_near[2 * b + 1]];
-            onfly_buf = (double *)pool_alloc(tot * sizeof(double), s);
+            onfly_buf = (double *)pool_alloc(plan->near_total * sizeof(double), s);
             if (onfly_buf == nullptr) {
-                cudaEventDestroy(ev);
                 return cuda_fail(cudaErrorMemoryAllocation, "onfly blocks");
             }
             std::vector<BlockJob> jobs;
@@ -656,47 +932,44 @@ int dmml_device(STARSH_blrm *M, int nrhs, double alpha,
                 const STARSH_int i = F->block_near[2 * b], j = F->block_near[2 * b + 1];
                 BlockJob jb{R->start[i], C->start[j], (int)R->size[i],
                             (int)C->size[j], onfly_buf + off};
-                nearD[b] = onfly_buf + off;
                 off += (size_t)jb.m * jb.n;
                 jobs.push_back(jb);
             }
             if ((info = gen_blocks(rec->points->K, jobs, s))) {
                 pool_free(onfly_buf);
-                cudaEventDestroy(ev);
                 return info;
             }
+            nearD = onfly_buf;
         } else {
-            for (STARSH_int b = 0; b < F->nblocks_near; ++b) nearD[b] = rec->dD[b];
+            nearD = rec->dD[0];
         }
     }
-    // per call: T (rows of every block row x nrhs) and the near pointers
+    // per call: T (rows of every block row x nrhs)
     const size_t tbytes = (size_t)plan->trows * nrhs * sizeof(double);
-    const size_t nbytes = nearD.size() * sizeof(double *);
     char *scratch = nullptr;
-    if (tbytes + nbytes > 0) {
-        scratch = (char *)pool_alloc((tbytes + 255) / 256 * 256 + nbytes, s);
+    if (tbytes > 0) {
+        scratch = (char *)pool_alloc(tbytes, s);
         if (scratch == nullptr) {
             if (onfly_buf) pool_free(onfly_buf);
-            cudaEventDestroy(ev);
             return cuda_fail(cudaErrorMemoryAllocation, "product scratch");
         }
     }
     double *T = (double *)scratch;
-    const double **dnear = (const double **)(scratch + (tbytes + 255) / 256 * 256);
-    if (nbytes)
-        cudaMemcpyAsync(dnear, nearD.data(), nbytes, cudaMemcpyHostToDevice, s);
-    if (nrhs > 32)
-        launch_products<4>(plan->j1, plan->n1, plan->vcol, plan->rowt, plan->j2,
-                           plan->n2, plan->ucol, plan->near, dnear, dA, lda, T, dB,
-                           ldb, nrhs, alpha, s);
-    else if (nrhs > 16)
-        launch_products<2>(plan->j1, plan->n1, plan->vcol, plan->rowt, plan->j2,
-                           plan->n2, plan->ucol, plan->near, dnear, dA, lda, T, dB,
-                           ldb, nrhs, alpha, s);
-    else
-        launch_products<1>(plan->j1, plan->n1, plan->vcol, plan->rowt, plan->j2,
-                           plan->n2, plan->ucol, plan->near, dnear, dA, lda, T, dB,
-                           ldb, nrhs, alpha, s);
+    auto tiles = [&](auto fn) {
+        fn(plan->j1, plan->n1, plan->vcol, plan->rowt, plan->j2, plan->n2, plan->ucol,
+           plan->near, nearD, dA, lda, T, dB, ldb, nrhs, alpha, beta, s);
+    };
+    if (nrhs <= kGemvRhs) {
+        if (nrhs == 1) tiles(launch_gemv<1>);
+        else if (nrhs == 2) tiles(launch_gemv<2>);
+        else tiles(launch_gemv<kGemvRhs>);
+    } else if (nrhs > 32) {
+        tiles(launch_products<4>);
+    } else if (nrhs > 16) {
+        tiles(launch_products<2>);
+    } else {
+        tiles(launch_products<1>);
+    }
     if (scratch) pool_free(scratch);
     if (onfly_buf) pool_free(onfly_buf);
     cudaError_t e = cudaGetLastError();
@@ -704,7 +977,6 @@ int dmml_device(STARSH_blrm *M, int nrhs, double alpha,
         cudaEventRecord(ev, s);
         cudaStreamWaitEvent(user_stream, ev, 0);
     }
-    cudaEventDestroy(ev);
     if (e != cudaSuccess) return cuda_fail(e, "dmml kernels");
     return STARSH_SUCCESS;
 }
@@ -717,65 +989,164 @@ struct DfeJob {
     const double *U, *V, *D;   // D: stored dense block or null
 };
 
-// Each CTA stores its 64 x 64 piece's ||D||^2 and ||D - U V^T||^2 in its own
-// slot of `part` (slot = (job, tile row, tile column)); k_dfe_sum adds a
-// job's slots in a fixed order, so the error is the same on every run.
-__global__ void __launch_bounds__(256)
-k_dfe(DevKernel K, const DfeJob *__restrict__ jobs, double *__restrict__ part)
+// Each CTA takes 64 rows and cb 64-column blocks (4, or 1 where that leaves
+// too few CTAs) of a job: U V^T on the
+// FP64 tensor path (8 warps of 32 x 16 outputs), and the block's entries
+// evaluated by the thread that holds the same output in its accumulators, so
+// nothing but the factors is read (or, for a stored dense block, its
+// entries).  Coordinates are staged once per CTA, the kernel family is
+// compiled in, and the factors' next K step of 16 is copied while the
+// entries of the current block are evaluated.  The entries' FP64 work is
+// what bounds it (the generator's bound without its store): N = 25600
+// square exponential, tol 1e-7, 3.4 ms, against 11.2 with scalar products
+// from shared memory and a family switch and two index loads per entry.
+// The CTA's ||D||^2 and ||D - U V^T||^2 go to its own slot of `part` (slot =
+// (job, tile row, column group)); k_dfe_sum adds a job's slots in a fixed
+// order, so the error is the same on every run.
+constexpr int kDfeCb = 4, kDfeLd = 68, kDfeDim = 4;
+constexpr size_t kDfeStage = 2 * (size_t)kPBK * kDfeLd;   // doubles
+
+// Entries (row i, columns c) of one block against the accumulators.
+template <int FAM, int NDIM>
+__device__ __forceinline__ void dfe_entries(
+    const DevKernel &K, const DfeJob &jb, const double (*rc)[64],
+    const double (*cc)[64 * kDfeCb], const long long *ri, const long long *ci,
+    int i0, int j0, int jb0, int wm, int wn, int g, int tig,
+    const double (&acc)[4][2][2], double &nrm, double &dif)
 {
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int lr = wm + 8 * i + g;
+        double xr[NDIM > 0 ? NDIM : 1];
+        if constexpr (NDIM > 0) {
+            #pragma unroll
+            for (int d = 0; d < NDIM; ++d) xr[d] = rc[d][lr];
+        }
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int lc = jb0 + wn + 8 * (q >> 1) + 2 * tig + (q & 1);
+            double v;
+            if (jb.D != nullptr) {
+                v = i0 + lr < jb.m && j0 + lc < jb.n
+                        ? jb.D[(size_t)(j0 + lc) * jb.m + i0 + lr] : 0.0;
+            } else {
+                double dist = 0.0;
+                if constexpr (NDIM > 0) {
+                    #pragma unroll
+                    for (int d = 0; d < NDIM; ++d) {
+                        const double t = __dsub_rn(xr[d], cc[d][lc]);
+                        dist = __dadd_rn(dist, __dmul_rn(t, t));
+                    }
+                } else if constexpr (NDIM == 0) {
+                    for (int d = 0; d < K.ndim; ++d) {
+                        const double t = __dsub_rn(rc[d][lr], cc[d][lc]);
+                        dist = __dadd_rn(dist, __dmul_rn(t, t));
+                    }
+                } else {
+                    dist = sq_dist(K, ri[lr], ci[lc]);
+                }
+                v = entry_fam<FAM>(K, dist, ri[lr], ci[lc]);
+            }
+            if (i0 + lr < jb.m && j0 + lc < jb.n) {
+                const double e = v - acc[i][q >> 1][q & 1];
+                nrm += v * v;
+                dif += e * e;
+            }
+        }
+    }
+}
+
+template <int FAM>
+__global__ void __launch_bounds__(256, 3)
+k_dfe(DevKernel K, const DfeJob *__restrict__ jobs, double *__restrict__ part,
+      int cb)
+{
+    extern __shared__ double dfe_sm[];         // [2][U 16 x 68, V 16 x 68]
+    __shared__ double rc[kDfeDim][64], cc[kDfeDim][64 * kDfeCb];
+    __shared__ long long ri[64], ci[64 * kDfeCb];
+    __shared__ double red[2][8];
     const DfeJob jb = jobs[blockIdx.z];
-    const int i0 = blockIdx.x * 64, j0 = blockIdx.y * 64;
+    const int i0 = blockIdx.x * 64, j0 = blockIdx.y * 64 * cb;
     double *slot = part + 2 * (((size_t)blockIdx.z * gridDim.y + blockIdx.y) *
                                gridDim.x + blockIdx.x);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     if (i0 >= jb.m || j0 >= jb.n) {
-        if (threadIdx.x == 0) slot[0] = slot[1] = 0.0;
+        if (t == 0) slot[0] = slot[1] = 0.0;
         return;
     }
-    __shared__ double Us[64][33];
-    __shared__ double Vs[64][33];
-    __shared__ double red[2][8];
-    const int t = threadIdx.x;
-    const int ii = t & 63, jj = t >> 6;
-    double acc[16] = {};
-    for (int p0 = 0; p0 < jb.r; p0 += 32) {
-        for (int q = t; q < 64 * 32; q += 256) {
-            const int row = q & 63, p = q >> 6;
-            const bool okp = p0 + p < jb.r;
-            Us[row][p] = (okp && i0 + row < jb.m)
-                             ? jb.U[(size_t)(p0 + p) * jb.m + i0 + row] : 0.0;
-            Vs[row][p] = (okp && j0 + row < jb.n)
-                             ? jb.V[(size_t)(p0 + p) * jb.n + j0 + row] : 0.0;
+    const int g = lane >> 2, tig = lane & 3;
+    const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16;
+    const bool staged = !K.aos && K.ndim <= kDfeDim;
+    if (t < 64) ri[t] = K.row_piv[jb.row0 + min(i0 + t, jb.m - 1)];
+    ci[t] = K.col_piv[jb.col0 + min(j0 + t, jb.n - 1)];
+    static_assert(64 * kDfeCb == 256, "a column index per thread");
+    __syncthreads();
+    if (staged)
+        for (int d = 0; d < K.ndim; ++d) {
+            if (t < 64) rc[d][t] = K.row_pt[d * K.row_count + ri[t]];
+            cc[d][t] = K.col_pt[d * K.col_count + ci[t]];
         }
-        __syncthreads();
-        #pragma unroll 4
-        for (int p = 0; p < 32; ++p) {
-            const double u = Us[ii][p];
-            #pragma unroll
-            for (int c = 0; c < 16; ++c) acc[c] += u * Vs[jj + 4 * c][p];
+    const int nblk = min(cb, (jb.n - j0 + 63) / 64);
+    const int ksteps = (jb.r + kPBK - 1) / kPBK;
+    const int steps = nblk * ksteps;           // (block, K step), block-major
+    auto issue = [&](int st) {
+        double *Us = dfe_sm + (st & 1) * kDfeStage, *Vs = Us + kPBK * kDfeLd;
+        const int b = st / ksteps, k0 = (st - b * ksteps) * kPBK;
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int row = t & 63, k = (t >> 6) + 4 * q, p = k0 + k;
+            const int i = i0 + row, j = j0 + b * 64 + row;
+            const bool okU = p < jb.r && i < jb.m, okV = p < jb.r && j < jb.n;
+            cp_async8(Us + k * kDfeLd + row, okU ? jb.U + (size_t)p * jb.m + i : jb.U, okU);
+            cp_async8(Vs + k * kDfeLd + row, okV ? jb.V + (size_t)p * jb.n + j : jb.V, okV);
         }
-        __syncthreads();
-    }
+    };
+    if (steps > 0) issue(0);
+    cp_async_commit();
     double nrm = 0.0, dif = 0.0;
-    const int i = i0 + ii;
-    if (i < jb.m) {
-        for (int c = 0; c < 16; ++c) {
-            const int j = j0 + jj + 4 * c;
-            if (j >= jb.n) continue;
-            const double d = jb.D ? jb.D[(size_t)j * jb.m + i]
-                                  : block_entry(K, jb.row0, jb.col0, i, j);
-            const double e = d - acc[c];
-            nrm += d * d;
-            dif += e * e;
+    int st = 0;
+    #pragma unroll 1
+    for (int b = 0; b < nblk; ++b) {
+        double acc[4][2][2] = {};
+        #pragma unroll 1
+        for (int k = 0; k < ksteps; ++k, ++st) {
+            asm volatile("cp.async.wait_group 0;\n" ::);
+            __syncthreads();                   // step st landed, st - 1 consumed
+            if (st + 1 < steps) issue(st + 1);
+            cp_async_commit();
+            const double *Us = dfe_sm + (st & 1) * kDfeStage, *Vs = Us + kPBK * kDfeLd;
+            #pragma unroll
+            for (int kk = 0; kk < kPBK; kk += 4) {
+                double af[4], bf[2];
+                #pragma unroll
+                for (int i = 0; i < 4; ++i) af[i] = Us[(kk + tig) * kDfeLd + wm + 8 * i + g];
+                #pragma unroll
+                for (int j = 0; j < 2; ++j) bf[j] = Vs[(kk + tig) * kDfeLd + wn + 8 * j + g];
+                #pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    #pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        dmma_884(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+            }
         }
+        if (b == 0) __syncthreads();           // coordinates
+        if (!staged)
+            dfe_entries<FAM, -1>(K, jb, rc, cc, ri, ci, i0, j0, b * 64, wm, wn, g, tig, acc, nrm, dif);
+        else if (K.ndim == 2)
+            dfe_entries<FAM, 2>(K, jb, rc, cc, ri, ci, i0, j0, b * 64, wm, wn, g, tig, acc, nrm, dif);
+        else if (K.ndim == 3)
+            dfe_entries<FAM, 3>(K, jb, rc, cc, ri, ci, i0, j0, b * 64, wm, wn, g, tig, acc, nrm, dif);
+        else
+            dfe_entries<FAM, 0>(K, jb, rc, cc, ri, ci, i0, j0, b * 64, wm, wn, g, tig, acc, nrm, dif);
     }
     #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         nrm += __shfl_down_sync(0xffffffffu, nrm, o);
         dif += __shfl_down_sync(0xffffffffu, dif, o);
     }
-    if ((t & 31) == 0) {
-        red[0][t >> 5] = nrm;
-        red[1][t >> 5] = dif;
+    if (lane == 0) {
+        red[0][warp] = nrm;
+        red[1][warp] = dif;
     }
     __syncthreads();
     if (t == 0) {
@@ -789,20 +1160,46 @@ k_dfe(DevKernel K, const DfeJob *__restrict__ jobs, double *__restrict__ part)
     }
 }
 
-// out[2 job + {0, 1}] = the sums of the job's nslot slots, in slot order.
+// out[2 job + {0, 1}] = the sums of the job's nslot slots: one warp per job,
+// lane l adds slots l, l + 32, ..., then a tree over the lanes.
 __global__ void k_dfe_sum(const double *__restrict__ part, int nslot,
                           long long njobs, double *__restrict__ out)
 {
-    const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long j = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (j >= njobs) return;
-    const double *p = part + 2 * (size_t)j * nslot;
+    const double2 *p = reinterpret_cast<const double2 *>(part) + (size_t)j * nslot;
     double a = 0.0, b = 0.0;
-    for (int q = 0; q < nslot; ++q) {
-        a += p[2 * q];
-        b += p[2 * q + 1];
+    for (int q = lane; q < nslot; q += 32) {
+        const double2 v = p[q];
+        a += v.x;
+        b += v.y;
     }
-    out[2 * j] = a;
-    out[2 * j + 1] = b;
+    #pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) {
+        out[2 * j] = a;
+        out[2 * j + 1] = b;
+    }
+}
+
+static void launch_dfe(const DevKernel &K, dim3 grid, const DfeJob *jobs,
+                       double *part, int cb, cudaStream_t s)
+{
+    constexpr size_t smem = 2 * kDfeStage * sizeof(double);
+    switch (K.family) {
+    case FAM_EXP: k_dfe<FAM_EXP><<<grid, 256, smem, s>>>(K, jobs, part, cb); break;
+    case FAM_SQREXP: k_dfe<FAM_SQREXP><<<grid, 256, smem, s>>>(K, jobs, part, cb); break;
+    case FAM_MATERN: k_dfe<FAM_MATERN><<<grid, 256, smem, s>>>(K, jobs, part, cb); break;
+    case FAM_MATERN2: k_dfe<FAM_MATERN2><<<grid, 256, smem, s>>>(K, jobs, part, cb); break;
+    case FAM_COULOMB: k_dfe<FAM_COULOMB><<<grid, 256, smem, s>>>(K, jobs, part, cb); break;
+    case FAM_SIN: k_dfe<FAM_SIN><<<grid, 256, smem, s>>>(K, jobs, part, cb); break;
+    case FAM_COS: k_dfe<FAM_COS><<<grid, 256, smem, s>>>(K, jobs, part, cb); break;
+    default: k_dfe<FAM_RBF><<<grid, 256, smem, s>>>(K, jobs, part, cb);
+    }
 }
 
 // The weighted sums sum ||D_b - U_b V_b^T||_F^2 (far blocks) and
@@ -837,7 +1234,9 @@ static int dfe_sums_device(STARSH_blrm *M, Context &ctx, double *diff2,
         mmax = std::max(mmax, j.m);
         nmax = std::max(nmax, j.n);
     }
-    const int gx = (mmax + 63) / 64, gy = (nmax + 63) / 64;
+    const int gx = (mmax + 63) / 64, gy1 = (nmax + 63) / 64;
+    const int cb = (size_t)gx * ((gy1 + kDfeCb - 1) / kDfeCb) * njobs < 888 ? 1 : kDfeCb;
+    const int gy = (gy1 + cb - 1) / cb;
     const size_t nslot = (size_t)gx * gy;
     double *sums = (double *)pool_alloc(2 * njobs * sizeof(double), s);
     double *part = (double *)pool_alloc(2 * njobs * nslot * sizeof(double), s);
@@ -853,11 +1252,10 @@ static int dfe_sums_device(STARSH_blrm *M, Context &ctx, double *diff2,
     for (size_t b0 = 0; b0 < njobs; b0 += 65535) {
         const unsigned nb = (unsigned)std::min<size_t>(65535, njobs - b0);
         dim3 grid(gx, gy, nb);
-        k_dfe<<<grid, 256, 0, s>>>(rec->points->K, dj + b0,
-                                   part + 2 * b0 * nslot);
+        launch_dfe(rec->points->K, grid, dj + b0, part + 2 * b0 * nslot, cb, s);
         count_launch();
     }
-    k_dfe_sum<<<(unsigned)((njobs + 255) / 256), 256, 0, s>>>(
+    k_dfe_sum<<<(unsigned)((njobs + 7) / 8), 256, 0, s>>>(
         part, (int)nslot, (long long)njobs, sums);
     count_launch();
     std::vector<double> h(2 * njobs);
