@@ -28,7 +28,6 @@ struct Context {
     cudaStream_t copy = nullptr;   // device-to-host copies of finished batches
     DeviceBuffer workspace;    // per-slot scratch of the engine
     DeviceBuffer tiles;        // TileWork array of a batch
-    DeviceBuffer descs;        // GemmDesc array of a batch
     DeviceBuffer omega;        // Gaussian sketch matrix
     DeviceBuffer flag;         // round flag of the adaptive sketch
     DeviceBuffer act;          // a round's sampling tiles, by round slot

@@ -198,7 +198,6 @@ void context_free_private(Context *c)
     }
     c->workspace.release();
     c->tiles.release();
-    c->descs.release();
     c->omega.release();
     c->flag.release();
     c->act.release();
@@ -903,7 +902,6 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     if (!ctx.workspace.reserve(ws_need, s))
         return cuda_fail(cudaErrorMemoryAllocation, "workspace");
     if (!ctx.tiles.reserve((size_t)max_slots * sizeof(TileWork), s) ||
-        !ctx.descs.reserve((size_t)max_slots * sizeof(GemmDesc), s) ||
         !ctx.flag.reserve(256, s) ||
         !ctx.act.reserve((size_t)max_slots * (1 + kSvdBins) * sizeof(int), s))
         return cuda_fail(cudaErrorMemoryAllocation, "batch arrays");
@@ -933,7 +931,6 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     };
     Workspace ws{};
     TileWork *dt = (TileWork *)ctx.tiles.ptr;
-    GemmDesc *dd = (GemmDesc *)ctx.descs.ptr;
 
     // ev[0..1] sketch GEMM, ev[2..3] projection GEMM, ev[4] generation
     // start, ev[5] basis start, ev[6] SVD end, ev[7..8] output
@@ -948,15 +945,16 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     OutArena none{nullptr, nullptr};
     int info = STARSH_SUCCESS;
 
-    // round_count >= 0: the steps of an adaptive round whose sampling
-    // tiles (round_count of them, known from the round flag) have compact
-    // descriptors; -1: one descriptor per tile of the batch
+    // round_count >= 0: the steps of an adaptive round run over its sampling
+    // tiles (round_count of them, known from the round's counts) alone; -1:
+    // over every tile of the batch
     int round_count = -1;
     auto gemm = [&](GemmStep step, bool ta, bool tb, int nt, int mm, int nn,
                     OutArena out) -> int {
         const bool compact = round_count >= 0;
-        make_gemm_descs(step, dt, nt, ws, omega, n_max, out, dd, s, compact);
-        count_launch(2);
+        const GemmArgs args{step, dt, compact ? (const int *)ctx.act.ptr : nullptr, ws,
+                            omega, n_max, out};
+        count_launch();
         // the transposed products of the adaptive rounds (outputs of a few
         // basis or sample columns, K = the tile height) and the Gram B B^T
         // of the small SVD (K = the tile width) split K inside the CTA
@@ -965,7 +963,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
                              step == STEP_A_RES_Z2 || step == STEP_A_GRAM2 ||
                              step == STEP_A_ORTH_Z || step == STEP_A_GRAM_R ||
                              step == STEP_GRAM_B;
-        return gemm_f64_batched(ta, tb, dd, compact ? round_count : nt, mm, nn,
+        return gemm_f64_batched(ta, tb, args, compact ? round_count : nt, mm, nn,
                                 s, split_k) == cudaSuccess
                    ? STARSH_SUCCESS
                    : cuda_fail(cudaGetLastError(), "gemm_f64_batched");
@@ -1078,16 +1076,18 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         const int *act = (const int *)ctx.act.ptr;
         auto rcount = [&]() { return round_count >= 0 ? round_count : nt; };
         auto ract = [&]() { return round_count >= 0 ? act : nullptr; };
-        auto append = [&](int bmax) -> int {
+        auto append = [&](int bmax, int k_max, bool empty) -> int {
             // orthonormalise the selected residual columns (kb of them)
-            // against the basis and append them: CholQR of R_J, one more
-            // projection, CholQR again (CGS2)
+            // against the basis (empty: there is none yet) and append them:
+            // CholQR of R_J, one more projection, CholQR again (CGS2)
             int e;
             launch_gather_cols(1, dt, rcount(), ws, s, ract());
             count_launch();
             if ((e = gemm(STEP_A_Q1B, false, false, nt, m_max, bmax, none))) return e;
-            if ((e = gemm(STEP_A_ORTH_Z, true, false, nt, k_max, bmax, none))) return e;
-            if ((e = gemm(STEP_A_ORTH_R, false, false, nt, m_max, bmax, none))) return e;
+            if (!empty) {
+                if ((e = gemm(STEP_A_ORTH_Z, true, false, nt, k_max, bmax, none))) return e;
+                if ((e = gemm(STEP_A_ORTH_R, false, false, nt, m_max, bmax, none))) return e;
+            }
             if ((e = gemm(STEP_A_GRAM_R, true, false, nt, bmax, bmax, none))) return e;
             launch_chol_inv(1, dt, rcount(), ws, bmax, s, ract());
             count_launch();
@@ -1096,9 +1096,17 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             count_launch();
             return STARSH_SUCCESS;
         };
+        // a pass adds at most its sample's columns to a tile's basis (a
+        // repeat pass searches the same sample once more): the bound of the
+        // rounds' outputs onto the basis (every CTA of a launch beyond a
+        // tile's own basis only starts and leaves)
+        int sampled = 0;
         for (int round = 0; info == STARSH_SUCCESS; ++round) {
             const int block = round == 0 ? ep.block : ep.block_next;
             const int bmax = std::min(block, k_max);
+            const int k_old = std::min(k_max, sampled);
+            sampled += may_repeat ? 2 * bmax : bmax;
+            const int k_new = std::min(k_max, sampled);
             const bool pre_sketched = fused && round == 0;
             round_count = -1;
             if (!pre_sketched) {
@@ -1137,21 +1145,21 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             }
             cudaEventRecord(ev[1], s);
             if (round > 0) {
-                if ((info = gemm(STEP_A_RES_Z, true, false, nt, k_max, bmax, none))) break;
+                if ((info = gemm(STEP_A_RES_Z, true, false, nt, k_old, bmax, none))) break;
                 if ((info = gemm(STEP_A_RES_Y, false, false, nt, m_max, bmax, none))) break;
             }
             if ((info = gemm(STEP_A_GRAM, true, false, nt, bmax, bmax, none))) break;
             launch_round_pivchol(dt, rcount(), ws, 0, bmax, s, ract());
             count_launch();
-            if ((info = append(bmax))) break;
+            if ((info = append(bmax, k_old, round == 0))) break;
             if (may_repeat) {
                 // same sample, projected off the grown basis once more
-                if ((info = gemm(STEP_A_RES_Z2, true, false, nt, k_max, bmax, none))) break;
+                if ((info = gemm(STEP_A_RES_Z2, true, false, nt, k_new, bmax, none))) break;
                 if ((info = gemm(STEP_A_RES_Y2, false, false, nt, m_max, bmax, none))) break;
                 if ((info = gemm(STEP_A_GRAM2, true, false, nt, bmax, bmax, none))) break;
                 launch_round_pivchol(dt, rcount(), ws, 1, bmax, s, ract());
                 count_launch();
-                if ((info = append(bmax))) break;
+                if ((info = append(bmax, k_new, false))) break;
             }
             launch_round_end(dt, nt, ep.verify, s);
             count_launch();
@@ -1166,6 +1174,17 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         round_count = -1;
         if (info) break;
         }
+        // The adaptive engine's last round set-up, which the host has read,
+        // counted and listed the tiles by basis size: bound of the products
+        // with the basis, and the small SVD's lists.
+        const bool listed = ep.engine == STARSH_B200_MIXED;
+        int bins[kSvdBins], k_basis = k_max;
+        if (listed) {
+            memcpy(bins, (const int *)ctx.mapped + 1, sizeof(bins));
+            k_basis = 1;
+            for (int b = 0; b < kSvdBins; ++b)
+                if (bins[b] > 0) k_basis = std::min(k_max, svd_bin_hi(b));
+        }
         // projection (tiles with at most 64 basis columns on the tensor
         // cores, the others FP64) and small SVD
         cudaEventRecord(ev[2], s);
@@ -1178,17 +1197,12 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             }
             count_launch(2);
         }
-        if ((info = gemm(STEP_PROJECT, true, false, nt, k_max, plan[pi].n, none))) break;
+        if ((info = gemm(STEP_PROJECT, true, false, nt, k_basis, plan[pi].n, none))) break;
         cudaEventRecord(ev[3], s);
-        if ((info = gemm(STEP_GRAM_B, false, true, nt, k_max, k_max, none))) break;
-        // the adaptive engine's last round set-up, which the host has read,
-        // counted and listed the tiles by basis size
-        const bool listed = ep.engine == STARSH_B200_MIXED;
-        int bins[kSvdBins];
-        if (listed) memcpy(bins, (const int *)ctx.mapped + 1, sizeof(bins));
+        if ((info = gemm(STEP_GRAM_B, false, true, nt, k_basis, k_basis, none))) break;
         count_launch(launch_small_svd(dt, nt, ws, s, ctx.lanes, listed ? bins : nullptr,
                                       listed ? (const int *)ctx.act.ptr + nt : nullptr, nt));
-        if ((info = gemm(STEP_ROTATE, true, false, nt, k_max, plan[pi].n, none))) break;
+        if ((info = gemm(STEP_ROTATE, true, false, nt, k_basis, plan[pi].n, none))) break;
         launch_rank_cut(dt, nt, ws, s);
         count_launch();
         cudaEventRecord(ev[6], s);
@@ -1219,6 +1233,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         // mirror is a concatenation of its parts), shared by the records
         // of the problems with tiles here.
         std::vector<size_t> nu(jobs.size(), 0), nv(jobs.size(), 0);
+        int r_max = 0;
         for (int t = 0; t < nt; ++t) {
             TileWork &w = all[b0 + t];
             st.sketch_flops += 2.0 * w.m * w.n *
@@ -1246,6 +1261,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             }
             jobs[w.prob].rank[owner[b0 + t].second] = w.rank;
             if (w.rank > 0) {
+                r_max = std::max(r_max, w.rank);
                 nu[w.prob] += (size_t)w.m * w.rank;
                 nv[w.prob] += (size_t)w.n * w.rank;
             }
@@ -1300,7 +1316,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             cudaEventRecord(ev[7], s);
             launch_select_w(dt, nt, ws, s);
             count_launch();
-            if ((info = gemm(STEP_OUT_U, false, false, nt, m_max, k_max, out))) break;
+            if ((info = gemm(STEP_OUT_U, false, false, nt, m_max, r_max, out))) break;
             launch_write_v(dt, nt, ws, out, s);
             count_launch();
             cudaEventRecord(ev[8], s);

@@ -138,11 +138,30 @@ struct OutArena {
     double *V;
 };
 
-// Builds the descriptors of `step` for every tile of the batch.
-void make_gemm_descs(GemmStep step, const TileWork *d_tiles, int ntiles,
-                     Workspace ws, const double *d_omega, int ld_omega,
-                     OutArena out, GemmDesc *d_desc, cudaStream_t stream,
-                     bool compact = false);
+// One GEMM step over the tiles of a batch: the operands and shapes of each
+// tile's product follow from its record (gemm_step.cuh), read by the GEMM
+// kernels themselves.  act (optional): the launch covers the tiles listed
+// there instead of the first ones.
+struct GemmArgs {
+    GemmStep step;
+    const TileWork *tiles;
+    const int *act;
+    Workspace ws;
+    const double *omega;
+    int ld_omega;
+    OutArena out;
+};
+
+// Launches one product per tile of `args` (`count` of them); entries whose
+// M, N or K is 0 are skipped.  max_m/max_n bound the shapes of all entries.
+// split_k (A^T B and A B^T): every entry runs on 64 x 64 CTA tiles whatever
+// the bounds, and a tile with few rows or columns of its own splits K over
+// the spare warps; an entry's result then depends on its own shape alone,
+// never on the bounds of the batch it is in.  Returns the CUDA error of the
+// launch.
+cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int count,
+                             int max_m, int max_n, cudaStream_t stream,
+                             bool split_k = false);
 
 // Per-tile kernels (one CTA per tile).
 // Thresholds come from each tile's tol and maxrank; the generator reads

@@ -12,7 +12,7 @@
 // steps past its K (those would add exact zeros).
 #include <cstdint>
 #include <mutex>
-#include "gemm_f64.cuh"
+#include "gemm_step.cuh"
 
 namespace b200 {
 
@@ -30,14 +30,14 @@ __device__ __forceinline__ void dmma_8x8x4(double &c0, double &c1, double a,
 // three CTAs per SM: their short K makes them latency-bound.
 template <bool TA, bool TB, int BM, int BN>
 __global__ void __launch_bounds__(kGemmThreads, (!TA && !TB) ? 3 : 0)
-k_gemm_f64(const GemmDesc *__restrict__ descs, int tiles_n)
+k_gemm_f64(const __grid_constant__ GemmArgs args, int tiles_n)
 {
     // 8 warps of 32 x 16 output each, BM / 32 along M and BN / 16 along N
     constexpr int WARPS_M = BM / 32;
     static_assert(WARPS_M * (BN / 16) == kGemmThreads / 32, "warp grid");
     constexpr int RA = BM * kGemmBK / kGemmThreads;   // A loads per thread
     constexpr int RB = BN * kGemmBK / kGemmThreads;   // B loads per thread
-    const GemmDesc d = descs[blockIdx.y];
+    const GemmDesc d = gemm_desc(args, blockIdx.y);
     const int tm = blockIdx.x / tiles_n;
     const int tn = blockIdx.x % tiles_n;
     const int m0 = tm * BM, n0 = tn * BN;
@@ -222,13 +222,62 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool pr
                  :: "r"(sa), "l"(gmem), "r"(n));
 }
 
+// A thread's share of an operand tile that is contiguous along k: rows t / 8 +
+// 32 r (r < R) of the tile, k pair t % 8 of each K step, in stages of
+// [row][kGemmLds], `pitch` rows apart.  What a row needs is worked out once (a K step of the
+// pipelined kernels is short, and addresses and bounds worked out per piece
+// took more issue slots than its products); rows outside the operand are
+// zeroed in every stage at the start and not copied.
+template <int R>
+struct PipeRows {
+    const double *src[R];
+    double *dst;
+    bool row_ok[R], even;
+
+    __device__ __forceinline__ void init(const double *base, int ld, int g0, int lim,
+                                         double *stages, int pitch, int tile_rows)
+    {
+        const int row = threadIdx.x >> 3, kk = (threadIdx.x & 7) * 2;
+        even = (ld & 1) == 0 && ((uintptr_t)base & 15) == 0;
+        dst = stages + row * kGemmLds + kk;
+        #pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int g = g0 + row + 32 * r;
+            row_ok[r] = row + 32 * r < tile_rows && g < lim;
+            src[r] = base + (size_t)(row_ok[r] ? g : g0) * ld + kk;
+            if (!row_ok[r] && row + 32 * r < tile_rows)
+                for (int s = 0; s < kTnStages; ++s) {
+                    double *z = dst + (s * pitch + 32 * r) * kGemmLds;
+                    z[0] = z[1] = 0.0;
+                }
+        }
+    }
+    // The K step at k0 into the stage whose first row is `at`.
+    __device__ __forceinline__ void copy(int at, int k0, int K) const
+    {
+        const int gk = k0 + (threadIdx.x & 7) * 2;
+        if (even && gk + 1 < K) {
+            #pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (row_ok[r])
+                    cp_async16(dst + (at + 32 * r) * kGemmLds, src[r] + k0, true);
+        } else {
+            #pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (row_ok[r]) {
+                    double *q = dst + (at + 32 * r) * kGemmLds;
+                    q[0] = gk < K ? src[r][k0] : 0.0;
+                    q[1] = gk + 1 < K ? src[r][k0 + 1] : 0.0;
+                }
+        }
+    }
+};
+
 __global__ void __launch_bounds__(kGemmThreads)
-k_gemm_f64_tn_pipe(const GemmDesc *__restrict__ descs, int tiles_n, int split_k)
+k_gemm_f64_tn_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split_k)
 {
     constexpr int BM = 64, BN = 64, WARPS_M = BM / 32;
-    // 16-byte pieces of the two operand tiles (BM and BN rows of 16 k)
-    constexpr int PA = BM * kGemmBK / 2, PIECES = (BM + BN) * kGemmBK / 2;
-    const GemmDesc d = descs[blockIdx.y];
+    const GemmDesc d = gemm_desc(args, blockIdx.y);
     const int tm = blockIdx.x / tiles_n, tn = blockIdx.x % tiles_n;
     const int m0 = tm * BM, n0 = tn * BN;
     if (m0 >= d.M || n0 >= d.N) return;
@@ -263,39 +312,14 @@ k_gemm_f64_tn_pipe(const GemmDesc *__restrict__ descs, int tiles_n, int split_k)
     for (int i = 0; i < 4; ++i)
         #pragma unroll
         for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    // the A tile (BM rows x 16 k) is pieces 0 .. PA - 1, the B tile (BN
-    // rows) the rest; thread t copies pieces t, t + 256, ... (row = piece
-    // / 8 within its tile, k pair = piece % 8)
-    const bool evenA = (d.lda & 1) == 0 && ((uintptr_t)d.A & 15) == 0;
-    const bool evenB = (d.ldb & 1) == 0 && ((uintptr_t)d.B & 15) == 0;
+    // 16-byte pieces: rows t / 8 and t / 8 + 32 of A and of B, k pair t % 8
+    PipeRows<2> ra, rb;
+    ra.init(d.A, d.lda, m0, d.M, As, BM, BM);
+    rb.init(d.B, d.ldb, n0, d.N, Bs, BN, BN);
     auto issue = [&](int kt) {
         const int st = kt % kTnStages, k0 = kt * kGemmBK;
-        #pragma unroll
-        for (int r = 0; r < PIECES / kGemmThreads; ++r) {
-            const int piece = t + kGemmThreads * r;
-            if (piece < PA) {
-                const int row = piece >> 3, kk = (piece & 7) * 2;
-                const int gm = m0 + row, gk = k0 + kk;
-                double *dst = As + (st * BM + row) * kGemmLds + kk;
-                if (evenA && gm < d.M && gk + 1 < d.K) {
-                    cp_async16(dst, d.A + (size_t)gm * d.lda + gk, true);
-                } else {
-                    dst[0] = (gm < d.M && gk < d.K) ? d.A[(size_t)gm * d.lda + gk] : 0.0;
-                    dst[1] = (gm < d.M && gk + 1 < d.K) ? d.A[(size_t)gm * d.lda + gk + 1] : 0.0;
-                }
-            } else {
-                const int q = piece - PA;
-                const int row = q >> 3, kk = (q & 7) * 2;
-                const int gn = n0 + row, gk = k0 + kk;
-                double *dst = Bs + (st * BN + row) * kGemmLds + kk;
-                if (evenB && gn < d.N && gk + 1 < d.K) {
-                    cp_async16(dst, d.B + (size_t)gn * d.ldb + gk, true);
-                } else {
-                    dst[0] = (gn < d.N && gk < d.K) ? d.B[(size_t)gn * d.ldb + gk] : 0.0;
-                    dst[1] = (gn < d.N && gk + 1 < d.K) ? d.B[(size_t)gn * d.ldb + gk + 1] : 0.0;
-                }
-            }
-        }
+        ra.copy(st * BM, k0, d.K);
+        rb.copy(st * BN, k0, d.K);
         asm volatile("cp.async.commit_group;");
     };
     const int ktiles = (d.K + kGemmBK - 1) / kGemmBK;
@@ -392,32 +416,14 @@ __device__ __forceinline__ void tn_wide(const GemmDesc &d, int m0, int n0,
     constexpr int STAGE = (kWideM + kWideN) * kGemmLds;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3, wn = warp * 16;
-    const bool evenA = (d.lda & 1) == 0 && ((uintptr_t)d.A & 15) == 0;
-    const bool evenB = (d.ldb & 1) == 0 && ((uintptr_t)d.B & 15) == 0;
-    // 16-byte pieces: row t / 8 + 32 r, k pair t % 8
-    const int row = t >> 3, kk = (t & 7) * 2;
-    auto piece = [&](double *dst, const double *src, int ld, int gr, int lim, int gk,
-                     bool even) {
-        const double *p = src + (size_t)gr * ld + gk;
-        if (even && gr < lim && gk + 1 < d.K) {
-            cp_async16(dst, p, true);
-        } else {
-            dst[0] = gr < lim && gk < d.K ? p[0] : 0.0;
-            dst[1] = gr < lim && gk + 1 < d.K ? p[1] : 0.0;
-        }
-    };
+    PipeRows<(MF + 3) / 4> ra;
+    PipeRows<kWideN / 32> rb;
+    ra.init(d.A, d.lda, m0, d.M, smem, kWideM + kWideN, MF * 8);
+    rb.init(d.B, d.ldb, n0, d.N, smem + kWideM * kGemmLds, kWideM + kWideN, kWideN);
     auto issue = [&](int kt) {
-        double *A = smem + kt % kTnStages * STAGE, *B = A + kWideM * kGemmLds;
-        const int gk = kt * kGemmBK + kk;
-        #pragma unroll
-        for (int r = 0; r < (MF + 3) / 4; ++r)
-            if (r * 32 + row < MF * 8)
-                piece(A + (r * 32 + row) * kGemmLds + kk, d.A, d.lda, m0 + r * 32 + row,
-                      d.M, gk, evenA);
-        #pragma unroll
-        for (int r = 0; r < kWideN / 32; ++r)
-            piece(B + (r * 32 + row) * kGemmLds + kk, d.B, d.ldb, n0 + r * 32 + row,
-                  d.N, gk, evenB);
+        const int at = kt % kTnStages * (kWideM + kWideN), k0 = kt * kGemmBK;
+        ra.copy(at, k0, d.K);
+        rb.copy(at, k0, d.K);
         asm volatile("cp.async.commit_group;");
     };
     double acc[MF][2][2] = {};
@@ -467,10 +473,10 @@ __device__ __forceinline__ void tn_wide(const GemmDesc &d, int m0, int n0,
 }
 
 __global__ void __launch_bounds__(kGemmThreads, 2)
-k_gemm_f64_tn_wide(const GemmDesc *__restrict__ descs, int tiles_n)
+k_gemm_f64_tn_wide(const __grid_constant__ GemmArgs args, int tiles_n)
 {
     extern __shared__ double gemm_smem[];
-    const GemmDesc d = descs[blockIdx.y];
+    const GemmDesc d = gemm_desc(args, blockIdx.y);
     const int m0 = blockIdx.x / tiles_n * kWideM, n0 = blockIdx.x % tiles_n * kWideN;
     if (m0 >= d.M || n0 >= d.N) return;
     switch (min(kWideM, d.M - m0) + 7 >> 3) {
@@ -497,10 +503,10 @@ k_gemm_f64_tn_wide(const GemmDesc *__restrict__ descs, int tiles_n)
 constexpr int kNtLds = 64 + 4;
 
 __global__ void __launch_bounds__(kGemmThreads)
-k_gemm_f64_nt_pipe(const GemmDesc *__restrict__ descs, int tiles_n, int split_k)
+k_gemm_f64_nt_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split_k)
 {
     constexpr int BM = 64, BN = 64;
-    const GemmDesc d = descs[blockIdx.y];
+    const GemmDesc d = gemm_desc(args, blockIdx.y);
     const int tm = blockIdx.x / tiles_n, tn = blockIdx.x % tiles_n;
     const int m0 = tm * BM, n0 = tn * BN;
     if (m0 >= d.M || n0 >= d.N) return;
@@ -529,30 +535,42 @@ k_gemm_f64_nt_pipe(const GemmDesc *__restrict__ descs, int tiles_n, int split_k)
     for (int i = 0; i < 4; ++i)
         #pragma unroll
         for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    // 16-byte pieces: rows 2 (t % 32) and the next, k = t / 32 and + 8 of a
+    // K step, of A and of B.  Pointers and bounds are worked out once; rows
+    // outside the operand are zeroed in every stage and not copied.
+    const int row = (t & 31) * 2, kk = t >> 5;
+    auto rows_in = [&](int g0, int lim) { return max(0, min(2, lim - g0 - row)); };
+    const int na = rows_in(m0, d.M), nb = rows_in(n0, d.N);
+    const double *pa = d.A + (na ? m0 + row : 0) + (size_t)kk * d.lda;
+    const double *pb = d.B + (nb ? n0 + row : 0) + (size_t)kk * d.ldb;
     const bool evenA = (d.lda & 1) == 0 && ((uintptr_t)d.A & 15) == 0;
     const bool evenB = (d.ldb & 1) == 0 && ((uintptr_t)d.B & 15) == 0;
-    // pieces 0 .. 511: A (row pair = piece % 32, k = piece / 32), 512 ..
-    // 1023: B the same way; thread t copies t, t + 256, t + 512, t + 768
+    double *qa = As + kk * kNtLds + row, *qb = Bs + kk * kNtLds + row;
+    for (int s = 0; s < kTnStages; ++s)
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int at = (s * kGemmBK + 8 * h) * kNtLds;
+            if (na < 2) qa[at + 1] = 0.0;
+            if (na < 1) qa[at] = 0.0;
+            if (nb < 2) qb[at + 1] = 0.0;
+            if (nb < 1) qb[at] = 0.0;
+        }
+    auto piece = [&](double *dst, const double *src, int n, bool even, bool in) {
+        if (n == 2 && even && in) {
+            cp_async16(dst, src, true);
+        } else {
+            if (n > 0) dst[0] = in ? src[0] : 0.0;
+            if (n > 1) dst[1] = in ? src[1] : 0.0;
+        }
+    };
     auto issue = [&](int kt) {
         const int st = kt % kTnStages, k0 = kt * kGemmBK;
         #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int piece = t + kGemmThreads * r;
-            const bool isA = piece < 512;
-            const int q = isA ? piece : piece - 512;
-            const int row = (q & 31) * 2, kk = q >> 5;
-            const int gk = k0 + kk;
-            const double *src = isA ? d.A : d.B;
-            const int ld = isA ? d.lda : d.ldb;
-            const int lim = isA ? d.M : d.N;
-            const int g0 = (isA ? m0 : n0) + row;
-            double *dst = (isA ? As : Bs) + (st * kGemmBK + kk) * kNtLds + row;
-            if ((isA ? evenA : evenB) && g0 + 1 < lim && gk < d.K) {
-                cp_async16(dst, src + (size_t)gk * ld + g0, true);
-            } else {
-                dst[0] = (g0 < lim && gk < d.K) ? src[(size_t)gk * ld + g0] : 0.0;
-                dst[1] = (g0 + 1 < lim && gk < d.K) ? src[(size_t)gk * ld + g0 + 1] : 0.0;
-            }
+        for (int h = 0; h < 2; ++h) {
+            const bool in = k0 + kk + 8 * h < d.K;
+            const int at = (st * kGemmBK + 8 * h) * kNtLds;
+            piece(qa + at, pa + (size_t)(k0 + 8 * h) * d.lda, na, evenA, in);
+            piece(qb + at, pb + (size_t)(k0 + 8 * h) * d.ldb, nb, evenB, in);
         }
         asm volatile("cp.async.commit_group;");
     };
@@ -629,7 +647,7 @@ k_gemm_f64_nt_pipe(const GemmDesc *__restrict__ descs, int tiles_n, int split_k)
 }
 
 template <int BM, int BN>
-static void launch_shape(bool ta, bool tb, const GemmDesc *dd, int nb,
+static void launch_shape(bool ta, bool tb, const GemmArgs &args, int nb,
                          int tiles_m, int tiles_n, cudaStream_t stream)
 {
     dim3 grid(tiles_m * tiles_n, nb);
@@ -638,7 +656,7 @@ static void launch_shape(bool ta, bool tb, const GemmDesc *dd, int nb,
         if (smem > 48 * 1024)
             cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
-        fn<<<grid, kGemmThreads, smem, stream>>>(dd, tiles_n);
+        fn<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n);
     };
     if (!ta && !tb) go(k_gemm_f64<false, false, BM, BN>);
     else if (ta && !tb) go(k_gemm_f64<true, false, BM, BN>);
@@ -646,9 +664,9 @@ static void launch_shape(bool ta, bool tb, const GemmDesc *dd, int nb,
     else go(k_gemm_f64<true, true, BM, BN>);
 }
 
-cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmDesc *d_desc,
-                             int batch, int max_m, int max_n,
-                             cudaStream_t stream, bool split_k)
+cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int batch,
+                             int max_m, int max_n, cudaStream_t stream,
+                             bool split_k)
 {
     if (batch <= 0 || max_m <= 0 || max_n <= 0) return cudaSuccess;
     split_k = split_k && ta != tb;
@@ -662,9 +680,9 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmDesc *d_desc,
     const int bn = wide ? kWideN : bm == 128 ? 32 : 64;
     const int tiles_m = (max_m + bm - 1) / bm;
     const int tiles_n = (max_n + bn - 1) / bn;
-    for (int b0 = 0; b0 < batch; b0 += 65535) {
-        const int nb = batch - b0 < 65535 ? batch - b0 : 65535;
-        const GemmDesc *dd = d_desc + b0;
+    {
+        // (a batch has at most a few thousand tiles: one launch)
+        const int nb = batch;
         dim3 grid(tiles_m * tiles_n, nb);
         if (ta && !tb && bm == 64) {
             constexpr size_t smem = (size_t)kTnStages * 128 * kGemmLds * sizeof(double);
@@ -680,9 +698,9 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmDesc *d_desc,
                                      (int)smem_wide);
             });
             if (wide)
-                k_gemm_f64_tn_wide<<<grid, kGemmThreads, smem_wide, stream>>>(dd, tiles_n);
+                k_gemm_f64_tn_wide<<<grid, kGemmThreads, smem_wide, stream>>>(args, tiles_n);
             else
-                k_gemm_f64_tn_pipe<<<grid, kGemmThreads, smem, stream>>>(dd, tiles_n, split_k ? 1 : 0);
+                k_gemm_f64_tn_pipe<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n, split_k ? 1 : 0);
         } else if (!ta && tb && bm == 64) {
             constexpr size_t smem = (size_t)kTnStages * 2 * kGemmBK * kNtLds * sizeof(double);
             static std::once_flag attr_nt;
@@ -691,9 +709,9 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmDesc *d_desc,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem);
             });
-            k_gemm_f64_nt_pipe<<<grid, kGemmThreads, smem, stream>>>(dd, tiles_n, split_k ? 1 : 0);
-        } else if (bm == 128) launch_shape<128, 32>(ta, tb, dd, nb, tiles_m, tiles_n, stream);
-        else launch_shape<64, 64>(ta, tb, dd, nb, tiles_m, tiles_n, stream);
+            k_gemm_f64_nt_pipe<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n, split_k ? 1 : 0);
+        } else if (bm == 128) launch_shape<128, 32>(ta, tb, args, nb, tiles_m, tiles_n, stream);
+        else launch_shape<64, 64>(ta, tb, args, nb, tiles_m, tiles_n, stream);
     }
     return cudaGetLastError();
 }

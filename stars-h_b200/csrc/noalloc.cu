@@ -47,9 +47,8 @@ constexpr size_t kSlotDoubles =
     slot_doubles(kNoAllocMaxDim, kNoAllocMaxDim, kNoAllocMaxK);
 constexpr size_t kOmegaDoubles = round32((size_t)kNoAllocMaxDim * kNoAllocMaxK);
 constexpr size_t kTileDoubles = round32((sizeof(TileWork) + 7) / 8);
-constexpr size_t kDescDoubles = round32((sizeof(GemmDesc) + 7) / 8);
 constexpr size_t kScratchDoubles =
-    kSlotDoubles + kOmegaDoubles + kTileDoubles + kDescDoubles;
+    kSlotDoubles + kOmegaDoubles + kTileDoubles;
 
 // The scratch.  Host code must not use this symbol as an address: on the
 // host it is only a stand-in; the device address comes from
@@ -142,7 +141,6 @@ extern "C" int starsh_b200_dense_rsvd_noalloc(const double *dD, int nrows,
     ws.stride = stride;
     double *omega = scratch + kSlotDoubles;
     TileWork *dt = (TileWork *)(omega + kOmegaDoubles);
-    GemmDesc *dd = (GemmDesc *)((double *)dt + kTileDoubles);
 
     k_noalloc_tile<<<1, 1, 0, s>>>(dt, nrows, ncols, k, maxrank, tol);
     B200_CUDA(cudaMemcpy2DAsync(ws.D(0), (size_t)ws.ldD() * sizeof(double), dD,
@@ -156,8 +154,8 @@ extern "C" int starsh_b200_dense_rsvd_noalloc(const double *dD, int nrows,
     const OutArena out{dU, dV};
     auto gemm = [&](GemmStep step, bool ta, bool tb, int mm, int nn,
                     OutArena o) -> int {
-        make_gemm_descs(step, dt, 1, ws, omega, ncols, o, dd, s);
-        return gemm_f64_batched(ta, tb, dd, 1, mm, nn, s) == cudaSuccess
+        const GemmArgs args{step, dt, nullptr, ws, omega, ncols, o};
+        return gemm_f64_batched(ta, tb, args, 1, mm, nn, s) == cudaSuccess
                    ? STARSH_SUCCESS
                    : cuda_fail(cudaGetLastError(), "no-alloc gemm");
     };
