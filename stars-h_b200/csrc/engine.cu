@@ -1081,8 +1081,6 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             // against the basis (empty: there is none yet) and append them:
             // CholQR of R_J, one more projection, CholQR again (CGS2)
             int e;
-            launch_gather_cols(1, dt, rcount(), ws, s, ract());
-            count_launch();
             if ((e = gemm(STEP_A_Q1B, false, false, nt, m_max, bmax, none))) return e;
             if (!empty) {
                 if ((e = gemm(STEP_A_ORTH_Z, true, false, nt, k_max, bmax, none))) return e;

@@ -126,7 +126,7 @@ enum GemmStep : int {
     STEP_A_RES_Z2,       // second projection of the same sample (repeat
     STEP_A_RES_Y2,       //   pass, tiles flagged need_pass_b)
     STEP_A_GRAM2,
-    STEP_A_Q1B,          // R  = Q1 T   (gathered residual columns)
+    STEP_A_Q1B,          // R  = Y[:, piv] T (residual columns kept)
     STEP_A_ORTH_Z,       // S  = Q^T R
     STEP_A_ORTH_R,       // R -= Q S
     STEP_A_GRAM_R,       // S  = R^T R

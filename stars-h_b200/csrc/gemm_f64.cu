@@ -212,7 +212,11 @@ k_gemm_f64(const __grid_constant__ GemmArgs args, int tiles_n)
 // results are identical to it; in a launch that asks for it (split_k), a
 // tile with at most 32 rows or 48 columns of its own splits K over the
 // spare warps (fixed slice order, deterministic).
-constexpr int kTnStages = 3;
+// Stages of the pipelined kernels: three, or five where the launch has at
+// most two CTAs per SM, whose K steps (16 deep, 64 x 64) then wait on the
+// latency of the copies (16 tiles of 1024 rows: 0.5 us a step with three).
+constexpr int kShallow = 3, kDeep = 5;
+constexpr int kDeepGrid = 296;
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool pred)
 {
@@ -228,7 +232,7 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool pr
 // pipelined kernels is short, and addresses and bounds worked out per piece
 // took more issue slots than its products); rows outside the operand are
 // zeroed in every stage at the start and not copied.
-template <int R>
+template <int R, int STAGES>
 struct PipeRows {
     const double *src[R];
     double *dst;
@@ -246,7 +250,7 @@ struct PipeRows {
             row_ok[r] = row + 32 * r < tile_rows && g < lim;
             src[r] = base + (size_t)(row_ok[r] ? g : g0) * ld + kk;
             if (!row_ok[r] && row + 32 * r < tile_rows)
-                for (int s = 0; s < kTnStages; ++s) {
+                for (int s = 0; s < STAGES; ++s) {
                     double *z = dst + (s * pitch + 32 * r) * kGemmLds;
                     z[0] = z[1] = 0.0;
                 }
@@ -273,6 +277,7 @@ struct PipeRows {
     }
 };
 
+template <int STAGES>
 __global__ void __launch_bounds__(kGemmThreads)
 k_gemm_f64_tn_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split_k)
 {
@@ -284,7 +289,7 @@ k_gemm_f64_tn_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split
     extern __shared__ double gemm_smem[];
     // [stage][64 rows][kGemmLds] for A^T, then the same for B^T
     double *As = gemm_smem;
-    double *Bs = gemm_smem + kTnStages * BM * kGemmLds;
+    double *Bs = gemm_smem + STAGES * BM * kGemmLds;
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3;
@@ -313,29 +318,29 @@ k_gemm_f64_tn_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split
         #pragma unroll
         for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
     // 16-byte pieces: rows t / 8 and t / 8 + 32 of A and of B, k pair t % 8
-    PipeRows<2> ra, rb;
+    PipeRows<2, STAGES> ra, rb;
     ra.init(d.A, d.lda, m0, d.M, As, BM, BM);
     rb.init(d.B, d.ldb, n0, d.N, Bs, BN, BN);
     auto issue = [&](int kt) {
-        const int st = kt % kTnStages, k0 = kt * kGemmBK;
+        const int st = kt % STAGES, k0 = kt * kGemmBK;
         ra.copy(st * BM, k0, d.K);
         rb.copy(st * BN, k0, d.K);
         asm volatile("cp.async.commit_group;");
     };
     const int ktiles = (d.K + kGemmBK - 1) / kGemmBK;
     #pragma unroll
-    for (int p = 0; p < kTnStages - 1; ++p) {
+    for (int p = 0; p < STAGES - 1; ++p) {
         if (p < ktiles) issue(p);
         else asm volatile("cp.async.commit_group;");
     }
     for (int kt = 0; kt < ktiles; ++kt) {
-        // the group of step kt has landed (at most kTnStages - 2 newer ones
+        // the group of step kt has landed (at most STAGES - 2 newer ones
         // still in flight)
-        asm volatile("cp.async.wait_group %0;" :: "n"(kTnStages - 2));
+        asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 2));
         __syncthreads();
-        if (kt + kTnStages - 1 < ktiles) issue(kt + kTnStages - 1);
+        if (kt + STAGES - 1 < ktiles) issue(kt + STAGES - 1);
         else asm volatile("cp.async.commit_group;");
-        const int st = kt % kTnStages;
+        const int st = kt % STAGES;
         const double *Ab = As + st * BM * kGemmLds;
         const double *Bb = Bs + st * BN * kGemmLds;
         #pragma unroll
@@ -416,12 +421,12 @@ __device__ __forceinline__ void tn_wide(const GemmDesc &d, int m0, int n0,
     constexpr int STAGE = (kWideM + kWideN) * kGemmLds;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3, wn = warp * 16;
-    PipeRows<(MF + 3) / 4> ra;
-    PipeRows<kWideN / 32> rb;
+    PipeRows<(MF + 3) / 4, kShallow> ra;
+    PipeRows<kWideN / 32, kShallow> rb;
     ra.init(d.A, d.lda, m0, d.M, smem, kWideM + kWideN, MF * 8);
     rb.init(d.B, d.ldb, n0, d.N, smem + kWideM * kGemmLds, kWideM + kWideN, kWideN);
     auto issue = [&](int kt) {
-        const int at = kt % kTnStages * (kWideM + kWideN), k0 = kt * kGemmBK;
+        const int at = kt % kShallow * (kWideM + kWideN), k0 = kt * kGemmBK;
         ra.copy(at, k0, d.K);
         rb.copy(at, k0, d.K);
         asm volatile("cp.async.commit_group;");
@@ -429,16 +434,16 @@ __device__ __forceinline__ void tn_wide(const GemmDesc &d, int m0, int n0,
     double acc[MF][2][2] = {};
     const int ktiles = (d.K + kGemmBK - 1) / kGemmBK;
     #pragma unroll
-    for (int p = 0; p < kTnStages - 1; ++p) {
+    for (int p = 0; p < kShallow - 1; ++p) {
         if (p < ktiles) issue(p);
         else asm volatile("cp.async.commit_group;");
     }
     for (int kt = 0; kt < ktiles; ++kt) {
-        asm volatile("cp.async.wait_group %0;" :: "n"(kTnStages - 2));
+        asm volatile("cp.async.wait_group %0;" :: "n"(kShallow - 2));
         __syncthreads();
-        if (kt + kTnStages - 1 < ktiles) issue(kt + kTnStages - 1);
+        if (kt + kShallow - 1 < ktiles) issue(kt + kShallow - 1);
         else asm volatile("cp.async.commit_group;");
-        const double *A = smem + kt % kTnStages * STAGE, *B = A + kWideM * kGemmLds;
+        const double *A = smem + kt % kShallow * STAGE, *B = A + kWideM * kGemmLds;
         #pragma unroll
         for (int k4 = 0; k4 < kGemmBK; k4 += 4) {
             double af[MF], bf[2];
@@ -502,6 +507,7 @@ k_gemm_f64_tn_wide(const __grid_constant__ GemmArgs args, int tiles_n)
 // regions as in the transposed kernel.
 constexpr int kNtLds = 64 + 4;
 
+template <int STAGES>
 __global__ void __launch_bounds__(kGemmThreads)
 k_gemm_f64_nt_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split_k)
 {
@@ -513,7 +519,7 @@ k_gemm_f64_nt_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split
     extern __shared__ double gemm_smem[];
     // [stage][16 k][kNtLds] for A, then the same for B
     double *As = gemm_smem;
-    double *Bs = gemm_smem + kTnStages * kGemmBK * kNtLds;
+    double *Bs = gemm_smem + STAGES * kGemmBK * kNtLds;
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3;
@@ -546,7 +552,7 @@ k_gemm_f64_nt_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split
     const bool evenA = (d.lda & 1) == 0 && ((uintptr_t)d.A & 15) == 0;
     const bool evenB = (d.ldb & 1) == 0 && ((uintptr_t)d.B & 15) == 0;
     double *qa = As + kk * kNtLds + row, *qb = Bs + kk * kNtLds + row;
-    for (int s = 0; s < kTnStages; ++s)
+    for (int s = 0; s < STAGES; ++s)
         #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int at = (s * kGemmBK + 8 * h) * kNtLds;
@@ -564,7 +570,7 @@ k_gemm_f64_nt_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split
         }
     };
     auto issue = [&](int kt) {
-        const int st = kt % kTnStages, k0 = kt * kGemmBK;
+        const int st = kt % STAGES, k0 = kt * kGemmBK;
         #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const bool in = k0 + kk + 8 * h < d.K;
@@ -576,16 +582,16 @@ k_gemm_f64_nt_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split
     };
     const int ktiles = (d.K + kGemmBK - 1) / kGemmBK;
     #pragma unroll
-    for (int p = 0; p < kTnStages - 1; ++p) {
+    for (int p = 0; p < STAGES - 1; ++p) {
         if (p < ktiles) issue(p);
         else asm volatile("cp.async.commit_group;");
     }
     for (int kt = 0; kt < ktiles; ++kt) {
-        asm volatile("cp.async.wait_group %0;" :: "n"(kTnStages - 2));
+        asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 2));
         __syncthreads();
-        if (kt + kTnStages - 1 < ktiles) issue(kt + kTnStages - 1);
+        if (kt + STAGES - 1 < ktiles) issue(kt + STAGES - 1);
         else asm volatile("cp.async.commit_group;");
-        const int st = kt % kTnStages;
+        const int st = kt % STAGES;
         const double *Ab = As + st * kGemmBK * kNtLds;
         const double *Bb = Bs + st * kGemmBK * kNtLds;
         #pragma unroll
@@ -646,6 +652,160 @@ k_gemm_f64_nt_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split
     }
 }
 
+// A B with a short K (the basis updates: K and N a round's columns or the
+// basis so far; U = Q W).  A CTA takes `iters` blocks of 64 rows and up to 64
+// columns; K steps of 32 of the (row block, K step) sequence run through
+// three cp.async stages, so a block's loads -- most often one step -- are in
+// flight two blocks ahead, and the tile's record is read once for all of
+// them.  The eight warps split the 64 rows finer where the tile has few
+// columns (16 columns and 8, 16 or 32 rows a warp).  The register-staged
+// kernel above waited a memory round trip in every K step of 16, and once
+// more for C: 256 tiles of 1024 rows and about 25 columns 57 us.  Per
+// element the K order is the same (bit-identical).
+constexpr int kNnK = 32, kNnRows = 64, kNnStages = 3;
+constexpr int kNnLdA = kNnRows + 4, kNnLdB = kNnK + 4;   // [k][row], [n][k]
+constexpr int kNnStage = kNnK * kNnLdA + 64 * kNnLdB;
+
+template <int MI>
+__device__ __forceinline__ void nn_short(const GemmDesc &d, int m_first, int m_last,
+                                         int n0, double *smem)
+{
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int g = lane >> 2, tig = lane & 3;
+    constexpr int WM = kNnRows / (8 * MI);           // warps along the rows
+    const int wm = warp % WM * 8 * MI, wn = warp / WM * 16;
+    const bool live = n0 + wn < d.N;
+    const int ksteps = max(1, (d.K + kNnK - 1) / kNnK);
+    const int blocks = (m_last - m_first + kNnRows - 1) / kNnRows;
+    const int total = blocks * ksteps;
+    const bool evenA = (d.lda & 1) == 0 && ((uintptr_t)d.A & 15) == 0;
+    const bool evenB = (d.ldb & 1) == 0 && ((uintptr_t)d.B & 15) == 0;
+    // copies of A: rows 2 (t % 32) and the next, k = t / 32 + 8 r; of B: k
+    // pair t % 16, columns t / 16 + 16 r
+    const int ar = (t & 31) * 2, ak = t >> 5, bk = (t & 15) * 2, bn = t >> 4;
+    int blk = 0, kst = 0;                            // next step to copy
+    auto issue = [&](int st) {
+        double *A = smem + st % kNnStages * kNnStage, *B = A + kNnK * kNnLdA;
+        const int k0 = kst * kNnK, row = m_first + blk * kNnRows + ar;
+        #pragma unroll
+        for (int r = 0; r < kNnK / 8; ++r) {
+            const int k = k0 + ak + 8 * r;
+            double *dst = A + (ak + 8 * r) * kNnLdA + ar;
+            if (k < d.K) {
+                const double *src = d.A + row + (size_t)(d.gather ? d.gather[k] : k) * d.lda;
+                if (evenA && row + 1 < m_last) {
+                    cp_async16(dst, src, true);
+                } else {
+                    dst[0] = row < m_last ? src[0] : 0.0;
+                    dst[1] = row + 1 < m_last ? src[1] : 0.0;
+                }
+            } else {
+                dst[0] = dst[1] = 0.0;
+            }
+        }
+        #pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int n = bn + 16 * r;
+            if (n0 + n >= (d.N + 15) / 16 * 16) break;
+            double *dst = B + n * kNnLdB + bk;
+            const int k = k0 + bk;
+            const double *src = d.B + (size_t)(n0 + n) * d.ldb + k;
+            const bool in = n0 + n < d.N;
+            if (in && evenB && k + 1 < d.K) {
+                cp_async16(dst, src, true);
+            } else {
+                dst[0] = in && k < d.K ? src[0] : 0.0;
+                dst[1] = in && k + 1 < d.K ? src[1] : 0.0;
+            }
+        }
+        if (++kst == ksteps) {
+            kst = 0;
+            ++blk;
+        }
+    };
+    #pragma unroll
+    for (int p = 0; p < kNnStages - 1; ++p) {
+        if (p < total) issue(p);
+        asm volatile("cp.async.commit_group;");
+    }
+    const bool upd = d.beta != 0.0;
+    int st = 0;
+    #pragma unroll 1
+    for (int b = 0; b < blocks; ++b) {
+        const int m0 = m_first + b * kNnRows + wm;
+        double acc[MI][2][2] = {}, cold[MI][2][2];
+        // the old C of an update is read before the products need to be done
+        if (upd) {
+            #pragma unroll
+            for (int i = 0; i < MI; ++i)
+                #pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int gm = m0 + i * 8 + g, gn = n0 + wn + j * 8 + 2 * tig + h;
+                        cold[i][j][h] = gm < m_last && gn < d.N
+                                            ? d.C[(size_t)gn * d.ldc + gm] : 0.0;
+                    }
+        }
+        #pragma unroll 1
+        for (int ks = 0; ks < ksteps; ++ks, ++st) {
+            asm volatile("cp.async.wait_group %0;" :: "n"(kNnStages - 2));
+            __syncthreads();
+            if (st + kNnStages - 1 < total) issue(st + kNnStages - 1);
+            asm volatile("cp.async.commit_group;");
+            if (!live) continue;
+            const double *A = smem + st % kNnStages * kNnStage, *B = A + kNnK * kNnLdA;
+            const int kend = min(kNnK, d.K - ks * kNnK);
+            #pragma unroll
+            for (int kk = 0; kk < kNnK; kk += 4) {
+                if (kk >= kend) break;
+                double af[MI], bf[2];
+                #pragma unroll
+                for (int i = 0; i < MI; ++i) af[i] = A[(kk + tig) * kNnLdA + wm + i * 8 + g];
+                #pragma unroll
+                for (int j = 0; j < 2; ++j) bf[j] = B[(wn + j * 8 + g) * kNnLdB + kk + tig];
+                #pragma unroll
+                for (int i = 0; i < MI; ++i)
+                    #pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        dmma_8x8x4(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+            }
+        }
+        if (!live) continue;
+        #pragma unroll
+        for (int i = 0; i < MI; ++i) {
+            const int gm = m0 + i * 8 + g;
+            if (gm >= m_last) continue;
+            #pragma unroll
+            for (int j = 0; j < 2; ++j)
+                #pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int gn = n0 + wn + j * 8 + 2 * tig + h;
+                    if (gn >= d.N) continue;
+                    double v = d.alpha * acc[i][j][h];
+                    if (upd) v += d.beta * cold[i][j][h];
+                    d.C[(size_t)gn * d.ldc + gm] = v;
+                }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;");
+}
+
+__global__ void __launch_bounds__(kGemmThreads, 2)
+k_gemm_f64_nn_short(const __grid_constant__ GemmArgs args, int tiles_n, int iters)
+{
+    extern __shared__ __align__(16) double nn_smem[];
+    const GemmDesc d = gemm_desc(args, blockIdx.y);
+    const int m_first = blockIdx.x / tiles_n * iters * kNnRows;
+    const int n0 = blockIdx.x % tiles_n * 64;
+    if (m_first >= d.M || n0 >= d.N) return;
+    const int m_last = min(d.M, m_first + iters * kNnRows);
+    const int cols = min(64, d.N - n0);
+    if (cols <= 16) nn_short<1>(d, m_first, m_last, n0, nn_smem);
+    else if (cols <= 32) nn_short<2>(d, m_first, m_last, n0, nn_smem);
+    else nn_short<4>(d, m_first, m_last, n0, nn_smem);
+}
+
 template <int BM, int BN>
 static void launch_shape(bool ta, bool tb, const GemmArgs &args, int nb,
                          int tiles_m, int tiles_n, cudaStream_t stream)
@@ -675,6 +835,23 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int batch,
     // has a basis much narrower than the batch maximum as its rows, the
     // fitted 64 x 128 kernel; 128 x 32 for narrow outputs (sketch blocks of
     // 32 columns)
+    const bool sketch = args.step == STEP_SKETCH || args.step == STEP_A_SKETCH;
+    if (!ta && !tb && !sketch) {
+        // four row blocks to a CTA where that still leaves two rounds of
+        // CTAs, else one
+        const int tiles_n = (max_n + 63) / 64;
+        const int blocks = (max_m + kNnRows - 1) / kNnRows;
+        const int iters = (size_t)((blocks + 3) / 4) * tiles_n * batch >= 592 ? 4 : 1;
+        constexpr size_t smem = (size_t)kNnStages * kNnStage * sizeof(double);
+        static std::once_flag attr;
+        std::call_once(attr, [] {
+            cudaFuncSetAttribute(k_gemm_f64_nn_short,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        });
+        k_gemm_f64_nn_short<<<dim3((blocks + iters - 1) / iters * tiles_n, batch),
+                              kGemmThreads, smem, stream>>>(args, tiles_n, iters);
+        return cudaGetLastError();
+    }
     const bool wide = ta && !tb && !split_k && max_n >= 256;
     const int bm = !wide && !split_k && max_n <= 32 && max_m >= 128 ? 128 : 64;
     const int bn = wide ? kWideN : bm == 128 ? 32 : 64;
@@ -684,32 +861,28 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int batch,
         // (a batch has at most a few thousand tiles: one launch)
         const int nb = batch;
         dim3 grid(tiles_m * tiles_n, nb);
-        if (ta && !tb && bm == 64) {
-            constexpr size_t smem = (size_t)kTnStages * 128 * kGemmLds * sizeof(double);
-            constexpr size_t smem_wide =
-                (size_t)kTnStages * (kWideM + kWideN) * kGemmLds * sizeof(double);
+        const bool deep = (size_t)grid.x * nb <= kDeepGrid;
+        if (wide) {
+            constexpr size_t smem =
+                (size_t)kShallow * (kWideM + kWideN) * kGemmLds * sizeof(double);
             static std::once_flag attr;
             std::call_once(attr, [] {
-                cudaFuncSetAttribute(k_gemm_f64_tn_pipe,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem);
                 cudaFuncSetAttribute(k_gemm_f64_tn_wide,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_wide);
-            });
-            if (wide)
-                k_gemm_f64_tn_wide<<<grid, kGemmThreads, smem_wide, stream>>>(args, tiles_n);
-            else
-                k_gemm_f64_tn_pipe<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n, split_k ? 1 : 0);
-        } else if (!ta && tb && bm == 64) {
-            constexpr size_t smem = (size_t)kTnStages * 2 * kGemmBK * kNtLds * sizeof(double);
-            static std::once_flag attr_nt;
-            std::call_once(attr_nt, [] {
-                cudaFuncSetAttribute(k_gemm_f64_nt_pipe,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem);
             });
-            k_gemm_f64_nt_pipe<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n, split_k ? 1 : 0);
+            k_gemm_f64_tn_wide<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n);
+        } else if (ta != tb && bm == 64) {
+            auto go = [&](auto fn, int stages, size_t stage_doubles) {
+                const size_t smem = stages * stage_doubles * sizeof(double);
+                cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem);
+                fn<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n, split_k ? 1 : 0);
+            };
+            if (ta && deep) go(k_gemm_f64_tn_pipe<kDeep>, kDeep, 128 * kGemmLds);
+            else if (ta) go(k_gemm_f64_tn_pipe<kShallow>, kShallow, 128 * kGemmLds);
+            else if (deep) go(k_gemm_f64_nt_pipe<kDeep>, kDeep, 2 * kGemmBK * kNtLds);
+            else go(k_gemm_f64_nt_pipe<kShallow>, kShallow, 2 * kGemmBK * kNtLds);
         } else if (bm == 128) launch_shape<128, 32>(ta, tb, args, nb, tiles_m, tiles_n, stream);
         else launch_shape<64, 64>(ta, tb, args, nb, tiles_m, tiles_n, stream);
     }

@@ -16,6 +16,7 @@ struct GemmDesc {
     int M, N, K;
     int lda, ldb, ldc;
     double alpha, beta;
+    const int *gather;   // A B form: column k of A is column gather[k] (or null)
 };
 
 constexpr int kGemmBM = 64;

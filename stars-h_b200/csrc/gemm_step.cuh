@@ -18,6 +18,7 @@ __device__ __forceinline__ GemmDesc gemm_desc(const GemmArgs &a, int index)
     d.A = d.B = nullptr;
     d.C = nullptr;
     d.lda = d.ldb = d.ldc = 1;
+    d.gather = nullptr;
     const int ldm = ws.ldM(), ldk = ws.ldK();
     switch (a.step) {
     case STEP_SKETCH:
@@ -178,9 +179,9 @@ __device__ __forceinline__ GemmDesc gemm_desc(const GemmArgs &a, int index)
         d.C = ws.S(s); d.ldc = ldk;
         d.M = tw.bcur; d.N = tw.bcur; d.K = tw.m;
         break;
-    case STEP_A_Q1B:    // NN: R = Q1buf(gathered residual columns) T
+    case STEP_A_Q1B:    // NN: R = (pivot columns of the residual) T
         if (tw.kb <= 0) break;
-        d.A = ws.Q1(s); d.lda = ldm;
+        d.A = ws.Y(s); d.lda = ldm; d.gather = ws.Piv(s);
         d.B = ws.T(s); d.ldb = ldk;
         d.C = ws.R(s); d.ldc = ldm;
         d.M = tw.m; d.N = tw.kb; d.K = tw.kb;
