@@ -727,6 +727,27 @@ struct ProductPlan {
     }
 };
 
+// A far block's place in the plan (or its mirror's).
+struct PlanBlock {
+    const double *U, *V;
+    long long P, rho;      // first T row of its block row; its first phase-1 row
+    int m, n, r, kap, S;   // sizes, rank, place in the block row's S columns
+};
+
+// The block's r columns in both phases' lists.  The lists have one entry per
+// factor column (5e5 for 16384 blocks), which took the host 10 ms to fill;
+// it now prepares one record per block.
+__global__ void k_plan_columns(const PlanBlock *__restrict__ blocks,
+                               const double **vcol, RowT *rowt, const double **ucol)
+{
+    const PlanBlock b = blocks[blockIdx.x];
+    for (int c = threadIdx.x; c < b.r; c += blockDim.x) {
+        vcol[b.rho + c] = b.V + (size_t)c * b.n;
+        rowt[b.rho + c] = RowT{b.P, b.kap + c, b.S};
+        ucol[b.P + b.kap + c] = b.U + (size_t)c * b.m;
+    }
+}
+
 template <class T>
 static size_t put(std::vector<char> &buf, const std::vector<T> &v)
 {
@@ -766,34 +787,25 @@ static int build_plan(STARSH_blrm *M, const Record &rec, cudaStream_t s,
     }
     for (STARSH_int i = 0; i < nbr; ++i) P[i + 1] = P[i] + S[i];
     const long long trows = P[nbr];
-    std::vector<const double *> ucol(trows);
-    for (size_t p = 0; p < prods.size(); ++p) {
-        const Prod &q = prods[p];
-        for (int c = 0; c < q.r; ++c)
-            ucol[P[q.orow] + kap[p] + c] = q.U + (size_t)c * q.m;
-    }
     // phase 1: products grouped by input block, list order within a group
     std::vector<std::vector<int>> bycol(nbc);
     for (size_t p = 0; p < prods.size(); ++p) bycol[prods[p].icol].push_back((int)p);
-    std::vector<const double *> vcol;
-    std::vector<RowT> rowt;
+    // (the columns themselves are spread out on the device, k_plan_columns)
+    std::vector<PlanBlock> blocks(prods.size());
     std::vector<Job1> j1;
-    vcol.reserve(trows);
-    rowt.reserve(trows);
+    long long rho = 0;
     for (STARSH_int j = 0; j < nbc; ++j) {
         if (bycol[j].empty()) continue;
-        const int rho0 = (int)vcol.size();
+        const long long rho0 = rho;
         for (int p : bycol[j]) {
             const Prod &q = prods[p];
-            for (int c = 0; c < q.r; ++c) {
-                vcol.push_back(q.V + (size_t)c * q.n);
-                rowt.push_back(RowT{P[q.orow], kap[p] + c, S[q.orow]});
-            }
+            blocks[p] = PlanBlock{q.U, q.V, P[q.orow], rho, q.m, q.n, q.r, kap[p], S[q.orow]};
+            rho += q.r;
         }
-        const int cnt = (int)vcol.size() - rho0;
+        const int cnt = (int)(rho - rho0);
         const Prod &q0 = prods[bycol[j][0]];
         for (int r0 = 0; r0 < cnt; r0 += kPBM)
-            j1.push_back(Job1{rho0 + r0, std::min(kPBM, cnt - r0), q0.n, q0.in0});
+            j1.push_back(Job1{(int)rho0 + r0, std::min(kPBM, cnt - r0), q0.n, q0.in0});
     }
     // near pieces per output row, in near-block order
     // (stored blocks by their place after the first one, regenerated ones
@@ -827,12 +839,17 @@ static int build_plan(STARSH_blrm *M, const Record &rec, cudaStream_t s,
     }
     // one device allocation for every array
     std::vector<char> buf;
-    const size_t o_vcol = put(buf, vcol), o_rowt = put(buf, rowt),
-                 o_ucol = put(buf, ucol), o_j1 = put(buf, j1), o_j2 = put(buf, j2),
-                 o_near = put(buf, near);
+    const size_t o_j1 = put(buf, j1), o_j2 = put(buf, j2), o_near = put(buf, near),
+                 o_blk = put(buf, blocks);
+    // (behind the uploaded arrays: what the device fills)
+    auto round256 = [](size_t n) { return (n + 255) / 256 * 256; };
+    const size_t o_rowt = round256(buf.size());
+    const size_t o_vcol = o_rowt + round256(trows * sizeof(RowT));
+    const size_t o_ucol = o_vcol + round256(trows * sizeof(double *));
+    const size_t all = o_ucol + trows * sizeof(double *);
     auto *plan = new ProductPlan();
     if (!buf.empty()) {
-        char *d = (char *)pool_alloc(buf.size(), s);
+        char *d = (char *)pool_alloc(all, s);
         if (d == nullptr) {
             delete plan;
             return cuda_fail(cudaErrorMemoryAllocation, "product plan");
@@ -850,6 +867,11 @@ static int build_plan(STARSH_blrm *M, const Record &rec, cudaStream_t s,
         plan->j1 = (Job1 *)(d + o_j1);
         plan->j2 = (Job2 *)(d + o_j2);
         plan->near = (NearPiece *)(d + o_near);
+        if (!blocks.empty()) {
+            k_plan_columns<<<(unsigned)blocks.size(), 64, 0, s>>>(
+                (const PlanBlock *)(d + o_blk), plan->vcol, plan->rowt, plan->ucol);
+            count_launch();
+        }
         // products on any stream wait for the upload
         if (cudaEventCreateWithFlags(&plan->ready, cudaEventDisableTiming) !=
                 cudaSuccess ||

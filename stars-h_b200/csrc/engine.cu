@@ -808,9 +808,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         all.swap(a2);
         owner.swap(o2);
     }
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    size_t budget = std::min<size_t>(free_b / 2, (size_t)24 << 30);
+    size_t budget = (size_t)24 << 30;
     if (const char *e = getenv("STARSH_B200_WORKSPACE_MB"))
         budget = std::min<size_t>(budget, (size_t)atoll(e) << 20);
     budget = std::min(budget, ctx.workspace_cap);
@@ -850,26 +848,42 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     bool proj_i8 = false;
     if (const char *e = getenv("STARSH_B200_PROJ"))
         proj_i8 = use_i8 && ep.engine == STARSH_B200_MIXED && strcmp(e, "i8") == 0;
-    for (long long b0 = 0; b0 < ntot;) {
-        Workspace probe{};
-        int bm = all[b0].m, bn = all[b0].n, bk = all[b0].k;
-        size_t stride = workspace_layout(probe, bm, bn, bk, true, proj_i8);
-        long long cap = (long long)(budget / (stride * sizeof(double)));
-        cap = std::max<long long>(1, std::min<long long>({cap, ntot - b0, kMaxBatchTiles, part}));
-        for (long long q = b0; q < b0 + cap; ++q) {
-            bm = std::max(bm, all[q].m);
-            bn = std::max(bn, all[q].n);
-            bk = std::max(bk, all[q].k);
+    auto make_plan = [&](size_t budget) {
+        plan.clear();
+        ws_need = 0;
+        max_slots = 1;
+        for (long long b0 = 0; b0 < ntot;) {
+            Workspace probe{};
+            int bm = all[b0].m, bn = all[b0].n, bk = all[b0].k;
+            size_t stride = workspace_layout(probe, bm, bn, bk, true, proj_i8);
+            long long cap = (long long)(budget / (stride * sizeof(double)));
+            cap = std::max<long long>(1, std::min<long long>({cap, ntot - b0, kMaxBatchTiles, part}));
+            for (long long q = b0; q < b0 + cap; ++q) {
+                bm = std::max(bm, all[q].m);
+                bn = std::max(bn, all[q].n);
+                bk = std::max(bk, all[q].k);
+            }
+            // even leading dimension (16-byte column strides for the TMA)
+            bm = (bm + 7) / 8 * 8;
+            stride = workspace_layout(probe, bm, bn, bk, true, proj_i8);
+            long long fit = (long long)(budget / (stride * sizeof(double)));
+            const int nt = (int)std::max<long long>(1, std::min(cap, fit));
+            plan.push_back({b0, nt, bm, bn, bk, stride});
+            ws_need = std::max(ws_need, (size_t)nt * stride * sizeof(double));
+            max_slots = std::max<long long>(max_slots, nt);
+            b0 += nt;
         }
-        // even leading dimension (16-byte column strides for the TMA)
-        bm = (bm + 7) / 8 * 8;
-        stride = workspace_layout(probe, bm, bn, bk, true, proj_i8);
-        long long fit = (long long)(budget / (stride * sizeof(double)));
-        const int nt = (int)std::max<long long>(1, std::min(cap, fit));
-        plan.push_back({b0, nt, bm, bn, bk, stride});
-        ws_need = std::max(ws_need, (size_t)nt * stride * sizeof(double));
-        max_slots = std::max<long long>(max_slots, nt);
-        b0 += nt;
+    };
+    make_plan(budget);
+    // What the lanes already hold needs no look at the free memory (the
+    // driver's answer takes 0.1 ms and, on a busy host, tens of
+    // milliseconds); to grow, take at most half of it.
+    const size_t held = std::min(ctx.workspace.bytes,
+                                 helper ? helper->workspace.bytes : (size_t)-1);
+    if (ws_need > held) {
+        size_t free_b = 0, total_b = 0;
+        cudaMemGetInfo(&free_b, &total_b);
+        if (free_b / 2 / lanes < budget) make_plan(free_b / 2 / lanes);
     }
     // what the lanes' streams read was uploaded on this one
     cudaEvent_t ready = nullptr;
