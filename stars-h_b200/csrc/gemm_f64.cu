@@ -200,24 +200,25 @@ k_gemm_f64(const __grid_constant__ GemmArgs args, int tiles_n)
     }
 }
 
-// A^T B with 64 x 64 CTA tiles and a three-stage cp.async pipeline: the
-// transposed products (Grams and projections onto the basis in the rounds)
-// have outputs of a few tiles and K = the tile height, so one CTA walks a
-// long K; the register-staged kernel above keeps one K step in flight and
-// waits on memory latency every step.  Operand tiles land in shared memory
-// directly (16-byte cp.async, k contiguous in both operands), two steps
-// ahead of the multiply (60 KB of shared memory).  Where a tile fills every
-// warp's output region, the per-element accumulation order is that of
-// k_gemm_f64 (K steps of 16 in order, the DMMA's k-order inside a step), so
-// results are identical to it; in a launch that asks for it (split_k), a
-// tile with at most 32 rows or 48 columns of its own splits K over the
-// spare warps (fixed slice order, deterministic).
-// Stages of the pipelined kernels: three, or five where the launch has at
-// most two CTAs per SM, whose K steps (16 deep, 64 x 64) then wait on the
-// latency of the copies (16 tiles of 1024 rows: 0.5 us a step with three).
-constexpr int kShallow = 3, kDeep = 5;
-constexpr int kDeepGrid = 296;
-
+// A^T B with 64 x 64 CTA tiles and a cp.async pipeline: the transposed
+// products (Grams and projections onto the basis in the rounds) have outputs
+// of a few tiles and K = the tile height, so one CTA walks a long K; the
+// register-staged kernel above keeps one K step in flight and waits on
+// memory latency every step.  Operand tiles land in shared memory directly
+// (16-byte cp.async, k contiguous in both operands).  Where a tile fills
+// every warp's output region, the per-element accumulation order is that of
+// k_gemm_f64 (the DMMA's k order, k4 steps in order), so results are
+// identical to it; in a launch that asks for it (split_k), a tile with at
+// most 32 rows or 48 columns of its own splits K over the spare warps (fixed
+// slice order, deterministic).
+//
+// With few rows a step has little to multiply, and the instructions around
+// it bound the kernel (16 tiles of 1024 rows, 32 columns: 212 a warp and
+// step of 16, 0.7 us): a step is 32 deep, a warp walks its own k4 steps only,
+// and copies advance their pointers.
+constexpr int kShallow = 3;            // stages of the fitted 64 x 128 kernel
+constexpr int kPipeK = 32;
+constexpr int kPipeLds = kPipeK + 4;   // [row][k]: fragment reads free of conflicts
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool pred)
 {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
@@ -277,88 +278,149 @@ struct PipeRows {
     }
 };
 
+// Output regions of 32 x 16, one per warp when the tile's own rows and
+// columns fill the CTA tile.  A 64 x 64 tile with fewer (the products onto a
+// narrow basis, Grams of a few columns) gives the spare warps a share of K
+// instead: nreg regions (rounded up to rp, a power of two), warp w works on
+// region w % rp over the k4 steps q = w / rp modulo nsl = 8 / rp, and the nsl
+// partial sums are added in slice order through shared memory.  Every
+// scheduler keeps the same share of the DMMA work.
+struct PipeSplit {
+    int rh = 2, rp = 8, nsl = 1;
+    __device__ __forceinline__ PipeSplit(int rows, int cols, int split_k)
+    {
+        if (!split_k) return;
+        rh = rows > 32 ? 2 : 1;
+        const int nreg = rh * min(4, (cols + 15) / 16);
+        rp = nreg <= 1 ? 1 : nreg <= 2 ? 2 : nreg <= 4 ? 4 : 8;
+        nsl = 8 / rp;
+    }
+};
+
+// acc += the k4 step at offset k4 of a stage: fragments A(wm + 8 i + g, k4 +
+// tig), B(wn + 8 j + g, k4 + tig) at a + 8 i * ra, b + 8 j * rb.
+__device__ __forceinline__ void pipe_k4(double (&acc)[4][2][2], const double *a, int ra,
+                                        const double *b, int rb)
+{
+    double af[4], bf[2];
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) af[i] = a[i * 8 * ra];
+    #pragma unroll
+    for (int j = 0; j < 2; ++j) bf[j] = b[j * 8 * rb];
+    #pragma unroll
+    for (int i = 0; i < 4; ++i)
+        #pragma unroll
+        for (int j = 0; j < 2; ++j)
+            dmma_8x8x4(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+}
+
+// STAGES: three where the launch has at most one CTA per SM, else two (two
+// CTAs per SM).
 template <int STAGES>
 __global__ void __launch_bounds__(kGemmThreads)
 k_gemm_f64_tn_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split_k)
 {
-    constexpr int BM = 64, BN = 64, WARPS_M = BM / 32;
+    constexpr int BM = 64, BN = 64;
     const GemmDesc d = gemm_desc(args, blockIdx.y);
     const int tm = blockIdx.x / tiles_n, tn = blockIdx.x % tiles_n;
     const int m0 = tm * BM, n0 = tn * BN;
     if (m0 >= d.M || n0 >= d.N) return;
     extern __shared__ double gemm_smem[];
-    // [stage][64 rows][kGemmLds] for A^T, then the same for B^T
-    double *As = gemm_smem;
-    double *Bs = gemm_smem + STAGES * BM * kGemmLds;
+    // [stage][64 rows of A^T, 64 rows of B^T][kPipeLds]
+    constexpr int STAGE = (BM + BN) * kPipeLds;
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3;
-    // Output regions of 32 x 16, one per warp when the tile's own rows and
-    // columns fill the CTA tile.  A 64 x 64 tile with fewer (the products
-    // onto a narrow basis, Grams of a few columns) gives the spare warps a
-    // share of K instead: nreg regions (rounded up to rp, a power of two),
-    // warp w works on region w % rp over the k4 steps q = w / rp modulo
-    // nsl = 8 / rp, and the nsl partial sums are added in slice order
-    // through shared memory.  Every scheduler keeps the same share of the
-    // DMMA work.
-    int rh = WARPS_M, rp = 8, nsl = 1;
-    if (split_k) {
-        rh = d.M - m0 > 32 ? 2 : 1;
-        const int cq = min(4, (d.N - n0 + 15) / 16);
-        const int nreg = rh * cq;
-        rp = nreg <= 1 ? 1 : nreg <= 2 ? 2 : nreg <= 4 ? 4 : 8;
-        nsl = 8 / rp;
-    }
+    const PipeSplit sp(d.M - m0, d.N - n0, split_k);
+    const int rh = sp.rh, rp = sp.rp, nsl = sp.nsl;
     const int reg = warp % rp, slice = warp / rp;
     const int wm = (reg % rh) * 32, wn = (reg / rh) * 16;
     const bool live = wm < BM && wn < BN && m0 + wm < d.M && n0 + wn < d.N;
-    double acc[4][2][2];
+    double acc[4][2][2] = {};
+    // 16-byte pieces: rows t / 16 + 16 r of A and of B, k pair t % 16; rows
+    // outside the operand are zeroed in every stage and not copied
+    const int row = t >> 4, kk = (t & 15) * 2;
+    const double *pa[4], *pb[4];
+    bool oa[4], ob[4];
+    double *dst = gemm_smem + row * kPipeLds + kk;
     #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int r = 0; r < 4; ++r) {
+        const int ga = m0 + row + 16 * r, gb = n0 + row + 16 * r;
+        oa[r] = ga < d.M;
+        ob[r] = gb < d.N;
+        pa[r] = d.A + (size_t)(oa[r] ? ga : m0) * d.lda + kk;
+        pb[r] = d.B + (size_t)(ob[r] ? gb : n0) * d.ldb + kk;
         #pragma unroll
-        for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    // 16-byte pieces: rows t / 8 and t / 8 + 32 of A and of B, k pair t % 8
-    PipeRows<2, STAGES> ra, rb;
-    ra.init(d.A, d.lda, m0, d.M, As, BM, BM);
-    rb.init(d.B, d.ldb, n0, d.N, Bs, BN, BN);
-    auto issue = [&](int kt) {
-        const int st = kt % STAGES, k0 = kt * kGemmBK;
-        ra.copy(st * BM, k0, d.K);
-        rb.copy(st * BN, k0, d.K);
-        asm volatile("cp.async.commit_group;");
+        for (int s = 0; s < STAGES; ++s) {
+            double *z = dst + s * STAGE + 16 * r * kPipeLds;
+            if (!oa[r]) z[0] = z[1] = 0.0;
+            if (!ob[r]) z[BM * kPipeLds] = z[BM * kPipeLds + 1] = 0.0;
+        }
+    }
+    const bool even = (d.lda & 1) == 0 && ((uintptr_t)d.A & 15) == 0 &&
+                      (d.ldb & 1) == 0 && ((uintptr_t)d.B & 15) == 0;
+    int left = d.K - kk;                       // k indices from this thread's next pair
+    int ist = 0;                               // stage of the next copy
+    auto issue = [&]() {
+        double *q = dst + ist * STAGE;
+        if (even && left >= 2) {
+            #pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (oa[r]) cp_async16(q + 16 * r * kPipeLds, pa[r], true);
+                if (ob[r]) cp_async16(q + (BM + 16 * r) * kPipeLds, pb[r], true);
+            }
+        } else {
+            #pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                double *za = q + 16 * r * kPipeLds, *zb = za + BM * kPipeLds;
+                if (oa[r]) {
+                    za[0] = left >= 1 ? pa[r][0] : 0.0;
+                    za[1] = left >= 2 ? pa[r][1] : 0.0;
+                }
+                if (ob[r]) {
+                    zb[0] = left >= 1 ? pb[r][0] : 0.0;
+                    zb[1] = left >= 2 ? pb[r][1] : 0.0;
+                }
+            }
+        }
+        #pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            pa[r] += kPipeK;
+            pb[r] += kPipeK;
+        }
+        left -= kPipeK;
+        ist = ist + 1 == STAGES ? 0 : ist + 1;
     };
-    const int ktiles = (d.K + kGemmBK - 1) / kGemmBK;
+    const int ktiles = (d.K + kPipeK - 1) / kPipeK;
     #pragma unroll
     for (int p = 0; p < STAGES - 1; ++p) {
-        if (p < ktiles) issue(p);
-        else asm volatile("cp.async.commit_group;");
+        if (p < ktiles) issue();
+        asm volatile("cp.async.commit_group;");
     }
+    const double *fa = gemm_smem + (wm + g) * kPipeLds + tig;
+    const double *fb = gemm_smem + (BM + wn + g) * kPipeLds + tig;
+    int cst = 0;
     for (int kt = 0; kt < ktiles; ++kt) {
         // the group of step kt has landed (at most STAGES - 2 newer ones
         // still in flight)
         asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 2));
         __syncthreads();
-        if (kt + STAGES - 1 < ktiles) issue(kt + STAGES - 1);
-        else asm volatile("cp.async.commit_group;");
-        const int st = kt % STAGES;
-        const double *Ab = As + st * BM * kGemmLds;
-        const double *Bb = Bs + st * BN * kGemmLds;
-        #pragma unroll
-        for (int k4 = 0; k4 < kGemmBK / 4; ++k4) {
-            // this warp's k4 steps (warp-uniform)
-            if (!live || ((kt * (kGemmBK / 4) + k4 - slice) & (nsl - 1)) != 0) continue;
-            const int kk = k4 * 4;
-            double af[4], bf[2];
-            #pragma unroll
-            for (int i = 0; i < 4; ++i) af[i] = Ab[(wm + i * 8 + g) * kGemmLds + kk + tig];
-            #pragma unroll
-            for (int j = 0; j < 2; ++j) bf[j] = Bb[(wn + j * 8 + g) * kGemmLds + kk + tig];
-            #pragma unroll
-            for (int i = 0; i < 4; ++i)
+        if (kt + STAGES - 1 < ktiles) issue();
+        asm volatile("cp.async.commit_group;");
+        const double *a = fa + cst * STAGE, *b = fb + cst * STAGE;
+        if (live) {
+            if (nsl == 1) {
                 #pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    dmma_8x8x4(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+                for (int k4 = 0; k4 < kPipeK / 4; ++k4)
+                    pipe_k4(acc, a + 4 * k4, kPipeLds, b + 4 * k4, kPipeLds);
+            } else {
+                // this warp's k4 steps (8 per step, a multiple of nsl)
+                #pragma unroll 1
+                for (int k4 = slice; k4 < kPipeK / 4; k4 += nsl)
+                    pipe_k4(acc, a + 4 * k4, kPipeLds, b + 4 * k4, kPipeLds);
+            }
         }
+        cst = cst + 1 == STAGES ? 0 : cst + 1;
     }
     asm volatile("cp.async.wait_group 0;");
     if (nsl > 1) {
@@ -497,8 +559,7 @@ k_gemm_f64_tn_wide(const __grid_constant__ GemmArgs args, int tiles_n)
 }
 
 // A B^T with 64 x 64 CTA tiles (the Gram B B^T of the small SVD, K = the
-// tile width) through the same three-stage cp.async pipeline as the
-// transposed products.  Here rows are contiguous in both operands and k is
+// tile width) through the same cp.async pipeline as the transposed products.  Here rows are contiguous in both operands and k is
 // strided, so the tiles are staged as [k][row] (row stride 68 doubles:
 // fragment reads free of bank conflicts); a 16-byte piece is two
 // consecutive rows at one k.  Without split_k the per-element accumulation
@@ -517,98 +578,89 @@ k_gemm_f64_nt_pipe(const __grid_constant__ GemmArgs args, int tiles_n, int split
     const int m0 = tm * BM, n0 = tn * BN;
     if (m0 >= d.M || n0 >= d.N) return;
     extern __shared__ double gemm_smem[];
-    // [stage][16 k][kNtLds] for A, then the same for B
-    double *As = gemm_smem;
-    double *Bs = gemm_smem + STAGES * kGemmBK * kNtLds;
+    // [stage][32 k of A, 32 k of B][kNtLds]
+    constexpr int STAGE = 2 * kPipeK * kNtLds;
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3;
-    // output regions, K slices and 8-row fragments as in the transposed
-    // kernel above
-    int rh = 2, rp = 8, nsl = 1;
-    if (split_k) {
-        rh = d.M - m0 > 32 ? 2 : 1;
-        const int cq = min(4, (d.N - n0 + 15) / 16);
-        const int nreg = rh * cq;
-        rp = nreg <= 1 ? 1 : nreg <= 2 ? 2 : nreg <= 4 ? 4 : 8;
-        nsl = 8 / rp;
-    }
+    const PipeSplit sp(d.M - m0, d.N - n0, split_k);
+    const int rh = sp.rh, rp = sp.rp, nsl = sp.nsl;
     const int reg = warp % rp, slice = warp / rp;
     const int wm = (reg % rh) * 32, wn = (reg / rh) * 16;
     const bool live = wm < BM && wn < BN && m0 + wm < d.M && n0 + wn < d.N;
-    double acc[4][2][2];
-    #pragma unroll
-    for (int i = 0; i < 4; ++i)
-        #pragma unroll
-        for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    // 16-byte pieces: rows 2 (t % 32) and the next, k = t / 32 and + 8 of a
-    // K step, of A and of B.  Pointers and bounds are worked out once; rows
-    // outside the operand are zeroed in every stage and not copied.
+    double acc[4][2][2] = {};
+    // 16-byte pieces: rows 2 (t % 32) and the next, k = t / 32 + 8 r of a K
+    // step, of A and of B; rows outside the operand are zeroed in every
+    // stage and not copied
     const int row = (t & 31) * 2, kk = t >> 5;
-    auto rows_in = [&](int g0, int lim) { return max(0, min(2, lim - g0 - row)); };
-    const int na = rows_in(m0, d.M), nb = rows_in(n0, d.N);
-    const double *pa = d.A + (na ? m0 + row : 0) + (size_t)kk * d.lda;
-    const double *pb = d.B + (nb ? n0 + row : 0) + (size_t)kk * d.ldb;
-    const bool evenA = (d.lda & 1) == 0 && ((uintptr_t)d.A & 15) == 0;
-    const bool evenB = (d.ldb & 1) == 0 && ((uintptr_t)d.B & 15) == 0;
-    double *qa = As + kk * kNtLds + row, *qb = Bs + kk * kNtLds + row;
+    const int na = max(0, min(2, d.M - m0 - row)), nb = max(0, min(2, d.N - n0 - row));
+    const double *pa = d.A + m0 + (na ? row : 0) + (size_t)kk * d.lda;
+    const double *pb = d.B + n0 + (nb ? row : 0) + (size_t)kk * d.ldb;
+    const size_t sa = (size_t)8 * d.lda, sb = (size_t)8 * d.ldb;
+    double *dst = gemm_smem + kk * kNtLds + row;
+    #pragma unroll
     for (int s = 0; s < STAGES; ++s)
         #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int at = (s * kGemmBK + 8 * h) * kNtLds;
-            if (na < 2) qa[at + 1] = 0.0;
-            if (na < 1) qa[at] = 0.0;
-            if (nb < 2) qb[at + 1] = 0.0;
-            if (nb < 1) qb[at] = 0.0;
+        for (int r = 0; r < 4; ++r) {
+            double *z = dst + s * STAGE + 8 * r * kNtLds;
+            if (na < 2) z[1] = 0.0;
+            if (na < 1) z[0] = 0.0;
+            if (nb < 2) z[kPipeK * kNtLds + 1] = 0.0;
+            if (nb < 1) z[kPipeK * kNtLds] = 0.0;
         }
-    auto piece = [&](double *dst, const double *src, int n, bool even, bool in) {
-        if (n == 2 && even && in) {
-            cp_async16(dst, src, true);
-        } else {
-            if (n > 0) dst[0] = in ? src[0] : 0.0;
-            if (n > 1) dst[1] = in ? src[1] : 0.0;
-        }
-    };
-    auto issue = [&](int kt) {
-        const int st = kt % STAGES, k0 = kt * kGemmBK;
+    const bool even = (d.lda & 1) == 0 && ((uintptr_t)d.A & 15) == 0 &&
+                      (d.ldb & 1) == 0 && ((uintptr_t)d.B & 15) == 0;
+    const bool whole = even && na != 1 && nb != 1;
+    int left = d.K - kk;
+    int ist = 0;
+    auto issue = [&]() {
+        double *q = dst + ist * STAGE;
         #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const bool in = k0 + kk + 8 * h < d.K;
-            const int at = (st * kGemmBK + 8 * h) * kNtLds;
-            piece(qa + at, pa + (size_t)(k0 + 8 * h) * d.lda, na, evenA, in);
-            piece(qb + at, pb + (size_t)(k0 + 8 * h) * d.ldb, nb, evenB, in);
+        for (int r = 0; r < 4; ++r) {
+            double *za = q + 8 * r * kNtLds, *zb = za + kPipeK * kNtLds;
+            const bool in = left > 8 * r;
+            if (whole && in) {
+                if (na) cp_async16(za, pa, true);
+                if (nb) cp_async16(zb, pb, true);
+            } else {
+                if (na > 0) za[0] = in ? pa[0] : 0.0;
+                if (na > 1) za[1] = in ? pa[1] : 0.0;
+                if (nb > 0) zb[0] = in ? pb[0] : 0.0;
+                if (nb > 1) zb[1] = in ? pb[1] : 0.0;
+            }
+            pa += sa;
+            pb += sb;
         }
-        asm volatile("cp.async.commit_group;");
+        left -= kPipeK;
+        ist = ist + 1 == STAGES ? 0 : ist + 1;
     };
-    const int ktiles = (d.K + kGemmBK - 1) / kGemmBK;
+    const int ktiles = (d.K + kPipeK - 1) / kPipeK;
     #pragma unroll
     for (int p = 0; p < STAGES - 1; ++p) {
-        if (p < ktiles) issue(p);
-        else asm volatile("cp.async.commit_group;");
+        if (p < ktiles) issue();
+        asm volatile("cp.async.commit_group;");
     }
+    const double *fa = gemm_smem + tig * kNtLds + wm + g;
+    const double *fb = gemm_smem + (kPipeK + tig) * kNtLds + wn + g;
+    int cst = 0;
     for (int kt = 0; kt < ktiles; ++kt) {
         asm volatile("cp.async.wait_group %0;" :: "n"(STAGES - 2));
         __syncthreads();
-        if (kt + STAGES - 1 < ktiles) issue(kt + STAGES - 1);
-        else asm volatile("cp.async.commit_group;");
-        const int st = kt % STAGES;
-        const double *Ab = As + st * kGemmBK * kNtLds;
-        const double *Bb = Bs + st * kGemmBK * kNtLds;
-        #pragma unroll
-        for (int k4 = 0; k4 < kGemmBK / 4; ++k4) {
-            if (!live || ((kt * (kGemmBK / 4) + k4 - slice) & (nsl - 1)) != 0) continue;
-            const int kk = k4 * 4;
-            double af[4], bf[2];
-            #pragma unroll
-            for (int i = 0; i < 4; ++i) af[i] = Ab[(kk + tig) * kNtLds + wm + i * 8 + g];
-            #pragma unroll
-            for (int j = 0; j < 2; ++j) bf[j] = Bb[(kk + tig) * kNtLds + wn + j * 8 + g];
-            #pragma unroll
-            for (int i = 0; i < 4; ++i)
+        if (kt + STAGES - 1 < ktiles) issue();
+        asm volatile("cp.async.commit_group;");
+        const double *a = fa + cst * STAGE, *b = fb + cst * STAGE;
+        if (live) {
+            if (nsl == 1) {
                 #pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    dmma_8x8x4(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+                for (int k4 = 0; k4 < kPipeK / 4; ++k4)
+                    pipe_k4(acc, a + 4 * k4 * kNtLds, 1, b + 4 * k4 * kNtLds, 1);
+            } else {
+                #pragma unroll 1
+                for (int k4 = slice; k4 < kPipeK / 4; k4 += nsl)
+                    pipe_k4(acc, a + 4 * k4 * kNtLds, 1, b + 4 * k4 * kNtLds, 1);
+            }
         }
+        cst = cst + 1 == STAGES ? 0 : cst + 1;
     }
     asm volatile("cp.async.wait_group 0;");
     if (nsl > 1) {
@@ -861,7 +913,7 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int batch,
         // (a batch has at most a few thousand tiles: one launch)
         const int nb = batch;
         dim3 grid(tiles_m * tiles_n, nb);
-        const bool deep = (size_t)grid.x * nb <= kDeepGrid;
+        const bool alone = (size_t)grid.x * nb <= 148;
         if (wide) {
             constexpr size_t smem =
                 (size_t)kShallow * (kWideM + kWideN) * kGemmLds * sizeof(double);
@@ -879,10 +931,11 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int batch,
                                      (int)smem);
                 fn<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n, split_k ? 1 : 0);
             };
-            if (ta && deep) go(k_gemm_f64_tn_pipe<kDeep>, kDeep, 128 * kGemmLds);
-            else if (ta) go(k_gemm_f64_tn_pipe<kShallow>, kShallow, 128 * kGemmLds);
-            else if (deep) go(k_gemm_f64_nt_pipe<kDeep>, kDeep, 2 * kGemmBK * kNtLds);
-            else go(k_gemm_f64_nt_pipe<kShallow>, kShallow, 2 * kGemmBK * kNtLds);
+            constexpr size_t tn = 128 * kPipeLds, nt = 2 * kPipeK * kNtLds;
+            if (ta && alone) go(k_gemm_f64_tn_pipe<3>, 3, tn);
+            else if (ta) go(k_gemm_f64_tn_pipe<2>, 2, tn);
+            else if (alone) go(k_gemm_f64_nt_pipe<3>, 3, nt);
+            else go(k_gemm_f64_nt_pipe<2>, 2, nt);
         } else if (bm == 128) launch_shape<128, 32>(ta, tb, args, nb, tiles_m, tiles_n, stream);
         else launch_shape<64, 64>(ta, tb, args, nb, tiles_m, tiles_n, stream);
     }
