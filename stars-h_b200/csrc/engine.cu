@@ -1023,7 +1023,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             }
             if (!launch_gen_sketch_i8(d_kernels, dt, nt, ws, om8, ld_om8,
                                       k_max_all, bmax0, s) ||
-                !launch_sketch_i8(dt, nt, ws, om8, ld_om8, k_max_all, bmax0, s,
+                !launch_sketch_i8(dt, nt, nt, nullptr, ws, om8, ld_om8, k_max_all, bmax0, s,
                                   TILE_RESKETCH | TILE_GEN_SEPARATE)) {
                 set_error("no TMA tensor map for the fused sketch");
                 info = STARSH_UNKNOWN_ERROR;
@@ -1144,7 +1144,8 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             } else if (use_i8) {
                 // every batch has an even leading dimension (plan), so the
                 // tensor map exists unless the driver lacks the entry point
-                if (!launch_sketch_i8(dt, nt, ws, om8, ld_om8, k_max_all, bmax, s)) {
+                if (!launch_sketch_i8(dt, nt, rcount(), ract(), ws, om8, ld_om8, k_max_all,
+                                      bmax, s)) {
                     set_error("no TMA tensor map for the sketch");
                     info = STARSH_UNKNOWN_ERROR;
                     break;
@@ -1326,8 +1327,6 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             OutArena out{base, base};
             upload_tiles(b0, nt, 1);
             cudaEventRecord(ev[7], s);
-            launch_select_w(dt, nt, ws, s);
-            count_launch();
             if ((info = gemm(STEP_OUT_U, false, false, nt, m_max, r_max, out))) break;
             launch_write_v(dt, nt, ws, out, s);
             count_launch();

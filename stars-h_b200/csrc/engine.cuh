@@ -118,7 +118,7 @@ enum GemmStep : int {
     STEP_PROJECT,        // B  = Q^T D                    (k1 x n)
     STEP_GRAM_B,         // S  = B B^T                    (k1 x k1)
     STEP_ROTATE,         // C  = W^T B   (W in T)         (k2 x n)
-    STEP_OUT_U,          // U  = Q Wsel  (Wsel in L)      (m x r)
+    STEP_OUT_U,          // U  = Q W[:, ord]  (W in T)    (m x r)
     STEP_A_SKETCH,       // Y  = D Omega[:, c:c+b]        (m x b)    adaptive
     STEP_A_RES_Z,        // S  = Q^T Y                    (k1 x b)   adaptive
     STEP_A_RES_Y,        // Y -= Q S                      (m x b)    adaptive
@@ -225,8 +225,6 @@ void launch_round_end(TileWork *d_tiles, int ntiles, int verify,
 void launch_round_pivchol(TileWork *d_tiles, int ntiles, Workspace ws,
                           int repeat, int bmax, cudaStream_t stream,
                           const int *act = nullptr);
-void launch_select_w(const TileWork *d_tiles, int ntiles, Workspace ws,
-                     cudaStream_t stream);
 // Tensor-core projection B = Q^T D (proj_i8.cu) of the tiles with at most
 // 64 basis columns and 4096 rows: the preparation flags them
 // TILE_PROJ_I8 (the FP64 projection step skips them).  launch_proj_i8
@@ -245,9 +243,12 @@ void launch_write_v(const TileWork *d_tiles, int ntiles, Workspace ws,
 bool sketch_i8_fits(int ncols, int n_max);
 // Returns false (nothing launched) when the batch's layout cannot be
 // described to the TMA unit (odd leading dimension).
-bool launch_sketch_i8(const TileWork *d_tiles, int ntiles, Workspace ws,
-                      const int8_t *om8, int ld_om8, int om8_cols, int ncols,
-                      cudaStream_t stream, int need = 0);
+// `count` tiles: those listed in act (a round's sampling tiles), or the
+// first ones of the batch's ntiles.
+bool launch_sketch_i8(const TileWork *d_tiles, int ntiles, int count,
+                      const int *act, Workspace ws, const int8_t *om8,
+                      int ld_om8, int om8_cols, int ncols, cudaStream_t stream,
+                      int need = 0);
 // First sampling round with the generation fused in (gen_sketch_i8.cu):
 // D, its exact norms and row maxima, and Y(:, 0:bcur) = D Omega8(:, 0:nc)
 // with bound-based row scales; tiles whose bound missed are flagged

@@ -761,8 +761,9 @@ __device__ __forceinline__ void nn_short(const GemmDesc &d, int m_first, int m_l
             if (n0 + n >= (d.N + 15) / 16 * 16) break;
             double *dst = B + n * kNnLdB + bk;
             const int k = k0 + bk;
-            const double *src = d.B + (size_t)(n0 + n) * d.ldb + k;
             const bool in = n0 + n < d.N;
+            const double *src = d.B + k +
+                (size_t)(in && d.gather_b ? d.gather_b[n0 + n] : n0 + n) * d.ldb;
             if (in && evenB && k + 1 < d.K) {
                 cp_async16(dst, src, true);
             } else {

@@ -16,7 +16,9 @@ struct GemmDesc {
     int M, N, K;
     int lda, ldb, ldc;
     double alpha, beta;
-    const int *gather;   // A B form: column k of A is column gather[k] (or null)
+    // A B form: column k of A is column gather[k], column n of B column
+    // gather_b[n] (or null)
+    const int *gather, *gather_b;
 };
 
 constexpr int kGemmBM = 64;

@@ -18,7 +18,7 @@ __device__ __forceinline__ GemmDesc gemm_desc(const GemmArgs &a, int index)
     d.A = d.B = nullptr;
     d.C = nullptr;
     d.lda = d.ldb = d.ldc = 1;
-    d.gather = nullptr;
+    d.gather = d.gather_b = nullptr;
     const int ldm = ws.ldM(), ldk = ws.ldK();
     switch (a.step) {
     case STEP_SKETCH:
@@ -215,10 +215,10 @@ __device__ __forceinline__ GemmDesc gemm_desc(const GemmArgs &a, int index)
         d.C = ws.Q(s) + (size_t)tw.k1 * ldm; d.ldc = ldm;
         d.M = tw.m; d.N = tw.kb; d.K = tw.kb;
         break;
-    case STEP_OUT_U:    // NN: U = Q Wsel, Wsel in L
+    case STEP_OUT_U:    // NN: U = Q W(:, ord), W in T
         if (tw.rank <= 0) break;
         d.A = ws.Q(s); d.lda = ldm;
-        d.B = ws.L(s); d.ldb = ldk;
+        d.B = ws.T(s); d.ldb = ldk; d.gather_b = ws.Ord(s);
         d.C = a.out.U + tw.off_u; d.ldc = tw.m;
         d.M = tw.m; d.N = tw.rank; d.K = tw.k1;
         break;

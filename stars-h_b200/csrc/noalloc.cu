@@ -187,7 +187,6 @@ extern "C" int starsh_b200_dense_rsvd_noalloc(const double *dD, int nrows,
     launch_rank_cut(dt, 1, ws, s);
     // One tile: its factors start at offset 0 of the caller's buffers, so
     // the output kernels run without a host round trip (rank <= 0 skips).
-    launch_select_w(dt, 1, ws, s);
     if ((info = gemm(STEP_OUT_U, false, false, m, k, out))) return info;
     launch_write_v(dt, 1, ws, out, s);
     B200_CUDA(cudaMemcpyAsync(d_rank, &dt->rank, sizeof(int),

@@ -2427,7 +2427,13 @@ void launch_merge_basis(TileWork *d_tiles, int ntiles, cudaStream_t stream)
 // i.e. starsh_dense_dsvfr applied to the exact energies plus the energy the
 // Gram factor (tail_h) and the sketch (outside) left out (0 if D = 0).
 // rank = r if r <= maxrank, else -1.
-__global__ void __launch_bounds__(kSmallThreads)
+// A row's energy is the sum of 32 strided partial sums (columns l, l + 32,
+// ... each, then a tree over l); warp l takes the partial sums l of 32 rows
+// at a time, so that its loads run along C's columns (a warp per row read a
+// 32-byte sector for every 8 bytes: 81 tiles 60 us).
+constexpr int kRankThreads = 1024;
+
+__global__ void __launch_bounds__(kRankThreads)
 k_rank_cut(TileWork *__restrict__ tiles, Workspace ws)
 {
     TileWork &tw = tiles[blockIdx.x];
@@ -2437,20 +2443,34 @@ k_rank_cut(TileWork *__restrict__ tiles, Workspace ws)
     const int maxrank = tw.maxrank;
     __shared__ double e[kMaxK];
     __shared__ int ord[kMaxK];
+    __shared__ double part[32][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double *C = ws.C(s);
     const int ld = ws.ldK();
-    for (int c = warp; c < k2; c += blockDim.x >> 5) {
+    for (int c0 = 0; c0 < k2; c0 += 32) {
+        const int c = c0 + lane;
         double acc = 0.0;
-        for (int j = lane; j < tw.n; j += 32) {
-            const double v = C[(size_t)j * ld + c];
-            acc += v * v;
+        if (c < k2) {
+            const double *p = C + (size_t)warp * ld + c;
+            int j = warp;
+            for (; j + 96 < tw.n; j += 128, p += (size_t)128 * ld) {
+                double v[4];
+                #pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = p[(size_t)32 * u * ld];
+                #pragma unroll
+                for (int u = 0; u < 4; ++u) acc += v[u] * v[u];
+            }
+            for (; j < tw.n; j += 32, p += (size_t)32 * ld) acc += *p * *p;
         }
+        part[warp][lane] = acc;
+        __syncthreads();
+        // warp w: row c0 + w, lane l its partial sum l
+        double x = part[lane][warp];
         #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) e[c] = acc;
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0 && c0 + warp < k2) e[c0 + warp] = x;
+        __syncthreads();
     }
-    __syncthreads();
     // Position of c = number of entries ranked before it.
     for (int c = threadIdx.x; c < k2; c += blockDim.x) {
         int pos = 0;
@@ -2460,15 +2480,13 @@ k_rank_cut(TileWork *__restrict__ tiles, Workspace ws)
         ord[pos] = c;
     }
     __syncthreads();
+    int *gord = ws.Ord(s);
+    double *ge = ws.E(s);
+    for (int c = threadIdx.x; c < k2; c += blockDim.x) {
+        gord[c] = ord[c];
+        ge[c] = e[ord[c]];
+    }
     if (threadIdx.x == 0) {
-        int *gord = ws.Ord(s);
-        double *ge = ws.E(s);
-        double total = 0.0;
-        for (int c = 0; c < k2; ++c) {
-            gord[c] = ord[c];
-            ge[c] = e[ord[c]];
-            total += e[c];
-        }
         // With the block's exact ||D||_F^2 (dnorm2, from the generator) the
         // energy outside the sketched basis, ||D||^2 - ||B||^2, is known
         // too: it joins the tail, less an allowance for the rounding of the
@@ -2494,7 +2512,7 @@ k_rank_cut(TileWork *__restrict__ tiles, Workspace ws)
             r = -1;
             if (tail <= budget) r = k2;
             for (int c = k2 - 1; c >= 1; --c) {
-                tail += ge[c];
+                tail += e[ord[c]];
                 if (tail <= budget) r = c;
                 else break;
             }
@@ -2507,57 +2525,45 @@ k_rank_cut(TileWork *__restrict__ tiles, Workspace ws)
 void launch_rank_cut(TileWork *d_tiles, int ntiles, Workspace ws,
                      cudaStream_t stream)
 {
-    k_rank_cut<<<ntiles, kSmallThreads, 0, stream>>>(d_tiles, ws);
-}
-
-// Wsel(:, c) = W(:, ord[c]) for c < rank, into L(slot).
-__global__ void k_select_w(const TileWork *__restrict__ tiles, Workspace ws)
-{
-    const TileWork tw = tiles[blockIdx.x];
-    if (tw.rank <= 0) return;
-    const int s = tw.slot, ld = ws.ldK();
-    const int *ord = ws.Ord(s);
-    const double *W = ws.T(s);
-    double *dst = ws.L(s);
-    for (int c = 0; c < tw.rank; ++c)
-        for (int i = threadIdx.x; i < tw.k1; i += blockDim.x)
-            dst[(size_t)c * ld + i] = W[(size_t)ord[c] * ld + i];
-}
-
-void launch_select_w(const TileWork *d_tiles, int ntiles, Workspace ws,
-                     cudaStream_t stream)
-{
-    k_select_w<<<ntiles, 256, 0, stream>>>(d_tiles, ws);
+    k_rank_cut<<<ntiles, kRankThreads, 0, stream>>>(d_tiles, ws);
 }
 
 // V(j, c) = C(ord[c], j): V is n x rank, leading dimension n.  A CTA
-// transposes `cols` (8, 16 or 32) columns j of C at a time through shared
-// memory: it reads the k2 rows of those columns (contiguous in C) and
-// writes the rank selected rows as `cols` consecutive entries of each
-// column of V, so both sides are coalesced.
+// transposes `cols` columns j of C at a time through shared memory: it reads
+// their k2 rows (contiguous in C; every lane busy whatever k2) and writes
+// the rank selected rows as consecutive entries of each column of V, so both
+// sides are coalesced.  As many columns a pass as its shared memory holds
+// (a multiple of 8), so that a pass has some 4000 loads in flight: with a
+// warp per column and 32 columns a pass the N = 102400 square exponential
+// spent 2.6 ms here for 1.2 GB.
+constexpr int kWriteVDoubles = 5376;    // 42 KB
+
 __global__ void __launch_bounds__(256)
 k_write_v(const TileWork *__restrict__ tiles, Workspace ws, OutArena out,
-          int cols)
+          int doubles)
 {
-    extern __shared__ double wv_sm[];   // [cols][k2 + 1]
+    extern __shared__ double wv_sm[];   // [cols][k2 | 1]
     const TileWork tw = tiles[blockIdx.x];
     if (tw.rank <= 0) return;
     const int s = tw.slot, ld = ws.ldK();
     const int *ord = ws.Ord(s);
     const double *C = ws.C(s);
     double *V = out.V + tw.off_v;
-    const int kr = tw.k2, ls = kr + 1;   // rows of C; ord[c] < k2
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int kr = tw.k2, ls = kr | 1;   // rows of C; ord[c] < k2
+    const int cols = max(8, min(256, doubles / ls / 8 * 8));
+    const int t = threadIdx.x;
     for (int j0 = blockIdx.y * cols; j0 < tw.n; j0 += gridDim.y * cols) {
         const int nj = min(cols, tw.n - j0);
-        // warp w reads columns j0 + w, j0 + w + 8, ...: k2 contiguous rows
-        for (int jj = warp; jj < nj; jj += 8)
-            for (int i = lane; i < kr; i += 32)
-                wv_sm[jj * ls + i] = C[(size_t)(j0 + jj) * ld + i];
+        const double *Cj = C + (size_t)j0 * ld;
+        #pragma unroll 8
+        for (int q = t; q < nj * kr; q += 256) {
+            const int jj = q / kr, i = q - jj * kr;
+            wv_sm[jj * ls + i] = Cj[(size_t)jj * ld + i];
+        }
         __syncthreads();
-        for (int c = warp; c < tw.rank; c += 8) {
-            const int row = ord[c];
-            if (lane < nj) V[(size_t)c * tw.n + j0 + lane] = wv_sm[lane * ls + row];
+        for (int q = t; q < nj * tw.rank; q += 256) {
+            const int c = q / nj, jj = q - c * nj;
+            V[(size_t)c * tw.n + j0 + jj] = wv_sm[jj * ls + ord[c]];
         }
         __syncthreads();
     }
@@ -2566,16 +2572,14 @@ k_write_v(const TileWork *__restrict__ tiles, Workspace ws, OutArena out,
 void launch_write_v(const TileWork *d_tiles, int ntiles, Workspace ws,
                     OutArena out, cudaStream_t stream)
 {
-    // 32 columns per pass while the tile fits 96 KB, fewer for wide bases
-    int cols = 32;
-    while (cols > 8 && (size_t)cols * (ws.k_max + 1) * sizeof(double) > 96 * 1024)
-        cols /= 2;
-    const size_t smem = (size_t)cols * (ws.k_max + 1) * sizeof(double);
+    // wide bases: at least 8 columns a pass
+    const int doubles = std::max(kWriteVDoubles, 8 * (ws.k_max | 1));
+    const size_t smem = (size_t)doubles * sizeof(double);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(k_write_v, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
-    dim3 grid(ntiles, 8);
-    k_write_v<<<grid, 256, smem, stream>>>(d_tiles, ws, out, cols);
+    dim3 grid(ntiles, ntiles >= 148 ? 4 : 8);
+    k_write_v<<<grid, 256, smem, stream>>>(d_tiles, ws, out, doubles);
 }
 
 }  // namespace b200

@@ -163,8 +163,8 @@ __device__ __forceinline__ bool sk_active(const SkItem &w, int need)
 __global__ void __launch_bounds__(kSkThreads, 1)
 k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
             const __grid_constant__ CUtensorMap omap,
-            const TileWork *__restrict__ tiles, int ntiles, Workspace ws,
-            int nc, int need)
+            const TileWork *__restrict__ tiles, int ntiles,
+            const int *__restrict__ act, Workspace ws, int nc, int need)
 {
     extern __shared__ __align__(1024) uint8_t sk_smem_raw[];
     __shared__ __align__(8) uint64_t full[kStages];    // chunk landed
@@ -187,6 +187,10 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int rpt = (ws.m_max + kSkRows - 1) / kSkRows;
     const long long nitems = (long long)ntiles * rpt;
+    // the batch's tile of a work item (the round's sampling tiles, if listed)
+    auto tile_of = [&](long long item) {
+        return act ? act[item / rpt] : (int)(item / rpt);
+    };
     const uint32_t ncols_alloc = nc * kSlices <= 128 ? 128
                                : nc * kSlices <= 256 ? 256 : 512;
 
@@ -224,12 +228,11 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
         // ---------------------------------------------------- converters
         const int r = t & (kSkRows - 1), qd = t >> 7;
         const double magic = 0x1.8p52;
-        SkItem wn = sk_item(tiles, (int)(blockIdx.x / rpt));
+        SkItem wn = sk_item(tiles, tile_of(blockIdx.x));
         for (long long item = blockIdx.x; item < nitems; item += gridDim.x) {
-            const int tile = (int)(item / rpt);
             const SkItem w = wn;
             if (item + gridDim.x < nitems)   // the next item's fields, early
-                wn = sk_item(tiles, (int)((item + gridDim.x) / rpt));
+                wn = sk_item(tiles, tile_of(item + gridDim.x));
             const int row0 = (int)(item % rpt) * kSkRows;
             if (!sk_active(w, need) || row0 >= w.m) continue;
             const int nchunks = (w.n + kSkChunk - 1) / kSkChunk;
@@ -239,7 +242,7 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
             // __syncwarp)
             const bool eok = mbar_wait_or(&expready[it & 1], (uint32_t)(it >> 1) & 1, &failed);
             if (!__all_sync(0xffffffffu, eok ? 1 : 0)) {
-                fail_tile = tile;
+                fail_tile = tile_of(item);
                 failed = 1;
                 break;
             }
@@ -254,7 +257,7 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                 ok = ok && (gc < kAbufs ||
                             mbar_wait_or(&afree[b], (uint32_t)((gc >> 1) - 1) & 1, &failed));
                 if (!__all_sync(0xffffffffu, ok ? 1 : 0)) {
-                    fail_tile = tile;
+                    fail_tile = tile_of(item);
                     failed = 1;
                     break;
                 }
@@ -290,13 +293,12 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
         long long issued = 0;
         if (lane == 0) {
             const uint32_t bytes = kDStageBytes + 2 * 16 * nc;
-            SkItem wn = sk_item(tiles, (int)(blockIdx.x / rpt));
+            SkItem wn = sk_item(tiles, tile_of(blockIdx.x));
             for (long long item = blockIdx.x; item < nitems && !failed;
                  item += gridDim.x) {
-                const int tile = (int)(item / rpt);
                 const SkItem w = wn;
                 if (item + gridDim.x < nitems)
-                    wn = sk_item(tiles, (int)((item + gridDim.x) / rpt));
+                    wn = sk_item(tiles, tile_of(item + gridDim.x));
                 const int row0 = (int)(item % rpt) * kSkRows;
                 if (!sk_active(w, need) || row0 >= w.m) continue;
                 const int nchunks = (w.n + kSkChunk - 1) / kSkChunk;
@@ -304,7 +306,7 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                     const int sg = (int)(gc % kStages);
                     if (gc >= kStages &&
                         !mbar_wait_or(&empty[sg], (uint32_t)(gc / kStages - 1) & 1, &failed)) {
-                        fail_tile = tile;
+                        fail_tile = tile_of(item);
                         failed = 1;
                         break;
                     }
@@ -331,13 +333,12 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
         long long last = -1;
         if (lane == 0) {
             const uint32_t idu = idesc_i8(nc, false), ids = idesc_i8(nc, true);
-            SkItem wn = sk_item(tiles, (int)(blockIdx.x / rpt));
+            SkItem wn = sk_item(tiles, tile_of(blockIdx.x));
             for (long long item = blockIdx.x; item < nitems && !failed;
                  item += gridDim.x) {
-                const int tile = (int)(item / rpt);
                 const SkItem w = wn;
                 if (item + gridDim.x < nitems)
-                    wn = sk_item(tiles, (int)((item + gridDim.x) / rpt));
+                    wn = sk_item(tiles, tile_of(item + gridDim.x));
                 const int row0 = (int)(item % rpt) * kSkRows;
                 if (!sk_active(w, need) || row0 >= w.m) continue;
                 const int nchunks = (w.n + kSkChunk - 1) / kSkChunk;
@@ -366,7 +367,7 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                     last = gc;
                 }
                 if (!ok) {
-                    fail_tile = tile;
+                    fail_tile = tile_of(item);
                     failed = 1;
                     break;
                 }
@@ -394,7 +395,7 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
         };
         auto next_valid = [&](long long item, SkItem &w) {
             for (; item < nitems; item += gridDim.x) {
-                w = sk_item(tiles, (int)(item / rpt));
+                w = sk_item(tiles, tile_of(item));
                 if (valid(w, item)) break;
             }
             return item;
@@ -408,7 +409,6 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
         long long item = next_valid(blockIdx.x, w);
         if (item < nitems) post(item, w, 0);
         while (item < nitems) {
-            const int tile = (int)(item / rpt);
             SkItem wn{};
             const long long nx = next_valid(item + gridDim.x, wn);
             if (nx < nitems) post(nx, wn, (it + 1) & 1);
@@ -419,7 +419,7 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
             // or every lane stops
             const bool ok = mbar_wait_or(&accfull, (uint32_t)it & 1, &failed);
             if (!__all_sync(0xffffffffu, ok ? 1 : 0)) {
-                if (lane == 0) fail_tile = tile;
+                if (lane == 0) fail_tile = tile_of(item);
                 failed = 1;
                 break;
             }
@@ -529,9 +529,10 @@ bool i8_colmajor_map(CUtensorMap *map, const int8_t *om8, int ld_om8,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool launch_sketch_i8(const TileWork *d_tiles, int ntiles, Workspace ws,
-                      const int8_t *om8, int ld_om8, int om8_cols, int ncols,
-                      cudaStream_t stream, int need)
+bool launch_sketch_i8(const TileWork *d_tiles, int ntiles, int count,
+                      const int *act, Workspace ws, const int8_t *om8,
+                      int ld_om8, int om8_cols, int ncols, cudaStream_t stream,
+                      int need)
 {
     const int nc = (ncols + 15) / 16 * 16;
     CUtensorMap dmap, omap;
@@ -547,11 +548,11 @@ bool launch_sketch_i8(const TileWork *d_tiles, int ntiles, Workspace ws,
                              (int)sketch_i8_smem());
         sms = count > 0 ? count : 148;
     }
-    const long long items = (long long)ntiles * ((ws.m_max + kSkRows - 1) / kSkRows);
+    const long long items = (long long)count * ((ws.m_max + kSkRows - 1) / kSkRows);
     const int grid = (int)std::min<long long>(sms, items);
     if (grid <= 0) return true;
     k_sketch_i8<<<grid, kSkThreads, sketch_i8_smem(), stream>>>(
-        dmap, omap, d_tiles, ntiles, ws, nc, need);
+        dmap, omap, d_tiles, count, act, ws, nc, need);
     return true;
 }
 
