@@ -743,6 +743,8 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     int one_family = kernels.empty() ? 0 : kernels[0].family;
     for (const DevKernel &K : kernels)
         if (K.family != one_family) one_family = 0;
+    bool plain = true;
+    for (const DevKernel &K : kernels) plain = plain && K.sigma == 1.0 && K.noise == 0.0;
     // Gaussian sketch, shared by every tile (as the reference reuses the
     // same iseed for every block): n_max x k_max, ld n_max.
     if (ctx.omega_rows != n_max || ctx.omega_cols != k_max) {
@@ -1018,7 +1020,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
                                (int *)ctx.act.ptr, nt, s);
             if (any_separate) {
                 launch_gen_tiles(d_kernels, dt, nt, ws, s, TILE_GEN_SEPARATE,
-                                 one_family);
+                                 one_family, plain);
                 count_launch();
             }
             if (!launch_gen_sketch_i8(d_kernels, dt, nt, ws, om8, ld_om8,
@@ -1033,7 +1035,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
             const cudaError_t ce = cudaGetLastError();
             if (ce != cudaSuccess) { info = cuda_fail(ce, "k_gen_sketch_i8"); break; }
         } else {
-            launch_gen_tiles(d_kernels, dt, nt, ws, s, 0, one_family);
+            launch_gen_tiles(d_kernels, dt, nt, ws, s, 0, one_family, plain);
             count_launch();
         }
         cudaEventRecord(ev[5], s);

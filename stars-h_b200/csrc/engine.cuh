@@ -168,10 +168,10 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int count,
 // the tile's kernel from d_kernels[tile.prob].
 // need != 0: only tiles whose status has a bit of `need`.
 // family != 0: every tile has that kernel family (a kernel compiled for
-// it alone, where one exists).
+// it alone, where one exists); plain: with sigma = 1 and no noise.
 void launch_gen_tiles(const DevKernel *d_kernels, const TileWork *d_tiles,
                       int ntiles, Workspace ws, cudaStream_t stream,
-                      int need = 0, int family = 0);
+                      int need = 0, int family = 0, bool plain = false);
 // Phases A (0) and B (1) of the pivoted Cholesky.
 void launch_pivchol(int phase, TileWork *d_tiles, int ntiles, Workspace ws,
                     cudaStream_t s);

@@ -334,6 +334,16 @@ __device__ __forceinline__ double entry_fam(const DevKernel &K, double dist,
     }
 }
 
+// The exponential families with sigma = 1 and no noise (noise only enters at
+// distance zero, where the exponential is exactly 1): the same bits without
+// the test and the product.
+template <int FAM>
+__device__ __forceinline__ double entry_plain(const DevKernel &K, double dist)
+{
+    static_assert(FAM == FAM_EXP || FAM == FAM_SQREXP, "exponential families");
+    return exp(FAM == FAM_EXP ? sqrt(dist) * K.inv_neg_beta : dist * K.inv_neg_2beta2);
+}
+
 __device__ __forceinline__ double entry_from_dist(const DevKernel &K,
                                                   double dist, long long ir,
                                                   long long jc)
