@@ -52,13 +52,13 @@ __device__ __forceinline__ void dmma_884(double &c0, double &c1, double a,
 // ranks.  Each output element is written by one CTA, its sum in a fixed
 // order (deterministic).
 //
-// CTA tile 128 x BN (BN = 16 FN), 8 warps as 4 (m) x 2 (n), warp tile
-// 32 x 8 FN of FP64 mma.sync m8n8k4; K steps of 16 through a three-stage
-// cp.async pipeline.  Shared-memory layouts are chosen so that the
+// CTA tile 128 x BN (BN = 16 FN; phase 2 64 x BN), in phase 1 8 warps as 4
+// (m) x 2 (n), warp tile 32 x 8 FN of FP64 mma.sync m8n8k4; K steps of 16
+// through a three-stage cp.async pipeline.  Shared-memory layouts are chosen so that the
 // fragment reads and the copies are free of bank conflicts: B as [n][k]
 // (row stride 20 doubles); A as [m][k] (stride 20) in phase 1, whose
 // operand is contiguous along k in global memory, and as [k][m] (stride
-// 132) in phase 2, whose operand is contiguous along m.
+// 68) in phase 2, whose operand is contiguous along m.
 
 struct RowT {          // where phase 1 writes row rho of T
     long long base;    // first T row of the output block row (P_i)
@@ -89,7 +89,7 @@ struct Job2 {          // phase 2: up to 128 rows of one output block row
 };
 
 constexpr int kPBM = 128, kPBK = 16, kPStages = 3;
-constexpr int kPAStage = 2560;   // >= 128 * 20 (phase 1), 16 * 132 (phase 2)
+constexpr int kPAStage = 128 * 20;   // phase 1
 
 template <int FN>
 constexpr int prod_stage_doubles() { return kPAStage + 20 * 16 * FN; }
@@ -112,25 +112,26 @@ __device__ __forceinline__ void cp_async_wait_stages()
     asm volatile("cp.async.wait_group %0;\n" ::"n"(kPStages - 2));
 }
 
-// acc += A_stage B_stage for one K step (A_KMAJOR: A stored as [k][m]).
-template <int FN, bool A_KMAJOR>
+// acc += A_stage B_stage for one K step: MI x NJ fragments of the warp at
+// (wm, wn); A stored as [k][m] with stride LDA, or (LDA = 0) as [m][k].
+template <int MI, int NJ, int LDA>
 __device__ __forceinline__ void prod_step(const double *As, const double *Bs,
-                                          double (&acc)[4][FN][2], int wm,
+                                          double (&acc)[MI][NJ][2], int wm,
                                           int wn, int g, int tig)
 {
     #pragma unroll
     for (int kk = 0; kk < kPBK; kk += 4) {
-        double af[4], bf[FN];
+        double af[MI], bf[NJ];
         #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            af[i] = A_KMAJOR ? As[(kk + tig) * 132 + wm + 8 * i + g]
-                             : As[(wm + 8 * i + g) * 20 + kk + tig];
+        for (int i = 0; i < MI; ++i)
+            af[i] = LDA ? As[(kk + tig) * LDA + wm + 8 * i + g]
+                        : As[(wm + 8 * i + g) * 20 + kk + tig];
         #pragma unroll
-        for (int j = 0; j < FN; ++j) bf[j] = Bs[(wn + 8 * j + g) * 20 + kk + tig];
+        for (int j = 0; j < NJ; ++j) bf[j] = Bs[(wn + 8 * j + g) * 20 + kk + tig];
         #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < MI; ++i)
             #pragma unroll
-            for (int j = 0; j < FN; ++j)
+            for (int j = 0; j < NJ; ++j)
                 dmma_884(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
     }
 }
@@ -189,7 +190,7 @@ k_prod_t(const Job1 *__restrict__ jobs, const double *const *__restrict__ vcol,
             issue(s + kPStages - 1, (s + kPStages - 1) % kPStages);
         cp_async_commit();
         const double *As = sm + (s % kPStages) * STAGE;
-        prod_step<FN, false>(As, As + kPAStage, acc, wm, wn, g, tig);
+        prod_step<4, FN, 0>(As, As + kPAStage, acc, wm, wn, g, tig);
     }
     #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -215,9 +216,15 @@ __device__ __forceinline__ void update(double *out, double alpha, double v,
     *out = fma(alpha, v, old);
 }
 
-// Phase 2: rows m0 .. m0 + rows - 1 of one output block row.
+// Phase 2: 64 of a job's rows of one output block row (a block row's K is
+// long and uneven: with 128 rows a CTA, N = 32768 left 40 of 148 SMs half
+// idle for the whole launch, the DMMA pipe 58 % busy).
+constexpr int kPB2 = 64, kPB2Ld = kPB2 + 4;
 template <int FN>
-__global__ void __launch_bounds__(256, 2)
+constexpr int prod_b_stage() { return kPBK * kPB2Ld + 20 * 16 * FN; }
+
+template <int FN>
+__global__ void __launch_bounds__(256, 3)
 k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
          const double *__restrict__ T, int nrhs,
          const NearPiece *__restrict__ near, const double *__restrict__ nearD,
@@ -225,14 +232,20 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
          double alpha, double beta)
 {
     constexpr int BN = 16 * FN;
-    constexpr int STAGE = prod_stage_doubles<FN>();
+    constexpr int STAGE = prod_b_stage<FN>(), AST = kPBK * kPB2Ld;
+    // warps along the rows and the columns, fragments of a warp
+    constexpr int WM = FN == 1 ? 4 : 2, MI = kPB2 / (8 * WM), NJ = 2 * FN * WM / 8;
     extern __shared__ double sm[];
-    const Job2 jb = jobs[blockIdx.x];
+    Job2 jb = jobs[blockIdx.x];
+    jb.m0 += blockIdx.z * kPB2;
+    jb.rows = min(kPB2, jb.rows - (int)blockIdx.z * kPB2);
+    if (jb.rows <= 0) return;
+    jb.out0 += blockIdx.z * kPB2;
     const int n0 = blockIdx.y * BN;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3;
-    const int wm = (warp & 3) * 32, wn = (warp >> 2) * 8 * FN;
-    // A copies: rows am, am + 64 and columns ak + 4 q (q < 4) of the step;
+    const int wm = warp % WM * 8 * MI, wn = warp / WM * 8 * NJ;
+    // A copies: row am and columns ak + 4 q (q < 4) of the step;
     // B copies: column lk of the step, right-hand sides lr + 16 q
     const int am = t & 63, ak = t >> 6;
     const int lk = t & 15, lr = t >> 4;
@@ -259,17 +272,14 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
         fetch_ptrs();
     };
     auto issue = [&](int st) {
-        double *As = sm + st * STAGE, *Bs = As + kPAStage;
+        double *As = sm + st * STAGE, *Bs = As + AST;
         if (piece < 0) {
             #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int m = am + 64 * h;
-                    const bool ok = up[q] != nullptr && m < jb.rows;
-                    cp_async8(As + (ak + 4 * q) * 132 + m,
-                              ok ? up[q] + jb.m0 + m : A, ok);
-                }
+            for (int q = 0; q < 4; ++q) {
+                const bool ok = up[q] != nullptr && am < jb.rows;
+                cp_async8(As + (ak + 4 * q) * kPB2Ld + am,
+                          ok ? up[q] + jb.m0 + am : A, ok);
+            }
             #pragma unroll
             for (int q = 0; q < FN; ++q) {
                 const int col = n0 + lr + 16 * q, kap = k0 + lk;
@@ -281,16 +291,14 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
             const NearPiece np = near[piece];
             const double *D = nearD + np.off;
             #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int m = am + 64 * h, kap = k0 + ak + 4 * q;
-                    const bool ok = kap < np.K && m < jb.rows;
-                    const size_t off = np.trans
-                        ? (size_t)kap + (size_t)(jb.m0 + m) * np.ld
-                        : (size_t)(jb.m0 + m) + (size_t)kap * np.ld;
-                    cp_async8(As + (ak + 4 * q) * 132 + m, ok ? D + off : A, ok);
-                }
+            for (int q = 0; q < 4; ++q) {
+                const int kap = k0 + ak + 4 * q;
+                const bool ok = kap < np.K && am < jb.rows;
+                const size_t off = np.trans
+                    ? (size_t)kap + (size_t)(jb.m0 + am) * np.ld
+                    : (size_t)(jb.m0 + am) + (size_t)kap * np.ld;
+                cp_async8(As + (ak + 4 * q) * kPB2Ld + am, ok ? D + off : A, ok);
+            }
             #pragma unroll
             for (int q = 0; q < FN; ++q) {
                 const int col = n0 + lr + 16 * q, kap = k0 + lk;
@@ -301,7 +309,7 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
         }
     };
     fetch_ptrs();
-    double acc[4][FN][2] = {};
+    double acc[MI][NJ][2] = {};
     #pragma unroll
     for (int s = 0; s < kPStages - 1; ++s) {
         if (s < total) {
@@ -319,15 +327,15 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
         }
         cp_async_commit();
         const double *As = sm + (s % kPStages) * STAGE;
-        prod_step<FN, true>(As, As + kPAStage, acc, wm, wn, g, tig);
+        prod_step<MI, NJ, kPB2Ld>(As, As + AST, acc, wm, wn, g, tig);
     }
     #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < MI; ++i) {
         const int m = wm + 8 * i + g;
         if (m >= jb.rows) continue;
         double *out = B + jb.out0 + m;
         #pragma unroll
-        for (int j = 0; j < FN; ++j)
+        for (int j = 0; j < NJ; ++j)
             #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int col = n0 + wn + 8 * j + 2 * tig + h;
@@ -345,12 +353,13 @@ static void launch_products(const Job1 *j1, int n1, const double *const *vcol,
                             double beta, cudaStream_t s)
 {
     constexpr size_t smem = (size_t)kPStages * prod_stage_doubles<FN>() * sizeof(double);
+    constexpr size_t smem_b = (size_t)kPStages * prod_b_stage<FN>() * sizeof(double);
     static std::once_flag attr;
     std::call_once(attr, [] {
         cudaFuncSetAttribute(k_prod_t<FN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
         cudaFuncSetAttribute(k_prod_b<FN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+                             (int)smem_b);
     });
     const unsigned ny = (unsigned)((nrhs + 16 * FN - 1) / (16 * FN));
     if (n1 > 0) {
@@ -359,7 +368,7 @@ static void launch_products(const Job1 *j1, int n1, const double *const *vcol,
         count_launch();
     }
     if (n2 > 0) {
-        k_prod_b<FN><<<dim3((unsigned)n2, ny), 256, smem, s>>>(
+        k_prod_b<FN><<<dim3((unsigned)n2, ny, kPBM / kPB2), 256, smem_b, s>>>(
             j2, ucol, T, nrhs, near, nearD, A, lda, B, ldb, alpha, beta);
         count_launch();
     }
@@ -836,6 +845,21 @@ static int build_plan(STARSH_blrm *M, const Record &rec, cudaStream_t s,
         for (int m0 = 0; m0 < mi; m0 += kPBM)
             j2.push_back(Job2{(long long)R->start[i] + m0, m0, std::min(kPBM, mi - m0),
                               P[i], S[i], near0, (int)near.size()});
+    }
+    // longest K first: the CTAs of a launch start in this order
+    {
+        auto klen = [&](const Job2 &j) {
+            long long k = j.kfar;
+            for (int q = j.near0; q < j.near1; ++q) k += near[q].K;
+            return k;
+        };
+        std::vector<std::pair<long long, int>> order(j2.size());
+        for (size_t q = 0; q < j2.size(); ++q) order[q] = {-klen(j2[q]), (int)q};
+        std::stable_sort(order.begin(), order.end(),
+                         [](const auto &x, const auto &y) { return x.first < y.first; });
+        std::vector<Job2> sorted(j2.size());
+        for (size_t q = 0; q < j2.size(); ++q) sorted[q] = j2[order[q].second];
+        j2.swap(sorted);
     }
     // one device allocation for every array
     std::vector<char> buf;
