@@ -52,9 +52,8 @@ __device__ __forceinline__ void dmma_884(double &c0, double &c1, double a,
 // ranks.  Each output element is written by one CTA, its sum in a fixed
 // order (deterministic).
 //
-// CTA tile 128 x BN (BN = 16 FN; phase 2 64 x BN), in phase 1 8 warps as 4
-// (m) x 2 (n), warp tile 32 x 8 FN of FP64 mma.sync m8n8k4; K steps of 16
-// through a three-stage cp.async pipeline.  Shared-memory layouts are chosen so that the
+// CTA tile 64 x BN (BN = 16 FN), 8 warps of FP64 mma.sync m8n8k4 fragments;
+// K steps of 16 through a three-stage cp.async pipeline.  Shared-memory layouts are chosen so that the
 // fragment reads and the copies are free of bank conflicts: B as [n][k]
 // (row stride 20 doubles); A as [m][k] (stride 20) in phase 1, whose
 // operand is contiguous along k in global memory, and as [k][m] (stride
@@ -89,7 +88,8 @@ struct Job2 {          // phase 2: up to 128 rows of one output block row
 };
 
 constexpr int kPBM = 128, kPBK = 16, kPStages = 3;
-constexpr int kPAStage = 128 * 20;   // phase 1
+constexpr int kPRows = 64;             // rows of a CTA
+constexpr int kPAStage = kPRows * 20;  // phase 1
 
 template <int FN>
 constexpr int prod_stage_doubles() { return kPAStage + 20 * 16 * FN; }
@@ -136,10 +136,10 @@ __device__ __forceinline__ void prod_step(const double *As, const double *Bs,
     }
 }
 
-// Phase 1: T rows of one job (rows rho0 .. rho0 + rows - 1), columns
-// n0 .. n0 + BN - 1 of the right-hand sides.
+// Phase 1: 64 of the T rows of one job, columns n0 .. n0 + BN - 1 of the
+// right-hand sides.
 template <int FN>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, 3)
 k_prod_t(const Job1 *__restrict__ jobs, const double *const *__restrict__ vcol,
          const RowT *__restrict__ rowt, const double *__restrict__ A, int lda,
          double *__restrict__ T, int nrhs)
@@ -147,13 +147,18 @@ k_prod_t(const Job1 *__restrict__ jobs, const double *const *__restrict__ vcol,
     constexpr int BN = 16 * FN;
     constexpr int STAGE = prod_stage_doubles<FN>();
     extern __shared__ double sm[];
-    __shared__ const double *rowp[kPBM];
-    const Job1 jb = jobs[blockIdx.x];
+    // warps along the rows and the columns, fragments of a warp
+    constexpr int WM = FN == 1 ? 4 : 2, MI = kPRows / (8 * WM), NJ = 2 * FN * WM / 8;
+    __shared__ const double *rowp[kPRows];
+    Job1 jb = jobs[blockIdx.x];
+    jb.rho0 += blockIdx.z * kPRows;
+    jb.rows = min(kPRows, jb.rows - (int)blockIdx.z * kPRows);
+    if (jb.rows <= 0) return;
     const int n0 = blockIdx.y * BN;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3;
-    const int wm = (warp & 3) * 32, wn = (warp >> 2) * 8 * FN;
-    for (int r = t; r < kPBM; r += 256)
+    const int wm = warp % WM * 8 * MI, wn = warp / WM * 8 * NJ;
+    for (int r = t; r < kPRows; r += 256)
         rowp[r] = r < jb.rows ? vcol[jb.rho0 + r] : nullptr;
     __syncthreads();
     const int lk = t & 15, lr = t >> 4;
@@ -164,7 +169,7 @@ k_prod_t(const Job1 *__restrict__ jobs, const double *const *__restrict__ vcol,
         const int k = step * kPBK + lk;
         const bool kin = k < jb.K;
         #pragma unroll
-        for (int q = 0; q < 8; ++q) {
+        for (int q = 0; q < 4; ++q) {
             const double *p = rowp[lr + 16 * q];
             const bool ok = kin && p != nullptr;
             cp_async8(As + (lr + 16 * q) * 20 + lk, ok ? p + k : A, ok);
@@ -177,7 +182,7 @@ k_prod_t(const Job1 *__restrict__ jobs, const double *const *__restrict__ vcol,
                       ok ? Aj + k + (size_t)col * lda : A, ok);
         }
     };
-    double acc[4][FN][2] = {};
+    double acc[MI][NJ][2] = {};
     #pragma unroll
     for (int s = 0; s < kPStages - 1; ++s) {
         if (s < steps) issue(s, s);
@@ -190,16 +195,16 @@ k_prod_t(const Job1 *__restrict__ jobs, const double *const *__restrict__ vcol,
             issue(s + kPStages - 1, (s + kPStages - 1) % kPStages);
         cp_async_commit();
         const double *As = sm + (s % kPStages) * STAGE;
-        prod_step<4, FN, 0>(As, As + kPAStage, acc, wm, wn, g, tig);
+        prod_step<MI, NJ, 0>(As, As + kPAStage, acc, wm, wn, g, tig);
     }
     #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < MI; ++i) {
         const int r = wm + 8 * i + g;
         if (r >= jb.rows) continue;
         const RowT rt = rowt[jb.rho0 + r];
         double *out = T + (size_t)nrhs * rt.base + rt.kappa;
         #pragma unroll
-        for (int j = 0; j < FN; ++j)
+        for (int j = 0; j < NJ; ++j)
             #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int col = n0 + wn + 8 * j + 2 * tig + h;
@@ -219,9 +224,9 @@ __device__ __forceinline__ void update(double *out, double alpha, double v,
 // Phase 2: 64 of a job's rows of one output block row (a block row's K is
 // long and uneven: with 128 rows a CTA, N = 32768 left 40 of 148 SMs half
 // idle for the whole launch, the DMMA pipe 58 % busy).
-constexpr int kPB2 = 64, kPB2Ld = kPB2 + 4;
+constexpr int kPRowsLd = kPRows + 4;
 template <int FN>
-constexpr int prod_b_stage() { return kPBK * kPB2Ld + 20 * 16 * FN; }
+constexpr int prod_b_stage() { return kPBK * kPRowsLd + 20 * 16 * FN; }
 
 template <int FN>
 __global__ void __launch_bounds__(256, 3)
@@ -232,15 +237,15 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
          double alpha, double beta)
 {
     constexpr int BN = 16 * FN;
-    constexpr int STAGE = prod_b_stage<FN>(), AST = kPBK * kPB2Ld;
+    constexpr int STAGE = prod_b_stage<FN>(), AST = kPBK * kPRowsLd;
     // warps along the rows and the columns, fragments of a warp
-    constexpr int WM = FN == 1 ? 4 : 2, MI = kPB2 / (8 * WM), NJ = 2 * FN * WM / 8;
+    constexpr int WM = FN == 1 ? 4 : 2, MI = kPRows / (8 * WM), NJ = 2 * FN * WM / 8;
     extern __shared__ double sm[];
     Job2 jb = jobs[blockIdx.x];
-    jb.m0 += blockIdx.z * kPB2;
-    jb.rows = min(kPB2, jb.rows - (int)blockIdx.z * kPB2);
+    jb.m0 += blockIdx.z * kPRows;
+    jb.rows = min(kPRows, jb.rows - (int)blockIdx.z * kPRows);
     if (jb.rows <= 0) return;
-    jb.out0 += blockIdx.z * kPB2;
+    jb.out0 += blockIdx.z * kPRows;
     const int n0 = blockIdx.y * BN;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3;
@@ -277,7 +282,7 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
             #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const bool ok = up[q] != nullptr && am < jb.rows;
-                cp_async8(As + (ak + 4 * q) * kPB2Ld + am,
+                cp_async8(As + (ak + 4 * q) * kPRowsLd + am,
                           ok ? up[q] + jb.m0 + am : A, ok);
             }
             #pragma unroll
@@ -297,7 +302,7 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
                 const size_t off = np.trans
                     ? (size_t)kap + (size_t)(jb.m0 + am) * np.ld
                     : (size_t)(jb.m0 + am) + (size_t)kap * np.ld;
-                cp_async8(As + (ak + 4 * q) * kPB2Ld + am, ok ? D + off : A, ok);
+                cp_async8(As + (ak + 4 * q) * kPRowsLd + am, ok ? D + off : A, ok);
             }
             #pragma unroll
             for (int q = 0; q < FN; ++q) {
@@ -327,7 +332,7 @@ k_prod_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
         }
         cp_async_commit();
         const double *As = sm + (s % kPStages) * STAGE;
-        prod_step<MI, NJ, kPB2Ld>(As, As + AST, acc, wm, wn, g, tig);
+        prod_step<MI, NJ, kPRowsLd>(As, As + AST, acc, wm, wn, g, tig);
     }
     #pragma unroll
     for (int i = 0; i < MI; ++i) {
@@ -363,12 +368,12 @@ static void launch_products(const Job1 *j1, int n1, const double *const *vcol,
     });
     const unsigned ny = (unsigned)((nrhs + 16 * FN - 1) / (16 * FN));
     if (n1 > 0) {
-        k_prod_t<FN><<<dim3((unsigned)n1, ny), 256, smem, s>>>(j1, vcol, rowt, A,
+        k_prod_t<FN><<<dim3((unsigned)n1, ny, kPBM / kPRows), 256, smem, s>>>(j1, vcol, rowt, A,
                                                               lda, T, nrhs);
         count_launch();
     }
     if (n2 > 0) {
-        k_prod_b<FN><<<dim3((unsigned)n2, ny, kPBM / kPB2), 256, smem_b, s>>>(
+        k_prod_b<FN><<<dim3((unsigned)n2, ny, kPBM / kPRows), 256, smem_b, s>>>(
             j2, ucol, T, nrhs, near, nearD, A, lda, B, ldb, alpha, beta);
         count_launch();
     }
