@@ -655,9 +655,6 @@ static void add_stats(starsh_b200_stats &a, const starsh_b200_stats &b)
     a.mirror_wait_ms += b.mirror_wait_ms;
 }
 
-// Calls with fewer matrix entries run on one lane.
-constexpr long long kLaneEntries = 200000000;
-
 // Runs the device pipeline over the far blocks of every problem of `jobs`
 // in shared batches: tiles of different problems (kernels, sizes, tol,
 // maxrank) share every launch.  Fills each job's ranks and the per-block
@@ -814,36 +811,12 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     if (const char *e = getenv("STARSH_B200_WORKSPACE_MB"))
         budget = std::min<size_t>(budget, (size_t)atoll(e) << 20);
     budget = std::min(budget, ctx.workspace_cap);
-    // Two lanes: the batches are dealt, as they come free, to two host
-    // threads with their own streams and workspaces, so that the chains of
-    // small launches of one batch's rounds and small SVDs run beside the
-    // other's full-width kernels, and neither waits for the host's reads.
-    // A call that would be one batch is cut in three (the first part, the
-    // near-diagonal tiles, has the longest rounds and SVDs).  Calls below
-    // kLaneEntries matrix entries are bound by the chain of one batch, which
-    // more parts do not shorten (7e7 entries: 4.74 against 4.54 ms, 1.2e8:
-    // 14.2 against 13.9 .. 15.3), and stay on one lane; above it 3e8 entries
-    // go from 10.9 to 10.8 ms, with host mirrors 8.8 to 7.8 (the first parts
-    // download early), 24 mixed problems 68.7 to 58.7, N = 65536 1/r 108.1
-    // to 102.1, N = 102400 square exponential 116.8 to 112.5.  A serving
-    // worker's context has the other workers beside it.
-    // STARSH_B200_LANES (1 or 2) sets the number.
-    int lanes = ctx.may_help && st.entries >= kLaneEntries && ntot >= 64 ? 2 : 1;
-    long long part = ntot;
-    if (const char *e = getenv("STARSH_B200_LANES"))
-        lanes = ctx.may_help ? std::max(1, std::min(2, atoi(e))) : 1;
-    Context *helper = lanes > 1 ? context_helper(ctx) : nullptr;
-    if (helper == nullptr) lanes = 1;
-    if (lanes > 1) {
-        budget /= 2;
-        part = (ntot + 2) / 3;
-    }
     // Batch plan: each batch takes as many tiles as fit the budget with
     // the layout of its largest dimensions (at most 4096).
     struct BatchPlan { long long b0; int nt; int m, n, k; size_t stride; };
     std::vector<BatchPlan> plan;
     size_t ws_need = 0;
-    long long max_slots = 1;
+    long long max_slots = 1, part = ntot;
     // the adaptive engine's projection on the tensor cores (needs the
     // int8 path's row maxima and TMA descriptors)
     // (opt-in: STARSH_B200_PROJ=i8 until it beats the FP64 projection)
@@ -877,6 +850,31 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         }
     };
     make_plan(budget);
+    // Two lanes: the batches are dealt, as they come free, to two host
+    // threads with their own streams and workspaces (half the budget each),
+    // so that the chains of small launches of one batch's rounds and small
+    // SVDs run beside the other's full-width kernels, and neither waits for
+    // the host's reads.  Where the adaptive engine's tiles need several
+    // batches anyway, in at least three parts (the first, the near-diagonal
+    // tiles, has the longest rounds and SVDs): 24 mixed problems 64.0 to
+    // 54.9 ms, N = 65536 1/r 93.8 to 89.9, N = 102400 square exponential
+    // 98.4 to 95.2, and 1.02 to 1.12 times over nine other calls of two to
+    // five batches.  Not one batch cut in parts (each part repeats the chain
+    // of rounds: 0.71 to 1.14 times over 77 calls, slower in 62 of them) and
+    // not the fixed-width FP64 engine, whose kernels fill the GPU (0.97, 0.97
+    // and 1.01 times with two to four batches).  A serving worker's context has the
+    // other workers beside it.  STARSH_B200_LANES (1 or 2) sets the number.
+    int lanes = ctx.may_help && ep.engine == STARSH_B200_MIXED && plan.size() > 1 ? 2 : 1;
+    if (const char *e = getenv("STARSH_B200_LANES"))
+        lanes = ctx.may_help ? std::max(1, std::min(2, atoi(e))) : 1;
+    if (getenv("STARSH_B200_TILE_LOG")) lanes = 1;   // (its lines in batch order)
+    Context *helper = lanes > 1 ? context_helper(ctx) : nullptr;
+    if (helper == nullptr) lanes = 1;
+    if (lanes > 1) {
+        budget /= 2;
+        part = (ntot + 2) / 3;
+        make_plan(budget);
+    }
     // What the lanes already hold needs no look at the free memory (the
     // driver's answer takes 0.1 ms and, on a busy host, tens of
     // milliseconds); to grow, take at most half of it.

@@ -205,8 +205,7 @@ int launch_small_svd(TileWork *d_tiles, int ntiles, Workspace ws,
 // `act` (optional): the launch covers the `ntiles` tiles listed there (a
 // round's sampling tiles) instead of the first `ntiles` of the batch.
 void launch_gather_cols(int phase, const TileWork *d_tiles, int ntiles,
-                        Workspace ws, cudaStream_t stream,
-                        const int *act = nullptr);
+                        Workspace ws, cudaStream_t stream);
 void launch_chol_inv(int phase, TileWork *d_tiles, int ntiles, Workspace ws,
                      int nmax, cudaStream_t stream, const int *act = nullptr);
 void launch_rank_cut(TileWork *d_tiles, int ntiles, Workspace ws,

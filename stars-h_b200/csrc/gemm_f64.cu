@@ -1,15 +1,12 @@
-// Batched FP64 GEMM (see gemm_f64.cuh).
-//
-// CTA tile 64 x 64 or 128 x 32, K step 16, 8 warps of 32 x 16
-// output each (4 x 2 fragments of the m8n8k4 DMMA).  Operand tiles are staged
-// in shared memory double-buffered, the next K tile is fetched into
-// registers while the current one is multiplied.  Global loads are
-// coalesced along whichever dimension is contiguous for the given transpose
-// flag, and the staging layout follows it: [row][k] with row stride 20 where
-// k is contiguous, [k][row] with stride rows + 4 where rows are, so that
-// both the stores and the fragment reads are free of bank conflicts.  Warps
-// skip the DMMAs of output regions outside the tile's own M x N and of k4
-// steps past its K (those would add exact zeros).
+// Batched FP64 GEMM (see gemm_f64.cuh): FP64 mma.sync m8n8k4, eight warps a
+// CTA.  One kernel for each shape of product:
+//   sketch (A B, long K)           k_gemm_f64
+//   basis updates, U (A B, short K) k_gemm_f64_nn_short
+//   rounds' A^T B, Gram B B^T      k_gemm_f64_tn_pipe, k_gemm_f64_nt_pipe
+//   projection, rotation (A^T B, wide) k_gemm_f64_tn_wide
+// Warps skip the DMMAs of output regions outside the tile's own M x N and of
+// k4 steps past its K (those would add exact zeros); the order of each sum is
+// the same in all of them (one chain over K, but for split_k).
 #include <cstdint>
 #include <mutex>
 #include "gemm_step.cuh"
@@ -26,10 +23,16 @@ __device__ __forceinline__ void dmma_8x8x4(double &c0, double &c1, double a,
         : "d"(a), "d"(b));
 }
 
-// The A B products (basis updates with K <= 64 and beta updates) keep
-// three CTAs per SM: their short K makes them latency-bound.
-template <bool TA, bool TB, int BM, int BN>
-__global__ void __launch_bounds__(kGemmThreads, (!TA && !TB) ? 3 : 0)
+// A B with a long K, the sketch Y = D Omega: CTA tile 64 x 64 or (sketch
+// blocks of 32 columns) 128 x 32, K step 16.  Operand tiles are staged in
+// shared memory double-buffered, the next K step fetched into registers while
+// the current one is multiplied; A lies there as [k][row] with stride rows +
+// 4, B as [column][k] with stride 20, so that both the stores and the
+// fragment reads are free of bank conflicts.  Three CTAs an SM.  Bound by the
+// DMMA pipe (82 % busy); the three-stage cp.async kernel of the short
+// products is no faster here.
+template <int BM, int BN>
+__global__ void __launch_bounds__(kGemmThreads, 3)
 k_gemm_f64(const __grid_constant__ GemmArgs args, int tiles_n)
 {
     // 8 warps of 32 x 16 output each, BM / 32 along M and BN / 16 along N
@@ -63,63 +66,33 @@ k_gemm_f64(const __grid_constant__ GemmArgs args, int tiles_n)
         for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
     double ra[RA], rb[RB];
-    // Element e = t + 256 r of a tile, laid out along whichever dimension
-    // is contiguous in global memory (coalesced loads):
-    //   A: !TA rows fastest, TA k fastest;  B: !TB k fastest, TB cols fastest.
-    auto a_coord = [&](int r, int &row, int &kk) {
-        const int e = t + kGemmThreads * r;
-        if (!TA) { row = e % BM; kk = e / BM; }
-        else     { kk = e % kGemmBK; row = e / kGemmBK; }
-    };
-    auto b_coord = [&](int r, int &col, int &kk) {
-        const int e = t + kGemmThreads * r;
-        if (!TB) { kk = e % kGemmBK; col = e / kGemmBK; }
-        else     { col = e % BN; kk = e / BN; }
-    };
+    // element e = t + 256 r of a tile, along the contiguous dimension: A
+    // rows fastest, B k fastest
+    constexpr int LDA = BM + 4;
     auto load_tiles = [&](int k0) {
         #pragma unroll
         for (int r = 0; r < RA; ++r) {
-            int row, kk;
-            a_coord(r, row, kk);
-            const int gm = m0 + row, gk = k0 + kk;
-            double v = 0.0;
-            if (gm < d.M && gk < d.K)
-                v = TA ? d.A[(size_t)gm * d.lda + gk]
-                       : d.A[(size_t)gk * d.lda + gm];
-            ra[r] = v;
+            const int e = t + kGemmThreads * r;
+            const int gm = m0 + e % BM, gk = k0 + e / BM;
+            ra[r] = gm < d.M && gk < d.K ? d.A[(size_t)gk * d.lda + gm] : 0.0;
         }
         #pragma unroll
         for (int r = 0; r < RB; ++r) {
-            int col, kk;
-            b_coord(r, col, kk);
-            const int gn = n0 + col, gk = k0 + kk;
-            double v = 0.0;
-            if (gn < d.N && gk < d.K)
-                v = TB ? d.B[(size_t)gk * d.ldb + gn]
-                       : d.B[(size_t)gn * d.ldb + gk];
-            rb[r] = v;
+            const int e = t + kGemmThreads * r;
+            const int gn = n0 + e / kGemmBK, gk = k0 + e % kGemmBK;
+            rb[r] = gn < d.N && gk < d.K ? d.B[(size_t)gn * d.ldb + gk] : 0.0;
         }
-    };
-    // shared-memory index of (row, k) of A and (col, k) of B
-    constexpr int LDA_K = BM + 4, LDB_K = BN + 4;   // [k][row] strides
-    auto a_at = [](int row, int kk) {
-        return TA ? row * kGemmLds + kk : kk * LDA_K + row;
-    };
-    auto b_at = [](int col, int kk) {
-        return TB ? kk * LDB_K + col : col * kGemmLds + kk;
     };
     auto store_tiles = [&](int buf) {
         #pragma unroll
         for (int r = 0; r < RA; ++r) {
-            int row, kk;
-            a_coord(r, row, kk);
-            As[buf][a_at(row, kk)] = ra[r];
+            const int e = t + kGemmThreads * r;
+            As[buf][e / BM * LDA + e % BM] = ra[r];
         }
         #pragma unroll
         for (int r = 0; r < RB; ++r) {
-            int col, kk;
-            b_coord(r, col, kk);
-            Bs[buf][b_at(col, kk)] = rb[r];
+            const int e = t + kGemmThreads * r;
+            Bs[buf][e / kGemmBK * kGemmLds + e % kGemmBK] = rb[r];
         }
     };
 
@@ -134,20 +107,18 @@ k_gemm_f64(const __grid_constant__ GemmArgs args, int tiles_n)
     for (int kt = 0; kt < ktiles; ++kt) {
         const int buf = kt & 1;
         if (kt + 1 < ktiles) load_tiles((kt + 1) * kGemmBK);
-        // k4 steps of this warp in the K step (warp-uniform; A B products
-        // only, the other forms keep every step)
-        const int kend = (TA || TB) ? kGemmBK
-                         : live ? min(kGemmBK, d.K - kt * kGemmBK) : 0;
+        // k4 steps of this warp in the K step (warp-uniform)
+        const int kend = live ? min(kGemmBK, d.K - kt * kGemmBK) : 0;
         #pragma unroll
         for (int kk = 0; kk < kGemmBK; kk += 4) {
             if (kk >= kend) break;
             double af[4], bf[2];
             #pragma unroll
             for (int i = 0; i < 4; ++i)
-                af[i] = As[buf][a_at(wm + i * 8 + g, kk + tig)];
+                af[i] = As[buf][(kk + tig) * LDA + wm + i * 8 + g];
             #pragma unroll
             for (int j = 0; j < 2; ++j)
-                bf[j] = Bs[buf][b_at(wn + j * 8 + g, kk + tig)];
+                bf[j] = Bs[buf][(wn + j * 8 + g) * kGemmLds + kk + tig];
             #pragma unroll
             for (int i = 0; i < 4; ++i)
                 #pragma unroll
@@ -160,43 +131,19 @@ k_gemm_f64(const __grid_constant__ GemmArgs args, int tiles_n)
         __syncthreads();
     }
 
-    // Accumulator (i, j, h) holds C(wm + 8i + g, wn + 8j + 2 tig + h).
-    // With beta != 0 the old C values are all read before the first store
-    // (the stores may alias later loads, so loads interleaved with them
-    // would each wait a full memory round trip).
-    double cold[4][2][2];
-    const bool upd = d.beta != 0.0;
-    if (upd) {
-        #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int gm = m0 + wm + i * 8 + g;
-            #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int gn = n0 + wn + j * 8 + 2 * tig + h;
-                    cold[i][j][h] = gm < d.M && gn < d.N
-                                        ? d.C[(size_t)gn * d.ldc + gm] : 0.0;
-                }
-            }
-        }
-    }
+    // accumulator (i, j, h) holds C(wm + 8i + g, wn + 8j + 2 tig + h); a
+    // sketch has no old C
     #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int gm = m0 + wm + i * 8 + g;
         if (gm >= d.M) continue;
         #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < 2; ++j)
             #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int gn = n0 + wn + j * 8 + 2 * tig + h;
-                if (gn >= d.N) continue;
-                double *c = d.C + (size_t)gn * d.ldc + gm;
-                double v = d.alpha * acc[i][j][h];
-                if (upd) v += d.beta * cold[i][j][h];
-                *c = v;
+                if (gn < d.N) d.C[(size_t)gn * d.ldc + gm] = d.alpha * acc[i][j][h];
             }
-        }
     }
 }
 
@@ -859,40 +806,28 @@ k_gemm_f64_nn_short(const __grid_constant__ GemmArgs args, int tiles_n, int iter
     else nn_short<4>(d, m_first, m_last, n0, nn_smem);
 }
 
-template <int BM, int BN>
-static void launch_shape(bool ta, bool tb, const GemmArgs &args, int nb,
-                         int tiles_m, int tiles_n, cudaStream_t stream)
-{
-    dim3 grid(tiles_m * tiles_n, nb);
-    const size_t smem = 2 * (size_t)(BM + BN) * kGemmLds * sizeof(double);
-    auto go = [&](auto fn) {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
-        fn<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n);
-    };
-    if (!ta && !tb) go(k_gemm_f64<false, false, BM, BN>);
-    else if (ta && !tb) go(k_gemm_f64<true, false, BM, BN>);
-    else if (!ta && tb) go(k_gemm_f64<false, true, BM, BN>);
-    else go(k_gemm_f64<true, true, BM, BN>);
-}
-
 cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int batch,
                              int max_m, int max_n, cudaStream_t stream,
                              bool split_k)
 {
     if (batch <= 0 || max_m <= 0 || max_n <= 0) return cudaSuccess;
-    split_k = split_k && ta != tb;
-    // CTA shape: 64 x 64 (always with split_k); for A^T B whose output is
-    // wide and (as for the projection B = Q^T D and the rotation C = W^T B)
-    // has a basis much narrower than the batch maximum as its rows, the
-    // fitted 64 x 128 kernel; 128 x 32 for narrow outputs (sketch blocks of
-    // 32 columns)
-    const bool sketch = args.step == STEP_SKETCH || args.step == STEP_A_SKETCH;
-    if (!ta && !tb && !sketch) {
+    if (!ta && !tb) {
+        const int tiles_n = (max_n + 63) / 64;
+        if (args.step == STEP_SKETCH || args.step == STEP_A_SKETCH) {
+            // 128 x 32 tiles for sketch blocks of at most 32 columns
+            auto go = [&](auto fn, int bm, int bn) {
+                const int smem = 2 * (bm + bn) * kGemmLds * (int)sizeof(double);
+                if (smem > 48 * 1024)
+                    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                fn<<<dim3((max_m + bm - 1) / bm * tiles_n, batch), kGemmThreads, smem,
+                     stream>>>(args, tiles_n);
+            };
+            if (max_n <= 32 && max_m >= 128) go(k_gemm_f64<128, 32>, 128, 32);
+            else go(k_gemm_f64<64, 64>, 64, 64);
+            return cudaGetLastError();
+        }
         // four row blocks to a CTA where that still leaves two rounds of
         // CTAs, else one
-        const int tiles_n = (max_n + 63) / 64;
         const int blocks = (max_m + kNnRows - 1) / kNnRows;
         const int iters = (size_t)((blocks + 3) / 4) * tiles_n * batch >= 592 ? 4 : 1;
         constexpr size_t smem = (size_t)kNnStages * kNnStage * sizeof(double);
@@ -905,41 +840,36 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int batch,
                               kGemmThreads, smem, stream>>>(args, tiles_n, iters);
         return cudaGetLastError();
     }
-    const bool wide = ta && !tb && !split_k && max_n >= 256;
-    const int bm = !wide && !split_k && max_n <= 32 && max_m >= 128 ? 128 : 64;
-    const int bn = wide ? kWideN : bm == 128 ? 32 : 64;
-    const int tiles_m = (max_m + bm - 1) / bm;
-    const int tiles_n = (max_n + bn - 1) / bn;
-    {
-        // (a batch has at most a few thousand tiles: one launch)
-        const int nb = batch;
-        dim3 grid(tiles_m * tiles_n, nb);
-        const bool alone = (size_t)grid.x * nb <= 148;
-        if (wide) {
-            constexpr size_t smem =
-                (size_t)kShallow * (kWideM + kWideN) * kGemmLds * sizeof(double);
-            static std::once_flag attr;
-            std::call_once(attr, [] {
-                cudaFuncSetAttribute(k_gemm_f64_tn_wide,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem);
-            });
-            k_gemm_f64_tn_wide<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n);
-        } else if (ta != tb && bm == 64) {
-            auto go = [&](auto fn, int stages, size_t stage_doubles) {
-                const size_t smem = stages * stage_doubles * sizeof(double);
-                cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem);
-                fn<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n, split_k ? 1 : 0);
-            };
-            constexpr size_t tn = 128 * kPipeLds, nt = 2 * kPipeK * kNtLds;
-            if (ta && alone) go(k_gemm_f64_tn_pipe<3>, 3, tn);
-            else if (ta) go(k_gemm_f64_tn_pipe<2>, 2, tn);
-            else if (alone) go(k_gemm_f64_nt_pipe<3>, 3, nt);
-            else go(k_gemm_f64_nt_pipe<2>, 2, nt);
-        } else if (bm == 128) launch_shape<128, 32>(ta, tb, args, nb, tiles_m, tiles_n, stream);
-        else launch_shape<64, 64>(ta, tb, args, nb, tiles_m, tiles_n, stream);
+    if (ta == tb) return cudaErrorInvalidValue;   // (no step multiplies A^T B^T)
+    // A^T B whose output is wide and (as for the projection B = Q^T D and the
+    // rotation C = W^T B) has a basis much narrower than the batch maximum as
+    // its rows: the fitted 64 x 128 kernel.  Else 64 x 64.
+    const bool wide = ta && !split_k && max_n >= 256;
+    const int tiles_m = (max_m + 63) / 64;
+    const int tiles_n = (max_n + (wide ? kWideN : 64) - 1) / (wide ? kWideN : 64);
+    const dim3 grid(tiles_m * tiles_n, batch);
+    const bool alone = (size_t)grid.x * batch <= 148;
+    if (wide) {
+        constexpr size_t smem =
+            (size_t)kShallow * (kWideM + kWideN) * kGemmLds * sizeof(double);
+        static std::once_flag attr;
+        std::call_once(attr, [] {
+            cudaFuncSetAttribute(k_gemm_f64_tn_wide,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        });
+        k_gemm_f64_tn_wide<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n);
+        return cudaGetLastError();
     }
+    auto go = [&](auto fn, int stages, size_t stage_doubles) {
+        const size_t smem = stages * stage_doubles * sizeof(double);
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        fn<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n, split_k ? 1 : 0);
+    };
+    constexpr size_t tn = 128 * kPipeLds, nt = 2 * kPipeK * kNtLds;
+    if (ta && alone) go(k_gemm_f64_tn_pipe<3>, 3, tn);
+    else if (ta) go(k_gemm_f64_tn_pipe<2>, 2, tn);
+    else if (alone) go(k_gemm_f64_nt_pipe<3>, 3, nt);
+    else go(k_gemm_f64_nt_pipe<2>, 2, nt);
     return cudaGetLastError();
 }
 

@@ -885,7 +885,8 @@ __device__ __forceinline__ double row_sum(double x, double *red)
 // left-looking product, trees over 32 rows and over warps), so both give
 // the same bits.  Phases R, R2 (nn <= the round's columns) and H (tiles of
 // 32 (W - 1) < nn <= 32 W rows: nn_lo, nn_hi).  81 tiles, 64 columns:
-// 215 -> 30 us; 81 tiles of up to 128 rows in phase H 286 -> 49 us.
+// 215 -> 75 us; 81 tiles of up to 128 rows in phase H 286 us in one launch ->
+// 125 us for 97 .. 128 rows, with the narrower ranges beside it.
 template <int W>
 __global__ void __launch_bounds__(32 * W)
 k_pivchol_rows(TileWork *__restrict__ tiles, Workspace ws, int phase, int nn_lo,
@@ -1500,10 +1501,9 @@ void launch_pivchol(int phase, TileWork *d_tiles, int ntiles, Workspace ws,
 // Gathers the pivot columns of Y into the Q buffer (phase A) or the Q1
 // buffer (phase B).
 __global__ void k_gather_cols(const TileWork *__restrict__ tiles,
-                              Workspace ws, int phase,
-                              const int *__restrict__ act)
+                              Workspace ws, int phase)
 {
-    const TileWork tw = tiles[act ? act[blockIdx.x] : blockIdx.x];
+    const TileWork tw = tiles[blockIdx.x];
     const int s = tw.slot;
     const int cnt = phase == PH_A ? tw.k1 : tw.kb;
     if (cnt <= 0) return;
@@ -1519,10 +1519,10 @@ __global__ void k_gather_cols(const TileWork *__restrict__ tiles,
 }
 
 void launch_gather_cols(int phase, const TileWork *d_tiles, int ntiles,
-                        Workspace ws, cudaStream_t stream, const int *act)
+                        Workspace ws, cudaStream_t stream)
 {
     dim3 grid(ntiles, 16);
-    k_gather_cols<<<grid, 256, 0, stream>>>(d_tiles, ws, phase, act);
+    k_gather_cols<<<grid, 256, 0, stream>>>(d_tiles, ws, phase);
 }
 
 // Cholesky G = R^T R of the re-orthogonalisation Gram in S(slot)
