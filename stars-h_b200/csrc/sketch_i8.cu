@@ -81,13 +81,22 @@ __host__ __device__ constexpr uint32_t idesc_i8(int n, bool a_signed)
 __device__ __forceinline__ void digits8(const double (&y)[8],
                                         uint32_t (&w)[kSlices][2])
 {
+    // (only the low byte of a top word is used, so 0x43380000 is not taken off)
     uint32_t lo[8], hi[8];
+    int top = 0;
     #pragma unroll
     for (int c = 0; c < 8; ++c) {
         lo[c] = (uint32_t)__double2loint(y[c]);
-        int top = __double2hiint(y[c]) - 0x43380000;
-        if (top > 127) { top = 127; lo[c] = 0xFFFFFFFFu; }
-        hi[c] = (uint32_t)top;
+        hi[c] = (uint32_t)__double2hiint(y[c]);
+        top = max(top, (int)hi[c]);
+    }
+    if (top > 0x43380000 + 127) {       // some q is 2^39 (rare)
+        #pragma unroll
+        for (int c = 0; c < 8; ++c)
+            if ((int)hi[c] > 0x43380000 + 127) {
+                hi[c] = 127;
+                lo[c] = 0xFFFFFFFFu;
+            }
     }
     #pragma unroll
     for (int g = 0; g < 2; ++g) {
@@ -138,6 +147,19 @@ __device__ __forceinline__ int row_exponent(const Workspace &ws, int m,
     return e;
 }
 
+// A role's place in a ring of N buffers: index and phase parity of its next
+// use (worked out from a running count, they were two 64-bit divisions a
+// chunk and thread).
+template <int N>
+struct Ring {
+    int i = 0;
+    uint32_t ph = 0;
+    __device__ __forceinline__ void next()
+    {
+        if (++i == N) { i = 0; ph ^= 1; }
+    }
+};
+
 // The tile fields the kernel reads, loaded once per item.
 struct SkItem {
     int m, n, bcur, slot, cols_done, status;
@@ -155,6 +177,13 @@ __device__ __forceinline__ SkItem sk_item(const TileWork *tiles, int tile)
 __device__ __forceinline__ bool sk_active(const SkItem &w, int need)
 {
     return w.bcur > 0 && (need == 0 || (w.status & need) != 0);
+}
+
+// The double of a 32-bit integer (two's complement in v), by its bits and
+// one subtraction (the conversion instructions run at a fraction of its rate).
+__device__ __forceinline__ double int_double(uint32_t v)
+{
+    return __hiloint2double(0x43300000, (int)(v ^ 0x80000000u)) - 0x1.000008p52;
 }
 
 // Y(:, 0:bcur) of every tile with an active round = D * Omega8(:, cols_done
@@ -221,7 +250,10 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
     const uint32_t tmem = tmem_base;
 
     int fail_tile = -1;          // a tile whose item this thread gave up on
-    long long gc = 0;            // chunks seen by this role (all items)
+    // this role's next chunk (over all items).  A wait for the phase before
+    // a barrier's first returns at once, so the first uses need no case.
+    Ring<kStages> st;
+    Ring<kAbufs> ab;
     int it = 0;                  // items processed by this CTA
 
     if (warp < kConvThreads / 32) {
@@ -251,28 +283,33 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
             const int sh = 39 - rowexp[it & 1][r];
             const double s1 = sh > 1000 ? ldexp(1.0, sh - 1000) : 1.0;
             const double s2 = ldexp(1.0, sh > 1000 ? 1000 : sh);
-            for (int kc = 0; kc < nchunks; ++kc, ++gc) {
-                const int sg = (int)(gc % kStages), b = (int)(gc & 1);
-                bool ok = mbar_wait_or(&full[sg], (uint32_t)(gc / kStages) & 1, &failed);
-                ok = ok && (gc < kAbufs ||
-                            mbar_wait_or(&afree[b], (uint32_t)((gc >> 1) - 1) & 1, &failed));
+            // all of this warp's rows inside the tile, one factor enough
+            const bool whole = __all_sync(0xffffffffu, i < w.m && sh <= 1000);
+            for (int kc = 0; kc < nchunks; ++kc, st.next(), ab.next()) {
+                bool ok = mbar_wait_or(&full[st.i], st.ph, &failed);
+                ok = ok && mbar_wait_or(&afree[ab.i], ab.ph ^ 1, &failed);
                 if (!__all_sync(0xffffffffu, ok ? 1 : 0)) {
                     fail_tile = tile_of(item);
                     failed = 1;
                     break;
                 }
-                const double *st = Dst + (size_t)sg * (kSkRows * kSkChunk);
+                const double *sd = Dst + st.i * (kSkRows * kSkChunk) + 8 * qd * kSkRows + r;
                 double y[8];
-                #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const int j = kc * kSkChunk + 8 * qd + c;
-                    double v = (i < w.m && j < w.n) ? st[(8 * qd + c) * kSkRows + r] : 0.0;
-                    if (sh > 1000) v *= s1;
-                    y[c] = fma(v, s2, magic);
+                if (whole && (kc + 1) * kSkChunk <= w.n) {
+                    #pragma unroll
+                    for (int c = 0; c < 8; ++c) y[c] = fma(sd[c * kSkRows], s2, magic);
+                } else {
+                    #pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const int j = kc * kSkChunk + 8 * qd + c;
+                        double v = (i < w.m && j < w.n) ? sd[c * kSkRows] : 0.0;
+                        if (sh > 1000) v *= s1;
+                        y[c] = fma(v, s2, magic);
+                    }
                 }
                 uint32_t dg[kSlices][2];
                 digits8(y, dg);
-                uint8_t *A = Abuf + b * kAbufBytes;
+                uint8_t *A = Abuf + ab.i * kAbufBytes;
                 #pragma unroll
                 for (int s = 0; s < kSlices; ++s)
                     *reinterpret_cast<uint2 *>(A + s * (kSkRows * kSkChunk) +
@@ -283,7 +320,7 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                 // one arrival per warp
                 asm volatile("fence.proxy.async.shared::cta;");
                 __syncwarp();
-                if ((t & 31) == 0) mbar_arrive(&afull[b]);
+                if ((t & 31) == 0) mbar_arrive(&afull[ab.i]);
             }
             if (failed) break;
             ++it;
@@ -302,10 +339,9 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                 const int row0 = (int)(item % rpt) * kSkRows;
                 if (!sk_active(w, need) || row0 >= w.m) continue;
                 const int nchunks = (w.n + kSkChunk - 1) / kSkChunk;
-                for (int kc = 0; kc < nchunks; ++kc, ++gc) {
-                    const int sg = (int)(gc % kStages);
-                    if (gc >= kStages &&
-                        !mbar_wait_or(&empty[sg], (uint32_t)(gc / kStages - 1) & 1, &failed)) {
+                for (int kc = 0; kc < nchunks; ++kc, st.next()) {
+                    const int sg = st.i;
+                    if (!mbar_wait_or(&empty[sg], st.ph ^ 1, &failed)) {
                         fail_tile = tile_of(item);
                         failed = 1;
                         break;
@@ -317,7 +353,7 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                     tma_load_om(o, &omap, kc * kSkChunk, w.cols_done, &full[sg]);
                     tma_load_om(o + nc * 16, &omap, kc * kSkChunk + 16, w.cols_done,
                                 &full[sg]);
-                    issued = gc + 1;
+                    ++issued;
                 }
             }
             // after a failure: the copies still in flight land before the
@@ -330,7 +366,8 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
         }
     } else if (warp == kMmaWarp) {
         // ----------------------------------------------------------- MMA
-        long long last = -1;
+        int last_b = -1;
+        uint32_t last_ph = 0;
         if (lane == 0) {
             const uint32_t idu = idesc_i8(nc, false), ids = idesc_i8(nc, true);
             SkItem wn = sk_item(tiles, tile_of(blockIdx.x));
@@ -344,9 +381,9 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                 const int nchunks = (w.n + kSkChunk - 1) / kSkChunk;
                 // the previous item's accumulators have been read out
                 bool ok = it == 0 || mbar_wait_or(&accempty, (uint32_t)(it - 1) & 1, &failed);
-                for (int kc = 0; ok && kc < nchunks; ++kc, ++gc) {
-                    const int sg = (int)(gc % kStages), b = (int)(gc & 1);
-                    if (!mbar_wait_or(&afull[b], (uint32_t)(gc >> 1) & 1, &failed)) {
+                for (int kc = 0; ok && kc < nchunks; ++kc, st.next(), ab.next()) {
+                    const int sg = st.i, b = ab.i;
+                    if (!mbar_wait_or(&afull[b], ab.ph, &failed)) {
                         ok = false;
                         break;
                     }
@@ -364,7 +401,8 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                     mma_commit(&empty[sg]);
                     mma_commit(&afree[b]);
                     if (kc == nchunks - 1) mma_commit(&accfull);
-                    last = gc;
+                    last_b = b;
+                    last_ph = ab.ph;
                 }
                 if (!ok) {
                     fail_tile = tile_of(item);
@@ -374,9 +412,9 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                 ++it;
             }
             // after a failure: the MMAs issued finish before TMEM is freed
-            if (failed && last >= 0) {
+            if (failed && last_b >= 0) {
                 int dummy = 0;
-                mbar_wait_or(&afree[last & 1], (uint32_t)(last >> 1) & 1, &dummy);
+                mbar_wait_or(&afree[last_b], last_ph, &dummy);
             }
         }
     } else {
@@ -426,6 +464,9 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
             asm volatile("tcgen05.fence::after_thread_sync;");
             double *Y = ws.Y(w.slot);
             const int ldY = ws.ldM();
+            // 2^(e - 39), while that is a normal number
+            const bool tiny = e - 39 < -1022;
+            const double sc = ldexp(1.0, tiny ? 0 : e - 39);
             for (int g = 0; g < nc / 8; ++g) {
                 uint32_t v[kSlices][8];
                 #pragma unroll
@@ -436,12 +477,15 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                     #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         const int col = 8 * g + c;
-                        long long T = (long long)(int)v[kSlices - 1][c];
+                        // T = sum_s v_s 256^s, |v_s| < 2^28: the four low
+                        // terms add up exactly below 2^53, so the last fma
+                        // rounds T once
+                        double T = int_double(v[0][c]);
                         #pragma unroll
-                        for (int s = kSlices - 2; s >= 0; --s)
-                            T = T * 256 + (long long)(int)v[s][c];
+                        for (int s = 1; s < kSlices; ++s)
+                            T = fma(int_double(v[s][c]), (double)(1ll << 8 * s), T);
                         if (col < w.bcur)
-                            Y[(size_t)col * ldY + i] = ldexp((double)T, e - 39);
+                            Y[(size_t)col * ldY + i] = tiny ? ldexp(T, e - 39) : T * sc;
                     }
                 }
             }
