@@ -67,8 +67,12 @@ static std::atomic<long long> g_launches{0};
 
 static bool create_lanes(SvdLanes &l)
 {
-    for (cudaStream_t &s : l.s)
-        if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess)
+    int least = 0, greatest = 0;
+    cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    for (int q = 0; q < SvdLanes::kStreams; ++q)
+        if (cudaStreamCreateWithPriority(&l.s[q], cudaStreamNonBlocking,
+                                         std::min(least, greatest + SvdLanes::rank(q))) !=
+            cudaSuccess)
             return false;
     for (cudaEvent_t &e : l.done)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)

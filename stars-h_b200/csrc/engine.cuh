@@ -188,9 +188,20 @@ __host__ __device__ constexpr int svd_bin_lo(int b) { return b == 0 ? 0 : svd_bi
 __host__ __device__ int svd_bin(int rows);
 
 // Streams and events the small SVD spreads its size ranges over (all null:
-// one stream): one for each range above 64 rows, and one more.
+// one stream): one for each range above 128 rows, then 113 .. 128, 81 .. 96,
+// 97 .. 112 and 65 .. 80 rows, and one more.  The ranges take CTAs by
+// priority, the largest rows first: their chains are the longest, and left
+// to the order in which the queues happen to drain they started last in some
+// processes (496 tiles of 512, sin(kr)/r: 4.1 or 5.2 ms).
 struct SvdLanes {
     static constexpr int kStreams = kSvdBins - kSvdBinLarge + 5;
+    static constexpr int kMid = kSvdBins - kSvdBinLarge;   // stream of 113 .. 128 rows
+    // steps below the greatest priority
+    static constexpr int rank(int q)
+    {
+        return q < kMid || q > kMid + 3 ? 0 : q == kMid ? 1 : q == kMid + 2 ? 2
+             : q == kMid + 1 ? 3 : 4;
+    }
     cudaStream_t s[kStreams] = {};
     cudaEvent_t fork = nullptr, large = nullptr;
     cudaEvent_t done[kStreams] = {};

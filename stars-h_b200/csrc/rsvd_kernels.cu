@@ -2291,7 +2291,7 @@ __host__ __device__ int svd_bin(int rows)
 // Phase H of the pivoted Cholesky and the Jacobi SVD on its factor, by
 // ranges of rows (svd_bin) on their own streams: the ranges are independent
 // chains of a few long launches that seldom fill the GPU one by one (81
-// tiles: 1.40 ms of Jacobi one after another, the longest of them 1.12 ms).
+// tiles: 1.40 ms of Jacobi one after another, the longest of them 0.84).
 // `count` (host) and `list` (device, kSvdBins lists of `list_ld` tiles) tell
 // the tiles of each range, so that only they are launched; null: every
 // range is launched over the whole batch, each CTA taking its tile or
@@ -2369,7 +2369,7 @@ int launch_small_svd(TileWork *d_tiles, int ntiles, Workspace ws,
         ++launches;
     }
     // 65 .. 128 rows: two ranges of the Gram factor, four of the Jacobi
-    constexpr int kLane2 = kSvdBins - kSvdBinLarge, kLane1 = kLane2 + 1;
+    constexpr int kLane2 = SvdLanes::kMid, kLane1 = kLane2 + 1;
     if (num(kBin128)) {
         const cudaStream_t s = lane(kLane2);
         pivchol_rows_launch<4>(d_tiles, num(kBin128), ws, PH_H, 113, 128, s, act(kBin128));

@@ -15,8 +15,8 @@
 // Each digit matrix times Omega is an exact 8-bit x int8 -> int32 product
 // (|sum| <= 255 * 127 * n < 2^31 for n <= 8192) on tcgen05.mma kind::i8
 // (unsigned A for u_s, signed A for t), accumulated in TMEM, one
-// accumulator per digit.  The epilogue recombines the digits in int64
-// (exact) and converts once:
+// accumulator per digit.  The epilogue adds the digits' sums up with FMAs,
+// of which only the last one rounds:
 //     Y_ic = 2^(e_i - 39) T_ic,  T_ic = sum_{s<4} 256^s P_s + 2^32 P_t.
 // The only error is the rounding of q: 2^-40 of the row maximum per entry,
 // far below the tolerance-driven thresholds of the adaptive basis (the
@@ -37,6 +37,11 @@
 //   * warps 18-21 (epilogue) read an item's accumulators from TMEM, write
 //     Y and release TMEM to the next item, while the copies and the
 //     conversion of that item's first chunks go on.
+// What bounds it is HBM, D being read once: 10000 tiles of 1024 x 1024 in
+// 15.7 ms, 5.7 TB/s of reads and writes (18.8 ms while the converters issued
+// about twice the instructions a chunk and an item's epilogue, which the
+// next item's MMAs wait for, worked in 64-bit integers).  Three or four digit
+// buffers in place of a fifth stage are slower (16.3 ms).
 // Hand-over is by mbarriers only; every wait gives up after about two
 // seconds or as soon as another thread has given up, and the CTA then
 // marks its tile TILE_MMA_TIMEOUT, waits for its own copies and MMAs in
