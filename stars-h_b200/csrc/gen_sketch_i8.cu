@@ -44,6 +44,7 @@
 #include <cstdint>
 #include "engine.cuh"
 #include "tc_common.cuh"
+#include "smem_limit.cuh"
 
 namespace b200 {
 
@@ -755,16 +756,8 @@ bool launch_gen_sketch_i8(const DevKernel *d_kernels, TileWork *d_tiles,
     if (npad > ld_om8) return false;
     CUtensorMap omap;
     if (!i8_colmajor_map(&omap, om8, ld_om8, om8_cols, nc)) return false;
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0, count = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(k_gen_sketch_i8,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kGsSmemBytes);
-        sms = count > 0 ? count : 148;
-    }
+    allow_smem<k_gen_sketch_i8, kGsSmemBytes>();
+    static const int sms = sm_count();
     const long long items = (long long)ntiles * ((ws.m_max + kGsRows - 1) / kGsRows);
     const int grid = (int)std::min<long long>(sms, items);
     if (grid <= 0) return true;

@@ -47,6 +47,7 @@
 #include <cstdint>
 #include "engine.cuh"
 #include "tc_common.cuh"
+#include "smem_limit.cuh"
 
 namespace b200 {
 
@@ -576,15 +577,8 @@ bool launch_proj_i8(TileWork *d_tiles, int ntiles, Workspace ws,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return false;
     }
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0, count = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(k_proj_i8, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kPjSmemBytes);
-        sms = count > 0 ? count : 148;
-    }
+    allow_smem<k_proj_i8, kPjSmemBytes>();
+    static const int sms = sm_count();
     const long long items = (long long)ntiles * ((ws.n_max + kPjCols - 1) / kPjCols);
     const int grid = (int)std::min<long long>(sms, items);
     if (grid > 0)

@@ -22,6 +22,7 @@
 #include <climits>
 #include <cooperative_groups.h>
 #include "engine.cuh"
+#include "smem_limit.cuh"
 
 namespace b200 {
 
@@ -1104,11 +1105,11 @@ static void pivchol_rows_launch(TileWork *d_tiles, int ntiles, Workspace ws,
                                 int phase, int nn_lo, int nn_hi,
                                 cudaStream_t stream, const int *act)
 {
+    // (the rounds, with two matrices, are launched for at most 64 rows)
+    constexpr size_t most = (size_t)(W <= 2 ? 2 : 1) * (32 * W) * (32 * W + 1) * sizeof(double);
     const size_t smem = (size_t)(phase == PH_H ? 1 : 2) * nn_hi * (32 * W + 1) *
                         sizeof(double);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_pivchol_rows<W>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem<k_pivchol_rows<W>, most>();
     k_pivchol_rows<W><<<ntiles, 32 * W, smem, stream>>>(d_tiles, ws, phase, nn_lo,
                                                         nn_hi, act);
 }
@@ -1313,14 +1314,16 @@ k_pivchol_cluster(TileWork *__restrict__ tiles, Workspace ws, int nn_lo, int nn_
 }
 
 // Most rows k_pivchol_cluster<CS> takes: a CTA's share of the Gram within
-// its shared memory (kJacobiSmemMax).
+// its shared memory.
+constexpr size_t kClusterSmemMax = 208 * 1024;
+
 template <int CS>
 static int pivchol_cluster_fit(int kmax)
 {
     int nn = std::min(kmax, 32 * kClusterMaxChunks);
     while (nn > 0 && (pivchol_cluster_warps<CS>(nn) * 32 > kClusterRows ||
                       (size_t)nn * 32 * pivchol_cluster_warps<CS>(nn) * sizeof(double) >
-                          208 * 1024))
+                          kClusterSmemMax))
         --nn;
     return nn;
 }
@@ -1334,7 +1337,7 @@ static void pivchol_cluster_launch(TileWork *d_tiles, int ntiles, Workspace ws,
     for (int nn = nn_lo; nn <= nn_hi; ++nn)
         smem = std::max(smem, (size_t)nn * 32 * pivchol_cluster_warps<CS>(nn) * sizeof(double));
     auto *fn = k_pivchol_cluster<CS>;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem<k_pivchol_cluster<CS>, kClusterSmemMax>();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(ntiles * CS));
     cfg.blockDim = dim3(kClusterRows);
@@ -1661,9 +1664,7 @@ static void chol_small_launch(int phase, TileWork *d_tiles, int ntiles,
                               Workspace ws, cudaStream_t stream, const int *act)
 {
     constexpr size_t smem = (size_t)2 * N * (N + 1) * sizeof(double);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_chol_inv_small<N>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem<k_chol_inv_small<N>, smem>();
     k_chol_inv_small<N><<<ntiles, 4 * N, smem, stream>>>(d_tiles, ws, phase, act);
 }
 
@@ -2243,8 +2244,10 @@ static void jacobi_block_launch(TileWork *d_tiles, int ntiles, Workspace ws,
     const int kmax = ws.k_max;
     auto *fn = k_jacobi_block<CLASS, G, E>;
     const size_t smem = (size_t)2 * (512 / G) * (max_rows | 1) * sizeof(double);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+    // (max_rows: at most the class's, and so its columns)
+    constexpr size_t most =
+        (size_t)2 * (512 / G) * (jacobi_class_cols(CLASS) | 1) * sizeof(double);
+    allow_smem<k_jacobi_block<CLASS, G, E>, most>();
     cudaLaunchConfig_t cfg = {};
     const int cs = jacobi_cluster(CLASS, kmax, ntiles, act != nullptr);
     cfg.gridDim = dim3((unsigned)(ntiles * cs));
@@ -2270,13 +2273,15 @@ static void jacobi_rows_launch(TileWork *d_tiles, int ntiles, Workspace ws,
 {
     auto *fn = k_jacobi<CLASS, G, E, THREADS, MINB, PAIRED>;
     size_t smem = 0;
-    if (E > 0) {
+    if constexpr (E > 0) {
         const int r = std::min(rows_hi, ws.k_max);
-        smem = (size_t)jacobi_stride<G, (E > 0 ? E : 1), PAIRED>(r) * r * sizeof(double);
+        smem = (size_t)jacobi_stride<G, E, PAIRED>(r) * r * sizeof(double);
         if (!PAIRED) smem = std::min(smem, kJacobiSmemMax);
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
+        // (rows_hi <= G E)
+        constexpr size_t full =
+            (size_t)jacobi_stride<G, E, PAIRED>(G * E) * (G * E) * sizeof(double);
+        constexpr size_t most = !PAIRED && full > kJacobiSmemMax ? kJacobiSmemMax : full;
+        allow_smem<k_jacobi<CLASS, G, E, THREADS, MINB, PAIRED>, most>();
     }
     fn<<<ntiles, THREADS, smem, stream>>>(d_tiles, ws, rows_lo, rows_hi, act);
 }
@@ -2588,9 +2593,7 @@ void launch_write_v(const TileWork *d_tiles, int ntiles, Workspace ws,
     // wide bases: at least 8 columns a pass
     const int doubles = std::max(kWriteVDoubles, 8 * (ws.k_max | 1));
     const size_t smem = (size_t)doubles * sizeof(double);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_write_v, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+    allow_smem<k_write_v, (size_t)8 * (kMaxK | 1) * sizeof(double)>();
     dim3 grid(ntiles, ntiles >= 148 ? 4 : 8);
     k_write_v<<<grid, 256, smem, stream>>>(d_tiles, ws, out, doubles);
 }

@@ -47,10 +47,12 @@
 // marks its tile TILE_MMA_TIMEOUT, waits for its own copies and MMAs in
 // flight and releases TMEM.
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cuda.h>
 #include "engine.cuh"
 #include "tc_common.cuh"
+#include "smem_limit.cuh"
 
 namespace b200 {
 
@@ -512,7 +514,7 @@ k_sketch_i8(const __grid_constant__ CUtensorMap dmap,
                      :: "r"(tmem), "r"(ncols_alloc));
 }
 
-static size_t sketch_i8_smem()
+static constexpr size_t sketch_i8_smem()
 {
     return (size_t)kAbufs * kAbufBytes + (size_t)kStages * kDStageBytes +
            (size_t)kStages * kOmSlotBytes + 1024;
@@ -526,8 +528,8 @@ bool sketch_i8_fits(int nc, int n_max)
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 {
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-    if (encode == nullptr) {
+    static std::atomic<PFN_cuTensorMapEncodeTiled_v12000> encode{nullptr};
+    if (encode.load() == nullptr) {
         void *fn = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn,
@@ -538,7 +540,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
         }
         encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
     }
-    return encode;
+    return encode.load();
 }
 
 // Tensor map of the batch's D blocks as one 3-D FP64 tensor (rows, columns,
@@ -588,15 +590,8 @@ bool launch_sketch_i8(const TileWork *d_tiles, int ntiles, int count,
     if (!d_tensor_map(&dmap, ws, ntiles) ||
         !i8_colmajor_map(&omap, om8, ld_om8, om8_cols, nc))
         return false;
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0, count = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(k_sketch_i8, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sketch_i8_smem());
-        sms = count > 0 ? count : 148;
-    }
+    allow_smem<k_sketch_i8, sketch_i8_smem()>();
+    static const int sms = sm_count();
     const long long items = (long long)count * ((ws.m_max + kSkRows - 1) / kSkRows);
     const int grid = (int)std::min<long long>(sms, items);
     if (grid <= 0) return true;

@@ -1,0 +1,140 @@
+"""What several host threads share when they launch kernels: the lanes of one
+call, the serving workers."""
+import ctypes
+import os
+import re
+import subprocess
+from ctypes import POINTER, c_double, c_int
+
+import numpy as np
+import pytest
+
+import starsh_b200 as sb
+from test_gpu_edges import ExpProblem
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "stars-h_b200", "csrc")
+
+
+def source(name):
+    """A source file without its comments."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = re.sub(r"/\*.*?\*/", "", f.read(), flags=re.S)
+    return re.sub(r"//[^\n]*", "", text)
+
+
+# A stand-in for the CUDA runtime's three calls: `limit` is the device-wide
+# limit of each function, `sets` counts the calls that set it.
+LIMIT_CHECK = r"""
+#include <cstdio>
+#include <map>
+#include <mutex>
+#include <thread>
+#include <vector>
+#include "smem_limit.cuh"
+static thread_local int current = 0;
+static std::mutex mu;
+static std::map<std::pair<int, const void *>, int> limit;
+static int sets = 0, refuse = 0;
+extern "C" cudaError_t cudaGetDevice(int *d) { *d = current; return cudaSuccess; }
+extern "C" cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { *v = 7; return cudaSuccess; }
+extern "C" cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute, int v)
+{
+    std::lock_guard<std::mutex> g(mu);
+    ++sets;
+    if (refuse) { --refuse; return cudaErrorInvalidValue; }
+    limit[{current, f}] = v;
+    return cudaSuccess;
+}
+static void a(int) {}
+static void b(int) {}
+#define CHECK(x) if (!(x)) { printf("line %d: %s\n", __LINE__, #x); return 1; }
+int main()
+{
+    refuse = 1;                         // a refused setting is tried again
+    CHECK((b200::allow_smem<a, 1000>() == cudaErrorInvalidValue));
+    CHECK((b200::allow_smem<a, 1000>() == cudaSuccess));
+    CHECK(sets == 2);
+    std::vector<std::thread> th;        // threads on three devices
+    for (int t = 0; t < 12; ++t)
+        th.emplace_back([t] {
+            current = t % 3;
+            for (int q = 0; q < 1000; ++q) {
+                b200::allow_smem<a, 1000>();
+                b200::allow_smem<b, 2000>();
+            }
+        });
+    for (auto &x : th) x.join();
+    CHECK(limit.size() == 6);
+    for (auto &x : limit) CHECK(x.second == (x.first.second == (const void *)a ? 1000 : 2000));
+    CHECK(sets <= 2 + 2 * 12);          // not once a call
+    current = 70;                       // beyond the devices remembered
+    const int before = sets;
+    b200::allow_smem<a, 1000>();
+    b200::allow_smem<a, 1000>();
+    CHECK(sets == before + 2);
+    CHECK(b200::sm_count() == 7);
+    return 0;
+}
+"""
+
+
+def test_limit_is_one_number_per_kernel_and_device(tmp_path):
+    src, exe = tmp_path / "limit.cpp", tmp_path / "limit"
+    src.write_text(LIMIT_CHECK)
+    subprocess.run(["g++", "-std=c++17", "-pthread", "-I", CSRC, "-I",
+                    "/usr/local/cuda/include", str(src), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+
+
+@pytest.mark.parametrize("name", ["rsvd_kernels.cu", "sketch_i8.cu", "gen_sketch_i8.cu",
+                                  "proj_i8.cu"])
+def test_engine_kernels_take_their_limit_once(name):
+    """No launch of the kernels that lanes and workers share sets a limit of
+    its own, and no plain static is filled in by whichever thread is first."""
+    text = source(name)
+    assert "allow_smem<" in text
+    assert "cudaFuncSetAttribute" not in text
+    assert not re.search(r"static int sms = 0|static PFN\w+ encode", text)
+
+
+def batch(lib, probs, tols, maxrank):
+    k = len(probs)
+    lib.starsh_set_oversample(b"10")
+    formats = (POINTER(sb.Blrf) * k)()
+    for p, pr in enumerate(probs):
+        F = POINTER(sb.Blrf)()
+        assert lib.starsh_blrf_new_tlr(ctypes.byref(F), pr.P, b"N", pr.C, pr.C) == 0
+        formats[p] = F
+    M = (POINTER(sb.Blrm) * k)()
+    info = lib.starsh_b200_approximate_batch(k, M, formats, (c_int * k)(*[maxrank] * k),
+                                             (c_double * k)(*tols), None, sb.ENGINE_MIXED, 0)
+    assert info == 0, (info, lib.starsh_b200_last_error())
+    return M
+
+
+def ranks(M):
+    return [np.ctypeslib.as_array(m.contents.far_rank,
+                                  shape=(m.contents.format.contents.nblocks_far,)).copy()
+            for m in M]
+
+
+@pytest.mark.gpu
+def test_lanes_with_different_basis_sizes(lib, monkeypatch):
+    """Two lanes whose batches hold bases of every range of 65 .. 160 rows
+    (kernels that share a function and differ in their shared memory) succeed
+    call after call, with the same ranks."""
+    tols = [7e-2, 5e-2, 3e-2, 1.8e-2, 1.1e-2]     # bases of about 75 to 135
+    probs = [ExpProblem(lib, 2000, 200, 0.5, seed=s) for s in range(len(tols))]
+    monkeypatch.setenv("STARSH_B200_WORKSPACE_MB", "80")
+    want = None
+    for _ in range(40):
+        M = batch(lib, probs, tols, 180)
+        assert sb.stats(lib).batches > 10
+        got = ranks(M)
+        want = want or got
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(a, b)
+        for m in M:
+            lib.starsh_blrm_free(m)
