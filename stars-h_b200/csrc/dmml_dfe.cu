@@ -23,6 +23,7 @@
 #include "device_ctx.cuh"
 #include "engine.cuh"
 #include "records.cuh"
+#include "smem_limit.cuh"
 #include "starsh-b200.h"
 
 namespace b200 {
@@ -359,13 +360,8 @@ static void launch_products(const Job1 *j1, int n1, const double *const *vcol,
 {
     constexpr size_t smem = (size_t)kPStages * prod_stage_doubles<FN>() * sizeof(double);
     constexpr size_t smem_b = (size_t)kPStages * prod_b_stage<FN>() * sizeof(double);
-    static std::once_flag attr;
-    std::call_once(attr, [] {
-        cudaFuncSetAttribute(k_prod_t<FN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-        cudaFuncSetAttribute(k_prod_b<FN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_b);
-    });
+    allow_smem<k_prod_t<FN>, smem>();
+    allow_smem<k_prod_b<FN>, smem_b>();
     const unsigned ny = (unsigned)((nrhs + 16 * FN - 1) / (16 * FN));
     if (n1 > 0) {
         k_prod_t<FN><<<dim3((unsigned)n1, ny, kPBM / kPRows), 256, smem, s>>>(j1, vcol, rowt, A,
@@ -616,13 +612,8 @@ static void launch_gemv(const Job1 *j1, int n1, const double *const *vcol,
 {
     constexpr size_t smem_t = (size_t)kGvStagesT * gv_stage_t<NR>() * sizeof(double);
     constexpr size_t smem_b = (size_t)kGvStagesB * gv_stage_b<NR>() * sizeof(double);
-    static std::once_flag attr;
-    std::call_once(attr, [] {
-        cudaFuncSetAttribute(k_gemv_t<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_t);
-        cudaFuncSetAttribute(k_gemv_b<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_b);
-    });
+    allow_smem<k_gemv_t<NR>, smem_t>();
+    allow_smem<k_gemv_b<NR>, smem_b>();
     if (n1 > 0) {
         k_gemv_t<NR><<<dim3((unsigned)n1, kPBM / kGvRowsT), 128, smem_t, s>>>(
             j1, vcol, rowt, A, lda, T, nrhs);

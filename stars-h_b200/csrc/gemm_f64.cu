@@ -8,8 +8,8 @@
 // k4 steps past its K (those would add exact zeros); the order of each sum is
 // the same in all of them (one chain over K, but for split_k).
 #include <cstdint>
-#include <mutex>
 #include "gemm_step.cuh"
+#include "smem_limit.cuh"
 
 namespace b200 {
 
@@ -811,6 +811,16 @@ k_gemm_f64_nn_short(const __grid_constant__ GemmArgs args, int tiles_n, int iter
     else nn_short<4>(d, m_first, m_last, n0, nn_smem);
 }
 
+// One launch of Kernel with Smem bytes of dynamic shared memory.
+template <auto Kernel, size_t Smem, class... Rest>
+static cudaError_t launch_gemm(dim3 grid, cudaStream_t stream, const GemmArgs &args,
+                               Rest... rest)
+{
+    allow_smem<Kernel, Smem>();
+    Kernel<<<grid, kGemmThreads, Smem, stream>>>(args, rest...);
+    return cudaGetLastError();
+}
+
 cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int batch,
                              int max_m, int max_n, cudaStream_t stream,
                              bool split_k)
@@ -820,30 +830,22 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int batch,
         const int tiles_n = (max_n + 63) / 64;
         if (args.step == STEP_SKETCH || args.step == STEP_A_SKETCH) {
             // 128 x 32 tiles for sketch blocks of at most 32 columns
-            auto go = [&](auto fn, int bm, int bn) {
-                const int smem = 2 * (bm + bn) * kGemmLds * (int)sizeof(double);
-                if (smem > 48 * 1024)
-                    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-                fn<<<dim3((max_m + bm - 1) / bm * tiles_n, batch), kGemmThreads, smem,
-                     stream>>>(args, tiles_n);
+            constexpr auto smem = [](int bm, int bn) {
+                return 2 * (bm + bn) * kGemmLds * sizeof(double);
             };
-            if (max_n <= 32 && max_m >= 128) go(k_gemm_f64<128, 32>, 128, 32);
-            else go(k_gemm_f64<64, 64>, 64, 64);
-            return cudaGetLastError();
+            if (max_n <= 32 && max_m >= 128)
+                return launch_gemm<k_gemm_f64<128, 32>, smem(128, 32)>(
+                    dim3((max_m + 127) / 128 * tiles_n, batch), stream, args, tiles_n);
+            return launch_gemm<k_gemm_f64<64, 64>, smem(64, 64)>(
+                dim3((max_m + 63) / 64 * tiles_n, batch), stream, args, tiles_n);
         }
         // four row blocks to a CTA where that still leaves two rounds of
         // CTAs, else one
         const int blocks = (max_m + kNnRows - 1) / kNnRows;
         const int iters = (size_t)((blocks + 3) / 4) * tiles_n * batch >= 592 ? 4 : 1;
         constexpr size_t smem = (size_t)kNnStages * kNnStage * sizeof(double);
-        static std::once_flag attr;
-        std::call_once(attr, [] {
-            cudaFuncSetAttribute(k_gemm_f64_nn_short,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        });
-        k_gemm_f64_nn_short<<<dim3((blocks + iters - 1) / iters * tiles_n, batch),
-                              kGemmThreads, smem, stream>>>(args, tiles_n, iters);
-        return cudaGetLastError();
+        return launch_gemm<k_gemm_f64_nn_short, smem>(
+            dim3((blocks + iters - 1) / iters * tiles_n, batch), stream, args, tiles_n, iters);
     }
     if (ta == tb) return cudaErrorInvalidValue;   // (no step multiplies A^T B^T)
     // A^T B whose output is wide and (as for the projection B = Q^T D and the
@@ -857,25 +859,18 @@ cudaError_t gemm_f64_batched(bool ta, bool tb, const GemmArgs &args, int batch,
     if (wide) {
         constexpr size_t smem =
             (size_t)kShallow * (kWideM + kWideN) * kGemmLds * sizeof(double);
-        static std::once_flag attr;
-        std::call_once(attr, [] {
-            cudaFuncSetAttribute(k_gemm_f64_tn_wide,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        });
-        k_gemm_f64_tn_wide<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n);
-        return cudaGetLastError();
+        return launch_gemm<k_gemm_f64_tn_wide, smem>(grid, stream, args, tiles_n);
     }
-    auto go = [&](auto fn, int stages, size_t stage_doubles) {
-        const size_t smem = stages * stage_doubles * sizeof(double);
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        fn<<<grid, kGemmThreads, smem, stream>>>(args, tiles_n, split_k ? 1 : 0);
-    };
-    constexpr size_t tn = 128 * kPipeLds, nt = 2 * kPipeK * kNtLds;
-    if (ta && alone) go(k_gemm_f64_tn_pipe<3>, 3, tn);
-    else if (ta) go(k_gemm_f64_tn_pipe<2>, 2, tn);
-    else if (alone) go(k_gemm_f64_nt_pipe<3>, 3, nt);
-    else go(k_gemm_f64_nt_pipe<2>, 2, nt);
-    return cudaGetLastError();
+    const int split = split_k ? 1 : 0;
+    constexpr size_t tn = 128 * kPipeLds * sizeof(double);          // a stage
+    constexpr size_t nt = 2 * kPipeK * kNtLds * sizeof(double);
+    if (ta && alone)
+        return launch_gemm<k_gemm_f64_tn_pipe<3>, 3 * tn>(grid, stream, args, tiles_n, split);
+    if (ta)
+        return launch_gemm<k_gemm_f64_tn_pipe<2>, 2 * tn>(grid, stream, args, tiles_n, split);
+    if (alone)
+        return launch_gemm<k_gemm_f64_nt_pipe<3>, 3 * nt>(grid, stream, args, tiles_n, split);
+    return launch_gemm<k_gemm_f64_nt_pipe<2>, 2 * nt>(grid, stream, args, tiles_n, split);
 }
 
 }  // namespace b200

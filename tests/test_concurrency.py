@@ -99,6 +99,16 @@ def test_engine_kernels_take_their_limit_once(name):
     assert not re.search(r"static int sms = 0|static PFN\w+ encode", text)
 
 
+@pytest.mark.parametrize("name", ["gemm_f64.cu", "dmml_dfe.cu"])
+def test_limits_hold_on_every_device(name):
+    """A limit is a device's: set once a process, a kernel that asks for more
+    than 48 KB could run on the first device alone (the entry without
+    allocations runs on whichever device is current)."""
+    text = source(name)
+    assert "allow_smem<" in text
+    assert "cudaFuncSetAttribute" not in text and "once_flag" not in text
+
+
 def batch(lib, probs, tols, maxrank):
     k = len(probs)
     lib.starsh_set_oversample(b"10")
