@@ -981,10 +981,9 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
                              step == STEP_A_RES_Z2 || step == STEP_A_GRAM2 ||
                              step == STEP_A_ORTH_Z || step == STEP_A_GRAM_R ||
                              step == STEP_GRAM_B;
-        return gemm_f64_batched(ta, tb, args, compact ? round_count : nt, mm, nn,
-                                s, split_k) == cudaSuccess
-                   ? STARSH_SUCCESS
-                   : cuda_fail(cudaGetLastError(), "gemm_f64_batched");
+        const cudaError_t e = gemm_f64_batched(ta, tb, args, compact ? round_count : nt,
+                                               mm, nn, s, split_k);
+        return e == cudaSuccess ? STARSH_SUCCESS : cuda_fail(e, "gemm_f64_batched");
     };
 
     for (size_t pi; info == STARSH_SUCCESS && !failed &&
@@ -1219,6 +1218,8 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         if ((info = gemm(STEP_GRAM_B, false, true, nt, k_basis, k_basis, none))) break;
         count_launch(launch_small_svd(dt, nt, ws, s, ctx.lanes, listed ? bins : nullptr,
                                       listed ? (const int *)ctx.act.ptr + nt : nullptr, nt));
+        const cudaError_t svd_error = cudaGetLastError();
+        if (svd_error != cudaSuccess) { info = cuda_fail(svd_error, "small SVD"); break; }
         if ((info = gemm(STEP_ROTATE, true, false, nt, k_basis, plan[pi].n, none))) break;
         launch_rank_cut(dt, nt, ws, s);
         count_launch();

@@ -155,9 +155,8 @@ extern "C" int starsh_b200_dense_rsvd_noalloc(const double *dD, int nrows,
     auto gemm = [&](GemmStep step, bool ta, bool tb, int mm, int nn,
                     OutArena o) -> int {
         const GemmArgs args{step, dt, nullptr, ws, omega, ncols, o};
-        return gemm_f64_batched(ta, tb, args, 1, mm, nn, s) == cudaSuccess
-                   ? STARSH_SUCCESS
-                   : cuda_fail(cudaGetLastError(), "no-alloc gemm");
+        const cudaError_t e = gemm_f64_batched(ta, tb, args, 1, mm, nn, s);
+        return e == cudaSuccess ? STARSH_SUCCESS : cuda_fail(e, "no-alloc gemm");
     };
     const int m = nrows, n = ncols;
     if ((info = gemm(STEP_SKETCH, false, false, m, k, none))) return info;
@@ -183,6 +182,7 @@ extern "C" int starsh_b200_dense_rsvd_noalloc(const double *dD, int nrows,
     if ((info = gemm(STEP_PROJECT, true, false, k, n, none))) return info;
     if ((info = gemm(STEP_GRAM_B, false, true, k, k, none))) return info;
     launch_small_svd(dt, 1, ws, s, SvdLanes{});
+    B200_CUDA(cudaGetLastError(), "no-alloc small SVD");
     if ((info = gemm(STEP_ROTATE, true, false, k, n, none))) return info;
     launch_rank_cut(dt, 1, ws, s);
     // One tile: its factors start at offset 0 of the caller's buffers, so

@@ -109,6 +109,19 @@ def test_limits_hold_on_every_device(name):
     assert "cudaFuncSetAttribute" not in text and "once_flag" not in text
 
 
+@pytest.mark.parametrize("name", ["engine.cu", "noalloc.cu"])
+def test_a_refused_launch_is_reported_as_what_it_was(name):
+    """gemm_f64_batched returns the launch error and thereby clears it: asked
+    for once more, the runtime knows of none ("no error").  The small SVD's
+    launches are looked at before the next product's."""
+    text = source(name)
+    calls = re.findall(r"gemm_f64_batched\(ta.*?;\s*return[^;]*;", text, flags=re.S)
+    assert calls and all("cudaGetLastError" not in c and "cuda_fail(e," in c for c in calls)
+    for m in re.finditer(r"launch_small_svd\(", text):
+        after = text[m.end():m.end() + 500]
+        assert 0 <= after.find("cudaGetLastError()") < after.find("gemm(STEP_ROTATE")
+
+
 def batch(lib, probs, tols, maxrank):
     k = len(probs)
     lib.starsh_set_oversample(b"10")
