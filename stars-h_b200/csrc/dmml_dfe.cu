@@ -395,6 +395,7 @@ constexpr int kGvRowsT = 64;         // ... rows of T of a CTA
 constexpr int kGvStagesT = 3;
 constexpr int kGvKB = 32;            // phase 2: K of a stage
 constexpr int kGvRowsB = 64;         // ... rows of a CTA
+constexpr int kGvThreadsB = 2 * kGvRowsB;   // ... half of them sum, half copy
 constexpr int kGvStagesB = 4;
 constexpr int kGvAhead = 3;          // ... stages a column pointer is read ahead
 
@@ -484,12 +485,21 @@ struct GvStage {
     int ldx, k, rs;      // K indices in use; doubles between rows of col
 };
 
+// The copying and the summing warps meet once a stage, each in a loop of its
+// own: a named barrier, which counts threads wherever they arrive from
+// (__syncthreads() is one place that all threads of the CTA pass).  Warps
+// arrive whole: both loops' conditions are the warp's.
+__device__ __forceinline__ void gvb_sync()
+{
+    asm volatile("barrier.sync.aligned 1, %0;" ::"n"(kGvThreadsB) : "memory");
+}
+
 // Phase 2: 64 output rows (K over the row's left-factor columns, then its
 // near blocks).  Two warps own the chains, a row per lane, and do nothing
 // else; the other two keep the ring filled, their column pointers read
 // three stages ahead.
 template <int NR>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kGvThreadsB)
 k_gemv_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
          const double *__restrict__ T, int nrhs,
          const NearPiece *__restrict__ near, const double *__restrict__ nearD,
@@ -568,7 +578,7 @@ k_gemv_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
                 const int st = st0 + q;
                 if (st >= total) break;
                 asm volatile("cp.async.wait_group %0;\n" ::"n"(kGvStagesB - 2));
-                __syncthreads();
+                gvb_sync();
                 if (st + kGvStagesB - 1 < total) {
                     issue(g[q], st + kGvStagesB - 1);
                     g[q] = describe();
@@ -580,7 +590,7 @@ k_gemv_b(const Job2 *__restrict__ jobs, const double *const *__restrict__ ucol,
     }
     double acc[NR] = {};
     for (int st = 0; st < total; ++st) {
-        __syncthreads();               // landed, and the refilled one consumed
+        gvb_sync();                    // landed, and the refilled one consumed
         const double *S = gvb_sm + st % kGvStagesB * STAGE + t;
         const double2 *X = reinterpret_cast<const double2 *>(
             gvb_sm + st % kGvStagesB * STAGE + kGvRowsB * kGvKB);
@@ -620,7 +630,7 @@ static void launch_gemv(const Job1 *j1, int n1, const double *const *vcol,
         count_launch();
     }
     if (n2 > 0) {
-        k_gemv_b<NR><<<dim3((unsigned)n2, kPBM / kGvRowsB), 128, smem_b, s>>>(
+        k_gemv_b<NR><<<dim3((unsigned)n2, kPBM / kGvRowsB), kGvThreadsB, smem_b, s>>>(
             j2, ucol, T, nrhs, near, nearD, A, lda, B, ldb, alpha, beta);
         count_launch();
     }

@@ -122,6 +122,19 @@ def test_a_refused_launch_is_reported_as_what_it_was(name):
         assert 0 <= after.find("cudaGetLastError()") < after.find("gemm(STEP_ROTATE")
 
 
+def test_roles_of_a_cta_meet_at_a_named_barrier():
+    """k_gemv_b's copying and summing warps each run their own loop: they meet
+    at a barrier that counts arrivals (both sides, all of the CTA's threads),
+    not at two different __syncthreads()."""
+    text = source("dmml_dfe.cu")
+    body = text[text.index("k_gemv_b("):]
+    body = body[:body.index("static void launch_gemv")]
+    assert "__syncthreads" not in body and body.count("gvb_sync();") == 2
+    assert re.search(r'"barrier\.sync\.aligned 1, %0;" ::"n"\(kGvThreadsB\) : "memory"', text)
+    assert re.search(r"__launch_bounds__\(kGvThreadsB\)\s*k_gemv_b\(", text)
+    assert re.search(r"k_gemv_b<NR><<<dim3\([^;]*?\), kGvThreadsB,", text)
+
+
 def batch(lib, probs, tols, maxrank):
     k = len(probs)
     lib.starsh_set_oversample(b"10")
