@@ -20,7 +20,10 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <map>
+#include <string>
+#include <system_error>
 #include <unordered_map>
 #include <vector>
 
@@ -1385,19 +1388,38 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         if (ready) cudaEventDestroy(ready);
         return info;
     }
-    // the helper's lane; its error text and statistics join this thread's
+    // the helper's lane; its error text and statistics join this thread's.
+    // Without a thread for it (the system's limit), this lane takes every
+    // batch; no exception leaves the helper's, and its thread is waited for
+    // whatever this lane does.
     int info2 = STARSH_SUCCESS;
     std::string error2;
     starsh_b200_stats st2;
     memset(&st2, 0, sizeof(st2));
-    std::thread other([&] {
-        cudaSetDevice(helper->device);
-        info2 = run_lane(*helper, st2);
-        if (info2) {
+    struct Helper {
+        std::thread t;
+        std::atomic<bool> &failed;
+        void join() { if (t.joinable()) t.join(); }
+        ~Helper()
+        {
+            if (!t.joinable()) return;
             failed = true;
-            error2 = t_error;
+            t.join();
         }
-    });
+    } other{{}, failed};
+    try {
+        other.t = std::thread([&] {
+            try {
+                cudaSetDevice(helper->device);
+                info2 = run_lane(*helper, st2);
+                if (info2) error2 = t_error;
+            } catch (const std::exception &) {
+                info2 = STARSH_MALLOC_ERROR;
+            }
+            if (info2) failed = true;
+        });
+    } catch (const std::system_error &) {
+    }
     int info = run_lane(ctx, st);
     if (info) failed = true;
     other.join();
@@ -1405,7 +1427,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     add_stats(st, st2);
     if (info == STARSH_SUCCESS && info2) {
         info = info2;
-        t_error = error2;
+        t_error = error2.empty() ? "out of host memory in the second lane" : error2;
     }
     // the parts in the order of the batches, whichever lane was first
     for (ProblemJob &jb : jobs)

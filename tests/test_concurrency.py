@@ -4,6 +4,7 @@ import ctypes
 import os
 import re
 import subprocess
+import sys
 from ctypes import POINTER, c_double, c_int
 
 import numpy as np
@@ -133,6 +134,41 @@ def test_roles_of_a_cta_meet_at_a_named_barrier():
     assert re.search(r'"barrier\.sync\.aligned 1, %0;" ::"n"\(kGvThreadsB\) : "memory"', text)
     assert re.search(r"__launch_bounds__\(kGvThreadsB\)\s*k_gemv_b\(", text)
     assert re.search(r"k_gemv_b<NR><<<dim3\([^;]*?\), kGvThreadsB,", text)
+
+
+# Two lanes, then the same call where the system refuses every new thread (a
+# default stack larger than the address space).
+NO_THREAD = r"""
+import ctypes, sys
+sys.path[:0] = %r
+import numpy as np
+import starsh_b200 as sb
+import test_concurrency as tc
+from test_gpu_edges import ExpProblem
+lib = sb.load()
+assert lib.starsh_b200_set_device(0) == 0
+probs = [ExpProblem(lib, 2000, 200, 0.5, seed=s) for s in range(2)]
+def call():
+    M = tc.batch(lib, probs, [5e-2, 1.1e-2], 180)
+    assert sb.stats(lib).batches > 4
+    return np.concatenate(tc.ranks(M))
+want = call()
+libc = ctypes.CDLL(None)
+attr = ctypes.create_string_buffer(256)
+assert libc.pthread_attr_init(attr) == 0
+assert libc.pthread_attr_setstacksize(attr, ctypes.c_size_t(1 << 47)) == 0
+assert libc.pthread_setattr_default_np(attr) == 0
+np.testing.assert_array_equal(call(), want)
+print("done")
+"""
+
+
+@pytest.mark.gpu
+def test_one_lane_where_no_thread_can_be_had(lib):
+    code = NO_THREAD % [os.path.join(ROOT, d) for d in ("stars-h_b200", "oracle", "tests")]
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
+                       env=dict(os.environ, STARSH_B200_WORKSPACE_MB="80"))
+    assert r.returncode == 0 and "done" in r.stdout, r.stderr[-2000:]
 
 
 def batch(lib, probs, tols, maxrank):
