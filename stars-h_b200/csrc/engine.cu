@@ -858,10 +858,10 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     };
     make_plan(budget);
     // Two lanes: the batches are dealt, as they come free, to two host
-    // threads with their own streams and workspaces (half the budget each),
-    // so that the chains of small launches of one batch's rounds and small
-    // SVDs run beside the other's full-width kernels, and neither waits for
-    // the host's reads.  Where the adaptive engine's tiles need several
+    // threads with their own streams (and half of the workspace each), so
+    // that the chains of small launches of one batch's rounds and small SVDs
+    // run beside the other's full-width kernels, and neither waits for the
+    // host's reads.  Where the adaptive engine's tiles need several
     // batches anyway, in at least three parts (the first, the near-diagonal
     // tiles, has the longest rounds and SVDs): 24 mixed problems 64.0 to
     // 54.9 ms, N = 65536 1/r 93.8 to 89.9, N = 102400 square exponential
@@ -878,20 +878,25 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     Context *helper = lanes > 1 ? context_helper(ctx) : nullptr;
     if (helper == nullptr) lanes = 1;
     if (lanes > 1) {
-        budget /= 2;
         part = (ntot + 2) / 3;
-        make_plan(budget);
+        make_plan(budget / 2);
     }
-    // What the lanes already hold needs no look at the free memory (the
-    // driver's answer takes 0.1 ms and, on a busy host, tens of
-    // milliseconds); to grow, take at most half of it.
-    const size_t held = std::min(ctx.workspace.bytes,
-                                 helper ? helper->workspace.bytes : (size_t)-1);
-    if (ws_need > held) {
+    // One workspace, a part of it for each lane.  What is held already needs
+    // no look at the free memory (the driver's answer takes 0.1 ms and, on a
+    // busy host, tens of milliseconds); to grow, take at most half of the
+    // free memory, where that is more than what is held.
+    if (lanes * ws_need > ctx.workspace.bytes) {
         size_t free_b = 0, total_b = 0;
         cudaMemGetInfo(&free_b, &total_b);
-        if (free_b / 2 / lanes < budget) make_plan(free_b / 2 / lanes);
+        const size_t most = std::max(ctx.workspace.bytes, free_b / 2);
+        if (most < budget) make_plan(most / lanes);
     }
+    if (!ctx.workspace.reserve(lanes * ws_need, s)) {
+        lanes = 1;
+        if (!ctx.workspace.reserve(ws_need, s))
+            return cuda_fail(cudaErrorMemoryAllocation, "workspace");
+    }
+    double *const workspace = (double *)ctx.workspace.ptr;
     // what the lanes' streams read was uploaded on this one
     cudaEvent_t ready = nullptr;
     if (lanes > 1) {
@@ -901,7 +906,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     std::atomic<size_t> next_batch{0};
     std::atomic<bool> failed{false};
     std::mutex rec_lock;      // the records' lists of parts
-    auto run_lane = [&](Context &ctx, starsh_b200_stats &st) -> int {
+    auto run_lane = [&](Context &ctx, double *workspace, starsh_b200_stats &st) -> int {
     // every return waits for what the lane still has in flight: the batch
     // downloads, and on failure kernels (what they touch is freed with the
     // records)
@@ -920,8 +925,6 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     cudaStream_t s = ctx.stream;
     if (const int e = mapped_area(ctx)) return e;
     if (ready) cudaStreamWaitEvent(s, ready, 0);
-    if (!ctx.workspace.reserve(ws_need, s))
-        return cuda_fail(cudaErrorMemoryAllocation, "workspace");
     if (!ctx.tiles.reserve((size_t)max_slots * sizeof(TileWork), s) ||
         !ctx.flag.reserve(256, s) ||
         !ctx.act.reserve((size_t)max_slots * (1 + kSvdBins) * sizeof(int), s))
@@ -995,7 +998,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         const int nt = plan[pi].nt;
         const int m_max = plan[pi].m, k_max = plan[pi].k;
         workspace_layout(ws, plan[pi].m, plan[pi].n, plan[pi].k, true, proj_i8);
-        ws.base = (double *)ctx.workspace.ptr;
+        ws.base = workspace;
         ws.stride = plan[pi].stride;
         for (int t = 0; t < nt; ++t) all[b0 + t].slot = t;
         // Round 0 of the adaptive engine with the generation fused into the
@@ -1384,7 +1387,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     };
 
     if (lanes == 1 || plan.size() == 1) {
-        const int info = run_lane(ctx, st);
+        const int info = run_lane(ctx, workspace, st);
         if (ready) cudaEventDestroy(ready);
         return info;
     }
@@ -1411,7 +1414,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         other.t = std::thread([&] {
             try {
                 cudaSetDevice(helper->device);
-                info2 = run_lane(*helper, st2);
+                info2 = run_lane(*helper, workspace + ws_need / sizeof(double), st2);
                 if (info2) error2 = t_error;
             } catch (const std::exception &) {
                 info2 = STARSH_MALLOC_ERROR;
@@ -1420,7 +1423,7 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
         });
     } catch (const std::system_error &) {
     }
-    int info = run_lane(ctx, st);
+    int info = run_lane(ctx, workspace, st);
     if (info) failed = true;
     other.join();
     cudaEventDestroy(ready);

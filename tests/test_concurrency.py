@@ -136,6 +136,47 @@ def test_roles_of_a_cta_meet_at_a_named_barrier():
     assert re.search(r"k_gemv_b<NR><<<dim3\([^;]*?\), kGvThreadsB,", text)
 
 
+# The device memory a process holds after a one-lane call that fills the
+# workspace and a two-lane call after it.
+HELD = r"""
+import ctypes, sys
+sys.path[:0] = %r
+import starsh_b200 as sb
+import test_concurrency as tc
+from harness import approximate_b200
+from test_gpu_edges import ExpProblem
+lib = sb.load()
+assert lib.starsh_b200_set_device(0) == 0
+cu = ctypes.CDLL("libcuda.so.1")
+def used():
+    pool, v = ctypes.c_void_p(), ctypes.c_uint64()
+    assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    assert cu.cuMemPoolGetAttribute(pool, 7, ctypes.byref(v)) == 0   # used now
+    return v.value / 2.0**20
+pr = ExpProblem(lib, 4000, 500, 0.5)
+lib.starsh_blrm_free(approximate_b200(lib, pr.F, 180, 1e-1, engine=sb.ENGINE_FP64, flags=0))
+assert sb.stats(lib).batches > 1
+one = used()
+for M in tc.batch(lib, [ExpProblem(lib, 4000, 500, 0.5, seed=1)], [1e-1], 180):
+    lib.starsh_blrm_free(M)
+assert sb.stats(lib).batches > 1
+print("held", one, used())
+"""
+
+
+@pytest.mark.gpu
+def test_lanes_share_the_workspace(lib):
+    """400 MB for a call's batches in flight are 400 MB whichever lanes the
+    calls took (and a few MB of sketch matrices and tile records)."""
+    code = HELD % [os.path.join(ROOT, d) for d in ("stars-h_b200", "oracle", "tests")]
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
+                       env=dict(os.environ, STARSH_B200_WORKSPACE_MB="400"))
+    assert r.returncode == 0, r.stderr[-2000:]
+    line = [x for x in r.stdout.splitlines() if x.startswith("held")][0].split()
+    one, two = float(line[1]), float(line[2])
+    assert 350 < one < 440 and two < 440, line
+
+
 # Two lanes, then the same call where the system refuses every new thread (a
 # default stack larger than the address space).
 NO_THREAD = r"""
