@@ -31,6 +31,7 @@ With N > 1 (torchrun) every rank runs an independent replica on its own GPU
 (the path does not shard); value = all ranks' entries / max rank time.
 """
 import argparse
+import contextlib
 import ctypes
 import json
 import os
@@ -431,6 +432,9 @@ def run_c4(args, lib, stream, clocks, torch):
         worst = max(worst, err / probs[i]["tol"])
     free_all(Ms, Fs)
     t_dev = statistics.mean(times)
+    with one_lane():
+        Ms, Fs, _, st1 = batched(sb.ENGINE_MIXED)
+    free_all(Ms, Fs)
     Ms, Fs, t_fp64_batched, _ = batched(sb.ENGINE_FP64)
     free_all(Ms, Fs)
     t_seq_fp64 = sequential(sb.ENGINE_FP64)
@@ -465,9 +469,10 @@ def run_c4(args, lib, stream, clocks, torch):
                        "chosen_over_plain": t_seq_fp64 / t_dev},
         "mixed_one_at_a_time": {"value": entries / t_seq_mixed / 1e6,
                                 "ms": t_seq_mixed * 1e3},
-        "phases_ms": {"gen": st.gen_ms, "basis": st.basis_ms,
-                      "project": st.project_ms, "svd": st.svd_ms,
-                      "output": st.output_ms},
+        "phases_ms": {"gen": st1.gen_ms, "basis": st1.basis_ms,
+                      "project": st1.project_ms, "svd": st1.svd_ms,
+                      "output": st1.output_ms},
+        "phases_what": PHASES_WHAT,
         "gpu_launches": int(st.kernel_launches),
         "clocks": clocks.summary(),
     }
@@ -643,6 +648,23 @@ def run_c5(args, lib, clocks):
     }
     print(json.dumps(line))
 
+
+@contextlib.contextmanager
+def one_lane():
+    """The library's calls on one lane: with two, the phases of a call run
+    beside each other and their times, added up, are no kernel's own."""
+    saved = os.environ.get("STARSH_B200_LANES")
+    os.environ["STARSH_B200_LANES"] = "1"
+    try:
+        yield
+    finally:
+        if saved is None:
+            del os.environ["STARSH_B200_LANES"]
+        else:
+            os.environ["STARSH_B200_LANES"] = saved
+
+
+PHASES_WHAT = "one more, untimed call on one lane (STARSH_B200_LANES=1)"
 
 # ------------------------------------------------------------- clocks
 
@@ -1205,6 +1227,11 @@ def main():
     step_times = []
     t_dev, sts, err, kept = measure(chosen, clocks, keep=bool(wl.get("dmml_nrhs")))
     last = sts[-1]
+    # the phases' times and the rates of single kernels
+    with one_lane():
+        for _ in range(2):     # (the first may enlarge the workspace)
+            M, F, _, _, alone = step(chosen, 0)
+            free(M, F)
     if chosen != sb.ENGINE_FP64:
         t_plain, _, err_plain, _ = measure(sb.ENGINE_FP64)
     else:
@@ -1284,12 +1311,12 @@ def main():
     # D once per round from HBM (bound: HBM; algorithmic bytes = 8 m n per
     # tile and round + the Y columns written); the FP64 engine's sketch is
     # a DMMA GEMM (bound: FP64 tensor, 2 m n k flops per tile)
-    per_launch_s = last.sketch_ms / 1e3 / max(1, last.sketch_launches)
-    if last.fused_launches > 0:
+    per_launch_s = alone.sketch_ms / 1e3 / max(1, alone.sketch_launches)
+    if alone.fused_launches > 0:
         # the fused generation + first-round sketch: it writes D (8 m n per
         # tile) and the round's Y columns; its inputs are the points
-        per_launch_s = last.fused_ms / 1e3 / last.fused_launches
-        bytes_per_launch = last.fused_bytes / last.fused_launches
+        per_launch_s = alone.fused_ms / 1e3 / alone.fused_launches
+        bytes_per_launch = alone.fused_bytes / alone.fused_launches
         achieved = bytes_per_launch / per_launch_s / 1e9
         peak, peak_src = measured_hbm_gbs()
         roof = {"bound": "hbm",
@@ -1298,9 +1325,9 @@ def main():
                 "frac": achieved / peak, "peak_source": peak_src,
                 "algorithmic_bytes_per_launch": bytes_per_launch,
                 "traffic": None,
-                "resketch_tiles": int(last.resketch_tiles)}
-    elif last.sketch_int8:
-        bytes_per_launch = last.sketch_bytes / max(1, last.sketch_launches)
+                "resketch_tiles": int(alone.resketch_tiles)}
+    elif alone.sketch_int8:
+        bytes_per_launch = alone.sketch_bytes / max(1, alone.sketch_launches)
         achieved = bytes_per_launch / per_launch_s / 1e9
         peak, peak_src = measured_hbm_gbs()
         roof = {"bound": "hbm", "kernel": "k_sketch_i8 (tcgen05 int8 slices, Y = D Omega8)",
@@ -1313,7 +1340,7 @@ def main():
                 "traffic": bytes_per_launch * SKETCH_TRAFFIC_RATIO,
                 "traffic_source": "ncu capture of a 256-tile case, scaled by tiles"}
     else:
-        flops_per_launch = last.sketch_flops / max(1, last.sketch_launches)
+        flops_per_launch = alone.sketch_flops / max(1, alone.sketch_launches)
         achieved = flops_per_launch / per_launch_s / 1e12
         peak = fp64_peak_tflops(torch)
         roof = {"bound": "tensor", "kernel": "k_gemm_f64 (sketch Y = D Omega, FP64 DMMA)",
@@ -1355,12 +1382,14 @@ def main():
                 "last_step_device_phases_ms": {
                     "generation": e2e_st.gen_ms, "sketch": e2e_st.sketch_ms,
                     "basis": e2e_st.basis_ms, "project": e2e_st.project_ms,
-                    "svd": e2e_st.svd_ms, "output": e2e_st.output_ms}},
+                    "svd": e2e_st.svd_ms, "output": e2e_st.output_ms,
+                    "what": "added over the call's lanes, whose phases overlap"}},
         "gpu_launches": int(sum(s.kernel_launches for s in sts)),
-        "phases_ms": {"generation": last.gen_ms, "fused_gen_sketch": last.fused_ms,
-                      "sketch": last.sketch_ms, "basis": last.basis_ms,
-                      "project": last.project_ms, "svd": last.svd_ms,
-                      "output": last.output_ms, "total_host": last.total_ms},
+        "phases_ms": {"generation": alone.gen_ms, "fused_gen_sketch": alone.fused_ms,
+                      "sketch": alone.sketch_ms, "basis": alone.basis_ms,
+                      "project": alone.project_ms, "svd": alone.svd_ms,
+                      "output": alone.output_ms, "total_host": alone.total_ms},
+        "phases_what": PHASES_WHAT,
         "roofline": roof,
         "clocks": clocks.summary(),
     }
@@ -1369,22 +1398,22 @@ def main():
     # the other large kernels of the step, each against its own bound:
     # the generator writes D once (8 B per entry; its limit is FP64 issue),
     # the projection B = Q^T D is an FP64 DMMA contraction
-    if chosen == sb.ENGINE_MIXED and last.gen_ms > 0 and last.project_ms > 0:
+    if chosen == sb.ENGINE_MIXED and alone.gen_ms > 0 and alone.project_ms > 0:
         dgemm = dmml["dgemm_tflops_in_run"] if dmml else fp64_peak_tflops(torch)
         hbm_peak, hbm_src = measured_hbm_gbs()
-        gen_entries = float(last.entries)
+        gen_entries = float(alone.entries)
         line["rooflines_other"] = {
             "generation (k_gen_tiles)": {
                 "bound": "fp64 issue (an exp or Bessel evaluation per entry)",
-                "entries_per_s": gen_entries / (last.gen_ms / 1e3),
-                "d_write_gbs": 8.0 * gen_entries / (last.gen_ms / 1e3) / 1e9,
-                "frac_of_hbm": 8.0 * gen_entries / (last.gen_ms / 1e3) / 1e9 / hbm_peak,
+                "entries_per_s": gen_entries / (alone.gen_ms / 1e3),
+                "d_write_gbs": 8.0 * gen_entries / (alone.gen_ms / 1e3) / 1e9,
+                "frac_of_hbm": 8.0 * gen_entries / (alone.gen_ms / 1e3) / 1e9 / hbm_peak,
                 "hbm_peak_source": hbm_src},
-            "projection (k_gemm_f64 TN, B = Q^T D)": {
+            "projection (k_gemm_f64_tn_wide, B = Q^T D)": {
                 "bound": "tensor (FP64 DMMA)",
-                "achieved_tflops": last.project_flops / (last.project_ms / 1e3) / 1e12,
+                "achieved_tflops": alone.project_flops / (alone.project_ms / 1e3) / 1e12,
                 "peak_tflops": dgemm,
-                "frac": last.project_flops / (last.project_ms / 1e3) / 1e12 / dgemm,
+                "frac": alone.project_flops / (alone.project_ms / 1e3) / 1e12 / dgemm,
                 "peak_source": "cuBLAS DGEMM 4096^3 measured in this run"}}
     if args.precision_study and (key.startswith("c3") or key.startswith("c2")):
         line["precision_study"] = precision_study(lib, wl, prob, torch)

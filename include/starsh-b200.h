@@ -331,7 +331,14 @@ void *starsh_b200_stream(void);
 
 /* ------------------------------------------------------- diagnostics */
 
-/* Timings and counters of the last approximation on this host thread. */
+/* Timings and counters of the last approximation on this host thread.  The
+ * device times of the phases (device_ms, sketch_ms, project_ms, gen_ms,
+ * basis_ms, svd_ms, output_ms, fused_ms) are intervals on a lane's stream,
+ * added over the batches.  A call on two lanes (the adaptive engine with
+ * several batches) adds both lanes' intervals, each of which contains what
+ * the GPU did for the other lane meanwhile: their sum can exceed total_ms,
+ * and no rate of a kernel follows from them.  STARSH_B200_LANES=1 in the
+ * environment gives a kernel's own times. */
 typedef struct starsh_b200_stats
 {
     double total_ms;          /* whole call, host clock                 */

@@ -1,6 +1,7 @@
 """What several host threads share when they launch kernels: the lanes of one
 call, the serving workers."""
 import ctypes
+import json
 import os
 import re
 import subprocess
@@ -134,6 +135,22 @@ def test_roles_of_a_cta_meet_at_a_named_barrier():
     assert re.search(r'"barrier\.sync\.aligned 1, %0;" ::"n"\(kGvThreadsB\) : "memory"', text)
     assert re.search(r"__launch_bounds__\(kGvThreadsB\)\s*k_gemv_b\(", text)
     assert re.search(r"k_gemv_b<NR><<<dim3\([^;]*?\), kGvThreadsB,", text)
+
+
+@pytest.mark.gpu
+def test_phase_times_of_the_benchmark_do_not_overlap(lib):
+    """The benchmark's phases, and the kernels' rates that follow from them,
+    are of a call whose phases run one after another: together they take no
+    longer than the call."""
+    r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--workload",
+                        "c1-exp", "--steps", "2", "--warmup", "1", "--no-cpu"],
+                       capture_output=True, text=True, cwd=ROOT,
+                       env=dict(os.environ, STARSH_B200_WORKSPACE_MB="40"))
+    assert r.returncode == 0, r.stderr[-2000:]
+    line = [json.loads(x) for x in r.stdout.splitlines() if x.startswith("{")][0]
+    ph = line["phases_ms"]
+    together = sum(ph[k] for k in ("generation", "basis", "project", "svd", "output"))
+    assert 0 < together <= ph["total_host"], ph
 
 
 # The device memory a process holds after a one-lane call that fills the
