@@ -1355,11 +1355,21 @@ static void pivchol_cluster_launch(TileWork *d_tiles, int ntiles, Workspace ws,
 
 // Phase H above kPivcholSplit rows, `count` tiles (of `act`, or the first
 // ones of the batch).  A few tiles: clusters of four as far as their shared
-// memory reaches (at least 256 rows), of eight beyond; a cluster keeps four
-// SMs to itself, so with more tiles than about two rounds of clusters the
-// one-CTA kernel, two tiles to an SM, has more throughput (134 mixed tiles:
-// 1.51 -> 0.59 ms with clusters; 641 tiles of a batch: 4.70 ms against
-// 4.98).  Returns the number of launches.
+// memory reaches (277 rows), of eight from there (to 416); a cluster keeps
+// its SMs to itself, so with more tiles than about two rounds of clusters the
+// one-CTA kernel, two tiles to an SM, has more throughput.  The whole small
+// SVD with one CTA a tile over that with clusters, random points, nearly all
+// tiles in one range:
+//   rows      16    36    64    81   100   144   225   324 tiles
+//   138     1.06  1.06  1.05  1.05  1.05  1.31  1.01  0.99
+//   181     1.06  1.06  1.06  1.01  0.99  0.95  0.92  0.88
+//   232     1.12  1.09  1.05  0.97  0.94  0.95  0.93  0.92
+//   291     1.10  1.18  0.89  0.92     -  0.85     -     -   (eight)
+//   300     1.12  1.29  1.23  1.39     -  1.03     -     -   (eight)
+//   362     0.98  0.96  0.94  0.93  0.96  0.91  0.91  0.93   (eight)
+// (the last beside tiles of 509 rows, the longest chains, which no cluster
+// holds; four tiles of 390 rows beside twelve of 291, the longest there: 15.7
+// -> 12.9 ms).  Returns the number of launches.
 constexpr int kPivcholClusterTiles = 74;
 
 static int pivchol_large_launch(TileWork *d_tiles, int count, Workspace ws,
@@ -2032,10 +2042,19 @@ constexpr int kJacobiClusterMax = 8;
 
 // CTAs per tile.  With few tiles the chain of one tile is what the launch
 // takes: one CTA for each meeting of a round (blocks of 512 / G columns, at
-// most k1 of them).  With more tiles than SMs, meetings queue on the SMs
-// anyway and a CTA per meeting only adds idle ones: 2, or 4 for the classes
-// above 256 rows.  Without the tile count (no list) the batch's widest
-// factor decides, as measured: 4 where kmax > 256, else 2.
+// most k1 of them).  With more tiles, meetings queue on the SMs anyway and a
+// CTA per meeting only adds idle ones: 2, or 4 for the classes above 256 rows.
+// The whole small SVD with 2 or 4 over that with a CTA per meeting (as above):
+//   rows      16    36    64    81   121   144   169   225   324 tiles
+//   181     1.28  1.27  1.28  1.26  1.16  1.05  1.36  1.12  0.94
+//   232     1.54  1.40  1.13  1.34  1.05  1.21  1.06  1.03  0.94
+//   276     1.35  1.32  1.11  1.09  0.99  1.00  0.98  0.91  0.81
+//   362     1.25  1.27  1.11  0.99  0.95  0.91  0.89  0.82  0.82
+// so the line lies at the SM count, and above 320 rows, where a CTA per meeting
+// is a cluster of eight (blocks of 16 columns: up to 16 meetings) and not of
+// three to five, at half of it (100 tiles of 362 rows: 0.94).  Without the tile
+// count (no list) the batch's widest factor decides, as measured: 4 where kmax
+// > 256, else 2.
 // STARSH_B200_JACOBI_CLUSTER (1 .. 8) sets one size for all.
 static int jacobi_cluster(int cls, int kmax, int count, bool known)
 {
@@ -2046,7 +2065,7 @@ static int jacobi_cluster(int cls, int kmax, int count, bool known)
         return v;
     }();
     if (forced) return forced;
-    if (known && count <= 148) {
+    if (known && count <= (cls == 9 ? 74 : 148)) {
         const int b = cls == 9 ? 16 : 32;
         const int nb = (std::min(kmax, jacobi_class_cols(cls)) + b - 1) / b;
         return std::max(2, std::min(kJacobiClusterMax, (nb + 1) / 2));
