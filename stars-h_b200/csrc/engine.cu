@@ -863,14 +863,15 @@ static int compress_multi(Context &ctx, std::vector<ProblemJob> &jobs,
     // run beside the other's full-width kernels, and neither waits for the
     // host's reads.  Where the adaptive engine's tiles need several
     // batches anyway, in at least three parts (the first, the near-diagonal
-    // tiles, has the longest rounds and SVDs): 24 mixed problems 64.0 to
-    // 54.9 ms, N = 65536 1/r 93.8 to 89.9, N = 102400 square exponential
-    // 98.4 to 95.2, and 1.02 to 1.12 times over nine other calls of two to
+    // tiles, has the longest rounds and SVDs): 24 mixed problems 62.6 to
+    // 58.8 ms, N = 65536 1/r 91.9 to 88.2, N = 102400 square exponential
+    // 95.7 to 92.9, and 1.02 to 1.12 times over nine other calls of two to
     // five batches.  Not one batch cut in parts (each part repeats the chain
     // of rounds: 0.71 to 1.14 times over 77 calls, slower in 62 of them) and
     // not the fixed-width FP64 engine, whose kernels fill the GPU (0.97, 0.97
-    // and 1.01 times with two to four batches).  A serving worker's context has the
-    // other workers beside it.  STARSH_B200_LANES (1 or 2) sets the number.
+    // and 1.01 times with two to four batches).  A serving worker's context
+    // has the other workers beside it.  STARSH_B200_LANES (1 or 2) sets the
+    // number.
     int lanes = ctx.may_help && ep.engine == STARSH_B200_MIXED && plan.size() > 1 ? 2 : 1;
     if (const char *e = getenv("STARSH_B200_LANES"))
         lanes = ctx.may_help ? std::max(1, std::min(2, atoi(e))) : 1;

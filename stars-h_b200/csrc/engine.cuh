@@ -40,8 +40,6 @@ struct TileWork {
     double dnorm2;          // ||D||_F^2 of the block, exact (FP64)
     int cols_done;          // sketch columns consumed so far
     int bcur;               // columns of the current round (0: inactive)
-    int round_slot;         // its place among the round's sampling tiles,
-                            // or -1 (compacted GEMM descriptors)
     int done;               // sampling finished (converged or capped)
     int kround;             // directions the current round's sample added
     int k1_round;           // basis columns when the current round began
@@ -100,7 +98,7 @@ struct Workspace {
 size_t workspace_layout(Workspace &w, int m_max, int n_max, int k_max,
                         bool store_d, bool proj_digits = false);
 
-// GEMM steps of the pipeline, each turned into descriptors on the device.
+// GEMM steps of the pipeline.
 enum GemmStep : int {
     STEP_SKETCH = 0,     // Y  = D Omega                  (m x k)
     STEP_GRAM_Y,         // S  = Y^T Y                    (k x k)

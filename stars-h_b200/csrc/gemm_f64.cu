@@ -149,9 +149,9 @@ k_gemm_f64(const __grid_constant__ GemmArgs args, int tiles_n)
 
 // A^T B with 64 x 64 CTA tiles and a cp.async pipeline: the transposed
 // products (Grams and projections onto the basis in the rounds) have outputs
-// of a few tiles and K = the tile height, so one CTA walks a long K; the
-// a kernel that stages through registers has one K step in flight and waits
-// on memory latency every step.  Operand tiles land in shared memory directly
+// of a few tiles and K = the tile height, so one CTA walks a long K; a kernel
+// that stages through registers has one K step in flight and waits on memory
+// latency every step.  Operand tiles land in shared memory directly
 // (16-byte cp.async, k contiguous in both operands).  Where a tile fills
 // every warp's output region, the per-element accumulation order is that of
 // k_gemm_f64 (the DMMA's k order, k4 steps in order), so results are
@@ -507,10 +507,10 @@ k_gemm_f64_tn_wide(const __grid_constant__ GemmArgs args, int tiles_n)
 
 // A B^T with 64 x 64 CTA tiles (the Gram B B^T of the small SVD, K = the
 // tile width) through the same cp.async pipeline as the transposed
-// products.  Here rows are contiguous in both operands and k is strided, so the tiles are staged as [k][row] (row stride 68 doubles:
-// fragment reads free of bank conflicts); a 16-byte piece is two
-// consecutive rows at one k.  Without split_k the per-element accumulation
-// order is that of k_gemm_f64 (K steps of 16 in order), so results are
+// products.  Here rows are contiguous in both operands and k is strided, so
+// the tiles are staged as [k][row] (row stride 68 doubles: fragment reads free
+// of bank conflicts); a 16-byte piece is two consecutive rows at one k.  Without split_k the per-element accumulation
+// order is that of k_gemm_f64 (k4 steps in order), so results are
 // identical to it; with it, K is split over the warps of empty output
 // regions as in the transposed kernel.
 // Three CTAs per SM where the launch has more than one CTA per SM (in 80

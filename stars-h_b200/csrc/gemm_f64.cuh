@@ -3,7 +3,8 @@
 // shape, so one launch covers all tiles of a batch even when their ranks
 // differ:
 //     C = alpha * op(A) * op(B) + beta * C,   op(A): M x K, op(B): K x N,
-// all matrices column-major.  TA/TB select op = transpose at compile time.
+// all matrices column-major (gemm_f64.cu: one kernel for each shape of
+// product).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -21,8 +22,6 @@ struct GemmDesc {
     const int *gather, *gather_b;
 };
 
-constexpr int kGemmBM = 64;
-constexpr int kGemmBN = 64;
 constexpr int kGemmBK = 16;
 constexpr int kGemmThreads = 256;
 // Shared-memory row stride (doubles) of the [row][k] tiles: 20 puts the

@@ -1442,10 +1442,9 @@ void launch_block_norms(const TileWork *, TileWork *d_rw, int ntiles,
 }
 
 // Start of a sampling round: tiles not done sample min(block, k - cols)
-// more columns; counts[0] counts them (each takes the next round slot, in
-// any order: a slot only places the tile's GEMM descriptors).  counts[1 + b]
-// and the lists after act[0 .. ld - 1] collect the tiles by basis size
-// (svd_bin), for the small SVD when no tile samples any more.
+// more columns; counts[0] counts them and act lists them, in any order.
+// counts[1 + b] and the lists after act[0 .. ld - 1] collect the tiles by
+// basis size (svd_bin), for the small SVD when no tile samples any more.
 __global__ void k_round_setup(TileWork *__restrict__ tiles, int ntiles,
                               int block, int *counts, int *act, int ld)
 {
@@ -1457,14 +1456,12 @@ __global__ void k_round_setup(TileWork *__restrict__ tiles, int ntiles,
     if (tw.done || tw.cols_done >= tw.k) {
         tw.bcur = 0;
         tw.done = 1;
-        tw.round_slot = -1;
         return;
     }
     tw.bcur = min(block, tw.k - tw.cols_done);
     tw.k1_round = tw.k1;
     tw.trunc_round = 0;
-    tw.round_slot = atomicAdd(counts, 1);
-    act[tw.round_slot] = t;
+    act[atomicAdd(counts, 1)] = t;
 }
 
 void launch_round_setup(TileWork *d_tiles, int ntiles, int block,
