@@ -37,7 +37,7 @@ _libc = ctypes.CDLL("libc.so.6")
 def build():
     """Compiles the oracle (and the reference, when its sources exist)."""
     targets = ["_ref/liboracle.so"]
-    if os.path.isdir(REF_SRC):
+    if os.path.isdir(os.path.join(REF_SRC, "src")):
         targets.append("_ref/libstarsh_ref.so")
     subprocess.run(["make", "-C", HERE, "-s"] + targets, check=True)
 
