@@ -1000,6 +1000,18 @@ def fp64_peak_tflops(torch):
 
 # ------------------------------------------------------------------ main
 
+def reference_missing():
+    """Why the reference arm cannot run here, or None: its library is compiled
+    from the reference's own sources by oracle/Makefile."""
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle
+    if os.path.exists(oracle.REF_SO):
+        return None
+    return ("the reference library is not there and its sources are not, "
+            "to compile it from" if not os.path.isdir(os.path.join(oracle.REF_SRC, "src"))
+            else "the reference library has not been compiled (make -C oracle)")
+
+
 def reference_arm(args, key, wl, threads):
     """--impl reference: the reference's OpenMP RSVD on the host cores, one
     bounded sample of the workload (same tiles, sketch width, tol) per
@@ -1128,6 +1140,12 @@ def main():
     rank = int(os.environ.get("RANK", 0))
     world = int(os.environ.get("WORLD_SIZE", 1))
     local = int(os.environ.get("LOCAL_RANK", 0))
+    if args.impl == "reference":
+        why = reference_missing()
+        if why:
+            if rank == 0:
+                print(json.dumps({"impl": "reference", "unavailable": why}))
+            return
     if key in ("c4-batch", "c5-serve"):
         if args.impl == "reference":
             if rank == 0:
